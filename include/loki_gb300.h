@@ -112,20 +112,23 @@ int loki_brutefold(const float* ts_e, const float* ts_v, int64_t nsamps,
                    float* fold_out, void* stream);
 
 /* Scratch bytes with which loki_brutefold / loki_brutefold_unit_variance fold
- * all nfreqs frequencies in one pass. With nbins <= 256 that is the phase
- * map plus the chain layout (per frequency: segment_len bytes of map, then
- * per 512-sample time chunk the chunk's positions sorted by bin, 1 KiB, and
- * the bin starts); a smaller scratch folds in frequency chunks, and one too
- * small for a single frequency of the chain layout uses the map alone. No
- * reference counterpart. */
+ * nsamps samples at all nfreqs frequencies in one pass. With nbins <= 256 that
+ * is the series laid out by time chunk plus, per frequency and chunk, the
+ * chunk's positions sorted by bin; a smaller scratch takes the frequencies,
+ * then the segments, in chunks, and one too small for 32 segments and a
+ * frequency of that layout uses the phase map alone (segment_len bytes a
+ * frequency, twice that with nbins > 256). No reference counterpart. */
+int64_t loki_brutefold_series_scratch_bytes(int64_t nsamps, int64_t nfreqs,
+                                            int64_t segment_len, int32_t nbins,
+                                            int32_t unit_variance);
+/* The same for 64 segments of a series (longer ones are taken in chunks). */
 int64_t loki_brutefold_scratch_bytes(int64_t nfreqs, int64_t segment_len, int32_t nbins);
 
 /* loki_brutefold for a series whose ts_v is all ones (the normalised series
  * io/timeseries.py:198-236 from_tim produces). Every variance sum of the
  * reference is then the bin's sample count, exact in float32, and the same
- * for every full segment: it is written from one histogram of the phase map
- * per frequency, and only the ts_e sums run sample by sample (half the
- * shared memory per thread). The fold is bit-identical to loki_brutefold's
+ * for every full segment: it is counted once per frequency, and only the
+ * ts_e sums run sample by sample (half the work). The fold is bit-identical to loki_brutefold's
  * with ts_v = 1. segment_len < 2^24. No reference counterpart as an entry
  * point. */
 int loki_brutefold_unit_variance(const float* ts_e, int64_t nsamps, const double* freqs,

@@ -243,6 +243,7 @@ SIGNATURES: dict[str, tuple] = {
     "loki_brutefold_noalloc": (C.c_int, [_P, _P, _I64, _P, _I64, _I64, _I32, _D, _D, _P, _P]),
     "loki_brutefold_noalloc_scratch_bytes": (C.c_int64, []),
     "loki_brutefold_scratch_bytes": (C.c_int64, [_I64, _I64, _I32]),
+    "loki_brutefold_series_scratch_bytes": (C.c_int64, [_I64, _I64, _I64, _I32, _I32]),
     "loki_prune_run_blocks": (C.c_int, [_P, _I32, _P, _P, _P, _I32, C.POINTER(LokiScoreSpec),
                                         _I64, _I64, _P, _I64, _P]),
     "loki_prune_run_blocks_scratch_bytes": (C.c_int64, [_I32, _I32]),

@@ -1,15 +1,16 @@
 // Brute fold at the start of the FFA (core/fold.py:108-171 brutefold_start).
 //
-// Two paths give the same bit-identical sums. With nbins <= 256 and room for
-// the chain layout in the scratch, the chain path below (chain_order_kernel,
-// brutefold_chain_kernel). Otherwise the per-thread walk described next.
+// Two paths give the same bit-identical sums: with nbins <= 256 and room for
+// it in the scratch, the chain path below; otherwise the per-thread walk
+// described next.
 //
 // The reference computes a phase-bin map per (frequency, sample in segment)
 // and then, per segment and frequency, adds every sample into its bin in time
-// order. Here the map is built once per frequency chunk (phase_map_kernel, FP64
-// with the reference's rounding) and shared by all segments; the fold kernel
-// gives each thread one (segment, frequency) and walks the samples in time
-// order exactly like the reference loop, so every bin sum is bit-identical.
+// order. In the walk the map is built once per frequency chunk
+// (phase_map_kernel, FP64 with the reference's rounding) and shared by all
+// segments; the fold kernel gives each thread one (segment, frequency) and
+// walks the samples in time order exactly like the reference loop, so every
+// bin sum is bit-identical.
 //
 // Per thread the running sums of the current bin stay in registers; all 2 x
 // nbins sums live in shared memory laid out [bin][thread] (conflict-free).
@@ -201,224 +202,413 @@ brutefold_count_kernel(const T* __restrict__ map, int64_t nfreq_chunk, int64_t f
 
 
 // ---------------------------------------------------------------------------
-// Chain layout (nbins <= 256). Each (segment, frequency, bin) sum is a chain
-// of adds in sample order. The order in which a frequency's samples reach its
-// bins depends only on the sample position within a segment, so it is built
-// once per frequency (chain_order_kernel): the segment is cut into time
-// chunks of kChunk samples, and within a chunk the samples are listed bin by
-// bin, in time order, as byte offsets into a shared-memory row. Each bin's run
-// is padded to a multiple of 4 entries with the offset of a zero column, so a
-// 16-byte load yields 4 entries and adding the zeros leaves a sum unchanged
-// (a sum that starts at +0 and adds finite or infinite values is never -0, and
-// x + 0 = x for every other x). Walking a bin's entries chunk after chunk
-// visits its samples in the reference's order.
+// Chain path (nbins <= 256). Each (row, frequency, bin) sum is a chain of adds
+// in sample order, a row being one segment of ts_e or (general variance) of
+// ts_v. Which samples reach a bin depends only on the position within a
+// segment, so the order is built once per frequency, not once per row:
 //
-// brutefold_chain_kernel gives each lane one segment (32 segments per block)
-// and each warp a set of (frequency, bin) chains: all lanes step through the
-// same chain at once, so the entries are broadcasts, there is no divergence,
-// and the 32 segments' samples sit in 32 different shared-memory banks (rows
-// of kChunk + 1 floats, the last one the zero column). The chain sums live in
-// shared memory between chunks.
+// 1. series_rows_kernel lays the series out by time chunk: for a group of NS
+//    rows (32 V lanes' worth) and a chunk of T samples, [t][row], so that a
+//    chunk is one contiguous copy and the rows of one sample are one
+//    conflict-free shared-memory load.
+// 2. chain_list_kernel sorts each chunk's T positions by bin (stable) for one
+//    frequency and writes them as steps of two neighbouring bins: two
+//    positions of the even bin, two of the odd one, in time order, padded with
+//    position T, a row of zeros. Adding +0 leaves a sum unchanged (a sum that
+//    starts at +0 is never -0).
+// 3. brutefold_chain_kernel: each lane owns V rows, each warp up to 32 chains
+//    (consecutive bins of one frequency) whose sums stay in registers over the
+//    whole segment. A step loads its four positions (one broadcast) and four
+//    samples of V rows and adds them in order, two chains side by side.
+//
+// Bound: shared-memory bandwidth, 4 bytes per add at 128 bytes a clock and SM:
+// 4.6 ms with padding for 2^21 samples x 15 100 frequencies, 64 bins, 128
+// segments, where the walk takes 6.8 ms and the lists 1.1 ms. A walk of
+// 512-sample chunks with one row a lane and the sums in shared memory took
+// 13.6 ms (four loads of loop state per 10 samples of a chain), its float64
+// phase map 4.5 ms and the sort of it by warp matches 2.7 ms.
 // ---------------------------------------------------------------------------
 
-constexpr int kChunk = 512;        // samples per time chunk
-constexpr int kChainWarps = 16;    // warps per fold block
-constexpr int kChainRow = kChunk + 1;
-constexpr uint32_t kZeroOff = kChunk * 4;  // byte offset of the zero column
+constexpr int kChains = 32;      // chains (bins) per warp, sums in registers
+constexpr int kChainWarps = 16;  // most warps per fold block
+constexpr int kMaxPer = 16;      // samples of a chunk per lane of the list kernel
 
-__host__ __device__ inline int chain_nbp(int nbins) { return (nbins + 1 + 7) & ~7; }
-// groups of 4 entries per (frequency, chunk): sum of ceil(n_b / 4) <= C/4 + nbins
-__host__ __device__ inline int chain_groups(int nbins) { return kChunk / 4 + nbins; }
+// Shape of one chain launch, fixed by nbins, the rows and the frequencies.
+struct ChainShape {
+  int V;    // rows per lane (0: the chain path does not apply)
+  int T;    // samples per time chunk, a multiple of 32, at most 32 kMaxPer
+  int wpf;  // warps per frequency
+  int bpw;  // bins per warp (even)
+  int F;    // frequencies per block
+  int LB;   // bytes of one (frequency, chunk) list
+};
 
-// One warp per (frequency, time chunk): order[f][t] = groups of 4 byte
-// offsets sorted by bin (stable, padded per bin); offs[f][t][b] = first group
-// of bin b, offs[f][t][nbins] = groups in use.
+// List of one (frequency, chunk): wpf 32-bit first entries, wpf x 16 step
+// counts (bytes), then the 16-bit entries (twice the position). A bin of n
+// positions takes ceil(n / 2) steps, a pair of bins the larger of the two, so
+// there are at most (T + nbins) / 2 steps of four entries.
+__host__ __device__ inline int list_counts_off(int wpf) { return (4 * wpf + 15) & ~15; }
+__host__ __device__ inline int list_entries_off(int wpf) {
+  return list_counts_off(wpf) + kChains / 2 * wpf;
+}
+__host__ __device__ inline int list_bytes(int T, int nbins, int wpf) {
+  return (list_entries_off(wpf) + 4 * (T + nbins) + 15) & ~15;
+}
+
+// Rows [0, nseg) are the segments of ts_e, rows [nseg, 2 nseg) those of ts_v.
+// out: [row group][chunk][t][NS], zeros beyond the series and the last row.
 __global__ void __launch_bounds__(256)
-chain_order_kernel(const uint8_t* __restrict__ map, int64_t nfreq, int64_t seg_len, int nbins,
-                   uint32_t* __restrict__ order, uint16_t* __restrict__ offs) {
-  __shared__ int cnt_all[8][256];
-  __shared__ int pos_all[8][256];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t nch = (seg_len + kChunk - 1) / kChunk;
-  const int64_t item = (int64_t)blockIdx.x * 8 + warp;
-  if (item >= nfreq * nch) return;  // no block-level synchronisation follows
-  const int64_t f = item / nch, t = item - f * nch;
-  const int nbp = chain_nbp(nbins), gc = chain_groups(nbins);
-  const int clen = (int)min((int64_t)kChunk, seg_len - t * kChunk);
-  const uint8_t* m = map + f * seg_len + t * kChunk;
-  int* cnt = cnt_all[warp];
-  int* pos = pos_all[warp];
-  for (int b = lane; b < nbins; b += 32) cnt[b] = 0;
-  __syncwarp();
-  const unsigned lt = (1u << lane) - 1u;
-  for (int s0 = 0; s0 < clen; s0 += 32) {  // counts per bin
-    const int s = s0 + lane;
-    const bool ok = s < clen;
-    const int b = ok ? (int)m[s] : -1 - lane;
-    const unsigned grp = __match_any_sync(0xFFFFFFFFu, b);
-    if (ok && (grp & lt) == 0) cnt[b] += __popc(grp);
-    __syncwarp();
-  }
-  // exclusive scan of the padded group counts: lane l owns bins [l*per, (l+1)*per)
-  const int per = (nbins + 31) / 32;
-  int local = 0;
-  for (int q = 0; q < per; ++q) {
-    const int b = lane * per + q;
-    if (b < nbins) local += (cnt[b] + 3) >> 2;
-  }
-  int incl = local;
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-    if (lane >= o) incl += y;
-  }
-  const int total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-  int run = incl - local;
-  uint16_t* of = offs + (f * nch + t) * nbp;
-  uint32_t* od = order + (f * nch + t) * (int64_t)gc * 4;
-  for (int q = 0; q < per; ++q) {
-    const int b = lane * per + q;
-    if (b < nbins) {
-      const int c = cnt[b], g = (c + 3) >> 2;
-      of[b] = (uint16_t)run;
-      pos[b] = 4 * run;  // the next free entry of bin b
-      for (int k = c; k < 4 * g; ++k) od[4 * run + k] = kZeroOff;  // padding
-      run += g;
-    }
-  }
-  for (int b = nbins + lane; b < nbp; b += 32) of[b] = (uint16_t)total;
-  __syncwarp();
-  for (int s0 = 0; s0 < clen; s0 += 32) {  // stable scatter
-    const int s = s0 + lane;
-    const bool ok = s < clen;
-    const int b = ok ? (int)m[s] : -1 - lane;
-    const unsigned grp = __match_any_sync(0xFFFFFFFFu, b);
-    if (ok) od[pos[b] + __popc(grp & lt)] = (uint32_t)s * 4u;
-    __syncwarp();
-    if (ok && (grp >> lane) == 1u) pos[b] += __popc(grp);  // highest lane of the group
-    __syncwarp();
-  }
-}
-
-__device__ __forceinline__ float lds_f32(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-  return v;
-}
-
-__device__ __forceinline__ uint4 lds_u32x4(uint32_t addr) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "r"(addr));
-  return v;
-}
-
-// Block: 32 segments (lanes) x F frequencies; chain c = f * nbins + b, warp w
-// walks chains w, w + 16, ... NC = 2 also sums ts_v. Shared memory, in order:
-// series rows [NC][32][kChainRow] f32, chain sums [NC][F * nbins][33] f32,
-// order groups [F][gc] uint4, chain table [F * nbins] u32, bin starts
-// [F][nbp] u16.
-template <int NC>
-__global__ void __launch_bounds__(kChainWarps * 32, NC == 1 ? 2 : 1)
-brutefold_chain_kernel(const float* __restrict__ ts_e, const float* __restrict__ ts_v,
-                       int64_t nsamps, const uint32_t* __restrict__ order,
-                       const uint16_t* __restrict__ offs, int64_t nfreq_chunk, int64_t f_offset,
-                       int64_t nfreq_total, int64_t seg_len, int64_t nseg, int nbins, int F,
-                       float* __restrict__ fold) {
-  extern __shared__ __align__(16) float csm[];
-  const int nbp = chain_nbp(nbins), gc = chain_groups(nbins);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t nsg = (nseg + 31) / 32;
-  const int64_t sg = blockIdx.x % nsg, fg = blockIdx.x / nsg;
-  const int64_t f0 = fg * F;
-  const int nfb = (int)min((int64_t)F, nfreq_chunk - f0);
-  const int nchains = nfb * nbins;
-  const int nct = F * nbins;  // chain slots
-  static_assert(kChunk == kChainWarps * 32, "one series sample per thread and row");
-  float* xs = csm;                        // [NC][32][kChainRow]
-  float* acc = xs + NC * 32 * kChainRow;  // [NC][nct][33]
-  const int fl = (NC * 32 * kChainRow + NC * nct * 33 + 3) & ~3;
-  uint4* ord_s = reinterpret_cast<uint4*>(csm + fl);
-  uint32_t* tab = reinterpret_cast<uint32_t*>(ord_s + F * gc);
-  uint16_t* off_s = reinterpret_cast<uint16_t*>(tab + nct);
-  const int64_t nch = (seg_len + kChunk - 1) / kChunk;
-  for (int r = tid; r < NC * 32; r += kChainWarps * 32) xs[r * kChainRow + kChunk] = 0.0f;
-  for (int i = tid; i < NC * nct * 33; i += kChainWarps * 32) acc[i] = 0.0f;
-  for (int c = tid; c < nchains; c += kChainWarps * 32) {
-    const int f = c / nbins, b = c - f * nbins;
-    tab[c] = (uint32_t)(f * gc) | ((uint32_t)(f * nbp + b) << 16);
-  }
-  // 32-bit shared addresses: the lane's series row, the order groups
-  const uint32_t xb = (uint32_t)__cvta_generic_to_shared(xs + lane * kChainRow);
-  const uint32_t ob = (uint32_t)__cvta_generic_to_shared(ord_s);
-  constexpr uint32_t kV = 32 * kChainRow * 4;  // ts_v rows follow the ts_e rows
-  const bool interior = sg * 32 + 32 < nseg;  // 32 full segments, none of them the last
-  for (int64_t t = 0; t < nch; ++t) {
-    const int clen = (int)min((int64_t)kChunk, seg_len - t * kChunk);
-    __syncthreads();  // the previous chunk's rows are consumed (and the setup is done)
-    // series rows: row r = segment sg * 32 + r; samples beyond nsamps (and
-    // rows beyond the last segment) are 0
-    const int64_t p0 = sg * 32 * seg_len + t * kChunk;
-    if (interior && clen == kChunk) {  // one sample of every row a thread, no checks
-      const float* pe = ts_e + p0 + tid;
-#pragma unroll 8
-      for (int r = 0; r < 32; ++r) {
-        xs[r * kChainRow + tid] = __ldg(pe + (int64_t)r * seg_len);
-        if constexpr (NC == 2)
-          xs[(32 + r) * kChainRow + tid] = __ldg(ts_v + p0 + tid + (int64_t)r * seg_len);
-      }
-    } else if (tid < clen) {
-      for (int r = 0; r < 32; ++r) {
-        const int64_t p = p0 + (int64_t)r * seg_len + tid;
-        const bool in = sg * 32 + r < nseg && p < nsamps;
-        xs[r * kChainRow + tid] = in ? __ldg(ts_e + p) : 0.0f;
-        if constexpr (NC == 2) xs[(32 + r) * kChainRow + tid] = in ? __ldg(ts_v + p) : 0.0f;
-      }
-    }
-    // this chunk's order groups and bin starts of the block's frequencies
-    for (int i = tid; i < nfb * gc; i += kChainWarps * 32) {
-      const int f = i / gc, q = i - f * gc;
-      ord_s[i] = __ldg(reinterpret_cast<const uint4*>(order + ((f0 + f) * nch + t) * gc * 4) + q);
-    }
-    for (int i = tid; i < nfb * nbp; i += kChainWarps * 32) {
-      const int f = i / nbp, q = i - f * nbp;
-      off_s[i] = offs[((f0 + f) * nch + t) * nbp + q];
+series_rows_kernel(const float* __restrict__ ts_e, const float* __restrict__ ts_v,
+                   int64_t nsamps, int64_t seg_len, int64_t nseg, int64_t nrows, int64_t rg0,
+                   int T, int NS, int64_t nch, float* __restrict__ out) {
+  __shared__ float tile[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t nt = T / 32;  // a block per 32 positions of a chunk; rg: within this launch
+  const int64_t tc = blockIdx.x / nt, t = tc % nch, rg = tc / nch;
+  const int t0 = (int)(blockIdx.x - tc * nt) * 32;
+  float* o = out + (rg * nch + t) * (int64_t)T * NS;
+  for (int r0 = 0; r0 < NS; r0 += 32) {
+    __syncthreads();
+    for (int q = ty; q < 32; q += 8) {
+      const int64_t row = (rg0 + rg) * NS + r0 + q;
+      const int64_t seg = row < nseg ? row : row - nseg;
+      const int64_t i = t * T + t0 + tx;  // position within the segment
+      const int64_t p = seg * seg_len + i;
+      float x = 0.0f;
+      if (row < nrows && i < seg_len && p < nsamps) x = __ldg((row < nseg ? ts_e : ts_v) + p);
+      tile[q][tx] = x;
     }
     __syncthreads();
-    for (int c = warp; c < nchains; c += kChainWarps) {
-      const uint32_t tb = tab[c];
-      const int oi = (int)(tb >> 16);
-      const uint32_t g0 = off_s[oi], g1 = off_s[oi + 1];
-      float a = acc[c * 33 + lane];
-      float v = NC == 2 ? acc[(nct + c) * 33 + lane] : 0.0f;
-      const uint32_t gend = ob + ((tb & 0xFFFFu) + g1) * 16u;
-      for (uint32_t ga = ob + ((tb & 0xFFFFu) + g0) * 16u; ga < gend; ga += 16u) {
-        const uint4 e = lds_u32x4(ga);
-        a = __fadd_rn(a, lds_f32(xb + e.x));
-        a = __fadd_rn(a, lds_f32(xb + e.y));
-        a = __fadd_rn(a, lds_f32(xb + e.z));
-        a = __fadd_rn(a, lds_f32(xb + e.w));
-        if constexpr (NC == 2) {
-          v = __fadd_rn(v, lds_f32(xb + kV + e.x));
-          v = __fadd_rn(v, lds_f32(xb + kV + e.y));
-          v = __fadd_rn(v, lds_f32(xb + kV + e.z));
-          v = __fadd_rn(v, lds_f32(xb + kV + e.w));
+    for (int q = ty; q < 32; q += 8) o[(int64_t)(t0 + q) * NS + r0 + tx] = tile[tx][q];
+  }
+}
+
+// Turns per sample (and at position 0) of one frequency as 64-bit fixed-point
+// fractions: the bin of position i is round(frac(i step + first) nbins). They
+// carry the exact product to 2^-64, the reference's float64 chain deviates
+// from it by at most 2^-50 of the turns counted from t_ref, and its float32
+// half-up rounding moves a bin edge by less than nbins 2^-23 bins. A position
+// farther than `margin` (2^-32 bins) from every edge therefore has a certain
+// bin; the others take the float64 chain (margin 2^31: every position does).
+struct BinStep {
+  unsigned long long step, first;
+  unsigned margin;
+};
+
+__device__ __forceinline__ unsigned long long turn_fraction(double a, double b) {
+  const double p = __dmul_rn(a, b), e = __fma_rn(a, b, -p);  // a b = p + e
+  const double fr = __dsub_rn(p, floor(p));                  // exact
+  unsigned long long u = fr >= 1.0 ? 0ull : (unsigned long long)__dmul_rn(fr, 0x1p64);
+  return u + (unsigned long long)(long long)__dmul_rn(e, 0x1p64);
+}
+
+__device__ __forceinline__ BinStep make_bin_step(double f, int64_t seg_len, int nbins,
+                                                 double tsamp, double t_ref) {
+  BinStep s{0, 0, 0x80000000u};
+  const double span = fmax((double)seg_len * tsamp, fabs(t_ref)) * f;  // turns
+  if (span >= 0.0 && span < 0x1p24) {  // false for NaN and for negative frequencies
+    s.step = turn_fraction(tsamp, f);
+    s.first = 0ull - turn_fraction(t_ref, f);
+    s.margin = (unsigned)((double)nbins * (0x1p10 + span * 0x1p-17)) + 64u;
+  }
+  return s;
+}
+
+// Bin of one position from the float64 chain (out of line: rarely taken).
+static __device__ __noinline__ int bin_exact(int64_t i, double f, int nbins, double tsamp,
+                                             double t_ref) {
+  const double pt = __dsub_rn(__dmul_rn((double)i, tsamp), t_ref);
+  const int b = round_shift(phase_idx(pt, f, nbins, 0.0), nbins);
+  return b < 0 || b >= nbins ? 0 : b;  // as phase_map_kernel
+}
+
+// One block per frequency, a warp per time chunk. counts (unit variance):
+// [frequency][2][nbins] sample counts of a full and of the last segment. The
+// bins are integer arithmetic kept in registers and sorted by per-lane counts
+// whose rows are padded to an odd number of words (without the padding 16-way
+// bank conflicts made it 2.2 ms instead of 1.0). Bound: instruction issue (79 %).
+constexpr int kCntRow = 36;    // bytes of a bin's 32 per-lane counts (9 words: no bank conflicts)
+constexpr int kPlaceRow = 34;  // 16-bit ranks of a bin's 32 lanes, its first entry (17 words)
+__host__ __device__ inline int list_warp_bytes(int nbins, int LB) {
+  return ((nbins * (kCntRow + 2 * kPlaceRow) + 15) & ~15) + LB;
+}
+
+__global__ void __launch_bounds__(256, 3)
+chain_list_kernel(const double* __restrict__ freqs, int64_t seg_len, int nbins, double tsamp,
+                  double t_ref, ChainShape cs, int64_t nch, int64_t last_len,
+                  uint8_t* __restrict__ lists, float* __restrict__ counts) {
+  extern __shared__ __align__(16) uint8_t lsm[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  const int per_warp = list_warp_bytes(nbins, cs.LB);  // list, counts u8, places u16
+  uint8_t* list = lsm + warp * per_warp;
+  uint8_t* cnt = list + cs.LB;
+  uint16_t* place = reinterpret_cast<uint16_t*>(cnt + nbins * kCntRow);
+  int* hist = reinterpret_cast<int*>(lsm + nwarps * per_warp);  // [2][nbins]
+  uint32_t* first = reinterpret_cast<uint32_t*>(list);
+  uint8_t* steps = list + list_counts_off(cs.wpf);
+  uint16_t* entry = reinterpret_cast<uint16_t*>(list + list_entries_off(cs.wpf));
+  const int64_t f = blockIdx.x;
+  const double fr = freqs[f];
+  const BinStep bs = make_bin_step(fr, seg_len, nbins, tsamp, t_ref);
+  const int per = cs.T / 32;
+  for (int k = tid; k < 2 * nbins; k += blockDim.x) hist[k] = 0;
+  for (int k = lane; k < list_entries_off(cs.wpf); k += 32) list[k] = 0;
+  __syncthreads();
+  for (int64_t t = warp; t < nch; t += nwarps) {
+    const int clen = (int)min((int64_t)cs.T, seg_len - t * cs.T);
+    for (int k = lane; k < nbins * (kCntRow / 4); k += 32) reinterpret_cast<uint32_t*>(cnt)[k] = 0;
+    __syncwarp();
+    // this lane's positions: bin, and rank among the lane's earlier ones
+    const int i0 = lane * per;
+    unsigned long long ph = bs.step * (unsigned long long)(t * cs.T + i0) + bs.first;
+    uint16_t br[kMaxPer];
+#pragma unroll
+    for (int k = 0; k < kMaxPer; ++k) {
+      br[k] = 0;
+      if (k < per && i0 + k < clen) {
+        const unsigned long long x =
+            (unsigned long long)(unsigned)(ph >> 32) * (unsigned)nbins + 0x80000000ull;
+        int b = (int)(x >> 32);
+        if (b >= nbins) b = 0;
+        if ((unsigned)x + bs.margin <= 2u * bs.margin - 1u)
+          b = bin_exact(t * cs.T + i0 + k, fr, nbins, tsamp, t_ref);
+        const int r = cnt[b * kCntRow + lane];
+        cnt[b * kCntRow + lane] = (uint8_t)(r + 1);
+        br[k] = (uint16_t)(b | (r << 8));
+        if (counts && last_len < seg_len && t * cs.T + i0 + k < last_len)
+          atomicAdd(&hist[nbins + b], 1);
+      }
+      ph += bs.step;
+    }
+    __syncwarp();
+    // per bin (a lane each): the rank of every lane's first position, the
+    // steps of its pair of bins and where they begin
+    int base = 0;  // steps of the bins before
+    for (int b0 = 0; b0 < nbins; b0 += 32) {
+      const int b = b0 + lane;
+      uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      int c = 0;
+      if (b < nbins) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          w[k] = reinterpret_cast<const uint32_t*>(cnt + b * kCntRow)[k];
+          c += (int)((w[k] * 0x01010101u) >> 24);
         }
       }
-      acc[c * 33 + lane] = a;
-      if constexpr (NC == 2) acc[(nct + c) * 33 + lane] = v;
+      const int g = (c + 1) >> 1;
+      const int st = max(g, __shfl_xor_sync(0xFFFFFFFFu, g, 1));
+      int incl = lane & 1 ? 0 : st;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (b < nbins) {
+        const int at = 4 * (base + incl - st);  // the pair's first entry
+        const int kb = b / cs.bpw, kc = b - kb * cs.bpw;
+        if (!(kc & 1)) steps[kb * (kChains / 2) + kc / 2] = (uint8_t)st;
+        if (kc == 0) first[kb] = (uint32_t)at;
+        if (counts) atomicAdd(&hist[b], c);
+        uint32_t run = 0;
+        uint32_t* o = reinterpret_cast<uint32_t*>(place + b * kPlaceRow);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const uint32_t in = w[k] * 0x01010101u, ex = in - w[k];  // per-byte prefix sums
+          o[2 * k] = (run + (ex & 0xFFu)) | ((run + ((ex >> 8) & 0xFFu)) << 16);
+          o[2 * k + 1] = (run + ((ex >> 16) & 0xFFu)) | ((run + (ex >> 24)) << 16);
+          run += in >> 24;
+        }
+        o[16] = (uint32_t)(at + 2 * (b & 1));
+      }
+      base += __shfl_sync(0xFFFFFFFFu, incl, 31);
+    }
+    const uint32_t pad = 2u * (uint32_t)cs.T * 0x10001u;  // the zero row
+    for (int k = lane; k < base; k += 32)
+      reinterpret_cast<uint2*>(entry)[k] = make_uint2(pad, pad);
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < kMaxPer; ++k)
+      if (k < per && i0 + k < clen) {
+        const uint16_t* o = place + (br[k] & 0xFF) * kPlaceRow;
+        const int r = o[lane] + (br[k] >> 8);
+        entry[o[32] + 4 * (r >> 1) + (r & 1)] = (uint16_t)(2 * (i0 + k));
+      }
+    __syncwarp();
+    uint4* dst = reinterpret_cast<uint4*>(lists + (f * nch + t) * cs.LB);
+    const int used = (list_entries_off(cs.wpf) + 8 * base + 15) / 16;
+    for (int k = lane; k < used; k += 32) dst[k] = reinterpret_cast<const uint4*>(list)[k];
+    __syncwarp();
+  }
+  if (!counts) return;
+  __syncthreads();
+  for (int b = tid; b < nbins; b += blockDim.x) {
+    counts[(f * 2) * nbins + b] = (float)hist[b];
+    counts[(f * 2 + 1) * nbins + b] = (float)hist[last_len < seg_len ? nbins + b : b];
+  }
+}
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+
+__device__ __forceinline__ uint2 lds_u32x2(uint32_t addr) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+  return v;
+}
+// One sample of this lane's V rows.
+__device__ __forceinline__ void lds_rows(uint32_t addr, float (&x)[1]) {
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x[0]) : "r"(addr));
+}
+__device__ __forceinline__ void lds_rows(uint32_t addr, float (&x)[2]) {
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(x[0]), "=f"(x[1]) : "r"(addr));
+}
+
+// Block: NS = 32 V rows x F frequencies, F * wpf warps. Shared memory, double
+// buffered by chunk: rows [T + 1][NS] f32 (row T zeros), lists [F][LB]; the
+// next chunk is copied while this one is walked. The sums leave through the
+// same memory, whole profiles at a time.
+template <int V>
+__global__ void __launch_bounds__(kChainWarps * 32, 1)
+brutefold_chain_kernel(const float* __restrict__ rows, const uint8_t* __restrict__ lists,
+                       const float* __restrict__ counts, ChainShape cs, int64_t nfreq_chunk,
+                       int64_t f_offset, int64_t nfreq_total, int64_t nch, int64_t nseg,
+                       int64_t nrows, int64_t rg0, int64_t nrg, int nbins,
+                       float* __restrict__ fold) {
+  constexpr int NS = 32 * V;
+  extern __shared__ __align__(16) uint8_t csm[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x;
+  const int64_t rg = blockIdx.x % nrg, f0 = blockIdx.x / nrg * cs.F;
+  const int nfb = (int)min((int64_t)cs.F, nfreq_chunk - f0);
+  const int rbytes = (cs.T + 1) * NS * 4, lbytes = cs.F * cs.LB + 16;
+  uint8_t* buf[2] = {csm, csm + rbytes + lbytes};
+  const float* src_r = rows + rg * nch * (int64_t)cs.T * NS;
+  auto fetch = [&](int64_t t) {
+    uint8_t* b = buf[t & 1];
+    const uint8_t* r = reinterpret_cast<const uint8_t*>(src_r + t * (int64_t)cs.T * NS);
+    for (int k = tid; k < cs.T * NS / 4; k += nthr) cp_async16(b + 16 * k, r + 16 * k);
+    const int lq = cs.LB / 16;
+    for (int k = tid; k < nfb * lq; k += nthr) {
+      const int fi = k / lq, q = k - fi * lq;
+      cp_async16(b + rbytes + 16 * k, lists + ((f0 + fi) * nch + t) * cs.LB + 16 * q);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int k = tid; k < NS; k += nthr)
+    for (int q = 0; q < 2; ++q) reinterpret_cast<float*>(buf[q])[cs.T * NS + k] = 0.0f;
+  float acc[kChains][V];
+#pragma unroll
+  for (int c = 0; c < kChains; ++c)
+#pragma unroll
+    for (int v = 0; v < V; ++v) acc[c][v] = 0.0f;
+  const int fi = warp / cs.wpf, kb = warp - fi * cs.wpf;
+  const bool active = fi < nfb;
+  fetch(0);
+  for (int64_t t = 0; t < nch; ++t) {
+    if (t + 1 < nch) {
+      fetch(t + 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    if (active) {
+      const uint8_t* l = buf[t & 1] + rbytes + fi * cs.LB;
+      const uint4 c4 = *reinterpret_cast<const uint4*>(l + list_counts_off(cs.wpf) +
+                                                       kb * (kChains / 2));
+      const uint32_t cw[4] = {c4.x, c4.y, c4.z, c4.w};
+      // 32-bit shared addresses: this lane's rows, the warp's entries
+      const uint32_t xb = (uint32_t)__cvta_generic_to_shared(buf[t & 1]) + lane * (4 * V);
+      uint32_t e = (uint32_t)__cvta_generic_to_shared(l) + list_entries_off(cs.wpf) +
+                   2 * reinterpret_cast<const uint32_t*>(l)[kb];
+      // a row's bytes are 64 V per unit of an entry: one 16 x 8-bit dot product per address
+      constexpr uint32_t kLo = 64 * V, kHi = kLo << 8;
+      uint2 next = lds_u32x2(e);  // one step ahead: the warp's steps are one run
+#pragma unroll
+      for (int c = 0; c < kChains; c += 2) {
+        const uint32_t end = e + ((cw[c >> 3] >> (8 * ((c >> 1) & 3))) & 0xFFu) * 8;
+        // One row a lane is where a walk has few warps and, at the low
+        // frequencies of few segments, long runs of one bin: four steps' loads
+        // in flight there (32 segments at 1-10 Hz: 0.66 -> 0.55 ms).
+        if constexpr (V == 1) {
+#pragma unroll 1
+          while (end - e >= 32) {
+            uint2 w[4];
+            w[0] = next;
+#pragma unroll
+            for (int k = 1; k < 4; ++k) w[k] = lds_u32x2(e + 8 * k);
+            e += 32;
+            next = lds_u32x2(e);
+            float x[4][4][V];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              lds_rows(__dp2a_lo(w[k].x, kLo, xb), x[k][0]);
+              lds_rows(__dp2a_lo(w[k].x, kHi, xb), x[k][1]);
+              lds_rows(__dp2a_lo(w[k].y, kLo, xb), x[k][2]);
+              lds_rows(__dp2a_lo(w[k].y, kHi, xb), x[k][3]);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              acc[c][0] = __fadd_rn(__fadd_rn(acc[c][0], x[k][0][0]), x[k][1][0]);
+              acc[c + 1][0] = __fadd_rn(__fadd_rn(acc[c + 1][0], x[k][2][0]), x[k][3][0]);
+            }
+          }
+        }
+#pragma unroll 1
+        while (e != end) {
+          const uint2 w = next;
+          e += 8;
+          next = lds_u32x2(e);
+          float a0[V], a1[V], b0[V], b1[V];
+          lds_rows(__dp2a_lo(w.x, kLo, xb), a0);
+          lds_rows(__dp2a_lo(w.x, kHi, xb), a1);
+          lds_rows(__dp2a_lo(w.y, kLo, xb), b0);
+          lds_rows(__dp2a_lo(w.y, kHi, xb), b1);
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+            acc[c][v] = __fadd_rn(__fadd_rn(acc[c][v], a0[v]), a1[v]);
+            acc[c + 1][v] = __fadd_rn(__fadd_rn(acc[c + 1][v], b0[v]), b1[v]);
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  // sums to shared memory [row][F nbins], then whole profiles to the fold
+  float* out_s = reinterpret_cast<float*>(csm);
+  const int fn = cs.F * nbins, stride = fn + 1;
+  if (active) {
+#pragma unroll
+    for (int c = 0; c < kChains; ++c) {
+      const int b = kb * cs.bpw + c;
+      if (c < cs.bpw && b < nbins)
+#pragma unroll
+        for (int v = 0; v < V; ++v) out_s[(lane * V + v) * stride + fi * nbins + b] = acc[c][v];
     }
   }
   __syncthreads();
-  // the block's sums, whole rows to the fold
-  for (int r = 0; r < 32; ++r) {
-    const int64_t g = sg * 32 + r;
-    if (g >= nseg) break;
-    for (int c = tid; c < nchains; c += kChainWarps * 32) {
-      const int f = c / nbins, b = c - f * nbins;
-      float* out = fold + ((size_t)g * nfreq_total + f_offset + f0 + f) * 2 * nbins;
-      out[b] = acc[c * 33 + r];
-      if constexpr (NC == 2) out[nbins + b] = acc[(nct + c) * 33 + r];
+  const int ncomp = counts ? 1 : 2;
+  for (int r = 0; r < NS; ++r) {
+    const int64_t row = (rg0 + rg) * NS + r;
+    if (row >= nrows) break;
+    const int64_t seg = row < nseg ? row : row - nseg;
+    float* o = fold + ((size_t)seg * nfreq_total + f_offset + f0) * 2 * nbins +
+               (row < nseg ? 0 : nbins);
+    if (ncomp == 1) {
+      const float* cn = counts + (f0 * 2 + (seg == nseg - 1 ? 1 : 0)) * nbins;
+      for (int k = tid; k < nfb * 2 * nbins; k += nthr) {
+        const int q = k / (2 * nbins), j = k - q * 2 * nbins;
+        o[k] = j < nbins ? out_s[r * stride + q * nbins + j]
+                         : __ldg(cn + q * 2 * nbins + j - nbins);
+      }
+    } else {
+      for (int k = tid; k < nfb * nbins; k += nthr) {
+        const int q = k / nbins;
+        o[q * 2 * nbins + (k - q * nbins)] = out_s[r * stride + k];
+      }
     }
   }
 }
@@ -429,75 +619,125 @@ using namespace loki;
 
 namespace loki {
 
-// Bytes per frequency of the chain layout: map, order groups, bin starts.
-static int64_t chain_bytes_per_freq(int64_t seg_len, int nbins) {
-  const int64_t nch = (seg_len + kChunk - 1) / kChunk;
-  return seg_len + nch * chain_groups(nbins) * 16 + nch * chain_nbp(nbins) * 2;
-}
-
 static int64_t round256(int64_t x) { return (x + 255) & ~int64_t(255); }
 
-static int chain_smem(int nbins, int nc, int F) {
-  const int nct = F * nbins;
-  const int fl = (nc * 32 * kChainRow + nc * nct * 33 + 3) & ~3;  // 16-byte aligned groups
-  return fl * 4 + F * chain_groups(nbins) * 16 + nct * 4 + F * chain_nbp(nbins) * 2;
+constexpr int kChainSmem = 226 * 1024;
+
+static int chain_smem(const ChainShape& c, int nbins) {
+  const int ns = 32 * c.V;
+  const int walk = 2 * ((c.T + 1) * ns * 4 + c.F * c.LB + 16);
+  const int out = ns * (c.F * nbins + 1) * 4;
+  return std::max(walk, out);
 }
 
-// Frequencies per fold block (F) and its shared memory; F = 0: the chain
-// kernel does not apply. Unit variance: two blocks per SM.
-static void chain_shape(int nbins, int nc, int* F, int* smem) {
-  *F = 0;
-  *smem = 0;
-  if (nbins < 1 || nbins > 256) return;
-  // unit variance: two blocks in the 228 KB of an SM (1 KB reserved per block)
-  const int limit = nc == 1 ? 114 * 1024 - 1024 : 220 * 1024;
-  int f = 16;
-  while (f > 0 && chain_smem(nbins, nc, f) > limit) --f;
-  *F = f;
-  *smem = f > 0 ? chain_smem(nbins, nc, f) : 0;
+// V: two rows a lane (64 rows share a list walk, 8-byte loads) once there are
+// more than 32. F: as many frequencies as 16 warps hold, fewer where that
+// leaves SMs without a block. T: the longest chunk two buffers of which
+// fit, since each (chain, chunk) pays a loop and half a padding entry.
+static ChainShape chain_shape(int nbins, int64_t nrows, int64_t nfreqs, int V) {
+  ChainShape c{0, 0, 0, 0, 0, 0};
+  if (nbins < 1 || nbins > 256) return c;
+  c.wpf = (nbins + kChains - 1) / kChains;
+  c.bpw = ((nbins + c.wpf - 1) / c.wpf + 1) & ~1;
+  c.F = kChainWarps / c.wpf;
+  const int64_t nrg = (nrows + 32 * V - 1) / (32 * V);
+  // waves of blocks times the work of one (its copies cost about 0.8 of a frequency's walk)
+  const int fmax = c.F;
+  double best = 0.0;
+  for (int f = fmax; f >= 1; --f) {
+    const int64_t blocks = nrg * ((nfreqs + f - 1) / f);
+    const double cost = (double)((blocks + 151) / 152) * (f + 0.8);
+    if (f == fmax || cost < best) {
+      best = cost;
+      c.F = f;
+    }
+  }
+  for (c.T = V == 1 ? 480 : 384; c.T >= 32; c.T -= 32) {
+    c.LB = list_bytes(c.T, nbins, c.wpf);
+    c.V = V;
+    if (chain_smem(c, nbins) <= kChainSmem) return c;
+  }
+  c.V = 0;
+  return c;
 }
 
-// Frequencies of the chain layout that fit in the scratch (0: none).
-static int64_t chain_chunk(int64_t scratch_bytes, int64_t seg_len, int nbins) {
-  const int64_t per = chain_bytes_per_freq(seg_len, nbins);
-  return std::max<int64_t>(0, (scratch_bytes - 3 * 256) / per);
+static int64_t chain_chunks(const ChainShape& c, int64_t seg_len) {
+  return (seg_len + c.T - 1) / c.T;
+}
+// Scratch bytes of one row group of the series layout, and of one frequency
+// (lists and counts).
+static int64_t chain_group_bytes(const ChainShape& c, int64_t seg_len) {
+  return chain_chunks(c, seg_len) * c.T * 32 * c.V * 4;
+}
+static int64_t chain_freq_bytes(const ChainShape& c, int64_t seg_len, int nbins) {
+  return chain_chunks(c, seg_len) * c.LB + 2 * nbins * 4;
 }
 
-// The chain path: per frequency chunk, the phase map, the chain order, the
-// chain fold and (unit) the count rows.
+// Scratch of the chain path: `groups` row groups of the series at a time (all
+// of them when they fit in half of it) and `chunk` frequencies.
+struct ChainPlan {
+  ChainShape c;
+  int64_t groups, chunk;
+};
+
+static ChainPlan chain_plan(int nbins, int64_t nrows, int64_t nfreqs, int64_t seg_len,
+                            int64_t scratch_bytes) {
+  for (int V = nrows > 32 ? 2 : 1; V >= 1; --V) {
+    const ChainShape c = chain_shape(nbins, nrows, nfreqs, V);
+    if (!c.V) continue;
+    const int64_t avail = scratch_bytes - 4 * 256;
+    const int64_t g = chain_group_bytes(c, seg_len), q = chain_freq_bytes(c, seg_len, nbins);
+    const int64_t nrg = (nrows + 32 * V - 1) / (32 * V);
+    if (avail < g + q) continue;
+    int64_t groups = nrg;
+    if (nrg * g + nfreqs * q > avail) groups = std::min(nrg, std::max<int64_t>(1, avail / 2 / g));
+    return {c, groups, std::min(nfreqs, std::max<int64_t>(1, (avail - groups * g) / q))};
+  }
+  return {{0, 0, 0, 0, 0, 0}, 0, 0};
+}
+
 static int brutefold_chain(const float* ts_e, const float* ts_v, bool unit, int64_t nsamps,
                            const double* freqs, int64_t nfreqs, int64_t seg_len, int nbins,
-                           double tsamp, double t_ref, char* scratch, int64_t chunk, int F,
-                           int smem, float* fold_out, cudaStream_t s) {
-  const int64_t nseg = (nsamps + seg_len - 1) / seg_len;
-  const int64_t nch = (seg_len + kChunk - 1) / kChunk;
-  auto kf = unit ? brutefold_chain_kernel<1> : brutefold_chain_kernel<2>;
-  if (set_smem_limit(kf, smem) != cudaSuccess)
+                           double tsamp, double t_ref, char* scratch, const ChainPlan& p,
+                           float* fold_out, cudaStream_t s) {
+  const ChainShape& c = p.c;
+  const int64_t nseg = (nsamps + seg_len - 1) / seg_len, nrows = nseg * (unit ? 1 : 2);
+  const int64_t nch = chain_chunks(c, seg_len), nrg = (nrows + 32 * c.V - 1) / (32 * c.V);
+  const int64_t last_len = nsamps - (nseg - 1) * seg_len;
+  auto kf = c.V == 1 ? brutefold_chain_kernel<1> : brutefold_chain_kernel<2>;
+  const int smem = chain_smem(c, nbins);
+  const int lwarps = nbins <= 128 ? 8 : 4;  // about 230 KB at 256 bins and 8 warps
+  const int lsmem = lwarps * list_warp_bytes(nbins, c.LB) + 2 * nbins * (int)sizeof(int);
+  if (set_smem_limit(kf, smem) != cudaSuccess ||
+      set_smem_limit(chain_list_kernel, lsmem) != cudaSuccess)
     return set_error(LOKI_ERR_CUDA, "cudaFuncSetAttribute failed");
-  uint8_t* map = reinterpret_cast<uint8_t*>(scratch);
-  uint32_t* order = reinterpret_cast<uint32_t*>(scratch + round256(chunk * seg_len));
-  uint16_t* offs = reinterpret_cast<uint16_t*>(
-      scratch + round256(chunk * seg_len) + round256(chunk * nch * chain_groups(nbins) * 16));
-  const int hsmem = 2 * nbins * (int)sizeof(int);
-  const int64_t nsg = (nseg + 31) / 32;
-  for (int64_t f0 = 0; f0 < nfreqs; f0 += chunk) {
-    const int64_t nf = std::min(chunk, nfreqs - f0);
-    const int64_t total = nf * seg_len;
-    const int mblocks = (int)std::min<int64_t>((total + 255) / 256, 152 * 64);
-    const int64_t oblocks = (nf * nch + 7) / 8;
-    const int64_t blocks = nsg * ((nf + F - 1) / F);
-    if (blocks > 0x7FFFFFFF || oblocks > 0x7FFFFFFF)
-      return set_error(LOKI_ERR_UNSUPPORTED, "grid too large");
-    for (int i = 0; i < (unit ? 4 : 3); ++i) note_launch();
-    phase_map_kernel<uint8_t><<<mblocks, 256, 0, s>>>(freqs + f0, nf, seg_len, nbins, tsamp,
-                                                     t_ref, map);
-    chain_order_kernel<<<(unsigned)oblocks, 256, 0, s>>>(map, nf, seg_len, nbins, order, offs);
-    kf<<<(unsigned)blocks, kChainWarps * 32, smem, s>>>(ts_e, ts_v, nsamps, order, offs, nf, f0,
-                                                        nfreqs, seg_len, nseg, nbins, F,
-                                                        fold_out);
-    if (unit)
-      brutefold_count_kernel<uint8_t><<<(unsigned)nf, 256, hsmem, s>>>(
-          map, nf, f0, nfreqs, seg_len, nsamps, nseg, nbins, fold_out);
+  float* rows = reinterpret_cast<float*>(scratch);
+  char* at = scratch + round256(p.groups * chain_group_bytes(c, seg_len));
+  float* counts = unit ? reinterpret_cast<float*>(at) : nullptr;
+  uint8_t* lists = reinterpret_cast<uint8_t*>(at + round256(p.chunk * 2 * nbins * 4));
+  const int threads = c.F * c.wpf * 32;
+  auto lay_out = [&](int64_t rg0, int64_t n) {
+    note_launch();
+    series_rows_kernel<<<(unsigned)(n * nch * (c.T / 32)), 256, 0, s>>>(ts_e, ts_v, nsamps, seg_len, nseg,
+                                                           nrows, rg0, c.T, 32 * c.V, nch, rows);
+  };
+  if (p.groups * nch * (c.T / 32) > 0x7FFFFFFF || p.chunk > 0x7FFFFFFF ||
+      p.groups * ((p.chunk + c.F - 1) / c.F) > 0x7FFFFFFF)
+    return set_error(LOKI_ERR_UNSUPPORTED, "grid too large");
+  if (p.groups == nrg) lay_out(0, nrg);
+  for (int64_t f0 = 0; f0 < nfreqs; f0 += p.chunk) {
+    const int64_t nf = std::min(p.chunk, nfreqs - f0);
+    note_launch();
+    chain_list_kernel<<<(unsigned)nf, 32 * lwarps, lsmem, s>>>(freqs + f0, seg_len, nbins, tsamp,
+                                                              t_ref, c, nch, last_len, lists,
+                                                              counts);
+    for (int64_t r0 = 0; r0 < nrg; r0 += p.groups) {
+      const int64_t n = std::min(p.groups, nrg - r0);
+      if (p.groups < nrg) lay_out(r0, n);
+      note_launch();
+      kf<<<(unsigned)(n * ((nf + c.F - 1) / c.F)), threads, smem, s>>>(
+          rows, lists, counts, c, nf, f0, nfreqs, nch, nseg, nrows, r0, n, nbins, fold_out);
+    }
     int rc = check_launch("brutefold_chain");
     if (rc) return rc;
   }
@@ -520,16 +760,13 @@ static int brutefold_impl(const float* ts_e, const float* ts_v, bool unit, int64
     return set_error(LOKI_ERR_UNSUPPORTED, "unit-variance counts need segments below 2^24");
   cudaStream_t s = (cudaStream_t)stream;
   const int nc = unit ? 1 : 2;
-  {  // the chain layout when it applies and one frequency of it fits
-    int F = 0, csmem = 0;
-    chain_shape(nbins, nc, &F, &csmem);
-    const int64_t cchunk = std::min(chain_chunk(scratch_bytes, segment_len, nbins), nfreqs);
-    if (F > 0 && cchunk > 0)
-      return brutefold_chain(ts_e, ts_v, unit, nsamps, freqs, nfreqs, segment_len, nbins, tsamp,
-                             t_ref, reinterpret_cast<char*>(phase_scratch), cchunk, F, csmem,
-                             fold_out, s);
-  }
   const int64_t nseg = (nsamps + segment_len - 1) / segment_len;
+  {  // the chain path when it applies and one row group and frequency of it fit
+    const ChainPlan p = chain_plan(nbins, nseg * nc, nfreqs, segment_len, scratch_bytes);
+    if (p.chunk > 0 && (reinterpret_cast<uintptr_t>(phase_scratch) & 15) == 0)
+      return brutefold_chain(ts_e, ts_v, unit, nsamps, freqs, nfreqs, segment_len, nbins, tsamp,
+                             t_ref, reinterpret_cast<char*>(phase_scratch), p, fold_out, s);
+  }
   const int elem = nbins <= 256 ? 1 : 2;
   int64_t chunk = scratch_bytes / (segment_len * elem);
   if (chunk < 1)
@@ -584,13 +821,21 @@ static int brutefold_impl(const float* ts_e, const float* ts_v, bool unit, int64
 
 }  // namespace loki
 
+extern "C" int64_t loki_brutefold_series_scratch_bytes(int64_t nsamps, int64_t nfreqs,
+                                                      int64_t segment_len, int32_t nbins,
+                                                      int32_t unit_variance) {
+  if (nsamps <= 0 || nfreqs <= 0 || segment_len <= 0 || nbins < 1) return 0;
+  const int64_t nrows = (nsamps + segment_len - 1) / segment_len * (unit_variance ? 1 : 2);
+  const int V = nrows > 32 ? 2 : 1;
+  const ChainShape c = chain_shape(nbins, nrows, nfreqs, V);
+  if (!c.V) return nfreqs * segment_len * (nbins <= 256 ? 1 : 2);
+  return 4 * 256 + (nrows + 32 * V - 1) / (32 * V) * chain_group_bytes(c, segment_len) +
+         nfreqs * chain_freq_bytes(c, segment_len, nbins);
+}
+
 extern "C" int64_t loki_brutefold_scratch_bytes(int64_t nfreqs, int64_t segment_len,
                                                 int32_t nbins) {
-  if (nfreqs <= 0 || segment_len <= 0 || nbins < 1) return 0;
-  int F = 0, smem = 0;
-  chain_shape(nbins, 1, &F, &smem);
-  if (F > 0) return 3 * 256 + nfreqs * chain_bytes_per_freq(segment_len, nbins);
-  return nfreqs * segment_len * (nbins <= 256 ? 1 : 2);
+  return loki_brutefold_series_scratch_bytes(segment_len * 64, nfreqs, segment_len, nbins, 1);
 }
 
 extern "C" int loki_brutefold(const float* ts_e, const float* ts_v, int64_t nsamps,
