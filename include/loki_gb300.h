@@ -995,11 +995,22 @@ int loki_downsample(const float* x, int64_t n, int32_t factor, float* out, void*
  * No allocation. */
 int loki_running_median(const float* x, int64_t n, int32_t window, int32_t subtract,
                         float* out, void* stream);
+/* The same with scratch of loki_running_median_scratch_bytes() device bytes
+ * (16-byte aligned; about 16 a sample): every output at once from a wavelet
+ * matrix instead of a window slid over the outputs one by one, two orders of
+ * magnitude faster. n + window <= 2^31. */
+int loki_running_median_scratch(const float* x, int64_t n, int32_t window, int32_t subtract,
+                                float* out, void* scratch, int64_t scratch_bytes, void* stream);
+int64_t loki_running_median_scratch_bytes(int64_t n, int32_t window);
 
 /* k-th smallest element (0-based) of x into *out (device), by a radix select
  * over the float order; scratch of loki_select_scratch_bytes() device bytes. */
 int loki_select_kth(const float* x, int64_t n, int64_t k, float* out, void* scratch,
                     int64_t scratch_bytes, void* stream);
+/* Up to four order statistics of the same array in the same passes; ranks is
+ * a host array, out nranks device floats. */
+int loki_select_ranks(const float* x, int64_t n, const int64_t* ranks, int32_t nranks,
+                      float* out, void* scratch, int64_t scratch_bytes, void* stream);
 int64_t loki_select_scratch_bytes(void);
 
 /* Sum of x (square == 0) or of x^2 (square != 0) accumulated in float64 into

@@ -289,6 +289,9 @@ SIGNATURES: dict[str, tuple] = {
                                   _I32, _P, _P, _P, _P]),
     "loki_downsample": (C.c_int, [_P, _I64, _I32, _P, _P]),
     "loki_running_median": (C.c_int, [_P, _I64, _I32, _I32, _P, _P]),
+    "loki_running_median_scratch": (C.c_int, [_P, _I64, _I32, _I32, _P, _P, _I64, _P]),
+    "loki_running_median_scratch_bytes": (C.c_int64, [_I64, _I32]),
+    "loki_select_ranks": (C.c_int, [_P, _I64, _P, _I32, _P, _P, _I64, _P]),
     "loki_select_kth": (C.c_int, [_P, _I64, _I64, _P, _P, _I64, _P]),
     "loki_select_scratch_bytes": (C.c_int64, []),
     "loki_sum_f64": (C.c_int, [_P, _I64, _I32, _P, _P, _I64, _P]),

@@ -26,17 +26,22 @@ class _Stats:
         self.stream = _lib.stream_ptr(torch.cuda.current_stream(dev))
         self._scratch = torch.empty(max(int(self.lib.loki_select_scratch_bytes()), 8192),
                                     dtype=torch.uint8, device=dev)
-        self._val = torch.empty(1, dtype=torch.float32, device=dev)
+        self._val = torch.empty(4, dtype=torch.float32, device=dev)
         self._dval = torch.empty(1, dtype=torch.float64, device=dev)
 
-    def kth(self, k: int, x=None) -> float:
+    def ranks(self, ks, x=None) -> list[float]:
+        """Order statistics of up to four ranks: one set of passes, one wait."""
         from pyloki_gb300 import _lib
 
         x = self.x if x is None else x
-        _lib.check(self.lib.loki_select_kth(_lib.ptr(x), x.numel(), int(k), _lib.ptr(self._val),
-                                            _lib.ptr(self._scratch), self._scratch.numel(),
-                                            self.stream))
-        return float(self._val.item())
+        ks = np.asarray(ks, dtype=np.int64)
+        _lib.check(self.lib.loki_select_ranks(_lib.ptr(x), x.numel(), ks.ctypes.data, len(ks),
+                                              _lib.ptr(self._val), _lib.ptr(self._scratch),
+                                              self._scratch.numel(), self.stream))
+        return self._val[: len(ks)].tolist()
+
+    def kth(self, k: int, x=None) -> float:
+        return self.ranks([int(k)], x)[0]
 
     def _sum(self, x, square: bool) -> float:
         from pyloki_gb300 import _lib
@@ -51,18 +56,25 @@ class _Stats:
 
     def median(self, x=None) -> float:
         n = self.n if x is None else int(x.numel())
-        lo = self.kth((n - 1) // 2, x)
-        hi = lo if n % 2 else self.kth(n // 2, x)
+        lo, hi = self.ranks([(n - 1) // 2, n // 2], x)
         return float(np.float32((np.float64(lo) + np.float64(hi)) / 2.0))
 
+    def percentiles(self, *qs: float) -> list[float]:
+        """numpy's ``percentile`` (linear interpolation) of the array, for one
+        or two percentages."""
+        pos = [(self.n - 1) * q / 100.0 for q in qs]
+        ks = [int(np.floor(p)) for p in pos]
+        v = self.ranks([k for k0 in ks for k in (k0, min(k0 + 1, self.n - 1))])
+        out = []
+        for i, (p, k) in enumerate(zip(pos, ks)):
+            t = p - k
+            a = np.float64(v[2 * i])
+            b = np.float64(v[2 * i + 1]) if t > 0 else a
+            out.append(float(a + (b - a) * t) if t < 0.5 else float(b - (b - a) * (1.0 - t)))
+        return out
+
     def percentile(self, q: float) -> float:
-        """numpy's ``percentile`` (linear interpolation) of the array."""
-        pos = (self.n - 1) * q / 100.0
-        k = int(np.floor(pos))
-        t = pos - k
-        a = np.float64(self.kth(k))
-        b = np.float64(self.kth(min(k + 1, self.n - 1))) if t > 0 else a
-        return float(a + (b - a) * t) if t < 0.5 else float(b - (b - a) * (1.0 - t))
+        return self.percentiles(q)[0]
 
     def _dev(self, loc: float, absolute: bool):
         import torch
@@ -238,9 +250,15 @@ class TimeSeries:
             msg = "deredden needs a finite series (no NaN or inf)"
             raise ValueError(msg)
         out = torch.empty_like(e)
-        _lib.check(_lib.load().loki_running_median(
-            _lib.ptr(e), e.numel(), nwin, 1, _lib.ptr(out),
-            _lib.stream_ptr(torch.cuda.current_stream(dev))))
+        lib, stream = _lib.load(), _lib.stream_ptr(torch.cuda.current_stream(dev))
+        need = int(lib.loki_running_median_scratch_bytes(e.numel(), nwin))
+        if need:
+            scratch = torch.empty(need, dtype=torch.uint8, device=dev)
+            _lib.check(lib.loki_running_median_scratch(
+                _lib.ptr(e), e.numel(), nwin, 1, _lib.ptr(out), _lib.ptr(scratch), need, stream))
+        else:  # a size only the sliding window takes, or its error
+            _lib.check(lib.loki_running_median(_lib.ptr(e), e.numel(), nwin, 1, _lib.ptr(out),
+                                               stream))
         return TimeSeries(out.cpu().numpy() if host else out,
                           v.cpu().numpy() if host else v, self.tsamp)
 
@@ -275,7 +293,8 @@ class TimeSeries:
         if scale_method == "std":
             scale = st.std()
         elif scale_method == "iqr":
-            scale = (st.percentile(75.0) - st.percentile(25.0)) / 1.3489795003921634
+            hi, lo = st.percentiles(75.0, 25.0)
+            scale = (hi - lo) / 1.3489795003921634
         elif scale_method == "mad":
             scale = st.mad() * 1.482602218505602
         else:
