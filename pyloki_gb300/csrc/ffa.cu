@@ -189,11 +189,23 @@ __device__ __forceinline__ float4 add4(const float4 a, const float4 b) {
 
 // ---------------------------------------------------------------------------
 // DP level (unify_fold, dynamic/dyn_pffa.py:435-489 + shift_add
-// core/common.py:304-324). Each warp owns 32 consecutive output parameters;
-// lane k resolves parameter k once, then the warp streams the roll-add of
-// every segment pair, pair-major, so neighbouring parameters (neighbouring
-// frequencies) are read and written together.
+// core/common.py:304-324). Each warp owns `pw` consecutive output parameters
+// and a range of segment pairs; lane k resolves parameter k once, then the warp
+// streams the roll-add of its segment pairs, pair-major, so neighbouring
+// parameters (neighbouring frequencies) are read and written together.
+//
+// Large levels take 32 parameters and every pair a warp. A level whose warps
+// would not fill the GPU is split, first over the segment pairs, then to 8
+// parameters a warp: a warp's rows are a serial chain of loads of about 1 us,
+// and the levels of a 2^16-sample search (168 to 13 430 parameters) took 47 us
+// each with 1 to 53 blocks and take 4 to 9 us split.
 // ---------------------------------------------------------------------------
+
+// How a level is split over warps: parameters a warp, segment pairs a block.
+struct LevelSplit {
+  int pw;
+  int64_t pairs;
+};
 
 constexpr int kLevelWarps = 8;
 constexpr int kBatch = 4;
@@ -205,14 +217,15 @@ __device__ __forceinline__ void level64_warp(const LokiFFALevel& L, const LevelK
                                              const S* __restrict__ in, S* __restrict__ out,
                                              int32_t* err, const OtherTable& T, bool tab,
                                              const OtherRes* __restrict__ gtab,
-                                             int64_t n_other, int64_t q0) {
+                                             int64_t n_other, int64_t q0, int pw, int64_t ip0,
+                                             int64_t ip1) {
   const int lane = threadIdx.x & 31;
   const int64_t Q = n_out_params(L), P_in = n_in_params(L);
   if (q0 >= Q) return;
-  const LaneTrial me = lane_trial(L, K, T, tab, gtab, n_other, q0 + lane, Q, err);
-  const int kmax = (int)std::min<int64_t>(32, Q - q0);
-  const int64_t nseg_out = L.nseg_in / 2;
-  for (int64_t ip = 0; ip < nseg_out; ++ip) {
+  const int kmax = (int)std::min<int64_t>(pw, Q - q0);
+  const LaneTrial me =
+      lane_trial(L, K, T, tab, gtab, n_other, lane < kmax ? q0 + lane : Q, Q, err);
+  for (int64_t ip = ip0; ip < ip1; ++ip) {
     // rows of 32 four-value groups
     const size_t g_t = (size_t)(2 * ip) * P_in * 32;
     const size_t g_h = (size_t)(2 * ip + 1) * P_in * 32;
@@ -250,63 +263,86 @@ template <typename S>
 __global__ void __launch_bounds__(kLevelWarps * 32, 4)
 ffa_level64_kernel(LokiFFALevel L, LevelK K, const S* __restrict__ in, S* __restrict__ out,
                    int32_t* __restrict__ err, const OtherRes* __restrict__ gtab,
-                   int64_t n_other) {
+                   int64_t n_other, LevelSplit sp) {
   __shared__ OtherTable T;
   const int warp = threadIdx.x >> 5;
   const int64_t Q = n_out_params(L);
-  const int64_t qb = (int64_t)blockIdx.x * kLevelWarps * 32;
+  const int64_t qb = (int64_t)blockIdx.x * kLevelWarps * sp.pw;
   bool tab = false;
   if (!gtab) {  // uniform: the whole block takes the same branch
-    tab = build_table(T, L, K, qb, std::min<int64_t>(qb + kLevelWarps * 32, Q) - 1);
+    tab = build_table(T, L, K, qb, std::min<int64_t>(qb + kLevelWarps * sp.pw, Q) - 1);
     __syncthreads();
   }
-  level64_warp(L, K, in, out, err, T, tab, gtab, n_other, qb + warp * 32);
+  const int64_t ip0 = blockIdx.y * sp.pairs;
+  level64_warp(L, K, in, out, err, T, tab, gtab, n_other, qb + warp * sp.pw, sp.pw, ip0,
+               std::min<int64_t>(ip0 + sp.pairs, L.nseg_in / 2));
 }
 
-// Any nbins: scalar, lane j handles bins j, j + 32, ...
+// Any nbins: scalar, lane j handles bins j, j + 32, ... of four parameters at a
+// time (16 loads in flight a lane; one parameter at a time left the level
+// waiting on each row: 3.0 -> 1.4 ms for the six levels of a 2^20 search with
+// 100 bins).
 template <typename S>
-__global__ void __launch_bounds__(kLevelWarps * 32, 4)
+__global__ void __launch_bounds__(kLevelWarps * 32, 3)
 ffa_level_kernel(LokiFFALevel L, LevelK K, const S* __restrict__ in, S* __restrict__ out,
                  int32_t* __restrict__ err, const OtherRes* __restrict__ gtab,
-                 int64_t n_other) {
+                 int64_t n_other, LevelSplit sp) {
   __shared__ OtherTable T;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t Q = n_out_params(L), P_in = n_in_params(L);
-  const int64_t qb = (int64_t)blockIdx.x * kLevelWarps * 32;
+  const int64_t qb = (int64_t)blockIdx.x * kLevelWarps * sp.pw;
   bool tab = false;
   if (!gtab) {  // uniform: the whole block takes the same branch
-    tab = build_table(T, L, K, qb, std::min<int64_t>(qb + kLevelWarps * 32, Q) - 1);
+    tab = build_table(T, L, K, qb, std::min<int64_t>(qb + kLevelWarps * sp.pw, Q) - 1);
     __syncthreads();
   }
-  const int64_t q0 = qb + warp * 32;
+  const int64_t q0 = qb + warp * sp.pw;
   if (q0 >= Q) return;
-  const LaneTrial me = lane_trial(L, K, T, tab, gtab, n_other, q0 + lane, Q, err);
+  const int kmax = (int)std::min<int64_t>(sp.pw, Q - q0);
+  const LaneTrial me =
+      lane_trial(L, K, T, tab, gtab, n_other, lane < kmax ? q0 + lane : Q, Q, err);
   const int nb = L.nbins;
-  const int kmax = (int)std::min<int64_t>(32, Q - q0);
-  const int64_t nseg_out = L.nseg_in / 2;
   const size_t row = (size_t)2 * nb;
-  for (int64_t ip = 0; ip < nseg_out; ++ip) {
+  const int64_t ip0 = blockIdx.y * sp.pairs;
+  const int64_t ip1 = std::min<int64_t>(ip0 + sp.pairs, L.nseg_in / 2);
+  for (int64_t ip = ip0; ip < ip1; ++ip) {
     const S* in_t = in + (size_t)(2 * ip) * P_in * row;
     const S* in_h = in + (size_t)(2 * ip + 1) * P_in * row;
     S* o_base = out + ((size_t)ip * Q + q0) * row;
-    for (int k = 0; k < kmax; ++k) {
-      const int64_t it = __shfl_sync(0xFFFFFFFFu, me.t, k);
-      const int64_t ih = __shfl_sync(0xFFFFFFFFu, me.h, k);
-      const int st = __shfl_sync(0xFFFFFFFFu, me.st, k);
-      const int sh = __shfl_sync(0xFFFFFFFFu, me.sh, k);
-      const bool ok = __shfl_sync(0xFFFFFFFFu, me.ok, k);
-      if (!ok) continue;
-      const S* t = in_t + (size_t)it * row;
-      const S* h = in_h + (size_t)ih * row;
-      S* o = o_base + (size_t)k * row;
+    for (int k0 = 0; k0 < kmax; k0 += kBatch) {
+      const S *t[kBatch], *h[kBatch];
+      int st[kBatch], sh[kBatch];
+      bool ok[kBatch];
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u) {
+        const int k = k0 + u, src = k < kmax ? k : 0;
+        t[u] = in_t + (size_t)__shfl_sync(0xFFFFFFFFu, me.t, src) * row;
+        h[u] = in_h + (size_t)__shfl_sync(0xFFFFFFFFu, me.h, src) * row;
+        st[u] = __shfl_sync(0xFFFFFFFFu, me.st, src);
+        sh[u] = __shfl_sync(0xFFFFFFFFu, me.sh, src);
+        ok[u] = __shfl_sync(0xFFFFFFFFu, me.ok, src) && k < kmax;
+      }
       for (int j = lane; j < nb; j += 32) {
-        int jt = j - st;
-        jt += (jt < 0) ? nb : 0;
-        int jh = j - sh;
-        jh += (jh < 0) ? nb : 0;
-        Store<S>::store(o + j, __fadd_rn(Store<S>::load(t + jt), Store<S>::load(h + jh)));
-        Store<S>::store(o + nb + j,
-                        __fadd_rn(Store<S>::load(t + nb + jt), Store<S>::load(h + nb + jh)));
+        float te[kBatch], tv[kBatch], he[kBatch], hv[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+          if (!ok[u]) continue;  // uniform across the warp
+          int jt = j - st[u];
+          jt += (jt < 0) ? nb : 0;
+          int jh = j - sh[u];
+          jh += (jh < 0) ? nb : 0;
+          te[u] = Store<S>::load(t[u] + jt);
+          tv[u] = Store<S>::load(t[u] + nb + jt);
+          he[u] = Store<S>::load(h[u] + jh);
+          hv[u] = Store<S>::load(h[u] + nb + jh);
+        }
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+          if (!ok[u]) continue;
+          S* o = o_base + (size_t)(k0 + u) * row;
+          Store<S>::store(o + j, __fadd_rn(te[u], he[u]));
+          Store<S>::store(o + nb + j, __fadd_rn(tv[u], hv[u]));
+        }
       }
     }
   }
@@ -465,7 +501,7 @@ band_union64_kernel(LokiFFALevel F, LevelK KF, const S* __restrict__ in_f,
                  (blockIdx.x - seg * nblk_f) * blockDim.x + warp * 32, tile, seg);
   } else {
     level64_warp(P, KP, in_p, out_p, err, T, false, tab_p, no_p,
-                 (int64_t)(blockIdx.x - nsc) * blockDim.x + warp * 32);
+                 (int64_t)(blockIdx.x - nsc) * blockDim.x + warp * 32, 32, 0, P.nseg_in / 2);
   }
 }
 
@@ -1002,16 +1038,28 @@ static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 template <typename S>
 static int launch_level_t(const LokiFFALevel& L, const LevelK& K, const S* in, S* out,
                           int32_t* err, cudaStream_t s, const OtherRes* gtab, int64_t n_other) {
-  const int64_t Q = n_out_params(L);
-  const int64_t blocks = (Q + kLevelWarps * 32 - 1) / (kLevelWarps * 32);
-  if (blocks > 0x7FFFFFFF) return set_error(LOKI_ERR_UNSUPPORTED, "grid too large");
+  const int64_t Q = n_out_params(L), pairs = L.nseg_in / 2;
+  // The GPU holds 152 SMs x 4 blocks of 8 warps. Pairs are split until there are
+  // four times as many (the last wave of a large level: 31.9 -> 28.5 ms for the
+  // seven levels of a 2^23 search); fewer parameters a warp resolve with fewer
+  // lanes, so only a level that does not fill the GPU once takes 8 (0.80 ms
+  // against 0.99 for the six levels of a 2^20 search otherwise).
+  constexpr int64_t kWant = 152 * 4 * kLevelWarps;
+  LevelSplit sp{32, pairs};
+  int64_t parts =
+      std::min<int64_t>({pairs, 65535, (4 * kWant + (Q + 31) / 32 - 1) / ((Q + 31) / 32)});
+  sp.pairs = (pairs + parts - 1) / parts;
+  parts = (pairs + sp.pairs - 1) / sp.pairs;
+  if (parts * ((Q + 31) / 32) < kWant) sp.pw = 8;
+  const int64_t blocks_x = (Q + kLevelWarps * sp.pw - 1) / (kLevelWarps * sp.pw);
+  if (blocks_x > 0x7FFFFFFF) return set_error(LOKI_ERR_UNSUPPORTED, "grid too large");
+  const dim3 blocks((unsigned)blocks_x, (unsigned)parts);
   note_launch();
   if (L.nbins == 64 && aligned16(in) && aligned16(out))
-    ffa_level64_kernel<S><<<(unsigned)blocks, kLevelWarps * 32, 0, s>>>(L, K, in, out, err,
-                                                                        gtab, n_other);
+    ffa_level64_kernel<S><<<blocks, kLevelWarps * 32, 0, s>>>(L, K, in, out, err, gtab, n_other,
+                                                              sp);
   else
-    ffa_level_kernel<S><<<(unsigned)blocks, kLevelWarps * 32, 0, s>>>(L, K, in, out, err, gtab,
-                                                                      n_other);
+    ffa_level_kernel<S><<<blocks, kLevelWarps * 32, 0, s>>>(L, K, in, out, err, gtab, n_other, sp);
   return LOKI_OK;
 }
 
