@@ -792,6 +792,12 @@ int64_t loki_scan_scratch_bytes(int64_t n);
 int loki_boxcar_snr(const float* profiles, int64_t nprof, int32_t nbins,
                     const LokiScoreSpec* spec, float* snr, void* stream);
 
+/* Boxcar S/N of (n, 2, nbins) folds, normalised e / sqrt(v) on the way:
+ * loki_fold_norm and loki_boxcar_snr in one pass, the same values (ffa.py:382-411
+ * and detection/scoring.py:99-153). */
+int loki_fold_snr(const float* folds, int64_t n, int32_t nbins, const LokiScoreSpec* spec,
+                  float* snr, void* stream);
+
 /* Score of (n, 2, nbins) folds: boxcar S/N of e / sqrt(v), max over widths
  * (detection/scoring.py:249-282 snr_score_batch_func). spec->mode is ignored. */
 int loki_snr_score_batch(const float* folds, int64_t n, int32_t nbins,

@@ -276,6 +276,7 @@ SIGNATURES: dict[str, tuple] = {
     "loki_ffa_final_tiled_scratch": (C.c_int64, [C.POINTER(LokiFFALevel),
                                                  C.POINTER(LokiFFALevel)]),
     "loki_boxcar_snr": (C.c_int, [_P, _I64, _I32, C.POINTER(LokiScoreSpec), _P, _P]),
+    "loki_fold_snr": (C.c_int, [_P, _I64, _I32, C.POINTER(LokiScoreSpec), _P, _P]),
     "loki_snr_score_batch": (C.c_int, [_P, _I64, _I32, C.POINTER(LokiScoreSpec), _P, _P]),
     "loki_fold_norm": (C.c_int, [_P, _I64, _I32, _P, _P]),
     "loki_f32_to_bf16": (C.c_int, [_P, _I64, _P, _P]),

@@ -46,15 +46,19 @@ __device__ __forceinline__ float prefix_row(float* row, int nbins, int wmax) {
   return last;  // prefix_sum[nbins - 1] == total
 }
 
-// S/N for one width given the prefix row (scoring.py:131-138).
-__device__ __forceinline__ double snr_width(const float* row, int nbins, int w,
-                                            double hb, double b, float total) {
-  float dmax = -FLT_MAX;
+// Largest differences P[i + w] - P[i] of up to four widths at once: the row is
+// walked once for all of them. A NaN difference is passed over, as the
+// reference's d > max does.
+__device__ __forceinline__ void dmax_widths(const float* row, int nbins, const int (&w)[4],
+                                            float (&m)[4]) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) m[q] = -FLT_MAX;
+#pragma unroll 4
   for (int i = 0; i < nbins; ++i) {
-    const float d = __fsub_rn(row[i + w], row[i]);
-    if (d > dmax) dmax = d;
+    const float p = row[i];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) m[q] = fmaxf(m[q], __fsub_rn(row[i + w[q]], p));
   }
-  return __dsub_rn(__dmul_rn(hb, (double)dmax), __dmul_rn(b, (double)total));
 }
 
 // ---- fast path: nbins == 64, widths 1, 2, 4, ..., 2^(nw-1) -----------------
@@ -221,21 +225,26 @@ __device__ __forceinline__ void score_row(float* row, int nbins, const LokiScore
                                           float* out) {
   const float total = prefix_row(row, nbins, sp.wmax);
   // (generic path: any nbins and width list, prefix in shared memory)
-  if (sp.mode == 0) {
-    for (int iw = 0; iw < sp.nwidths; ++iw) {
-      double s = snr_width(row, nbins, sp.widths[iw], sp.hb[iw], sp.b[iw], total);
-      out[iw] = __double2float_rn(__dmul_rn(s, sp.inv_stdnoise));
+  double best = -(double)FLT_MAX;
+  for (int w0 = 0; w0 < sp.nwidths; w0 += 4) {
+    int w[4];
+    float m[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) w[q] = sp.widths[min(w0 + q, sp.nwidths - 1)];
+    dmax_widths(row, nbins, w, m);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int iw = w0 + q;
+      if (iw >= sp.nwidths) break;
+      // S/N of one width (scoring.py:131-138)
+      const double s = __dmul_rn(__dsub_rn(__dmul_rn(sp.hb[iw], (double)m[q]),
+                                           __dmul_rn(sp.b[iw], (double)total)),
+                                 sp.inv_stdnoise);
+      if (sp.mode == 0) out[iw] = __double2float_rn(s);
+      else if (s > best) best = s;
     }
-  } else {
-    double best = -(double)FLT_MAX;
-    for (int iw = 0; iw < sp.nwidths; ++iw) {
-      double s = __dmul_rn(
-          snr_width(row, nbins, sp.widths[iw], sp.hb[iw], sp.b[iw], total),
-          sp.inv_stdnoise);
-      if (s > best) best = s;
-    }
-    out[0] = __double2float_rn(best);
   }
+  if (sp.mode != 0) out[0] = __double2float_rn(best);
 }
 
 }  // namespace loki

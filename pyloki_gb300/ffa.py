@@ -381,6 +381,25 @@ class DynamicProgramming:
         self.launches += 1
         return out.reshape(*lead, self.nbins)
 
+    def fold_snr(self, widths=None, stdnoise: float = 1.0, *, iseg: int = 0) -> torch.Tensor:
+        """Boxcar S/N ``(*counts, nwidths)`` of one segment's folds of the
+        current level: ``boxcar_snr_nd(get_fold_norm(iseg), widths)``, for
+        time-domain float32 folds without writing the normalised profiles."""
+        widths = self.cfg.score_widths if widths is None else np.asarray(widths, np.int64)
+        if self.cfg.use_fourier or self._storage:
+            from pyloki_gb300.scoring import boxcar_snr_nd
+
+            return boxcar_snr_nd(self.get_fold_norm(iseg), widths, stdnoise)
+        fold = self.fold[iseg]
+        flat = fold.reshape(-1, 2, fold.shape[-1])
+        snr = torch.empty((flat.shape[0], len(widths)), dtype=torch.float32,
+                          device=self._device)
+        spec = _lib.score_spec(widths, self.nbins, stdnoise, mode=0)
+        _lib.check(self._lib.loki_fold_snr(_lib.ptr(flat), flat.shape[0], self.nbins, spec,
+                                           _lib.ptr(snr), self._stream()))
+        self.launches += 1
+        return snr.reshape(*fold.shape[:-2], len(widths))
+
     def get_complexity(self) -> list[int]:
         return [_cart_len(self.cfg.get_param_grid_count(lvl))
                 for lvl in range(self.cfg.niters_ffa + 1)]

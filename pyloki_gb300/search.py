@@ -140,9 +140,7 @@ def ffa_search(tseries: TimeSeries, search_cfg: PulsarSearchConfig, *, quiet: bo
     dyp.initialize()
     if materialize:
         dyp.execute(show_progress=show_progress)
-        from pyloki_gb300.scoring import boxcar_snr_nd
-
-        snrs = boxcar_snr_nd(dyp.get_fold_norm(), widths, 1.0)
+        snrs = dyp.fold_snr(widths)
     else:
         snrs = dyp.search(widths, 1.0, norm=norm)
     pgram = Periodogram(params={"width": widths, **dyp.param_arr_dict}, snrs=snrs,
