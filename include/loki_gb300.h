@@ -270,6 +270,19 @@ int loki_brutefold_complex(const float* ts_e, const float* ts_v, int64_t nsamps,
                            int32_t nbins, double tsamp, double t_ref, void* fold_out,
                            void* stream);
 
+/* The same on the tensor cores, with scratch of
+ * loki_brutefold_complex_scratch_bytes() device bytes (16-byte aligned) for
+ * the segments split into bfloat16 parts; float32 results, as close to float64
+ * as loki_brutefold_complex's. segment_len <= 2^24. A bounded wait that runs
+ * out sets LOKI_DEVERR_TIMEOUT. */
+int loki_brutefold_complex_scratch(const float* ts_e, const float* ts_v, int64_t nsamps,
+                                   const double* freqs, int64_t nfreqs, int64_t segment_len,
+                                   int32_t nbins, double tsamp, double t_ref, void* scratch,
+                                   int64_t scratch_bytes, void* fold_out, int32_t* dev_err,
+                                   void* stream);
+int64_t loki_brutefold_complex_scratch_bytes(int64_t nsamps, int64_t segment_len,
+                                             int32_t unit_variance);
+
 /* One complex DP level (dynamic/dyn_pffa.py:435-489 with shift_add_complex,
  * core/common.py:344-372): out[ipair, p] = tail * e^{-2 pi i k s_t / nbins}
  * + head * e^{-2 pi i k s_h / nbins} by phasor recurrence over k, the rows
@@ -277,6 +290,18 @@ int loki_brutefold_complex(const float* ts_e, const float* ts_v, int64_t nsamps,
  * levels only (no frequency window). */
 int loki_ffa_level_complex(const LokiFFALevel* lvl, const LokiFFACoord* plan,
                            const void* fold_in, void* fold_out, void* stream);
+
+/* The same level without a plan: the rows exactly, the shifts to float32
+ * rounding, resolved in the kernel; nbins <= 286. An index outside the grid
+ * sets LOKI_DEVERR_WINDOW in dev_err. */
+int loki_ffa_level_complex_rows(const LokiFFALevel* lvl, const void* fold_in, void* fold_out,
+                                int32_t* dev_err, void* stream);
+
+/* Boxcar S/N of (n, 2, 33) complex folds of 64 bins: loki_fold_norm_complex and
+ * loki_boxcar_snr in one pass (float32 transforms, within their rounding).
+ * Widths up to 70. */
+int loki_fold_snr_complex64(const void* folds, int64_t n, const LokiScoreSpec* spec, float* snr,
+                            void* stream);
 
 /* Normalised profiles of complex folds (ffa.py:401-411): irfft of both
  * components to nbins samples, then e / sqrt(v); folds (n, 2, nbins / 2 + 1)

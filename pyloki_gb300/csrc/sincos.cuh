@@ -1,0 +1,55 @@
+// Sine and cosine of the Fourier folds' float32 angles.
+#pragma once
+
+#include "loki_common.cuh"
+
+namespace loki {
+
+// sin and cos of a float32 angle by Cody and Waite's additive reduction
+// ("Software Manual for the Elementary Functions", 1980): 2 pi split into
+// three float32 parts, the first two with 8 significant bits so that k times
+// them is exact for |k| < 2^15 (angles up to about 2e5 rad), subtracted with
+// fused multiply-adds; sincosf of the reduced angle then stays on its short
+// path. The parts come from 2 pi to 60 digits: 0x1.92p+2 + 0x1.fbp-10 +
+// 0x1.5110b4p-20 (their sum is 2 pi to 2e-14).
+__device__ __forceinline__ void sincos_reduced(float a, float* s, float* c) {
+  constexpr float kC1 = 0x1.92p+2f, kC2 = 0x1.fbp-10f, kC3 = 0x1.5110b4p-20f;
+  const float k = rintf(__fmul_rn(a, 0.15915494f));
+  if (fabsf(k) < 32768.0f) {
+    float r = __fmaf_rn(-k, kC1, a);
+    r = __fmaf_rn(-k, kC2, r);
+    r = __fmaf_rn(-k, kC3, r);
+    sincosf(r, s, c);
+  } else {
+    sincosf(a, s, c);
+  }
+}
+
+// The same for a caller that knows |a| < 2e5: reduction by pi / 2 in four
+// parts (the first three with 7 significant bits, so k times them is exact for
+// |k| < 2^17 and the subtractions are exact; the parts, truncations of pi / 2
+// to 60 digits, sum to it within 6e-15), then minimax polynomials on [-pi/4,
+// pi/4] in r^2 (Remez exchange in float64, rounded: sin to 4e-9, cos to 1e-10
+// before rounding). Both results are within 1.3 x 2^-24 of the exact values:
+// as accurate as sincosf there, in about half its instructions.
+__device__ __forceinline__ void sincos_small(float a, float* s, float* c) {
+  const float kf = __fmaf_rn(a, 0x1.45f306p-1f, 12582912.0f);  // 2^23 + 2^22: k in the low bits
+  const unsigned q = __float_as_uint(kf);
+  const float k = __fsub_rn(kf, 12582912.0f);
+  float r = __fmaf_rn(-k, 0x1.9p+0f, a);
+  r = __fmaf_rn(-k, 0x1.0cp-7f, r);
+  r = __fmaf_rn(-k, 0x1.ecp-14f, r);
+  r = __fmaf_rn(-k, 0x1.5110b4p-22f, r);
+  const float r2 = __fmul_rn(r, r);
+  float p = __fmaf_rn(r2, -0x1.994cfap-13f, 0x1.11075cp-7f);
+  p = __fmaf_rn(r2, p, -0x1.555546p-3f);
+  const float sr = __fmaf_rn(__fmul_rn(r, r2), p, r);
+  float t = __fmaf_rn(r2, 0x1.9a00cep-16f, -0x1.6c0c86p-10f);
+  t = __fmaf_rn(r2, t, 0x1.55554ap-5f);
+  const float cr = __fmaf_rn(__fmul_rn(r2, r2), t, __fmaf_rn(r2, -0.5f, 1.0f));
+  const float sv = q & 1u ? cr : sr, cv = q & 1u ? sr : cr;
+  *s = __uint_as_float(__float_as_uint(sv) ^ ((q << 30) & 0x80000000u));
+  *c = __uint_as_float(__float_as_uint(cv) ^ (((q + 1u) << 30) & 0x80000000u));
+}
+
+}  // namespace loki

@@ -170,6 +170,11 @@ class DynamicProgramming:
         if nbatch > 1 and cfg.use_fourier:
             msg = "batched series are for time-domain folds"
             raise ValueError(msg)
+        # More than one final segment: the folds feed a pruning tree, whose
+        # survivor sets hang on every rounding of a complex fold, so those keep
+        # the direct sums and the phasor recurrence. A search's folds take the
+        # tensor cores and whole-row levels (2^20 samples: 147 -> 19 ms).
+        self._tree_folds = cfg.nsamps > cfg.bseg_ffa
         self.nbatch = nbatch
         self._ts_dev: tuple[torch.Tensor, torch.Tensor] | None = None
         self._ts_data = ts_data
@@ -297,13 +302,24 @@ class DynamicProgramming:
             nfreq = g0.dev[-1].numel()
             nbf = cfg.nbins // 2 + 1
             fold = torch.empty((nseg, nfreq, 2, nbf), dtype=torch.complex64, device=dev)
-            _lib.check(self._lib.loki_brutefold_complex(
-                _lib.ptr(ts_e), 0 if self._unit_var else _lib.ptr(ts_v), ts_e.numel(),
-                _lib.ptr(g0.dev[-1]), nfreq,
-                cfg.bseg_brute, cfg.nbins, cfg.tsamp, t_ref, _lib.ptr(fold), self._stream()))
+            self._err.zero_()
+            v_ptr = 0 if self._unit_var else _lib.ptr(ts_v)
+            need = int(self._lib.loki_brutefold_complex_scratch_bytes(
+                ts_e.numel(), cfg.bseg_brute, int(self._unit_var)))
+            if need and not self._tree_folds:
+                scratch = torch.empty(need, dtype=torch.uint8, device=dev)
+                _lib.check(self._lib.loki_brutefold_complex_scratch(
+                    _lib.ptr(ts_e), v_ptr, ts_e.numel(), _lib.ptr(g0.dev[-1]), nfreq,
+                    cfg.bseg_brute, cfg.nbins, cfg.tsamp, t_ref, _lib.ptr(scratch), need,
+                    _lib.ptr(fold), _lib.ptr(self._err), self._stream()))
+                self.launches += 1
+            else:
+                _lib.check(self._lib.loki_brutefold_complex(
+                    _lib.ptr(ts_e), v_ptr, ts_e.numel(), _lib.ptr(g0.dev[-1]), nfreq,
+                    cfg.bseg_brute, cfg.nbins, cfg.tsamp, t_ref, _lib.ptr(fold),
+                    self._stream()))
             self.launches += 1
             self._fold = fold.reshape(nseg, *([1] * (cfg.nparams - 1)), nfreq, 2, nbf)
-            self._err.zero_()
             self._ffa_level = 0
             return
         self._fold, nl = _brutefold(ts_e, ts_v, g0.dev[-1], cfg.bseg_brute, cfg.nbins,
@@ -339,14 +355,20 @@ class DynamicProgramming:
         if self.cfg.use_fourier:  # shift_add_complex (core/common.py:344-372)
             nbf = self.nbins // 2 + 1
             desc = level_desc(self.cfg, cur, prev, nseg_in)
-            plan = torch.empty((cur.size, 4), dtype=torch.int32, device=self._device)
-            _lib.check(self._lib.loki_ffa_plan(desc, _lib.ptr(plan), _lib.ptr(self._err),
-                                               self._stream()))
             out = torch.empty((nseg_in // 2, cur.size, 2, nbf), dtype=torch.complex64,
                               device=self._device)
-            _lib.check(self._lib.loki_ffa_level_complex(desc, _lib.ptr(plan), _lib.ptr(fold_in),
-                                                        _lib.ptr(out), self._stream()))
-            self.launches += 2
+            if self.nbins <= 286 and not self._tree_folds:
+                _lib.check(self._lib.loki_ffa_level_complex_rows(
+                    desc, _lib.ptr(fold_in), _lib.ptr(out), _lib.ptr(self._err),
+                    self._stream()))
+                self.launches += 1
+            else:
+                plan = torch.empty((cur.size, 4), dtype=torch.int32, device=self._device)
+                _lib.check(self._lib.loki_ffa_plan(desc, _lib.ptr(plan), _lib.ptr(self._err),
+                                                   self._stream()))
+                _lib.check(self._lib.loki_ffa_level_complex(
+                    desc, _lib.ptr(plan), _lib.ptr(fold_in), _lib.ptr(out), self._stream()))
+                self.launches += 2
             self._fold = out.reshape(nseg_in // 2, *cur.counts.tolist(), 2, nbf)
             self._ffa_level += 1
             return
@@ -384,9 +406,11 @@ class DynamicProgramming:
     def fold_snr(self, widths=None, stdnoise: float = 1.0, *, iseg: int = 0) -> torch.Tensor:
         """Boxcar S/N ``(*counts, nwidths)`` of one segment's folds of the
         current level: ``boxcar_snr_nd(get_fold_norm(iseg), widths)``, for
-        time-domain float32 folds without writing the normalised profiles."""
+        float32 folds, and complex ones of 64 bins, without writing the
+        normalised profiles."""
         widths = self.cfg.score_widths if widths is None else np.asarray(widths, np.int64)
-        if self.cfg.use_fourier or self._storage:
+        fourier = self.cfg.use_fourier
+        if self._storage or (fourier and (self.nbins != 64 or int(widths.max()) > 70)):
             from pyloki_gb300.scoring import boxcar_snr_nd
 
             return boxcar_snr_nd(self.get_fold_norm(iseg), widths, stdnoise)
@@ -395,8 +419,12 @@ class DynamicProgramming:
         snr = torch.empty((flat.shape[0], len(widths)), dtype=torch.float32,
                           device=self._device)
         spec = _lib.score_spec(widths, self.nbins, stdnoise, mode=0)
-        _lib.check(self._lib.loki_fold_snr(_lib.ptr(flat), flat.shape[0], self.nbins, spec,
-                                           _lib.ptr(snr), self._stream()))
+        if fourier:
+            _lib.check(self._lib.loki_fold_snr_complex64(_lib.ptr(flat), flat.shape[0], spec,
+                                                         _lib.ptr(snr), self._stream()))
+        else:
+            _lib.check(self._lib.loki_fold_snr(_lib.ptr(flat), flat.shape[0], self.nbins, spec,
+                                               _lib.ptr(snr), self._stream()))
         self.launches += 1
         return snr.reshape(*fold.shape[:-2], len(widths))
 
@@ -514,9 +542,7 @@ class DynamicProgramming:
         if cfg.use_fourier:  # every level materialised, then irfft norm + boxcar
             self.execute()
             mark("levels")
-            from pyloki_gb300.scoring import boxcar_snr_nd
-
-            snr = boxcar_snr_nd(self.get_fold_norm(), widths, stdnoise)
+            snr = self.fold_snr(widths, stdnoise)
             if mode != 0:
                 snr = snr.amax(dim=-1)
             mark("final")
