@@ -623,7 +623,8 @@ typedef struct {
   LokiPruneWork work;           /* par_cap >= max_sugg, ovf_cap >= max_sugg + child_cap + 1;
                                    host_words and the events are not used */
   int64_t* counts;              /* 8 words: parents, children, survivors, backtrack rows,
-                                   valid children of the level */
+                                   valid children of the level; the last three are the
+                                   emission's (parents, first backtrack row, best) */
   int32_t* ovf_flag;            /* 1 word */
   LokiPruneLevelStats* stats;   /* nlevels records */
   double* best_leaves;          /* nlevels rows of (poly_order + 2) * 2, or NULL */

@@ -409,7 +409,7 @@ fold_snr_complex64_kernel(const float2* __restrict__ folds, int64_t n, LokiScore
   }
   const int nout = sp.mode == 0 ? sp.nwidths : 1;
   if (SK.pow2_64) score_row64_pow2(x, sp, SK, out + (size_t)(p0 + tid) * nout);
-  else score_row(x, 64, sp, out + (size_t)(p0 + tid) * nout);
+  else score_row(x, 64, sp, SK, out + (size_t)(p0 + tid) * nout);
 }
 
 // get_fold_norm for Fourier folds (ffa.py:401-411): irfft of each component

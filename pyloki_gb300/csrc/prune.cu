@@ -210,12 +210,18 @@ __device__ __forceinline__ int64_t axis_index(double v, double vmin, double inv,
 // Child leaf parameters [d_P .. d_1] from the parent's branching info.
 __device__ __forceinline__ void child_params(const LokiBranchInfo& B, int P, int64_t local,
                                              double* pv) {
+  // a parent has at most branch_max^P children: 32-bit arithmetic, and none for
+  // the parameters that did not split
+  uint32_t rest = (uint32_t)local;
   for (int j = P - 1; j >= 0; --j) {
-    const int64_t c = B.count[j];
-    const int64_t k = local % c;
-    local /= c;
-    pv[j] = (c == 1 && k == 0) ? B.first[j]
-                               : __dadd_rn(B.first[j], __dmul_rn((double)k, B.dact[j]));
+    const uint32_t c = (uint32_t)B.count[j];
+    if (c == 1) {
+      pv[j] = B.first[j];
+      continue;
+    }
+    const uint32_t q = rest / c, k = rest - q * c;
+    rest = q;
+    pv[j] = __dadd_rn(B.first[j], __dmul_rn((double)k, B.dact[j]));
   }
 }
 
@@ -407,6 +413,37 @@ __device__ __forceinline__ int64_t find_parent(const int64_t* offsets, int64_t n
   return lo;
 }
 
+// find_parent for a warp: lanes k < kmax hold ascending children c. The first
+// lane's parent by a 32-way search, the others' among the 32 parents after it
+// (a few windows; a lane beyond them searches alone). Four to five dependent
+// loads where a binary search of every lane takes 12 to 16.
+__device__ __forceinline__ int64_t warp_find_parents(const int64_t* __restrict__ offsets,
+                                                     int64_t n, int64_t c, int kmax) {
+  const int lane = threadIdx.x & 31;
+  const int64_t c0 = __shfl_sync(0xFFFFFFFFu, c, 0);
+  if (lane >= kmax) c = c0;
+  int64_t lo = 0, hi = n;  // offsets[lo] <= c0 < offsets[hi]
+  while (hi - lo > 32) {
+    const int64_t step = (hi - lo + 31) / 32, i = lo + lane * step;
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, i < hi && offsets[i] <= c0);
+    lo += (31 - __clz(m)) * step;
+    hi = min(hi, lo + step);
+  }
+  lo += __popc(__ballot_sync(0xFFFFFFFFu, lo + lane < hi && offsets[lo + lane] <= c0)) - 1;
+  int64_t par = -1;
+  for (int w = 0; w < 4; ++w, lo += 32) {
+    const int64_t off = offsets[min(lo + 1 + lane, n)];
+    int k = 0;  // entries of the window at or below c
+#pragma unroll
+    for (int s = 16; s >= 1; s >>= 1)
+      if (__shfl_sync(0xFFFFFFFFu, off, k + s - 1) <= c) k += s;
+    if (__shfl_sync(0xFFFFFFFFu, off, k) <= c) ++k;
+    if (par < 0 && k < 32) par = lo + k;
+    if (__ballot_sync(0xFFFFFFFFu, par < 0) == 0) break;
+  }
+  return par >= 0 ? par : find_parent(offsets, n, c);
+}
+
 __device__ __forceinline__ unsigned float_key(float x) {
   const unsigned u = __float_as_uint(x);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
@@ -416,37 +453,13 @@ __device__ __forceinline__ float key_float(unsigned k) {
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
 }
 
-// Children c0 .. c0 + 31 (those below n_children) of one warp.
-__device__ __forceinline__ void score_tile(const LokiPruneLevel& D, const double* __restrict__ leaves,
-                   const float* __restrict__ folds, int64_t n_parents,
-                   const LokiBranchInfo* __restrict__ info, const int64_t* __restrict__ offsets,
-                   int64_t n_children, const float* __restrict__ seg, const LokiScoreSpec& sp,
-                   const ScoreK& SK, float* __restrict__ scores, int32_t* __restrict__ cidx,
-                   double* __restrict__ cphase, unsigned* __restrict__ minmax_keys,
-                   float* tile, int64_t c0) {
+// Rows of 32 children (parent row, segment row and roll held lane by lane):
+// shift-add, e / sqrt(v), one normalised profile per tile row.
+__device__ __forceinline__ void gather_norm_rows(const float* __restrict__ folds,
+                                                 const float* __restrict__ seg, int64_t my_par,
+                                                 int64_t my_row, int my_shift, int kmax, int nb,
+                                                 float* tile, int stride) {
   const int lane = threadIdx.x & 31;
-  const int nb = D.nbins, P = D.poly_order;
-  const int stride = score_stride(nb, sp.wmax);
-  const int kmax = (int)std::min<int64_t>(32, n_children - c0);
-  // lane k resolves child c0 + k
-  int64_t my_par = 0, my_row = 0;
-  int my_shift = 0;
-  if (lane < kmax) {
-    const int64_t c = c0 + lane;
-    const int64_t par = find_parent(offsets, n_parents, c);
-    const LokiBranchInfo B = info[par];
-    const double* lf = leaves + par * (P + 2) * 2;
-    double pv[LOKI_MAX_PARAMS + 1];
-    child_params(B, P, c - offsets[par], pv);
-    pv[P] = B.d0;  // d_0 (alpha_0 in the current domain for Chebyshev)
-    const ChildRes r = resolve_child(D, pv, lf[(P + 1) * 2]);
-    cidx[2 * c] = r.ia;
-    cidx[2 * c + 1] = r.iff;
-    cphase[c] = r.phase;
-    my_par = par;
-    my_row = (int64_t)r.ia * D.n_freq + r.iff;
-    my_shift = round_shift(r.phase, nb);
-  }
   if (nb == 64) {
     // eight children's rows in flight per lane (bins lane and lane + 32)
     constexpr int kU = 8;
@@ -504,17 +517,63 @@ __device__ __forceinline__ void score_tile(const LokiPruneLevel& D, const double
     }
   }
   __syncwarp();
+}
+
+// Lane k scores row k of the tile; the level's score range is reduced over the
+// warp before it reaches the run's two words.
+__device__ __forceinline__ void score_tile_rows(float* tile, int stride, int nb,
+                                                const LokiScoreSpec& sp, const ScoreK& SK,
+                                                float* __restrict__ scores, int kmax,
+                                                unsigned* __restrict__ minmax_keys) {
+  const int lane = threadIdx.x & 31;
+  unsigned lo = 0xFFFFFFFFu, hi = 0u;
   if (lane < kmax) {
     float* row = tile + lane * stride;
     float s;
     if (SK.pow2_64) score_row64_pow2(row, sp, SK, &s);
-    else score_row(row, nb, sp, &s);
-    scores[c0 + lane] = s;
-    if (s == s) {  // NaN scores do not enter min/max (like np.min on finite data)
-      atomicMin(minmax_keys, float_key(s));
-      atomicMax(minmax_keys + 1, float_key(s));
-    }
+    else score_row(row, nb, sp, SK, &s);
+    scores[lane] = s;
+    if (s == s) lo = hi = float_key(s);  // NaN scores do not enter min/max (like np.min)
   }
+  lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+  hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+  if (lane == 0 && lo != 0xFFFFFFFFu) {
+    atomicMin(minmax_keys, lo);
+    atomicMax(minmax_keys + 1, hi);
+  }
+}
+
+// Children c0 .. c0 + 31 (those below n_children) of one warp.
+__device__ __forceinline__ void score_tile(const LokiPruneLevel& D, const double* __restrict__ leaves,
+                   const float* __restrict__ folds, int64_t n_parents,
+                   const LokiBranchInfo* __restrict__ info, const int64_t* __restrict__ offsets,
+                   int64_t n_children, const float* __restrict__ seg, const LokiScoreSpec& sp,
+                   const ScoreK& SK, float* __restrict__ scores, int32_t* __restrict__ cidx,
+                   double* __restrict__ cphase, unsigned* __restrict__ minmax_keys,
+                   float* tile, int64_t c0) {
+  const int lane = threadIdx.x & 31;
+  const int nb = D.nbins, P = D.poly_order;
+  const int stride = score_stride(nb, sp.wmax);
+  const int kmax = (int)std::min<int64_t>(32, n_children - c0);
+  // lane k resolves child c0 + k
+  int64_t my_par = warp_find_parents(offsets, n_parents, c0 + lane, kmax), my_row = 0;
+  int my_shift = 0;
+  if (lane < kmax) {
+    const int64_t c = c0 + lane, par = my_par;
+    const LokiBranchInfo B = info[par];
+    const double* lf = leaves + par * (P + 2) * 2;
+    double pv[LOKI_MAX_PARAMS + 1];
+    child_params(B, P, c - offsets[par], pv);
+    pv[P] = B.d0;  // d_0 (alpha_0 in the current domain for Chebyshev)
+    const ChildRes r = resolve_child(D, pv, lf[(P + 1) * 2]);
+    cidx[2 * c] = r.ia;
+    cidx[2 * c + 1] = r.iff;
+    cphase[c] = r.phase;
+    my_row = (int64_t)r.ia * D.n_freq + r.iff;
+    my_shift = round_shift(r.phase, nb);
+  }
+  gather_norm_rows(folds, seg, my_par, my_row, my_shift, kmax, nb, tile, stride);
+  score_tile_rows(tile, stride, nb, sp, SK, scores + c0, kmax, minmax_keys);
 }
 
 __global__ void __launch_bounds__(kPruneWarps * 32)
@@ -803,6 +862,89 @@ select_overflow_kernel(const float* __restrict__ scores, const int64_t* __restri
 // emit: thread per survivor for the leaf, warp per 32 survivors for folds
 // ---------------------------------------------------------------------------
 
+// What the level-synchronous batch adds to an emission: the run's backtrack
+// history row of every survivor, and the level's best leaf.
+struct EmitExtra {
+  int32_t* bt_hist = nullptr;  // row of the level's first survivor
+  int64_t best = -1;           // survivor with the best score
+  double* best_leaf = nullptr;
+  float* best_score = nullptr;
+};
+
+__device__ __forceinline__ void emit_extra(const EmitExtra& X, int64_t s, const double* lo,
+                                           float sc, const int32_t* bt, int P) {
+  if (X.bt_hist) {
+    int32_t* h = X.bt_hist + s * (P + 2);
+    for (int j = 0; j < P + 2; ++j) h[j] = bt[j];
+  }
+  if (s == X.best) {
+    for (int j = 0; j < (P + 2) * 2; ++j) X.best_leaf[j] = lo[j];
+    *X.best_score = sc;
+  }
+}
+
+// Rows of 32 survivors (as gather_norm_rows): shift-added, written to fout.
+__device__ __forceinline__ void gather_add_rows(const float* __restrict__ folds,
+                                                const float* __restrict__ seg, int64_t my_par,
+                                                int64_t my_row, int my_shift, int kmax, int nb,
+                                                float* __restrict__ fout) {
+  const int lane = threadIdx.x & 31;
+  if (nb == 64) {
+    // four survivors' rows in flight per lane (bins lane and lane + 32)
+    constexpr int kU = 4;
+    for (int k0 = 0; k0 < kmax; k0 += kU) {
+      float pe[kU][2], pw[kU][2], se[kU][2], sw[kU][2];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const int k = k0 + u;
+        const int src = k < kmax ? k : 0;
+        const int64_t par = __shfl_sync(0xFFFFFFFFu, my_par, src);
+        const int64_t row = __shfl_sync(0xFFFFFFFFu, my_row, src);
+        const int sh = __shfl_sync(0xFFFFFFFFu, my_shift, src);
+        if (k < kmax) {
+          const float* pf = folds + par * 128;
+          const float* sf = seg + row * 128;
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const int j = lane + 32 * c;
+            const int js = (j - sh) & 63;
+            pe[u][c] = __ldg(pf + j);
+            pw[u][c] = __ldg(pf + 64 + j);
+            se[u][c] = __ldg(sf + js);
+            sw[u][c] = __ldg(sf + 64 + js);
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const int k = k0 + u;
+        if (k >= kmax) break;
+        float* o = fout + k * 128;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          o[lane + 32 * c] = __fadd_rn(pe[u][c], se[u][c]);
+          o[64 + lane + 32 * c] = __fadd_rn(pw[u][c], sw[u][c]);
+        }
+      }
+    }
+    return;
+  }
+  for (int k = 0; k < kmax; ++k) {
+    const int64_t par = __shfl_sync(0xFFFFFFFFu, my_par, k);
+    const int64_t row = __shfl_sync(0xFFFFFFFFu, my_row, k);
+    const int sh = __shfl_sync(0xFFFFFFFFu, my_shift, k);
+    const float* pf = folds + par * 2 * nb;
+    const float* sf = seg + row * 2 * nb;
+    float* o = fout + k * 2 * nb;
+    for (int j = lane; j < nb; j += 32) {
+      int js = j - sh;
+      js += (js < 0) ? nb : 0;
+      o[j] = __fadd_rn(pf[j], sf[js]);
+      o[nb + j] = __fadd_rn(pf[nb + j], sf[nb + js]);
+    }
+  }
+}
+
 // Survivors s0 .. s0 + 31 (those below n_surv) of one warp.
 __device__ __forceinline__ void emit_tile(const LokiPruneLevel& D, const double* __restrict__ leaves,
                   const float* __restrict__ folds, const LokiBranchInfo* __restrict__ info,
@@ -812,16 +954,15 @@ __device__ __forceinline__ void emit_tile(const LokiPruneLevel& D, const double*
                   const int32_t* __restrict__ cidx, const double* __restrict__ cphase,
                   double* __restrict__ lout, float* __restrict__ fout,
                   float* __restrict__ sout, float* __restrict__ seout,
-                  int32_t* __restrict__ bout, int64_t s0) {
+                  int32_t* __restrict__ bout, int64_t s0, const EmitExtra& X = EmitExtra()) {
   const int lane = threadIdx.x & 31;
   const int nb = D.nbins, P = D.poly_order, m = P + 1;
   const int kmax = (int)std::min<int64_t>(32, n_surv - s0);
-  int64_t my_par = 0, my_row = 0;
+  const int64_t my_c = surv[s0 + min(lane, kmax - 1)];
+  int64_t my_par = warp_find_parents(offsets, n_parents, my_c, kmax), my_row = 0;
   int my_shift = 0;
   if (lane < kmax) {
-    const int64_t s = s0 + lane;
-    const int64_t c = surv[s];
-    const int64_t par = find_parent(offsets, n_parents, c);
+    const int64_t s = s0 + lane, c = my_c, par = my_par;
     const LokiBranchInfo B = info[par];
     const double* lf = leaves + par * (P + 2) * 2;
     double pv[LOKI_MAX_PARAMS + 1], ev[LOKI_MAX_PARAMS + 1];
@@ -859,64 +1000,11 @@ __device__ __forceinline__ void emit_tile(const LokiPruneLevel& D, const double*
     bt[D.nparams_ffa - 1] = ia;  // column 1 + (nparams_ffa - 2)
     bt[D.nparams_ffa] = iff;     // column 1 + (nparams_ffa - 1)
     bt[P + 1] = (int32_t)cphase[c];
-    my_par = par;
+    emit_extra(X, s, lo, sc, bt, P);
     my_row = (int64_t)ia * D.n_freq + iff;
     my_shift = round_shift(cphase[c], nb);
   }
-  if (nb == 64) {
-    // four survivors' rows in flight per lane (bins lane and lane + 32)
-    constexpr int kU = 4;
-    for (int k0 = 0; k0 < kmax; k0 += kU) {
-      float pe[kU][2], pw[kU][2], se[kU][2], sw[kU][2];
-#pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const int k = k0 + u;
-        const int src = k < kmax ? k : 0;
-        const int64_t par = __shfl_sync(0xFFFFFFFFu, my_par, src);
-        const int64_t row = __shfl_sync(0xFFFFFFFFu, my_row, src);
-        const int sh = __shfl_sync(0xFFFFFFFFu, my_shift, src);
-        if (k < kmax) {
-          const float* pf = folds + par * 128;
-          const float* sf = seg + row * 128;
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            const int j = lane + 32 * c;
-            const int js = (j - sh) & 63;
-            pe[u][c] = __ldg(pf + j);
-            pw[u][c] = __ldg(pf + 64 + j);
-            se[u][c] = __ldg(sf + js);
-            sw[u][c] = __ldg(sf + 64 + js);
-          }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const int k = k0 + u;
-        if (k >= kmax) break;
-        float* o = fout + (s0 + k) * 128;
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          o[lane + 32 * c] = __fadd_rn(pe[u][c], se[u][c]);
-          o[64 + lane + 32 * c] = __fadd_rn(pw[u][c], sw[u][c]);
-        }
-      }
-    }
-    return;
-  }
-  for (int k = 0; k < kmax; ++k) {
-    const int64_t par = __shfl_sync(0xFFFFFFFFu, my_par, k);
-    const int64_t row = __shfl_sync(0xFFFFFFFFu, my_row, k);
-    const int sh = __shfl_sync(0xFFFFFFFFu, my_shift, k);
-    const float* pf = folds + par * 2 * nb;
-    const float* sf = seg + row * 2 * nb;
-    float* o = fout + (s0 + k) * 2 * nb;
-    for (int j = lane; j < nb; j += 32) {
-      int js = j - sh;
-      js += (js < 0) ? nb : 0;
-      o[j] = __fadd_rn(pf[j], sf[js]);
-      o[nb + j] = __fadd_rn(pf[nb + j], sf[nb + js]);
-    }
-  }
+  gather_add_rows(folds, seg, my_par, my_row, my_shift, kmax, nb, fout + s0 * 2 * nb);
 }
 
 __global__ void __launch_bounds__(kPruneWarps * 32)
@@ -1117,7 +1205,7 @@ __device__ __forceinline__ void ascend_tile(const LokiPruneLevel& D, const doubl
     float s;
     float* row = tile + lane * stride;
     if (SK.pow2_64) score_row64_pow2(row, sp, SK, &s);
-    else score_row(row, nb, sp, &s);
+    else score_row(row, nb, sp, SK, &s);
     scores[s0 + lane] = s;
   }
 }
@@ -1477,33 +1565,8 @@ __device__ __forceinline__ void circ_score_tile(const LokiPruneLevel& D, const d
     my_row = (int64_t)r.ia * D.n_freq + r.iff;
     my_shift = round_shift(r.phase, nb);
   }
-  for (int k = 0; k < kmax; ++k) {
-    const int64_t par = __shfl_sync(0xFFFFFFFFu, my_par, k);
-    const int64_t row = __shfl_sync(0xFFFFFFFFu, my_row, k);
-    const int sh = __shfl_sync(0xFFFFFFFFu, my_shift, k);
-    const float* pf = folds + par * 2 * nb;
-    const float* sf = seg + row * 2 * nb;
-    float* trow = tile + k * stride;
-    for (int j = lane; j < nb; j += 32) {
-      int js = j - sh;
-      js += (js < 0) ? nb : 0;
-      const float e = __fadd_rn(pf[j], sf[js]);
-      const float vv = __fadd_rn(pf[nb + j], sf[nb + js]);
-      trow[j] = __fdiv_rn(e, __fsqrt_rn(vv));
-    }
-  }
-  __syncwarp();
-  if (lane < kmax) {
-    float* row = tile + lane * stride;
-    float s;
-    if (SK.pow2_64) score_row64_pow2(row, sp, SK, &s);
-    else score_row(row, nb, sp, &s);
-    scores[v0 + lane] = s;
-    if (s == s) {
-      atomicMin(minmax_keys, float_key(s));
-      atomicMax(minmax_keys + 1, float_key(s));
-    }
-  }
+  gather_norm_rows(folds, seg, my_par, my_row, my_shift, kmax, nb, tile, stride);
+  score_tile_rows(tile, stride, nb, sp, SK, scores + v0, kmax, minmax_keys);
 }
 
 // With cnt (device counts) the valid children are pos_v[cnt[1]] (the
@@ -1556,7 +1619,8 @@ __device__ __forceinline__ void circ_emit_tile(const LokiPruneLevel& D, const do
                  const double* __restrict__ cphase, const int8_t* __restrict__ ccls,
                  const int32_t* __restrict__ batch_taylor, double* __restrict__ lout,
                  float* __restrict__ fout, float* __restrict__ sout,
-                 float* __restrict__ seout, int32_t* __restrict__ bout, int64_t s0) {
+                 float* __restrict__ seout, int32_t* __restrict__ bout, int64_t s0,
+                 const EmitExtra& X = EmitExtra()) {
   const int lane = threadIdx.x & 31;
   const int nb = D.nbins, P = 5, m = 6;
   const int kmax = (int)std::min<int64_t>(32, n_surv - s0);
@@ -1613,24 +1677,12 @@ __device__ __forceinline__ void circ_emit_tile(const LokiPruneLevel& D, const do
     bt[D.nparams_ffa - 1] = ia;
     bt[D.nparams_ffa] = iff;
     bt[P + 1] = (int32_t)cphase[v];
+    emit_extra(X, s, lo, sc, bt, P);
     my_par = ch.parent;
     my_row = (int64_t)ia * D.n_freq + iff;
     my_shift = round_shift(cphase[v], nb);
   }
-  for (int k = 0; k < kmax; ++k) {
-    const int64_t par = __shfl_sync(0xFFFFFFFFu, my_par, k);
-    const int64_t row = __shfl_sync(0xFFFFFFFFu, my_row, k);
-    const int sh = __shfl_sync(0xFFFFFFFFu, my_shift, k);
-    const float* pf = folds + par * 2 * nb;
-    const float* sf = seg + row * 2 * nb;
-    float* o = fout + (s0 + k) * 2 * nb;
-    for (int j = lane; j < nb; j += 32) {
-      int js = j - sh;
-      js += (js < 0) ? nb : 0;
-      o[j] = __fadd_rn(pf[j], sf[js]);
-      o[nb + j] = __fadd_rn(pf[nb + j], sf[nb + js]);
-    }
-  }
+  gather_add_rows(folds, seg, my_par, my_row, my_shift, kmax, nb, fout + s0 * 2 * nb);
 }
 
 __global__ void __launch_bounds__(kPruneWarps * 32)
@@ -1745,7 +1797,7 @@ __host__ __device__ inline size_t cplx_warp_floats(int nbins, int stride) {
 __device__ __forceinline__ void score_child_complex(
     const LokiPruneLevel& D, const double* __restrict__ leaves, const float2* __restrict__ folds,
     int64_t n_parents, const LokiBranchInfo* __restrict__ info,
-    const int64_t* __restrict__ offsets, const float2* __restrict__ seg, const LokiScoreSpec& sp,
+    const int64_t* __restrict__ offsets, const float2* __restrict__ seg, const LokiScoreSpec& sp, const ScoreK& SK,
     float* __restrict__ scores, int32_t* __restrict__ cidx, double* __restrict__ cphase,
     unsigned* __restrict__ minmax_keys, const float* tw, float2* comb, float* trow, int64_t c) {
   const int nb = D.nbins, nbf = nb / 2 + 1, P = D.poly_order;
@@ -1763,7 +1815,7 @@ __device__ __forceinline__ void score_child_complex(
   rotate_add(seg + row * 2 * nbf, folds + par * 2 * nbf, prune_phasor(r.phase, nb), nbf, comb);
   irfft_norm(comb, nb, nbf, tw, trow);
   float s;
-  score_row(trow, nb, sp, &s);
+  score_row(trow, nb, sp, SK, &s);
   scores[c] = s;
   if (s == s) {
     atomicMin(minmax_keys, float_key(s));
@@ -1791,25 +1843,30 @@ prune_score_complex_kernel(LokiPruneLevel D, const double* __restrict__ leaves,
   float* tile = wbase + (size_t)32 * 2 * nbf * 2;
   const int64_t c = ((int64_t)blockIdx.x * kPruneWarps + warp) * 32 + lane;
   if (c >= n_children) return;
-  score_child_complex(D, leaves, folds, n_parents, info, offsets, seg, sp, scores, cidx, cphase,
+  score_child_complex(D, leaves, folds, n_parents, info, offsets, seg, sp, SK, scores, cidx, cphase,
                       minmax_keys, tw, comb, tile + lane * stride, c);
 }
 
 // Survivors of the complex tree: transform / backtrack exactly as
 // prune_emit_kernel, the fold written as the complex sum.
-// One survivor of the complex tree: transform, backtrack and the complex
-// sum of its fold.
-__device__ __forceinline__ void emit_one_complex(
-    const LokiPruneLevel& D, const double* __restrict__ leaves, const float2* __restrict__ folds,
+// The rows one survivor's fold is made of.
+struct EmitRow {
+  int64_t par, row;
+  double phase;
+};
+
+// One survivor of the complex tree: transform and backtrack, its fold's rows
+// returned.
+
+__device__ __forceinline__ EmitRow emit_one_complex_leaf(
+    const LokiPruneLevel& D, const double* __restrict__ leaves,
     const LokiBranchInfo* __restrict__ info, const int64_t* __restrict__ offsets,
-    int64_t n_parents, const float2* __restrict__ seg, const int64_t* __restrict__ surv,
-    const float* __restrict__ cscores, const int32_t* __restrict__ cidx,
-    const double* __restrict__ cphase, double* __restrict__ lout, float2* __restrict__ fout,
-    float* __restrict__ sout, float* __restrict__ seout, int32_t* __restrict__ bout,
-    int64_t s) {
-  const int nb = D.nbins, nbf = nb / 2 + 1, P = D.poly_order, m = P + 1;
+    const int64_t* __restrict__ surv, const float* __restrict__ cscores,
+    const int32_t* __restrict__ cidx, const double* __restrict__ cphase,
+    double* __restrict__ lout, float* __restrict__ sout, float* __restrict__ seout,
+    int32_t* __restrict__ bout, int64_t s, int64_t par, const EmitExtra& X = EmitExtra()) {
+  const int P = D.poly_order, m = P + 1;
   const int64_t c = surv[s];
-  const int64_t par = find_parent(offsets, n_parents, c);
   const LokiBranchInfo B = info[par];
   const double* lf = leaves + par * (P + 2) * 2;
   double pv[LOKI_MAX_PARAMS + 1], ev[LOKI_MAX_PARAMS + 1];
@@ -1846,8 +1903,23 @@ __device__ __forceinline__ void emit_one_complex(
   bt[D.nparams_ffa - 1] = ia;
   bt[D.nparams_ffa] = iff;
   bt[P + 1] = (int32_t)cphase[c];
-  const int64_t row = (int64_t)ia * D.n_freq + iff;
-  rotate_add(seg + row * 2 * nbf, folds + par * 2 * nbf, prune_phasor(cphase[c], nb), nbf,
+  emit_extra(X, s, lo, cscores[c], bt, P);
+  return {par, (int64_t)ia * D.n_freq + iff, cphase[c]};
+}
+
+__device__ __forceinline__ void emit_one_complex(
+    const LokiPruneLevel& D, const double* __restrict__ leaves, const float2* __restrict__ folds,
+    const LokiBranchInfo* __restrict__ info, const int64_t* __restrict__ offsets,
+    int64_t n_parents, const float2* __restrict__ seg, const int64_t* __restrict__ surv,
+    const float* __restrict__ cscores, const int32_t* __restrict__ cidx,
+    const double* __restrict__ cphase, double* __restrict__ lout, float2* __restrict__ fout,
+    float* __restrict__ sout, float* __restrict__ seout, int32_t* __restrict__ bout,
+    int64_t s) {
+  const int nb = D.nbins, nbf = nb / 2 + 1;
+  const EmitRow r = emit_one_complex_leaf(D, leaves, info, offsets, surv, cscores, cidx, cphase,
+                                          lout, sout, seout, bout, s,
+                                          find_parent(offsets, n_parents, surv[s]));
+  rotate_add(seg + r.row * 2 * nbf, folds + r.par * 2 * nbf, prune_phasor(r.phase, nb), nbf,
              fout + s * 2 * nbf);
 }
 
@@ -1877,7 +1949,7 @@ __device__ __forceinline__ void ascend_one_complex(
     float* __restrict__ scores, float* __restrict__ scores_ep, int nseg,
     const double* __restrict__ tm_seg, const double* __restrict__ dt_seg,
     const int32_t* __restrict__ seg_idx, const float2* __restrict__ ffa, int64_t seg_stride,
-    const LokiScoreSpec& sp, const float* tw, float2* comb, float* trow, int64_t r) {
+    const LokiScoreSpec& sp, const ScoreK& SK, const float* tw, float2* comb, float* trow, int64_t r) {
   const int nb = D.nbins, nbf = nb / 2 + 1, P = D.poly_order, m = P + 1;
   const double* lf = leaves + r * (P + 2) * 2;
   double pv[LOKI_MAX_PARAMS + 1], ev[LOKI_MAX_PARAMS + 1];
@@ -1930,7 +2002,7 @@ __device__ __forceinline__ void ascend_one_complex(
   irfft_norm(comb, nb, nbf, tw, trow);
   scores_ep[r] = scores[r];
   float s;
-  score_row(trow, nb, sp, &s);
+  score_row(trow, nb, sp, SK, &s);
   scores[r] = s;
 }
 
@@ -1956,7 +2028,7 @@ prune_ascend_complex_kernel(LokiPruneLevel D, const double* __restrict__ leaves,
   const int64_t r = ((int64_t)blockIdx.x * kPruneWarps + warp) * 32 + lane;
   if (r >= n) return;
   ascend_one_complex(D, leaves, folds, scores, scores_ep, nseg, tm_seg, dt_seg, seg_idx, ffa,
-                     seg_stride, sp, tw, comb, tile + lane * stride, r);
+                     seg_stride, sp, SK, tw, comb, tile + lane * stride, r);
 }
 
 // ---------------------------------------------------------------------------
@@ -1973,7 +2045,7 @@ __device__ __forceinline__ void circ_score_one_complex(
     const LokiPruneLevel& D, const double* __restrict__ leaves, const float2* __restrict__ folds,
     int64_t batch, const LokiBranchInfo* __restrict__ info, const CircChild* __restrict__ map,
     const int64_t* __restrict__ valid_ids, const float2* __restrict__ seg,
-    const LokiScoreSpec& sp, const float* tw, float2* comb, float* trow,
+    const LokiScoreSpec& sp, const ScoreK& SK, const float* tw, float2* comb, float* trow,
     float* __restrict__ scores, int32_t* __restrict__ cidx, double* __restrict__ cphase,
     int8_t* __restrict__ ccls, int32_t* __restrict__ batch_taylor,
     unsigned* __restrict__ minmax_keys, int64_t v) {
@@ -1995,7 +2067,7 @@ __device__ __forceinline__ void circ_score_one_complex(
              prune_phasor(r.phase, nb), nbf, comb);
   irfft_norm(comb, nb, nbf, tw, trow);
   float s;
-  score_row(trow, nb, sp, &s);
+  score_row(trow, nb, sp, SK, &s);
   scores[v] = s;
   if (s == s) {
     atomicMin(minmax_keys, float_key(s));
@@ -2026,23 +2098,24 @@ circ_score_complex_kernel(LokiPruneLevel D, const double* __restrict__ leaves,
   float* tile = wbase + (size_t)32 * 2 * nbf * 2;
   const int64_t v = ((int64_t)blockIdx.x * kPruneWarps + warp) * 32 + lane;
   if (v >= n_valid) return;
-  circ_score_one_complex(D, leaves, folds, batch, info, map, valid_ids, seg, sp, tw, comb,
+  circ_score_one_complex(D, leaves, folds, batch, info, map, valid_ids, seg, sp, SK, tw, comb,
                          tile + lane * stride, scores, cidx, cphase, ccls, batch_taylor,
                          minmax_keys, v);
 }
 
 // Survivor s of the complex circular tree (circ_emit_one's leaves, basis
 // flag and backtracks; the fold written as the complex sum).
-__device__ __forceinline__ void circ_emit_one_complex(
-    const LokiPruneLevel& D, const double* __restrict__ leaves, const float2* __restrict__ folds,
-    int64_t batch, const LokiBranchInfo* __restrict__ info, const CircChild* __restrict__ map,
-    const int64_t* __restrict__ valid_ids, const float2* __restrict__ seg,
-    const int64_t* __restrict__ surv, const float* __restrict__ cscores,
+__device__ __forceinline__ EmitRow circ_emit_one_complex_leaf(
+    const LokiPruneLevel& D, const double* __restrict__ leaves, int64_t batch,
+    const LokiBranchInfo* __restrict__ info, const CircChild* __restrict__ map,
+    const int64_t* __restrict__ valid_ids, const int64_t* __restrict__ surv,
+    const float* __restrict__ cscores,
     const int32_t* __restrict__ cidx, const double* __restrict__ cphase,
     const int8_t* __restrict__ ccls, const int32_t* __restrict__ batch_taylor,
-    double* __restrict__ lout, float2* __restrict__ fout, float* __restrict__ sout,
-    float* __restrict__ seout, int32_t* __restrict__ bout, int64_t s) {
-  const int nb = D.nbins, nbf = nb / 2 + 1, P = 5, m = 6;
+    double* __restrict__ lout, float* __restrict__ sout,
+    float* __restrict__ seout, int32_t* __restrict__ bout, int64_t s,
+    const EmitExtra& X = EmitExtra()) {
+  const int P = 5, m = 6;
   const int64_t v = surv[s];
   const CircChild ch = map[valid_ids[v]];
   const LokiBranchInfo B = info[ch.parent];
@@ -2091,9 +2164,25 @@ __device__ __forceinline__ void circ_emit_one_complex(
   bt[D.nparams_ffa - 1] = ia;
   bt[D.nparams_ffa] = iff;
   bt[P + 1] = (int32_t)cphase[v];
-  const int64_t row = (int64_t)ia * D.n_freq + iff;
-  rotate_add(seg + row * 2 * nbf, folds + (int64_t)ch.parent * 2 * nbf,
-             prune_phasor(cphase[v], nb), nbf, fout + s * 2 * nbf);
+  emit_extra(X, s, lo, cscores[v], bt, P);
+  return {(int64_t)ch.parent, (int64_t)ia * D.n_freq + iff, cphase[v]};
+}
+
+__device__ __forceinline__ void circ_emit_one_complex(
+    const LokiPruneLevel& D, const double* __restrict__ leaves, const float2* __restrict__ folds,
+    int64_t batch, const LokiBranchInfo* __restrict__ info, const CircChild* __restrict__ map,
+    const int64_t* __restrict__ valid_ids, const float2* __restrict__ seg,
+    const int64_t* __restrict__ surv, const float* __restrict__ cscores,
+    const int32_t* __restrict__ cidx, const double* __restrict__ cphase,
+    const int8_t* __restrict__ ccls, const int32_t* __restrict__ batch_taylor,
+    double* __restrict__ lout, float2* __restrict__ fout, float* __restrict__ sout,
+    float* __restrict__ seout, int32_t* __restrict__ bout, int64_t s) {
+  const int nb = D.nbins, nbf = nb / 2 + 1;
+  const EmitRow r = circ_emit_one_complex_leaf(D, leaves, batch, info, map, valid_ids, surv,
+                                               cscores, cidx, cphase, ccls, batch_taylor, lout,
+                                               sout, seout, bout, s);
+  rotate_add(seg + r.row * 2 * nbf, folds + r.par * 2 * nbf, prune_phasor(r.phase, nb), nbf,
+             fout + s * 2 * nbf);
 }
 
 // Survivors of the complex circular tree: leaves, basis flag and backtracks as
@@ -2119,6 +2208,154 @@ circ_emit_complex_kernel(LokiPruneLevel D, const double* __restrict__ leaves,
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
+
+// ---------------------------------------------------------------------------
+// Complex rows of 32 children at a time, 64 bins. The warp stages one component
+// of its children's parent and segment rows in shared memory (whole rows, lane
+// by harmonic), then each lane combines and transforms its own child with the
+// arithmetic of rotate_add and irfft_norm: the phasor recurrence, and every bin
+// summed over the harmonics in order with each product and sum rounded. The
+// angles of bins j, 64 - j, 32 - j and 32 + j have the same cosine and sine up
+// to sign, so their four sums share two products, and the 64 sums are
+// independent registers. A lane walking its rows in global memory and the bins
+// one after the other took 56 ms for the 7.7e6 children of a 16-run search.
+// ---------------------------------------------------------------------------
+
+constexpr int kCplxRow = 33;  // float2 of one component; odd, so lanes miss each other's banks
+__host__ __device__ constexpr int cplx64_warp_bytes() { return 2 * 32 * kCplxRow * 8; }
+
+// One component of the rows of children k < kmax: par rows to A, seg rows to B.
+__device__ __forceinline__ void stage_rows64(const float2* __restrict__ folds,
+                                             const float2* __restrict__ seg, int64_t my_par,
+                                             int64_t my_row, int kmax, int comp, float2* A,
+                                             float2* B) {
+  const int lane = threadIdx.x & 31;
+  constexpr int kU = 8;
+  for (int k0 = 0; k0 < kmax; k0 += kU) {
+    float2 a[kU], b[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int k = k0 + u, src = k < kmax ? k : 0;
+      const int64_t par = __shfl_sync(0xFFFFFFFFu, my_par, src);
+      const int64_t row = __shfl_sync(0xFFFFFFFFu, my_row, src);
+      if (k < kmax) {
+        a[u] = __ldg(folds + par * 66 + comp * 33 + lane);
+        b[u] = __ldg(seg + row * 66 + comp * 33 + lane);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u)
+      if (k0 + u < kmax) {
+        A[(k0 + u) * kCplxRow + lane] = a[u];
+        B[(k0 + u) * kCplxRow + lane] = b[u];
+      }
+  }
+  if (lane < kmax) {
+    A[lane * kCplxRow + 32] = __ldg(folds + my_par * 66 + comp * 33 + 32);
+    B[lane * kCplxRow + 32] = __ldg(seg + my_row * 66 + comp * 33 + 32);
+  }
+  __syncwarp();
+}
+
+// rotate_add of one component in place: a = b phasor^k + a.
+__device__ __forceinline__ void combine64(float2* a, const float2* b, float2 delta) {
+  float2 ph = make_float2(1.0f, 0.0f);
+#pragma unroll 3
+  for (int k = 0; k < 33; ++k) {
+    const float2 r = cmul_rn(b[k], ph), p = a[k];
+    a[k] = make_float2(__fadd_rn(r.x, p.x), __fadd_rn(r.y, p.y));
+    ph = cmul_rn(ph, delta);
+  }
+}
+
+// irfft_norm's sums of one component (unscaled); tw = (cos, sin) of 2 pi t / 64.
+__device__ __forceinline__ void irfft64_sums(const float2* __restrict__ X,
+                                             const float2* __restrict__ tw, float (&acc)[64]) {
+  const float x0 = X[0].x, nyq = X[32].x;
+#pragma unroll
+  for (int j = 0; j < 64; ++j) acc[j] = (j & 1) ? __fsub_rn(x0, nyq) : __fadd_rn(x0, nyq);
+#pragma unroll 1
+  for (int m = 1; m < 32; ++m) {
+    const float2 x = X[m];
+    const bool odd = m & 1;
+    const float sg = odd ? -2.0f : 2.0f;
+    // bins 0, 32 and 16, 48: angles that are multiples of a quarter turn
+    acc[0] = __fmaf_rn(2.0f, x.x, acc[0]);
+    acc[32] = __fmaf_rn(sg, x.x, acc[32]);
+    const float v = (m & 2) ? -2.0f : 2.0f;
+    acc[16] = __fmaf_rn(odd ? -v : v, odd ? x.y : x.x, acc[16]);
+    acc[48] = __fmaf_rn(v, odd ? x.y : x.x, acc[48]);
+    int t = 0;
+#pragma unroll
+    for (int j = 1; j < 16; ++j) {
+      t = (t + m) & 63;
+      const float2 w = tw[t];
+      const float a = __fmul_rn(x.x, w.x), b = __fmul_rn(x.y, w.y);
+      const float u = __fsub_rn(a, b), z = __fadd_rn(a, b);
+      // doubling is exact: 2 t + acc rounds once, as the sum of the doubled term
+      acc[j] = __fmaf_rn(2.0f, u, acc[j]);
+      acc[64 - j] = __fmaf_rn(2.0f, z, acc[64 - j]);
+      acc[32 - j] = __fmaf_rn(sg, z, acc[32 - j]);
+      acc[32 + j] = __fmaf_rn(sg, u, acc[32 + j]);
+    }
+  }
+}
+
+__device__ __forceinline__ void load_twiddles64(float2* tw) {
+  for (int t = threadIdx.x; t < 64; t += blockDim.x) {
+    double s, c;
+    sincospi(2.0 * (double)t / 64.0, &s, &c);
+    tw[t] = make_float2((float)c, (float)s);
+  }
+}
+
+// Scores of the warp's children (rows and phasor held lane by lane).
+__device__ __forceinline__ void cplx64_score(const float2* __restrict__ folds,
+                                             const float2* __restrict__ seg, int64_t my_par,
+                                             int64_t my_row, float2 delta, int kmax,
+                                             const float2* tw, float2* buf,
+                                             const LokiScoreSpec& sp, const ScoreK& SK,
+                                             float* __restrict__ scores,
+                                             unsigned* __restrict__ minmax_keys) {
+  const int lane = threadIdx.x & 31;
+  float2 *A = buf, *B = buf + 32 * kCplxRow;
+  const float inv = 1.0f / 64.0f;
+  float e[64], v[64];
+  stage_rows64(folds, seg, my_par, my_row, kmax, 0, A, B);
+  combine64(A + lane * kCplxRow, B + lane * kCplxRow, delta);
+  irfft64_sums(A + lane * kCplxRow, tw, e);
+  __syncwarp();
+  stage_rows64(folds, seg, my_par, my_row, kmax, 1, A, B);
+  combine64(A + lane * kCplxRow, B + lane * kCplxRow, delta);
+  irfft64_sums(A + lane * kCplxRow, tw, v);
+  __syncwarp();  // every lane has read its rows: the buffer becomes the score tile
+  const int stride = score_stride(64, sp.wmax);
+  float* tile = reinterpret_cast<float*>(buf);
+#pragma unroll
+  for (int j = 0; j < 64; ++j)
+    tile[lane * stride + j] = __fdiv_rn(__fmul_rn(e[j], inv), __fsqrt_rn(__fmul_rn(v[j], inv)));
+  __syncwarp();
+  score_tile_rows(tile, stride, 64, sp, SK, scores, kmax, minmax_keys);
+}
+
+// Complex sums of the warp's survivors, whole rows to fout.
+__device__ __forceinline__ void cplx64_emit(const float2* __restrict__ folds,
+                                            const float2* __restrict__ seg, int64_t my_par,
+                                            int64_t my_row, float2 delta, int kmax, float2* buf,
+                                            float2* __restrict__ fout) {
+  const int lane = threadIdx.x & 31;
+  float2 *A = buf, *B = buf + 32 * kCplxRow;
+  for (int comp = 0; comp < 2; ++comp) {
+    stage_rows64(folds, seg, my_par, my_row, kmax, comp, A, B);
+    if (lane < kmax) combine64(A + lane * kCplxRow, B + lane * kCplxRow, delta);
+    __syncwarp();
+    for (int k = 0; k < kmax; ++k) {
+      fout[k * 66 + comp * 33 + lane] = A[k * kCplxRow + lane];
+      if (lane == 0) fout[k * 66 + comp * 33 + 32] = A[k * kCplxRow + 32];
+    }
+    __syncwarp();
+  }
+}
 
 static int check_prune(const LokiPruneLevel* D) {
   if (!D) return set_error(LOKI_ERR_INVALID, "null prune level descriptor");
@@ -3314,10 +3551,11 @@ struct BatchTabs {
   int32_t nlevels;
 };
 
-__device__ __forceinline__ int64_t* job_pos(const LokiPruneWork& w) {
-  const int64_t sums = (int64_t)max((int64_t)1, (w.child_cap + kScanBlock - 1) / kScanBlock) * 8;
-  return reinterpret_cast<int64_t*>(reinterpret_cast<char*>(w.sscan) + sums);
-}
+// counts[] of a job between the kernels of a level: parents, children (0 when
+// they exceed the workspace), survivors, backtrack rows of the levels before,
+// valid children (circular tree), and for the emission the parents, the first
+// backtrack row and the best survivor of the level.
+enum { kCntPar, kCntChild, kCntSurv, kCntBt, kCntValid, kCntOldPar, kCntBtRow, kCntBest };
 
 __global__ void bj_seed_kernel(BatchTabs T) {
   const LokiPruneJob& J = T.jobs[blockIdx.x];
@@ -3330,459 +3568,635 @@ __global__ void bj_seed_kernel(BatchTabs T) {
   *J.run.ovf_flag = 0;
 }
 
-__global__ void bj_branch_kernel(BatchTabs T, int l) {
-  const LokiPruneJob& J = T.jobs[blockIdx.y];
-  const LokiPruneLevel& D = T.levels[(size_t)blockIdx.y * T.nlevels + (l - 1)];
-  const LokiPruneWork& w = J.run.work;
-  const int64_t n = J.run.counts[0];
-  const double* leaves = J.run.trees[(l - 1) & 1].leaves;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    branch_one(D, leaves, i, reinterpret_cast<LokiBranchInfo*>(w.info), w.offsets, J.dev_err,
-               nullptr);
-}
+// ---- work of a level's wide kernels -------------------------------------------
+//
+// A wide kernel (branch, map, score, emit) runs one block per resident slot of
+// the GPU over the tiles of up to kQueueJobs jobs: every block sums the jobs'
+// tile counts (from one of their counters) and takes an equal run of
+// consecutive tiles, so most blocks see one job. A job's level descriptor
+// (2.3 KB of matrices and limits, read by every step of the resolve) is copied
+// to shared memory when the block turns to it. With a grid of blocks per job
+// instead, sized for the largest job, most blocks only read their job's
+// counters and left (60 us a level for 64 jobs in branch alone), and the
+// descriptor's lines were fetched one dependent load after another.
+constexpr int kQueueJobs = 256;
+constexpr int kTile = kPruneWarps * 32;  // parents, children or survivors a tile
 
-// The scans of a level, per job. Counts (in place, scratch w.scan): mode 0
-// the parents' child counts (offsets), mode 2 the circular tree's crackle
-// expansion counts (exp_off), both over counts[0] parents. Flags (into the
-// positions after w.sscan's sums): mode 1 score >= threshold over counts[1]
-// children, mode 3 the circular tree's validity flags over counts[1]
-// children, mode 4 score >= threshold over counts[4] valid children.
-__device__ __forceinline__ void bj_scan_args(const BatchTabs& T, int l, int mode,
-                                             const void** in, int64_t** out, int64_t** sums,
-                                             int64_t* n, double* thr) {
-  const LokiPruneJob& J = T.jobs[blockIdx.y];
-  const LokiPruneWork& w = J.run.work;
-  if (mode == 0 || mode == 2) {
-    int64_t* a = mode == 0 ? w.offsets : J.run.exp_off;
-    *in = a;
-    *out = a;
-    *sums = reinterpret_cast<int64_t*>(w.scan);
-    *n = J.run.counts[0];
-    *thr = 0.0;
-  } else {
-    *in = mode == 3 ? static_cast<const void*>(J.run.valid_flags)
-                    : static_cast<const void*>(w.child_scores);
-    *out = job_pos(w);
-    *sums = reinterpret_cast<int64_t*>(w.sscan);
-    *n = J.run.counts[mode == 4 ? 4 : 1];
-    *thr = mode == 3 ? 0.5 : T.thr[(size_t)blockIdx.y * T.nlevels + (l - 1)];
-  }
-}
+struct JobQueue {
+  alignas(16) LokiPruneLevel lvl;
+  int pre[kQueueJobs + 1];  // tiles before each job
+};
 
-template <bool FLAGS>
-__global__ void __launch_bounds__(kScanBlock) bj_scan_block_kernel(BatchTabs T, int l, int mode) {
-  __shared__ int64_t warp_tot[32];
-  const void* in;
-  int64_t *out, *sums, n;
-  double thr;
-  bj_scan_args(T, l, mode, &in, &out, &sums, &n, &thr);
-  const int64_t ntiles = (n + kScanBlock - 1) / kScanBlock;
-  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x)
-    scan_tile<FLAGS>(in, n, thr, out, sums, t, warp_tot);
-}
-
-template <bool FLAGS>
-__global__ void __launch_bounds__(kScanBlock) bj_scan_sums_kernel(BatchTabs T, int l, int mode) {
-  __shared__ int64_t warp_tot[32];
-  __shared__ int64_t carry;
-  const void* in;
-  int64_t *out, *sums, n;
-  double thr;
-  bj_scan_args(T, l, mode, &in, &out, &sums, &n, &thr);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t nblocks = (n + kScanBlock - 1) / kScanBlock;
-  if (threadIdx.x == 0) carry = 0;
+// Tiles [t0, t1) of this block over jobs j0 .. j0 + nj, counts[idx] items each.
+__device__ __forceinline__ void queue_open(JobQueue& Q, const BatchTabs& T, int j0, int nj,
+                                           int idx, int* t0, int* t1) {
+  const int lane = threadIdx.x & 31;
+  for (int t = threadIdx.x; t < nj; t += blockDim.x)
+    Q.pre[t + 1] = (int)((T.jobs[j0 + t].run.counts[idx] + kTile - 1) / kTile);
+  if (threadIdx.x == 0) Q.pre[0] = 0;
   __syncthreads();
-  for (int64_t base = 0; base < nblocks; base += kScanBlock) {
-    const int64_t i = base + threadIdx.x;
-    const int64_t x = i < nblocks ? sums[i] : 0;
-    int64_t v = x;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int64_t y = __shfl_up_sync(0xFFFFFFFFu, v, o);
-      if (lane >= o) v += y;
-    }
-    if (lane == 31) warp_tot[warp] = v;
-    __syncthreads();
-    if (warp == 0) {
-      int64_t w = warp_tot[lane];
+  if (threadIdx.x < 32) {
+    int carry = 0;
+    for (int base = 0; base < nj; base += 32) {
+      int v = base + lane < nj ? Q.pre[base + lane + 1] : 0;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const int64_t y = __shfl_up_sync(0xFFFFFFFFu, w, o);
-        if (lane >= o) w += y;
+        const int y = __shfl_up_sync(0xFFFFFFFFu, v, o);
+        if (lane >= o) v += y;
       }
-      warp_tot[lane] = w;
+      if (base + lane < nj) Q.pre[base + lane + 1] = v + carry;
+      carry += __shfl_sync(0xFFFFFFFFu, v, 31);
     }
-    __syncthreads();
-    const int64_t incl = v + (warp ? warp_tot[warp - 1] : 0);
-    const int64_t c = carry;
-    if (i < nblocks) sums[i] = c + incl - x;
-    __syncthreads();
-    if (threadIdx.x == kScanBlock - 1) carry = c + incl;
-    __syncthreads();
   }
-  if (threadIdx.x == 0) out[n] = carry;
-}
-
-template <bool FLAGS>
-__global__ void __launch_bounds__(kScanBlock) bj_scan_add_kernel(BatchTabs T, int l, int mode) {
-  const void* in;
-  int64_t *out, *sums, n;
-  double thr;
-  bj_scan_args(T, l, mode, &in, &out, &sums, &n, &thr);
-  for (int64_t i = (int64_t)blockIdx.x * kScanBlock + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * kScanBlock)
-    out[i] += sums[i / kScanBlock];
-}
-
-__global__ void __launch_bounds__(kPruneWarps * 32, 4)
-bj_score_kernel(BatchTabs T, int l, LokiScoreSpec sp, ScoreK SK) {
-  extern __shared__ float tiles[];
-  const LokiPruneJob& J = T.jobs[blockIdx.y];
-  const size_t li = (size_t)blockIdx.y * T.nlevels + (l - 1);
-  const LokiPruneLevel& D = T.levels[li];
-  const LokiPruneRun& R = J.run;
-  const LokiPruneWork& w = R.work;
-  const LokiPruneTree& in = R.trees[(l - 1) & 1];
-  const float* seg = J.ffa_fold + (int64_t)T.seg_idx[li] * J.seg_stride;
-  const int warp = threadIdx.x >> 5;
-  float* tile = tiles + (size_t)warp * 32 * score_stride(D.nbins, sp.wmax);
-  int64_t* cnt = R.counts;
-  const int64_t n_par = cnt[0];
-  const int64_t total = w.offsets[n_par];
-  const int64_t n_child = total > w.child_cap ? 0 : total;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    cnt[1] = n_child;
-    LokiPruneLevelStats* st = R.stats + (l - 1);
-    st->n_parents = n_par;
-    st->n_children = total;
-    st->n_valid = total;
-    if (total > w.child_cap) atomicOr(J.dev_err, LOKI_DEVERR_CAPACITY);
-  }
-  for (int64_t t = (int64_t)blockIdx.x * kPruneWarps + warp; t * 32 < n_child;
-       t += (int64_t)gridDim.x * kPruneWarps) {
-    score_tile(D, in.leaves, in.folds, n_par, reinterpret_cast<LokiBranchInfo*>(w.info),
-               w.offsets, n_child, seg, sp, SK, w.child_scores, w.child_idx, w.child_phase,
-               reinterpret_cast<unsigned*>(w.minmax), tile, t * 32);
-    __syncwarp();
-  }
-}
-
-// mode 1: survivors among counts[1] children; mode 3: the circular tree's
-// valid children (valid_ids) among counts[1]; mode 4: survivors among
-// counts[4] valid children.
-__global__ void bj_scatter_kernel(BatchTabs T, int l, int mode) {
-  const LokiPruneJob& J = T.jobs[blockIdx.y];
-  const LokiPruneWork& w = J.run.work;
-  const double thr = mode == 3 ? 0.5 : T.thr[(size_t)blockIdx.y * T.nlevels + (l - 1)];
-  const float* f = mode == 3 ? J.run.valid_flags : w.child_scores;
-  int64_t* ids = mode == 3 ? J.run.valid_ids : w.surv;
-  const int64_t n = J.run.counts[mode == 4 ? 4 : 1];
-  const int64_t* pos = job_pos(w);
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    if ((double)f[i] >= thr) ids[pos[i]] = i;
-}
-
-// one block per job: the survivor count, and the overflow rule when it
-// exceeds max_sugg
-__global__ void __launch_bounds__(kSelThreads)
-bj_overflow_kernel(BatchTabs T, int l, int64_t max_sugg, int64_t batch, int circ) {
-  const LokiPruneJob& J = T.jobs[blockIdx.x];
-  const LokiPruneRun& R = J.run;
-  const LokiPruneWork& w = R.work;
-  int64_t* cnt = R.counts;
-  const int64_t n_sel = job_pos(w)[cnt[circ ? 4 : 1]];
-  const int64_t n_par = cnt[0];
-  __syncthreads();  // every thread has read the counters
-  if (threadIdx.x == 0) cnt[2] = n_sel;
-  if (n_sel <= max_sugg) return;  // uniform over the block
-  if (threadIdx.x == 0) *R.ovf_flag = 1;
-  // the circular tree's batches are over its valid children
-  select_overflow_block(w.child_scores, circ ? R.batch_offsets : w.offsets, n_par, batch,
-                        T.thr[(size_t)blockIdx.x * T.nlevels + (l - 1)], max_sugg, w.surv,
-                        cnt + 2, w.ovf_thr, w.ovf_ids, reinterpret_cast<unsigned*>(w.ovf_keys));
-}
-
-__global__ void __launch_bounds__(kPruneWarps * 32) bj_emit_kernel(BatchTabs T, int l) {
-  const LokiPruneJob& J = T.jobs[blockIdx.y];
-  const size_t li = (size_t)blockIdx.y * T.nlevels + (l - 1);
-  const LokiPruneLevel& D = T.levels[li];
-  const LokiPruneRun& R = J.run;
-  const LokiPruneWork& w = R.work;
-  const LokiPruneTree& in = R.trees[(l - 1) & 1];
-  const LokiPruneTree& out = R.trees[l & 1];
-  const float* seg = J.ffa_fold + (int64_t)T.seg_idx[li] * J.seg_stride;
-  const int warp = threadIdx.x >> 5;
-  const int64_t n_par = R.counts[0], n_surv = R.counts[2];
-  for (int64_t t = (int64_t)blockIdx.x * kPruneWarps + warp; t * 32 < n_surv;
-       t += (int64_t)gridDim.x * kPruneWarps)
-    emit_tile(D, in.leaves, in.folds, reinterpret_cast<LokiBranchInfo*>(w.info), w.offsets,
-              n_par, seg, w.surv, n_surv, w.child_scores, w.child_idx, w.child_phase,
-              out.leaves, out.folds, out.scores, out.scores_ep, out.backtracks, t * 32);
-}
-
-// complex (Fourier-domain) trees: the per-child functions of the complex
-// level kernels, grid-stride over each job's device counts. The jobs' fold
-// rows and segment strides are in complex (float2) units.
-__global__ void __launch_bounds__(kPruneWarps * 32)
-bj_score_complex_kernel(BatchTabs T, int l, LokiScoreSpec sp) {
-  extern __shared__ float smem[];
-  const LokiPruneJob& J = T.jobs[blockIdx.y];
-  const size_t li = (size_t)blockIdx.y * T.nlevels + (l - 1);
-  const LokiPruneLevel& D = T.levels[li];
-  const LokiPruneRun& R = J.run;
-  const LokiPruneWork& w = R.work;
-  const LokiPruneTree& in = R.trees[(l - 1) & 1];
-  const float2* seg = reinterpret_cast<const float2*>(J.ffa_fold) + (int64_t)T.seg_idx[li] *
-                                                                        J.seg_stride;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nb = D.nbins, nbf = nb / 2 + 1;
-  const int stride = score_stride(nb, sp.wmax);
-  float* tw = smem;
-  load_twiddles(tw, nb);
   __syncthreads();
-  float* wbase = smem + 2 * nb + (size_t)warp * cplx_warp_floats(nb, stride);
-  float2* comb = reinterpret_cast<float2*>(wbase) + (size_t)lane * 2 * nbf;
-  float* trow = wbase + (size_t)32 * 2 * nbf * 2 + lane * stride;
-  int64_t* cnt = R.counts;
-  const int64_t n_par = cnt[0];
-  const int64_t total = w.offsets[n_par];
-  const int64_t n_child = total > w.child_cap ? 0 : total;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    cnt[1] = n_child;
-    LokiPruneLevelStats* st = R.stats + (l - 1);
-    st->n_parents = n_par;
-    st->n_children = total;
-    st->n_valid = total;
-    if (total > w.child_cap) atomicOr(J.dev_err, LOKI_DEVERR_CAPACITY);
+  const int total = Q.pre[nj], per = (total + (int)gridDim.x - 1) / (int)gridDim.x;
+  *t0 = min((int)blockIdx.x * per, total);
+  *t1 = min(*t0 + per, total);
+}
+
+// Job of tile t; its level descriptor in Q.lvl (loaded when the job changes:
+// every thread of the block comes here for every tile). Returns the job.
+__device__ __forceinline__ int queue_job(JobQueue& Q, const BatchTabs& T, int j0, int nj, int l,
+                                         int t, int cur) {
+  int lo = 0, hi = nj;  // pre[lo] <= t < pre[hi]
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (Q.pre[mid] <= t) lo = mid;
+    else hi = mid;
   }
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n_child;
-       c += (int64_t)gridDim.x * blockDim.x)
-    score_child_complex(D, in.leaves, reinterpret_cast<const float2*>(in.folds), n_par,
-                        reinterpret_cast<LokiBranchInfo*>(w.info), w.offsets, seg, sp,
-                        w.child_scores, w.child_idx, w.child_phase,
-                        reinterpret_cast<unsigned*>(w.minmax), tw, comb, trow, c);
+  if (lo != cur) {
+    __syncthreads();  // the previous job's descriptor is no longer read
+    static_assert(sizeof(LokiPruneLevel) % 8 == 0, "copied by 8-byte words");
+    const uint64_t* src = reinterpret_cast<const uint64_t*>(
+        T.levels + (size_t)(j0 + lo) * T.nlevels + (l - 1));
+    uint64_t* dst = reinterpret_cast<uint64_t*>(&Q.lvl);
+    for (int k = threadIdx.x; k < (int)(sizeof(LokiPruneLevel) / 8); k += blockDim.x)
+      dst[k] = src[k];
+    __syncthreads();
+  }
+  return lo;
 }
 
-__global__ void __launch_bounds__(kPruneWarps * 32) bj_emit_complex_kernel(BatchTabs T, int l) {
-  const LokiPruneJob& J = T.jobs[blockIdx.y];
-  const size_t li = (size_t)blockIdx.y * T.nlevels + (l - 1);
-  const LokiPruneLevel& D = T.levels[li];
-  const LokiPruneRun& R = J.run;
-  const LokiPruneWork& w = R.work;
-  const LokiPruneTree& in = R.trees[(l - 1) & 1];
-  const LokiPruneTree& out = R.trees[l & 1];
-  const float2* seg = reinterpret_cast<const float2*>(J.ffa_fold) + (int64_t)T.seg_idx[li] *
-                                                                        J.seg_stride;
-  const int64_t n_par = R.counts[0], n_surv = R.counts[2];
-  for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n_surv;
-       s += (int64_t)gridDim.x * blockDim.x)
-    emit_one_complex(D, in.leaves, reinterpret_cast<const float2*>(in.folds),
-                     reinterpret_cast<LokiBranchInfo*>(w.info), w.offsets, n_par, seg, w.surv,
-                     w.child_scores, w.child_idx, w.child_phase, out.leaves,
-                     reinterpret_cast<float2*>(out.folds), out.scores, out.scores_ep,
-                     out.backtracks, s);
+// Runs body(job index, tile within the job, level descriptor) over this block's
+// tiles.
+template <typename F>
+__device__ __forceinline__ void queue_run(JobQueue& Q, const BatchTabs& T, int l, int j0, int nj,
+                                          int idx, F body) {
+  int t0, t1, cur = -1;
+  queue_open(Q, T, j0, nj, idx, &t0, &t1);
+  for (int t = t0; t < t1; ++t) {
+    cur = queue_job(Q, T, j0, nj, l, t, cur);
+    body(j0 + cur, (int64_t)(t - Q.pre[cur]));
+  }
 }
 
-// circular-orbit tree (real folds): the steps of circ_level_dev per job
-__global__ void bj_circ_branch_kernel(BatchTabs T, int l) {
-  const LokiPruneJob& J = T.jobs[blockIdx.y];
-  const LokiPruneLevel& D = T.levels[(size_t)blockIdx.y * T.nlevels + (l - 1)];
-  const LokiPruneRun& R = J.run;
-  const int64_t n = R.counts[0];
-  const double* leaves = R.trees[(l - 1) & 1].leaves;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    circ_branch_one(D, leaves, i, reinterpret_cast<LokiBranchInfo*>(R.work.info),
-                    R.work.offsets, R.exp_off, J.dev_err);
+__device__ __forceinline__ const void* job_segment(const BatchTabs& T, const LokiPruneJob& J,
+                                                   int job, int l, int bytes) {
+  const size_t li = (size_t)job * T.nlevels + (l - 1);
+  return reinterpret_cast<const char*>(J.ffa_fold) +
+         (int64_t)T.seg_idx[li] * J.seg_stride * bytes;
 }
 
-// the batch-ordered child map and validity flags; counts[1] = every child,
-// or 0 above the workspace (flagged)
-__global__ void bj_circ_map_kernel(BatchTabs T, int l, int64_t batch) {
-  const LokiPruneJob& J = T.jobs[blockIdx.y];
-  const LokiPruneLevel& D = T.levels[(size_t)blockIdx.y * T.nlevels + (l - 1)];
+__global__ void __launch_bounds__(kTile) bj_branch_kernel(BatchTabs T, int l, int j0, int nj) {
+  __shared__ JobQueue Q;
+  queue_run(Q, T, l, j0, nj, kCntPar, [&](int job, int64_t tile) {
+    const LokiPruneJob& J = T.jobs[job];
+    const int64_t i = tile * kTile + threadIdx.x;
+    if (i < J.run.counts[kCntPar])
+      branch_one(Q.lvl, J.run.trees[(l - 1) & 1].leaves, i,
+                 reinterpret_cast<LokiBranchInfo*>(J.run.work.info), J.run.work.offsets,
+                 J.dev_err, nullptr);
+  });
+}
+
+// ---- per-job kernels: one block of 1024 threads a job ---------------------------
+
+constexpr int kJobThreads = 1024;
+constexpr int kJobPer = 8;  // consecutive items a thread takes per pass
+
+// Exclusive block scan of one value a thread; the total to *tot.
+__device__ __forceinline__ int64_t job_scan(int64_t x, int64_t* wsum, int64_t* tot) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int64_t v = x;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int64_t y = __shfl_up_sync(0xFFFFFFFFu, v, o);
+    if (lane >= o) v += y;
+  }
+  __syncthreads();  // wsum of the previous pass has been read
+  if (lane == 31) wsum[warp] = v;
+  __syncthreads();
+  int64_t before = 0, total = 0;
+  const int64_t w = wsum[lane];
+  int64_t z = w;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int64_t y = __shfl_up_sync(0xFFFFFFFFu, z, o);
+    if (lane >= o) z += y;
+  }
+  total = __shfl_sync(0xFFFFFFFFu, z, 31);
+  before = __shfl_sync(0xFFFFFFFFu, z - w, warp);
+  *tot = total;
+  return before + v - x;
+}
+
+// Exclusive scan in place of the n counts at a; a[n] = the total.
+__device__ __forceinline__ int64_t job_scan_counts(int64_t* a, int64_t n, int64_t* wsum) {
+  int64_t carry = 0;
+  for (int64_t base = 0; base < n; base += kJobThreads * kJobPer) {
+    const int64_t i0 = base + (int64_t)threadIdx.x * kJobPer;
+    int64_t c[kJobPer], sum = 0;
+#pragma unroll
+    for (int k = 0; k < kJobPer; ++k) {
+      c[k] = i0 + k < n ? a[i0 + k] : 0;
+      sum += c[k];
+    }
+    int64_t tot, run = carry + job_scan(sum, wsum, &tot);
+#pragma unroll
+    for (int k = 0; k < kJobPer; ++k) {
+      if (i0 + k < n) a[i0 + k] = run;
+      run += c[k];
+    }
+    carry += tot;
+  }
+  if (threadIdx.x == 0) a[n] = carry;
+  return carry;
+}
+
+// After branch: the children's offsets (and, circular tree, the expansions'),
+// their number and the level's record; the circular tree's batch flags cleared.
+__global__ void __launch_bounds__(kJobThreads) bj_scan_kernel(BatchTabs T, int l, int j0,
+                                                              int circ, int64_t batch) {
+  __shared__ int64_t wsum[32];
+  const LokiPruneJob& J = T.jobs[j0 + blockIdx.x];
   const LokiPruneRun& R = J.run;
-  const LokiPruneWork& w = R.work;
   int64_t* cnt = R.counts;
-  const int64_t n = cnt[0];
-  const int64_t total = w.offsets[n] + R.exp_off[n];
-  const bool fits = total <= w.child_cap;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    cnt[1] = fits ? total : 0;
+  const int64_t n = cnt[kCntPar];
+  int64_t total = job_scan_counts(R.work.offsets, n, wsum);
+  if (circ) {
+    total += job_scan_counts(R.exp_off, n, wsum);
+    for (int64_t i = threadIdx.x; i <= n / batch; i += blockDim.x) R.batch_taylor[i] = 0;
+  }
+  if (threadIdx.x == 0) {
+    cnt[kCntChild] = total > R.work.child_cap ? 0 : total;
     LokiPruneLevelStats* st = R.stats + (l - 1);
     st->n_parents = n;
     st->n_children = total;
-    if (!fits) atomicOr(J.dev_err, LOKI_DEVERR_CAPACITY);
-  }
-  if (!fits) return;
-  const double* leaves = R.trees[(l - 1) & 1].leaves;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    circ_map_one(D, leaves, n, batch, reinterpret_cast<const LokiBranchInfo*>(w.info),
-                 w.offsets, R.exp_off, reinterpret_cast<CircChild*>(R.child_map),
-                 R.valid_flags, i);
-}
-
-// the per-batch "holds Taylor children" flags of the current parents
-__global__ void bj_circ_clear_kernel(BatchTabs T, int64_t batch) {
-  const LokiPruneRun& R = T.jobs[blockIdx.y].run;
-  const int64_t nb = R.counts[0] / batch + 1;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nb;
-       i += (int64_t)gridDim.x * blockDim.x)
-    R.batch_taylor[i] = 0;
-}
-
-__global__ void __launch_bounds__(kPruneWarps * 32)
-bj_circ_score_kernel(BatchTabs T, int l, LokiScoreSpec sp, ScoreK SK, int64_t batch) {
-  extern __shared__ float tiles[];
-  const LokiPruneJob& J = T.jobs[blockIdx.y];
-  const size_t li = (size_t)blockIdx.y * T.nlevels + (l - 1);
-  const LokiPruneLevel& D = T.levels[li];
-  const LokiPruneRun& R = J.run;
-  const LokiPruneWork& w = R.work;
-  const LokiPruneTree& in = R.trees[(l - 1) & 1];
-  const float* seg = J.ffa_fold + (int64_t)T.seg_idx[li] * J.seg_stride;
-  const int warp = threadIdx.x >> 5;
-  float* tile = tiles + (size_t)warp * 32 * score_stride(D.nbins, sp.wmax);
-  int64_t* cnt = R.counts;
-  const int64_t n_valid = job_pos(w)[cnt[1]];
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    cnt[4] = n_valid;
-    R.stats[l - 1].n_valid = n_valid;
-  }
-  for (int64_t t = (int64_t)blockIdx.x * kPruneWarps + warp; t * 32 < n_valid;
-       t += (int64_t)gridDim.x * kPruneWarps) {
-    circ_score_tile(D, in.leaves, in.folds, batch,
-                    reinterpret_cast<const LokiBranchInfo*>(w.info),
-                    reinterpret_cast<const CircChild*>(R.child_map), R.valid_ids, n_valid, seg,
-                    sp, SK, w.child_scores, w.child_idx, w.child_phase, R.child_class,
-                    R.batch_taylor, reinterpret_cast<unsigned*>(w.minmax), tile, t * 32);
-    __syncwarp();
+    if (!circ) st->n_valid = total;
+    if (total > R.work.child_cap) atomicOr(J.dev_err, LOKI_DEVERR_CAPACITY);
   }
 }
 
-// valid-child offsets at the parents (the overflow rule reads those at
-// batch boundaries)
-__global__ void bj_circ_boff_kernel(BatchTabs T) {
-  const LokiPruneRun& R = T.jobs[blockIdx.y].run;
-  const int64_t n = R.counts[0], n_valid = R.counts[4];
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p <= n;
-       p += (int64_t)gridDim.x * blockDim.x)
-    R.batch_offsets[p] = lower_bound64(R.valid_ids, n_valid, R.work.offsets[p] + R.exp_off[p]);
-}
-
-__global__ void __launch_bounds__(kPruneWarps * 32)
-bj_circ_emit_kernel(BatchTabs T, int l, int64_t batch) {
-  const LokiPruneJob& J = T.jobs[blockIdx.y];
-  const size_t li = (size_t)blockIdx.y * T.nlevels + (l - 1);
-  const LokiPruneLevel& D = T.levels[li];
-  const LokiPruneRun& R = J.run;
-  const LokiPruneWork& w = R.work;
-  const LokiPruneTree& in = R.trees[(l - 1) & 1];
-  const LokiPruneTree& out = R.trees[l & 1];
-  const float* seg = J.ffa_fold + (int64_t)T.seg_idx[li] * J.seg_stride;
-  const int warp = threadIdx.x >> 5;
-  const int64_t n_surv = R.counts[2];
-  for (int64_t t = (int64_t)blockIdx.x * kPruneWarps + warp; t * 32 < n_surv;
-       t += (int64_t)gridDim.x * kPruneWarps)
-    circ_emit_tile(D, in.leaves, in.folds, batch,
-                   reinterpret_cast<const LokiBranchInfo*>(w.info),
-                   reinterpret_cast<const CircChild*>(R.child_map), R.valid_ids, seg, w.surv,
-                   n_surv, w.child_scores, w.child_idx, w.child_phase, R.child_class,
-                   R.batch_taylor, out.leaves, out.folds, out.scores, out.scores_ep,
-                   out.backtracks, t * 32);
-}
-
-// the circular tree over complex folds: lane per valid child / survivor
-__global__ void __launch_bounds__(kPruneWarps * 32)
-bj_circ_score_complex_kernel(BatchTabs T, int l, LokiScoreSpec sp, int64_t batch) {
-  extern __shared__ float smem[];
-  const LokiPruneJob& J = T.jobs[blockIdx.y];
-  const size_t li = (size_t)blockIdx.y * T.nlevels + (l - 1);
-  const LokiPruneLevel& D = T.levels[li];
-  const LokiPruneRun& R = J.run;
-  const LokiPruneWork& w = R.work;
-  const LokiPruneTree& in = R.trees[(l - 1) & 1];
-  const float2* seg =
-      reinterpret_cast<const float2*>(J.ffa_fold) + (int64_t)T.seg_idx[li] * J.seg_stride;
+// Indices of the n values v with v >= thr, in order, to ids; returns how many.
+// *best: position among them of the largest, the first of equals (-1: none).
+__device__ __forceinline__ int64_t job_compact(const float* __restrict__ v, int64_t n, double thr,
+                                               int64_t* __restrict__ ids, int64_t* wsum,
+                                               int64_t* best) {
+  int64_t carry = 0, bi = -1;
+  float bv = 0.0f;
+  for (int64_t base = 0; base < n; base += kJobThreads * kJobPer) {
+    const int64_t i0 = base + (int64_t)threadIdx.x * kJobPer;
+    float x[kJobPer];
+    unsigned f = 0;
+    if (i0 + kJobPer <= n && (reinterpret_cast<uintptr_t>(v) & 15) == 0) {
+#pragma unroll
+      for (int k = 0; k < kJobPer; k += 4) {
+        const float4 q = *reinterpret_cast<const float4*>(v + i0 + k);
+        x[k] = q.x, x[k + 1] = q.y, x[k + 2] = q.z, x[k + 3] = q.w;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < kJobPer; ++k) x[k] = i0 + k < n ? v[i0 + k] : nanf("");
+    }
+#pragma unroll
+    for (int k = 0; k < kJobPer; ++k) f |= (double)x[k] >= thr ? 1u << k : 0u;
+    int64_t tot, at = carry + job_scan(__popc(f), wsum, &tot);
+#pragma unroll
+    for (int k = 0; k < kJobPer; ++k)
+      if (f >> k & 1u) {
+        if (bi < 0 || x[k] > bv) {
+          bv = x[k];
+          bi = at;
+        }
+        ids[at++] = i0 + k;
+      }
+    carry += tot;
+  }
+  // the block's best: a thread's own is its first maximum already
+  __shared__ float sv[32];
+  __shared__ int64_t si[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nb = D.nbins, nbf = nb / 2 + 1;
-  const int stride = score_stride(nb, sp.wmax);
-  float* tw = smem;
-  load_twiddles(tw, nb);
-  __syncthreads();
-  float* wbase = smem + 2 * nb + (size_t)warp * cplx_warp_floats(nb, stride);
-  float2* comb = reinterpret_cast<float2*>(wbase) + (size_t)lane * 2 * nbf;
-  float* trow = wbase + (size_t)32 * 2 * nbf * 2 + lane * stride;
-  int64_t* cnt = R.counts;
-  const int64_t n_valid = job_pos(w)[cnt[1]];
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    cnt[4] = n_valid;
-    R.stats[l - 1].n_valid = n_valid;
+  auto fold = [&]() {
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ov = __shfl_down_sync(0xFFFFFFFFu, bv, o);
+      const int64_t oi = __shfl_down_sync(0xFFFFFFFFu, bi, o);
+      if (oi >= 0 && (bi < 0 || ov > bv || (ov == bv && oi < bi))) {
+        bv = ov;
+        bi = oi;
+      }
+    }
+  };
+  fold();
+  if (lane == 0) {
+    sv[warp] = bv;
+    si[warp] = bi;
   }
-  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n_valid;
-       v += (int64_t)gridDim.x * blockDim.x)
-    circ_score_one_complex(D, in.leaves, reinterpret_cast<const float2*>(in.folds), batch,
-                           reinterpret_cast<const LokiBranchInfo*>(w.info),
-                           reinterpret_cast<const CircChild*>(R.child_map), R.valid_ids, seg, sp,
-                           tw, comb, trow, w.child_scores, w.child_idx, w.child_phase,
-                           R.child_class, R.batch_taylor, reinterpret_cast<unsigned*>(w.minmax),
-                           v);
+  __syncthreads();
+  bv = sv[lane];
+  bi = si[lane];
+  fold();
+  *best = __shfl_sync(0xFFFFFFFFu, bi, 0);
+  __syncthreads();
+  return carry;
 }
 
-__global__ void __launch_bounds__(kPruneWarps * 32)
-bj_circ_emit_complex_kernel(BatchTabs T, int l, int64_t batch) {
-  const LokiPruneJob& J = T.jobs[blockIdx.y];
-  const size_t li = (size_t)blockIdx.y * T.nlevels + (l - 1);
-  const LokiPruneLevel& D = T.levels[li];
+// Circular tree: the valid children in order and their number.
+__global__ void __launch_bounds__(kJobThreads) bj_circ_valid_kernel(BatchTabs T, int l, int j0) {
+  __shared__ int64_t wsum[32];
+  const LokiPruneRun& R = T.jobs[j0 + blockIdx.x].run;
+  int64_t best;
+  const int64_t n = job_compact(R.valid_flags, R.counts[kCntChild], 0.5, R.valid_ids, wsum, &best);
+  if (threadIdx.x == 0) {
+    R.counts[kCntValid] = n;
+    R.stats[l - 1].n_valid = n;
+  }
+}
+
+// After score: the survivors in child order (by the overflow rule when they
+// exceed max_sugg), the best of them, the level's record, and the counters
+// turned to the next level.
+__global__ void __launch_bounds__(kJobThreads)
+bj_select_kernel(BatchTabs T, int l, int j0, int64_t max_sugg, int64_t batch, int circ) {
+  __shared__ int64_t wsum[32];
+  const int job = j0 + blockIdx.x;
+  const LokiPruneJob& J = T.jobs[job];
   const LokiPruneRun& R = J.run;
   const LokiPruneWork& w = R.work;
-  const LokiPruneTree& in = R.trees[(l - 1) & 1];
-  const LokiPruneTree& out = R.trees[l & 1];
-  const float2* seg =
-      reinterpret_cast<const float2*>(J.ffa_fold) + (int64_t)T.seg_idx[li] * J.seg_stride;
-  const int64_t n_surv = R.counts[2];
-  for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n_surv;
-       s += (int64_t)gridDim.x * blockDim.x)
-    circ_emit_one_complex(D, in.leaves, reinterpret_cast<const float2*>(in.folds), batch,
-                          reinterpret_cast<const LokiBranchInfo*>(w.info),
-                          reinterpret_cast<const CircChild*>(R.child_map), R.valid_ids, seg,
-                          w.surv, w.child_scores, w.child_idx, w.child_phase, R.child_class,
-                          R.batch_taylor, out.leaves, reinterpret_cast<float2*>(out.folds),
-                          out.scores, out.scores_ep, out.backtracks, s);
-}
-
-__global__ void bj_bt_kernel(BatchTabs T, int l, int row) {
-  const LokiPruneJob& J = T.jobs[blockIdx.y];
-  const LokiPruneRun& R = J.run;
-  if (!R.bt_hist) return;
-  const int64_t start = R.counts[3], rows = R.counts[2];
-  if (start + rows > R.bt_rows) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(J.dev_err, LOKI_DEVERR_CAPACITY);
-    return;
-  }
-  const int32_t* bt = R.trees[l & 1].backtracks;
-  int32_t* h = R.bt_hist + start * row;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < rows * row;
-       i += (int64_t)gridDim.x * blockDim.x)
-    h[i] = bt[i];
-}
-
-// one block per job: the best leaf of the new tree, then the level's end
-__global__ void __launch_bounds__(1024) bj_best_kernel(BatchTabs T, int l, int row_leaf) {
-  const LokiPruneJob& J = T.jobs[blockIdx.x];
-  const LokiPruneRun& R = J.run;
   int64_t* cnt = R.counts;
-  const int64_t n = cnt[2];
-  if (R.best_leaves && R.best_scores)
-    block_best(R.trees[l & 1].scores, n, R.trees[l & 1].leaves, row_leaf,
-               R.best_leaves + (int64_t)(l - 1) * row_leaf, R.best_scores + (l - 1));
-  __syncthreads();  // every thread has read the count
-  if (threadIdx.x == 0)
-    level_end(cnt, reinterpret_cast<unsigned*>(R.work.minmax), R.ovf_flag, R.stats + (l - 1));
+  const int64_t n_par = cnt[kCntPar], n_valid = cnt[kCntValid];
+  const double thr = T.thr[(size_t)job * T.nlevels + (l - 1)];
+  int64_t best;
+  int64_t n = job_compact(w.child_scores, circ ? n_valid : cnt[kCntChild], thr, w.surv, wsum,
+                          &best);
+  const bool ovf = n > max_sugg;
+  if (ovf) {
+    const int64_t* off = w.offsets;
+    if (circ) {  // the rule's batches are over the valid children
+      for (int64_t q = threadIdx.x; q <= (n_par + batch - 1) / batch; q += blockDim.x) {
+        const int64_t p = min(q * batch, n_par);
+        R.batch_offsets[p] = lower_bound64(R.valid_ids, n_valid, w.offsets[p] + R.exp_off[p]);
+      }
+      off = R.batch_offsets;
+    }
+    __syncthreads();
+    select_overflow_block(w.child_scores, off, n_par, batch, thr, max_sugg, w.surv, &wsum[0],
+                          w.ovf_thr, w.ovf_ids, reinterpret_cast<unsigned*>(w.ovf_keys));
+    n = wsum[0];
+    __syncthreads();
+    // the best of what the rule kept
+    unsigned long long* key = reinterpret_cast<unsigned long long*>(&wsum[1]);
+    if (threadIdx.x == 0) *key = 0ull;
+    __syncthreads();
+    for (int64_t i = threadIdx.x; i < n; i += blockDim.x)
+      // + 0.0f: zeros of either sign are equal
+      atomicMax(key, ((unsigned long long)float_key(w.child_scores[w.surv[i]] + 0.0f) << 32) |
+                         (0xFFFFFFFFu - (unsigned)i));
+    __syncthreads();
+    best = n > 0 ? (int64_t)(0xFFFFFFFFu - (unsigned)*key) : -1;
+  }
+  if (threadIdx.x != 0) return;
+  LokiPruneLevelStats* st = R.stats + (l - 1);
+  unsigned* keys = reinterpret_cast<unsigned*>(w.minmax);
+  cnt[kCntOldPar] = n_par;
+  cnt[kCntBtRow] = cnt[kCntBt];
+  cnt[kCntBest] = best;
+  cnt[kCntSurv] = n;
+  if (R.bt_hist && cnt[kCntBt] + n > R.bt_rows) atomicOr(J.dev_err, LOKI_DEVERR_CAPACITY);
+  *R.ovf_flag = ovf ? 1 : 0;
+  level_end(cnt, keys, R.ovf_flag, st);
+}
+
+// ---- score and emission ------------------------------------------------------
+
+__global__ void __launch_bounds__(kTile, 4)
+bj_score_kernel(BatchTabs T, int l, int j0, int nj, LokiScoreSpec sp, ScoreK SK) {
+  extern __shared__ float tiles[];
+  __shared__ JobQueue Q;
+  const int warp = threadIdx.x >> 5;
+  queue_run(Q, T, l, j0, nj, kCntChild, [&](int job, int64_t t) {
+    const LokiPruneJob& J = T.jobs[job];
+    const LokiPruneWork& w = J.run.work;
+    const LokiPruneTree& in = J.run.trees[(l - 1) & 1];
+    const int64_t n_child = J.run.counts[kCntChild], c0 = t * kTile + warp * 32;
+    if (c0 >= n_child) return;
+    float* tile = tiles + (size_t)warp * 32 * score_stride(Q.lvl.nbins, sp.wmax);
+    score_tile(Q.lvl, in.leaves, in.folds, J.run.counts[kCntPar],
+               reinterpret_cast<LokiBranchInfo*>(w.info), w.offsets, n_child,
+               static_cast<const float*>(job_segment(T, J, job, l, 4)), sp, SK, w.child_scores,
+               w.child_idx, w.child_phase, reinterpret_cast<unsigned*>(w.minmax), tile, c0);
+    __syncwarp();
+  });
+}
+
+// The emission's extras of a job: its backtrack history row and best survivor.
+__device__ __forceinline__ EmitExtra job_extra(const LokiPruneRun& R, int l, int P) {
+  EmitExtra X;
+  const int64_t row = R.counts[kCntBtRow];
+  if (R.bt_hist && row + R.counts[kCntSurv] <= R.bt_rows) X.bt_hist = R.bt_hist + row * (P + 2);
+  if (R.best_leaves && R.best_scores) {
+    X.best = R.counts[kCntBest];
+    X.best_leaf = R.best_leaves + (int64_t)(l - 1) * (P + 2) * 2;
+    X.best_score = R.best_scores + (l - 1);
+  }
+  return X;
+}
+
+__global__ void __launch_bounds__(kTile, 4) bj_emit_kernel(BatchTabs T, int l, int j0, int nj) {
+  __shared__ JobQueue Q;
+  const int warp = threadIdx.x >> 5;
+  queue_run(Q, T, l, j0, nj, kCntSurv, [&](int job, int64_t t) {
+    const LokiPruneJob& J = T.jobs[job];
+    const LokiPruneRun& R = J.run;
+    const LokiPruneWork& w = R.work;
+    const LokiPruneTree &in = R.trees[(l - 1) & 1], &out = R.trees[l & 1];
+    const int64_t n_surv = R.counts[kCntSurv], s0 = t * kTile + warp * 32;
+    if (s0 >= n_surv) return;
+    emit_tile(Q.lvl, in.leaves, in.folds, reinterpret_cast<LokiBranchInfo*>(w.info), w.offsets,
+              R.counts[kCntOldPar], static_cast<const float*>(job_segment(T, J, job, l, 4)),
+              w.surv, n_surv, w.child_scores, w.child_idx, w.child_phase, out.leaves, out.folds,
+              out.scores, out.scores_ep, out.backtracks, s0, job_extra(R, l, Q.lvl.poly_order));
+  });
+}
+
+// Shared memory of the complex kernels: twiddles, then per warp either the 64-bin
+// rows or (other bin counts) every lane's sums and score row.
+__host__ __device__ inline int cplx_smem_bytes(int nbins, int wmax, bool score) {
+  const int stride = score_stride(nbins, wmax);
+  if (nbins == 64)
+    return 512 + kPruneWarps * (score ? max(cplx64_warp_bytes(), 32 * stride * 4)
+                                      : cplx64_warp_bytes());
+  return score ? (int)((2 * nbins + kPruneWarps * cplx_warp_floats(nbins, stride)) * 4) : 0;
+}
+
+__global__ void __launch_bounds__(kTile)
+bj_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LokiScoreSpec sp, ScoreK SK, int nb) {
+  extern __shared__ __align__(16) float smem[];
+  __shared__ JobQueue Q;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int stride = score_stride(nb, sp.wmax), nbf = nb / 2 + 1;
+  if (nb == 64) load_twiddles64(reinterpret_cast<float2*>(smem));
+  else load_twiddles(smem, nb);
+  queue_run(Q, T, l, j0, nj, kCntChild, [&](int job, int64_t t) {
+    const LokiPruneJob& J = T.jobs[job];
+    const LokiPruneWork& w = J.run.work;
+    const LokiPruneTree& in = J.run.trees[(l - 1) & 1];
+    const LokiBranchInfo* info = reinterpret_cast<LokiBranchInfo*>(w.info);
+    const float2* folds = reinterpret_cast<const float2*>(in.folds);
+    const float2* seg = static_cast<const float2*>(job_segment(T, J, job, l, 8));
+    unsigned* keys = reinterpret_cast<unsigned*>(w.minmax);
+    const int64_t n_par = J.run.counts[kCntPar], n_child = J.run.counts[kCntChild];
+    const int64_t c0 = t * kTile + warp * 32, c = c0 + lane;
+    if (c0 >= n_child) return;
+    const int kmax = (int)min((int64_t)32, n_child - c0);
+    const LokiPruneLevel& D = Q.lvl;
+    if (nb != 64) {
+      float* wbase = smem + 2 * nb + (size_t)warp * cplx_warp_floats(nb, stride);
+      if (c < n_child)
+        score_child_complex(D, in.leaves, folds, n_par, info, w.offsets, seg, sp, SK,
+                            w.child_scores, w.child_idx, w.child_phase, keys, smem,
+                            reinterpret_cast<float2*>(wbase) + (size_t)lane * 2 * nbf,
+                            wbase + (size_t)32 * 2 * nbf * 2 + lane * stride, c);
+      return;
+    }
+    const int64_t par = warp_find_parents(w.offsets, n_par, c, kmax);
+    int64_t row = 0;
+    float2 delta = make_float2(1.0f, 0.0f);
+    if (lane < kmax) {
+      const int P = D.poly_order;
+      const LokiBranchInfo B = info[par];
+      double pv[LOKI_MAX_PARAMS + 1];
+      child_params(B, P, c - w.offsets[par], pv);
+      pv[P] = B.d0;
+      const ChildRes r = resolve_child(D, pv, in.leaves[(par * (P + 2) + P + 1) * 2]);
+      w.child_idx[2 * c] = r.ia;
+      w.child_idx[2 * c + 1] = r.iff;
+      w.child_phase[c] = r.phase;
+      row = (int64_t)r.ia * D.n_freq + r.iff;
+      delta = prune_phasor(r.phase, 64);
+    }
+    const int wb = max(cplx64_warp_bytes(), 32 * stride * 4);
+    cplx64_score(folds, seg, par, row, delta, kmax, reinterpret_cast<const float2*>(smem),
+                 reinterpret_cast<float2*>(reinterpret_cast<char*>(smem) + 512 + warp * wb), sp,
+                 SK, w.child_scores + c0, keys);
+    __syncwarp();
+  });
+}
+
+__global__ void __launch_bounds__(kTile, 4)
+bj_emit_complex_kernel(BatchTabs T, int l, int j0, int nj, int nb) {
+  extern __shared__ __align__(16) float smem[];
+  __shared__ JobQueue Q;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  queue_run(Q, T, l, j0, nj, kCntSurv, [&](int job, int64_t t) {
+    const LokiPruneJob& J = T.jobs[job];
+    const LokiPruneRun& R = J.run;
+    const LokiPruneWork& w = R.work;
+    const LokiPruneTree &in = R.trees[(l - 1) & 1], &out = R.trees[l & 1];
+    const LokiBranchInfo* info = reinterpret_cast<LokiBranchInfo*>(w.info);
+    const float2* folds = reinterpret_cast<const float2*>(in.folds);
+    const float2* seg = static_cast<const float2*>(job_segment(T, J, job, l, 8));
+    const int64_t n_surv = R.counts[kCntSurv], s0 = t * kTile + warp * 32, s = s0 + lane;
+    if (s0 >= n_surv) return;
+    const int kmax = (int)min((int64_t)32, n_surv - s0), nbf = nb / 2 + 1;
+    const int64_t par = warp_find_parents(w.offsets, R.counts[kCntOldPar],
+                                          w.surv[s0 + min(lane, kmax - 1)], kmax);
+    EmitRow r = {0, 0, 0.0};
+    if (lane < kmax)
+      r = emit_one_complex_leaf(Q.lvl, in.leaves, info, w.offsets, w.surv, w.child_scores,
+                                w.child_idx, w.child_phase, out.leaves, out.scores,
+                                out.scores_ep, out.backtracks, s, par,
+                                job_extra(R, l, Q.lvl.poly_order));
+    float2* fout = reinterpret_cast<float2*>(out.folds);
+    if (nb == 64)
+      cplx64_emit(folds, seg, r.par, r.row, prune_phasor(r.phase, nb), kmax,
+                  reinterpret_cast<float2*>(reinterpret_cast<char*>(smem) + 512 +
+                                            warp * cplx64_warp_bytes()),
+                  fout + s0 * 66);
+    else if (lane < kmax)
+      rotate_add(seg + r.row * 2 * nbf, folds + r.par * 2 * nbf, prune_phasor(r.phase, nb), nbf,
+                 fout + s * 2 * nbf);
+  });
+}
+
+// ---- circular-orbit tree -------------------------------------------------------
+
+__global__ void __launch_bounds__(kTile)
+bj_circ_branch_kernel(BatchTabs T, int l, int j0, int nj) {
+  __shared__ JobQueue Q;
+  queue_run(Q, T, l, j0, nj, kCntPar, [&](int job, int64_t tile) {
+    const LokiPruneJob& J = T.jobs[job];
+    const int64_t i = tile * kTile + threadIdx.x;
+    if (i < J.run.counts[kCntPar])
+      circ_branch_one(Q.lvl, J.run.trees[(l - 1) & 1].leaves, i,
+                      reinterpret_cast<LokiBranchInfo*>(J.run.work.info), J.run.work.offsets,
+                      J.run.exp_off, J.dev_err);
+  });
+}
+
+// the batch-ordered child map and validity flags (none of a level whose
+// children exceed the workspace)
+__global__ void __launch_bounds__(kTile)
+bj_circ_map_kernel(BatchTabs T, int l, int j0, int nj, int64_t batch) {
+  __shared__ JobQueue Q;
+  queue_run(Q, T, l, j0, nj, kCntPar, [&](int job, int64_t tile) {
+    const LokiPruneRun& R = T.jobs[job].run;
+    const int64_t i = tile * kTile + threadIdx.x, n = R.counts[kCntPar];
+    if (i < n && R.counts[kCntChild] > 0)
+      circ_map_one(Q.lvl, R.trees[(l - 1) & 1].leaves, n, batch,
+                   reinterpret_cast<const LokiBranchInfo*>(R.work.info), R.work.offsets,
+                   R.exp_off, reinterpret_cast<CircChild*>(R.child_map), R.valid_flags, i);
+  });
+}
+
+__global__ void __launch_bounds__(kTile)
+bj_circ_score_kernel(BatchTabs T, int l, int j0, int nj, LokiScoreSpec sp, ScoreK SK,
+                     int64_t batch) {
+  extern __shared__ float tiles[];
+  __shared__ JobQueue Q;
+  const int warp = threadIdx.x >> 5;
+  queue_run(Q, T, l, j0, nj, kCntValid, [&](int job, int64_t t) {
+    const LokiPruneJob& J = T.jobs[job];
+    const LokiPruneRun& R = J.run;
+    const LokiPruneWork& w = R.work;
+    const LokiPruneTree& in = R.trees[(l - 1) & 1];
+    const int64_t n_valid = R.counts[kCntValid], v0 = t * kTile + warp * 32;
+    if (v0 >= n_valid) return;
+    circ_score_tile(Q.lvl, in.leaves, in.folds, batch,
+                    reinterpret_cast<const LokiBranchInfo*>(w.info),
+                    reinterpret_cast<const CircChild*>(R.child_map), R.valid_ids, n_valid,
+                    static_cast<const float*>(job_segment(T, J, job, l, 4)), sp, SK,
+                    w.child_scores, w.child_idx, w.child_phase, R.child_class, R.batch_taylor,
+                    reinterpret_cast<unsigned*>(w.minmax),
+                    tiles + (size_t)warp * 32 * score_stride(Q.lvl.nbins, sp.wmax), v0);
+    __syncwarp();
+  });
+}
+
+__global__ void __launch_bounds__(kTile)
+bj_circ_emit_kernel(BatchTabs T, int l, int j0, int nj, int64_t batch) {
+  __shared__ JobQueue Q;
+  const int warp = threadIdx.x >> 5;
+  queue_run(Q, T, l, j0, nj, kCntSurv, [&](int job, int64_t t) {
+    const LokiPruneJob& J = T.jobs[job];
+    const LokiPruneRun& R = J.run;
+    const LokiPruneWork& w = R.work;
+    const LokiPruneTree &in = R.trees[(l - 1) & 1], &out = R.trees[l & 1];
+    const int64_t n_surv = R.counts[kCntSurv], s0 = t * kTile + warp * 32;
+    if (s0 >= n_surv) return;
+    circ_emit_tile(Q.lvl, in.leaves, in.folds, batch,
+                   reinterpret_cast<const LokiBranchInfo*>(w.info),
+                   reinterpret_cast<const CircChild*>(R.child_map), R.valid_ids,
+                   static_cast<const float*>(job_segment(T, J, job, l, 4)), w.surv, n_surv,
+                   w.child_scores, w.child_idx, w.child_phase, R.child_class, R.batch_taylor,
+                   out.leaves, out.folds, out.scores, out.scores_ep, out.backtracks, s0,
+                   job_extra(R, l, 5));
+  });
+}
+
+__global__ void __launch_bounds__(kTile)
+bj_circ_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LokiScoreSpec sp, ScoreK SK,
+                             int64_t batch, int nb) {
+  extern __shared__ __align__(16) float smem[];
+  __shared__ JobQueue Q;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int stride = score_stride(nb, sp.wmax), nbf = nb / 2 + 1;
+  if (nb == 64) load_twiddles64(reinterpret_cast<float2*>(smem));
+  else load_twiddles(smem, nb);
+  queue_run(Q, T, l, j0, nj, kCntValid, [&](int job, int64_t t) {
+    const LokiPruneJob& J = T.jobs[job];
+    const LokiPruneRun& R = J.run;
+    const LokiPruneWork& w = R.work;
+    const LokiPruneTree& in = R.trees[(l - 1) & 1];
+    const LokiBranchInfo* info = reinterpret_cast<const LokiBranchInfo*>(w.info);
+    const CircChild* map = reinterpret_cast<const CircChild*>(R.child_map);
+    const float2* folds = reinterpret_cast<const float2*>(in.folds);
+    const float2* seg = static_cast<const float2*>(job_segment(T, J, job, l, 8));
+    unsigned* keys = reinterpret_cast<unsigned*>(w.minmax);
+    const int64_t n_valid = R.counts[kCntValid], v0 = t * kTile + warp * 32, v = v0 + lane;
+    if (v0 >= n_valid) return;
+    const int kmax = (int)min((int64_t)32, n_valid - v0);
+    const LokiPruneLevel& D = Q.lvl;
+    if (nb != 64) {
+      float* wbase = smem + 2 * nb + (size_t)warp * cplx_warp_floats(nb, stride);
+      if (v < n_valid)
+        circ_score_one_complex(D, in.leaves, folds, batch, info, map, R.valid_ids, seg, sp, SK,
+                               smem, reinterpret_cast<float2*>(wbase) + (size_t)lane * 2 * nbf,
+                               wbase + (size_t)32 * 2 * nbf * 2 + lane * stride, w.child_scores,
+                               w.child_idx, w.child_phase, R.child_class, R.batch_taylor, keys,
+                               v);
+      return;
+    }
+    int64_t par = 0, row = 0;
+    float2 delta = make_float2(1.0f, 0.0f);
+    if (lane < kmax) {
+      const CircChild ch = map[R.valid_ids[v]];
+      const LokiBranchInfo I = info[ch.parent];
+      const double* lf = in.leaves + (int64_t)ch.parent * 14;
+      double pv[6], ev[6];
+      circ_child(I, lf, ch, pv, ev);
+      ChildRes r;
+      const int cls = circ_resolve(D, pv, ev, lf[12], &r);
+      if (cls == 0) atomicOr(R.batch_taylor + ch.parent / batch, 1);
+      w.child_idx[2 * v] = r.ia;
+      w.child_idx[2 * v + 1] = r.iff;
+      w.child_phase[v] = r.phase;
+      R.child_class[v] = (int8_t)cls;
+      par = ch.parent;
+      row = (int64_t)r.ia * D.n_freq + r.iff;
+      delta = prune_phasor(r.phase, 64);
+    }
+    const int wb = max(cplx64_warp_bytes(), 32 * stride * 4);
+    cplx64_score(folds, seg, par, row, delta, kmax, reinterpret_cast<const float2*>(smem),
+                 reinterpret_cast<float2*>(reinterpret_cast<char*>(smem) + 512 + warp * wb), sp,
+                 SK, w.child_scores + v0, keys);
+    __syncwarp();
+  });
+}
+
+__global__ void __launch_bounds__(kTile)
+bj_circ_emit_complex_kernel(BatchTabs T, int l, int j0, int nj, int64_t batch, int nb) {
+  extern __shared__ __align__(16) float smem[];
+  __shared__ JobQueue Q;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  queue_run(Q, T, l, j0, nj, kCntSurv, [&](int job, int64_t t) {
+    const LokiPruneJob& J = T.jobs[job];
+    const LokiPruneRun& R = J.run;
+    const LokiPruneWork& w = R.work;
+    const LokiPruneTree &in = R.trees[(l - 1) & 1], &out = R.trees[l & 1];
+    const float2* folds = reinterpret_cast<const float2*>(in.folds);
+    const float2* seg = static_cast<const float2*>(job_segment(T, J, job, l, 8));
+    const int64_t n_surv = R.counts[kCntSurv], s0 = t * kTile + warp * 32, s = s0 + lane;
+    if (s0 >= n_surv) return;
+    const int kmax = (int)min((int64_t)32, n_surv - s0), nbf = nb / 2 + 1;
+    EmitRow r = {0, 0, 0.0};
+    if (lane < kmax)
+      r = circ_emit_one_complex_leaf(Q.lvl, in.leaves, batch,
+                                     reinterpret_cast<const LokiBranchInfo*>(w.info),
+                                     reinterpret_cast<const CircChild*>(R.child_map),
+                                     R.valid_ids, w.surv, w.child_scores, w.child_idx,
+                                     w.child_phase, R.child_class, R.batch_taylor, out.leaves,
+                                     out.scores, out.scores_ep, out.backtracks, s,
+                                     job_extra(R, l, 5));
+    float2* fout = reinterpret_cast<float2*>(out.folds);
+    if (nb == 64)
+      cplx64_emit(folds, seg, r.par, r.row, prune_phasor(r.phase, nb), kmax,
+                  reinterpret_cast<float2*>(reinterpret_cast<char*>(smem) + 512 +
+                                            warp * cplx64_warp_bytes()),
+                  fout + s0 * 66);
+    else if (lane < kmax)
+      rotate_add(seg + r.row * 2 * nbf, folds + r.par * 2 * nbf, prune_phasor(r.phase, nb), nbf,
+                 fout + s * 2 * nbf);
+  });
 }
 
 }  // namespace loki
@@ -3877,22 +4291,22 @@ static int batch_enqueue(void* dev_scratch, int32_t njobs, int32_t nlevels,
                          const LokiScoreSpec* spec, int64_t max_sugg, int64_t batch_size,
                          const BatchShape& shape, cudaStream_t s,
                          cudaEvent_t* ev_score = nullptr) {
-  const int nb = shape.nbins, P = shape.poly_order;
+  const int nb = shape.nbins;
   const bool cplx = shape.fourier != 0;
   LokiScoreSpec sp = *spec;
   sp.mode = 1;
   const ScoreK SK = make_score_k(sp, nb);
-  const int smem =
-      cplx ? (int)((2 * nb + kPruneWarps * cplx_warp_floats(nb, score_stride(nb, sp.wmax))) *
-                   sizeof(float))
-           : score_smem_bytes(nb, sp.wmax, kPruneWarps);
+  const int smem = cplx ? cplx_smem_bytes(nb, sp.wmax, true)
+                        : score_smem_bytes(nb, sp.wmax, kPruneWarps);
+  const int smem_emit = cplx ? cplx_smem_bytes(nb, sp.wmax, false) : 0;
   if (smem > 200 * 1024)
     return set_error(LOKI_ERR_UNSUPPORTED, "nbins + wmax too large for pruning");
-  if (smem > 48 * 1024 &&
-      (cplx ? (shape.circ ? set_smem_limit(bj_circ_score_complex_kernel, smem)
+  if ((cplx ? (shape.circ ? set_smem_limit(bj_circ_score_complex_kernel, smem)
                           : set_smem_limit(bj_score_complex_kernel, smem))
             : shape.circ ? set_smem_limit(bj_circ_score_kernel, smem)
-                         : set_smem_limit(bj_score_kernel, smem)) != cudaSuccess)
+                         : set_smem_limit(bj_score_kernel, smem)) != cudaSuccess ||
+      (cplx && (shape.circ ? set_smem_limit(bj_circ_emit_complex_kernel, smem_emit)
+                           : set_smem_limit(bj_emit_complex_kernel, smem_emit)) != cudaSuccess))
     return set_error(LOKI_ERR_CUDA, "cudaFuncSetAttribute failed");
   int dev = 0, nsm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -3909,92 +4323,84 @@ static int batch_enqueue(void* dev_scratch, int32_t njobs, int32_t nlevels,
   T.seg_idx = reinterpret_cast<const int32_t*>(base + o_si);
   T.thr = reinterpret_cast<const double*>(base + o_th);
   T.nlevels = nlevels;
-  // Per-job grids. The jobs' sizes differ from level to level, so every job
-  // gets enough blocks for several times an even share of the GPU: blocks
-  // past a job's work retire at once, and the block scheduler spreads the
-  // busy jobs' blocks over the whole GPU.
-  auto per_job = [&](int64_t waves_blocks, int64_t cap_blocks) {
-    return (unsigned)std::max<int64_t>(
-        1, std::min<int64_t>(cap_blocks, (waves_blocks + njobs - 1) / njobs));
-  };
+  // Wide kernels: one block per resident slot (see JobQueue), no more than the
+  // largest workspace has tiles. Per-job kernels: one block a job.
   const int64_t max_par = shape.max_par, max_child = shape.max_child;
-  const int64_t spread = std::min<int64_t>(njobs, 16);
-  const unsigned g_par = per_job(8 * nsm * spread, (max_par + 255) / 256);
-  const unsigned g_scan_p = per_job(2 * nsm, (max_par + 1 + kScanBlock - 1) / kScanBlock);
-  const unsigned g_scan_c = per_job(2 * nsm, (max_child + kScanBlock - 1) / kScanBlock);
-  const unsigned g_score =
-      per_job(6 * nsm * spread, (max_child + kPruneWarps * 32 - 1) / (kPruneWarps * 32));
-  const unsigned g_flat = per_job(8 * nsm, (max_child + 255) / 256);
-  const unsigned g_emit =
-      per_job(6 * nsm * spread, (max_par + kPruneWarps * 32 - 1) / (kPruneWarps * 32));
-  const int row_bt = P + 2, row_leaf = (P + 2) * 2;
-  int l_cur = 1;
-  auto scan = [&](int mode, unsigned g) {
-    if (mode == 0 || mode == 2) {
-      bj_scan_block_kernel<false><<<dim3(g, njobs), kScanBlock, 0, s>>>(T, l_cur, mode);
-      bj_scan_sums_kernel<false><<<dim3(1, njobs), kScanBlock, 0, s>>>(T, l_cur, mode);
-      bj_scan_add_kernel<false><<<dim3(g, njobs), kScanBlock, 0, s>>>(T, l_cur, mode);
-    } else {
-      bj_scan_block_kernel<true><<<dim3(g, njobs), kScanBlock, 0, s>>>(T, l_cur, mode);
-      bj_scan_sums_kernel<true><<<dim3(1, njobs), kScanBlock, 0, s>>>(T, l_cur, mode);
-      bj_scan_add_kernel<true><<<dim3(g, njobs), kScanBlock, 0, s>>>(T, l_cur, mode);
-    }
+  auto wide = [&](const void* kern, int bytes, int64_t items, int nj, unsigned* g) {
+    int per = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kTile, bytes) != cudaSuccess)
+      return set_error(LOKI_ERR_CUDA, "occupancy query failed");
+    *g = (unsigned)std::max<int64_t>(
+        1, std::min<int64_t>((int64_t)nsm * std::max(1, per), (items + kTile - 1) / kTile * nj));
+    return (int)LOKI_OK;
   };
+  const void* k_branch = shape.circ ? (const void*)bj_circ_branch_kernel
+                                    : (const void*)bj_branch_kernel;
+  const void* k_score = shape.circ ? (cplx ? (const void*)bj_circ_score_complex_kernel
+                                           : (const void*)bj_circ_score_kernel)
+                                   : (cplx ? (const void*)bj_score_complex_kernel
+                                           : (const void*)bj_score_kernel);
+  const void* k_emit = shape.circ ? (cplx ? (const void*)bj_circ_emit_complex_kernel
+                                          : (const void*)bj_circ_emit_kernel)
+                                  : (cplx ? (const void*)bj_emit_complex_kernel
+                                          : (const void*)bj_emit_kernel);
   note_launch();
   bj_seed_kernel<<<(unsigned)njobs, 1, 0, s>>>(T);
+  unsigned g_branch = 1, g_map = 1, g_score = 1, g_emit = 1;
+  const int nj_max = std::min<int>(njobs, kQueueJobs);
+  if (int rc = wide(k_branch, 0, max_par, nj_max, &g_branch)) return rc;
+  if (shape.circ)
+    if (int rc = wide((const void*)bj_circ_map_kernel, 0, max_par, nj_max, &g_map)) return rc;
+  if (int rc = wide(k_score, smem, max_child, nj_max, &g_score)) return rc;
+  if (int rc = wide(k_emit, smem_emit, max_par, nj_max, &g_emit)) return rc;
   for (int l = 1; l <= nlevels; ++l) {
-    l_cur = l;
-    if (shape.circ) {
-      // circ_level_dev's steps for every job at once
-      for (int i = 0; i < 21; ++i) note_launch();
-      bj_circ_branch_kernel<<<dim3(g_par, njobs), 256, 0, s>>>(T, l);
-      scan(0, g_scan_p);
-      scan(2, g_scan_p);
-      bj_circ_map_kernel<<<dim3(g_par, njobs), 256, 0, s>>>(T, l, batch_size);
-      scan(3, g_scan_c);
-      bj_scatter_kernel<<<dim3(g_flat, njobs), 256, 0, s>>>(T, l, 3);
-      bj_circ_clear_kernel<<<dim3(g_par, njobs), 256, 0, s>>>(T, batch_size);
-      if (ev_score) cudaEventRecord(ev_score[2 * (l - 1)], s);
-      if (cplx)
-        bj_circ_score_complex_kernel<<<dim3(g_score, njobs), kPruneWarps * 32, smem, s>>>(
-            T, l, sp, batch_size);
-      else
-        bj_circ_score_kernel<<<dim3(g_score, njobs), kPruneWarps * 32, smem, s>>>(T, l, sp, SK,
-                                                                                 batch_size);
-      if (ev_score) cudaEventRecord(ev_score[2 * (l - 1) + 1], s);
-      bj_circ_boff_kernel<<<dim3(g_par, njobs), 256, 0, s>>>(T);
-      scan(4, g_scan_c);
-      bj_scatter_kernel<<<dim3(g_flat, njobs), 256, 0, s>>>(T, l, 4);
-      bj_overflow_kernel<<<(unsigned)njobs, kSelThreads, 0, s>>>(T, l, max_sugg, batch_size,
-                                                                 1);
-      if (cplx)
-        bj_circ_emit_complex_kernel<<<dim3(g_emit, njobs), kPruneWarps * 32, 0, s>>>(
-            T, l, batch_size);
-      else
-        bj_circ_emit_kernel<<<dim3(g_emit, njobs), kPruneWarps * 32, 0, s>>>(T, l, batch_size);
-    } else {
-      for (int i = 0; i < 11; ++i) note_launch();
-      bj_branch_kernel<<<dim3(g_par, njobs), 256, 0, s>>>(T, l);
-      scan(0, g_scan_p);
-      if (ev_score) cudaEventRecord(ev_score[2 * (l - 1)], s);
-      if (cplx)
-        bj_score_complex_kernel<<<dim3(g_score, njobs), kPruneWarps * 32, smem, s>>>(T, l, sp);
-      else
-        bj_score_kernel<<<dim3(g_score, njobs), kPruneWarps * 32, smem, s>>>(T, l, sp, SK);
-      if (ev_score) cudaEventRecord(ev_score[2 * (l - 1) + 1], s);
-      scan(1, g_scan_c);
-      bj_scatter_kernel<<<dim3(g_flat, njobs), 256, 0, s>>>(T, l, 1);
-      bj_overflow_kernel<<<(unsigned)njobs, kSelThreads, 0, s>>>(T, l, max_sugg, batch_size,
-                                                                 0);
-      if (cplx)
-        bj_emit_complex_kernel<<<dim3(g_emit, njobs), kPruneWarps * 32, 0, s>>>(T, l);
-      else
-        bj_emit_kernel<<<dim3(g_emit, njobs), kPruneWarps * 32, 0, s>>>(T, l);
+    // steps of the level for every job at once, kQueueJobs jobs a launch; the
+    // score launches come together so that their time can be taken
+    for (int step = 0; step < 7; ++step) {
+      if (step == 4 && ev_score) cudaEventRecord(ev_score[2 * (l - 1)], s);
+      if (step == 5 && ev_score) cudaEventRecord(ev_score[2 * (l - 1) + 1], s);
+      if (!shape.circ && (step == 2 || step == 3)) continue;
+      for (int j0 = 0; j0 < njobs; j0 += kQueueJobs) {
+        const int nj = std::min(kQueueJobs, njobs - j0);
+        note_launch();
+        switch (step) {
+          case 0:
+            if (shape.circ) bj_circ_branch_kernel<<<g_branch, kTile, 0, s>>>(T, l, j0, nj);
+            else bj_branch_kernel<<<g_branch, kTile, 0, s>>>(T, l, j0, nj);
+            break;
+          case 1:
+            bj_scan_kernel<<<(unsigned)nj, kJobThreads, 0, s>>>(T, l, j0, shape.circ, batch_size);
+            break;
+          case 2: bj_circ_map_kernel<<<g_map, kTile, 0, s>>>(T, l, j0, nj, batch_size); break;
+          case 3: bj_circ_valid_kernel<<<(unsigned)nj, kJobThreads, 0, s>>>(T, l, j0); break;
+          case 4:
+            if (shape.circ && cplx)
+              bj_circ_score_complex_kernel<<<g_score, kTile, smem, s>>>(T, l, j0, nj, sp, SK,
+                                                                        batch_size, nb);
+            else if (shape.circ)
+              bj_circ_score_kernel<<<g_score, kTile, smem, s>>>(T, l, j0, nj, sp, SK, batch_size);
+            else if (cplx)
+              bj_score_complex_kernel<<<g_score, kTile, smem, s>>>(T, l, j0, nj, sp, SK, nb);
+            else
+              bj_score_kernel<<<g_score, kTile, smem, s>>>(T, l, j0, nj, sp, SK);
+            break;
+          case 5:
+            bj_select_kernel<<<(unsigned)nj, kJobThreads, 0, s>>>(T, l, j0, max_sugg, batch_size,
+                                                                  shape.circ);
+            break;
+          default:
+            if (shape.circ && cplx)
+              bj_circ_emit_complex_kernel<<<g_emit, kTile, smem_emit, s>>>(T, l, j0, nj,
+                                                                           batch_size, nb);
+            else if (shape.circ)
+              bj_circ_emit_kernel<<<g_emit, kTile, 0, s>>>(T, l, j0, nj, batch_size);
+            else if (cplx)
+              bj_emit_complex_kernel<<<g_emit, kTile, smem_emit, s>>>(T, l, j0, nj, nb);
+            else
+              bj_emit_kernel<<<g_emit, kTile, 0, s>>>(T, l, j0, nj);
+        }
+      }
     }
-    note_launch();
-    note_launch();
-    bj_bt_kernel<<<dim3(g_flat, njobs), 256, 0, s>>>(T, l, row_bt);
-    bj_best_kernel<<<(unsigned)njobs, 1024, 0, s>>>(T, l, row_leaf);
     int rc = check_launch("prune_run_batch");
     if (rc) return rc;
   }
@@ -4128,7 +4534,7 @@ prune_ascend_batch_kernel(const LokiAscendJob* __restrict__ jobs, int nseg, Loki
 // The same over complex trees (folds and segment strides in float2 units).
 __global__ void __launch_bounds__(kPruneWarps * 32)
 prune_ascend_batch_complex_kernel(const LokiAscendJob* __restrict__ jobs, int nseg,
-                                  LokiScoreSpec sp) {
+                                  LokiScoreSpec sp, ScoreK SK) {
   extern __shared__ float smem[];
   const LokiAscendJob& J = jobs[blockIdx.y];
   const LokiPruneLevel& D = J.lvl;
@@ -4146,7 +4552,7 @@ prune_ascend_batch_complex_kernel(const LokiAscendJob* __restrict__ jobs, int ns
        r += (int64_t)gridDim.x * blockDim.x)
     ascend_one_complex(D, J.leaves, reinterpret_cast<float2*>(J.folds), J.scores, J.scores_ep,
                        nseg, J.tm_seg, J.dt_seg, J.seg_idx,
-                       reinterpret_cast<const float2*>(J.ffa_fold), J.seg_stride, sp, tw, comb,
+                       reinterpret_cast<const float2*>(J.ffa_fold), J.seg_stride, sp, SK, tw, comb,
                        trow, r);
 }
 
@@ -4225,7 +4631,7 @@ extern "C" int loki_prune_ascend_batch(const LokiAscendJob* jobs, int32_t njobs,
   note_launch();
   if (fourier)
     prune_ascend_batch_complex_kernel<<<dim3(bx, njobs), kPruneWarps * 32, smem, s>>>(
-        reinterpret_cast<const LokiAscendJob*>(dev_scratch), nseg, sp);
+        reinterpret_cast<const LokiAscendJob*>(dev_scratch), nseg, sp, SK);
   else
     prune_ascend_batch_kernel<<<dim3(bx, njobs), kPruneWarps * 32, smem, s>>>(
         reinterpret_cast<const LokiAscendJob*>(dev_scratch), nseg, sp, SK);
@@ -4293,7 +4699,7 @@ prune_seed_batch_kernel(const LokiSeedJob* __restrict__ jobs, int nb, int P, Lok
       float s;
       float* row = tile + lane * stride;
       if (SK.pow2_64) score_row64_pow2(row, sp, SK, &s);
-      else score_row(row, nb, sp, &s);
+      else score_row(row, nb, sp, SK, &s);
       J.scores_out[p0 + lane] = s;
       J.scores_ep_out[p0 + lane] = s;
       J.seed_scores_out[p0 + lane] = s;

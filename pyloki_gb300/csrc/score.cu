@@ -53,7 +53,7 @@ score_kernel(const float* __restrict__ in, int64_t nprof, int nb, LokiScoreSpec 
     const int nout = sp.mode == 0 ? sp.nwidths : 1;
     float* row = tile + lane * stride;
     if (SK.pow2_64) score_row64_pow2(row, sp, SK, out + (size_t)(p0 + lane) * nout);
-    else score_row(row, nb, sp, out + (size_t)(p0 + lane) * nout);
+    else score_row(row, nb, sp, SK, out + (size_t)(p0 + lane) * nout);
   }
 }
 

@@ -25,7 +25,15 @@ __host__ __device__ __forceinline__ int score_stride(int nbins, int wmax) {
 // Circular prefix sum of length nbins + wmax, in place (scoring.py:42-71).
 __device__ __forceinline__ float prefix_row(float* row, int nbins, int wmax) {
   float s = row[0];
-  for (int i = 1; i < nbins; ++i) {
+  int i = 1;
+  for (; i + 8 <= nbins; i += 8) {  // eight loads ahead of the eight stores
+    float x[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) x[k] = row[i + k];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) row[i + k] = s = __fadd_rn(s, x[k]);
+  }
+  for (; i < nbins; ++i) {
     s = __fadd_rn(s, row[i]);
     row[i] = s;
   }
@@ -222,10 +230,13 @@ __device__ __forceinline__ void score_row64_pow2(const float* row, const LokiSco
 // Score the row owned by this lane. mode 0 writes nwidths values at out,
 // mode 1 writes the max over widths at out[0].
 __device__ __forceinline__ void score_row(float* row, int nbins, const LokiScoreSpec& sp,
-                                          float* out) {
+                                          const ScoreK& K, float* out) {
   const float total = prefix_row(row, nbins, sp.wmax);
-  // (generic path: any nbins and width list, prefix in shared memory)
+  // (generic path: any nbins and width list, prefix in shared memory). With
+  // stdnoise 1 the S/N is snr_fast's float, the rounding of the same float64
+  // chain; the largest float is then the rounding of the largest float64.
   double best = -(double)FLT_MAX;
+  float best_f = -FLT_MAX;
   for (int w0 = 0; w0 < sp.nwidths; w0 += 4) {
     int w[4];
     float m[4];
@@ -236,6 +247,13 @@ __device__ __forceinline__ void score_row(float* row, int nbins, const LokiScore
     for (int q = 0; q < 4; ++q) {
       const int iw = w0 + q;
       if (iw >= sp.nwidths) break;
+      if (K.inv_one) {
+        const float f = snr_fast(m[q], total, K.hb_hi[iw], K.hb_lo[iw], K.b_hi[iw], K.b_lo[iw],
+                                 sp.hb[iw], sp.b[iw]);
+        if (sp.mode == 0) out[iw] = f;
+        else if (f > best_f) best_f = f;
+        continue;
+      }
       // S/N of one width (scoring.py:131-138)
       const double s = __dmul_rn(__dsub_rn(__dmul_rn(sp.hb[iw], (double)m[q]),
                                            __dmul_rn(sp.b[iw], (double)total)),
@@ -244,7 +262,7 @@ __device__ __forceinline__ void score_row(float* row, int nbins, const LokiScore
       else if (s > best) best = s;
     }
   }
-  if (sp.mode != 0) out[0] = __double2float_rn(best);
+  if (sp.mode != 0) out[0] = K.inv_one ? best_f : __double2float_rn(best);
 }
 
 }  // namespace loki

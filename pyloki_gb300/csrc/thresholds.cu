@@ -54,7 +54,7 @@ sim_score_kernel(const float* __restrict__ in, const int64_t* __restrict__ src_r
   if (lane < kmax) {
     float* row = tile + lane * stride;
     if (SK.pow2_64) score_row64_pow2(row, sp, SK, scores + r0 + lane);
-    else score_row(row, nb, sp, scores + r0 + lane);
+    else score_row(row, nb, sp, SK, scores + r0 + lane);
   }
 }
 
