@@ -207,6 +207,14 @@ __device__ __forceinline__ int64_t axis_index(double v, double vmin, double inv,
   return idx;
 }
 
+// The tree's order as a constant where the kernel has one (KP > 0): the loops
+// over it unroll and a child's parameters stay in registers instead of local
+// memory.
+template <int KP>
+__device__ __forceinline__ int tree_order(const LokiPruneLevel& D) {
+  return KP > 0 ? KP : D.poly_order;
+}
+
 // Child leaf parameters [d_P .. d_1] from the parent's branching info.
 __device__ __forceinline__ void child_params(const LokiBranchInfo& B, int P, int64_t local,
                                              double* pv) {
@@ -248,9 +256,10 @@ __device__ __forceinline__ void cheby_low3(const LokiPruneLevel& D, const double
 // Chebyshev resolve (core/chebyshev.py:180-277): shift the coefficients to
 // t_add (and t_init on the moving grid) at the current scale, then read the
 // Taylor accel / velocity / delay there.
-__device__ __forceinline__ void cheby_kinematics(const LokiPruneLevel& D, const double* pv,
-                                                 double* accel, double* vel, double* dd) {
-  const int m = D.poly_order + 1;
+__device__ __forceinline__ void cheby_kinematics(const LokiPruneLevel& D, int P,
+                                                 const double* pv, double* accel, double* vel,
+                                                 double* dd) {
+  const int m = P + 1;
   double a[LOKI_MAX_PARAMS + 1];
   for (int i = 0; i < m; ++i) a[i] = tdot(pv, D.tm_a, i, m);
   double a2, a1, a0;
@@ -270,12 +279,12 @@ __device__ __forceinline__ void cheby_kinematics(const LokiPruneLevel& D, const 
 
 // poly_taylor_resolve_batch (moving) / poly_taylor_fixed_resolve_batch
 // (core/taylor.py:172-277) for one child with params pv[0..P] (d_P..d_1, d_0).
-__device__ __forceinline__ ChildRes resolve_child(const LokiPruneLevel& D, const double* pv,
-                                                  double f0) {
-  const int P = D.poly_order, m = P + 1;
+__device__ __forceinline__ ChildRes resolve_child(const LokiPruneLevel& D, int P,
+                                                  const double* pv, double f0) {
+  const int m = P + 1;
   double accel, vel, dd;
   if (D.basis == 1) {
-    cheby_kinematics(D, pv, &accel, &vel, &dd);
+    cheby_kinematics(D, P, pv, &accel, &vel, &dd);
   } else if (D.moving) {
     accel = tdot(pv, D.tm_a, P - 2, m);
     vel = __dsub_rn(tdot(pv, D.tm_a, P - 1, m), tdot(pv, D.tm_i, P - 1, m));
@@ -300,13 +309,14 @@ __device__ __forceinline__ ChildRes resolve_child(const LokiPruneLevel& D, const
 
 // Parent i: per-parameter child counts, steps and first values (info[i]) and
 // its child count (counts[i]).
+template <int KP = 0>
 __device__ __forceinline__ void branch_one(const LokiPruneLevel& D,
                                            const double* __restrict__ leaves, int64_t i,
                                            LokiBranchInfo* __restrict__ info,
                                            int64_t* __restrict__ counts,
                                            int32_t* __restrict__ err,
                                            const uint8_t* __restrict__ mask) {
-  const int P = D.poly_order, m = P + 1;
+  const int P = tree_order<KP>(D), m = P + 1;
   const double* lf = leaves + i * (P + 2) * 2;
   const double f0 = lf[(P + 1) * 2];
   const double fscale = __ddiv_rn(f0, LOKI_C_VAL);
@@ -544,7 +554,9 @@ __device__ __forceinline__ void score_tile_rows(float* tile, int stride, int nb,
 }
 
 // Children c0 .. c0 + 31 (those below n_children) of one warp.
-__device__ __forceinline__ void score_tile(const LokiPruneLevel& D, const double* __restrict__ leaves,
+template <int KP = 0>
+__device__ __forceinline__ void score_tile(
+                   const LokiPruneLevel& D, const double* __restrict__ leaves,
                    const float* __restrict__ folds, int64_t n_parents,
                    const LokiBranchInfo* __restrict__ info, const int64_t* __restrict__ offsets,
                    int64_t n_children, const float* __restrict__ seg, const LokiScoreSpec& sp,
@@ -552,7 +564,7 @@ __device__ __forceinline__ void score_tile(const LokiPruneLevel& D, const double
                    double* __restrict__ cphase, unsigned* __restrict__ minmax_keys,
                    float* tile, int64_t c0) {
   const int lane = threadIdx.x & 31;
-  const int nb = D.nbins, P = D.poly_order;
+  const int nb = D.nbins, P = tree_order<KP>(D);
   const int stride = score_stride(nb, sp.wmax);
   const int kmax = (int)std::min<int64_t>(32, n_children - c0);
   // lane k resolves child c0 + k
@@ -565,7 +577,7 @@ __device__ __forceinline__ void score_tile(const LokiPruneLevel& D, const double
     double pv[LOKI_MAX_PARAMS + 1];
     child_params(B, P, c - offsets[par], pv);
     pv[P] = B.d0;  // d_0 (alpha_0 in the current domain for Chebyshev)
-    const ChildRes r = resolve_child(D, pv, lf[(P + 1) * 2]);
+    const ChildRes r = resolve_child(D, P, pv, lf[(P + 1) * 2]);
     cidx[2 * c] = r.ia;
     cidx[2 * c + 1] = r.iff;
     cphase[c] = r.phase;
@@ -946,7 +958,9 @@ __device__ __forceinline__ void gather_add_rows(const float* __restrict__ folds,
 }
 
 // Survivors s0 .. s0 + 31 (those below n_surv) of one warp.
-__device__ __forceinline__ void emit_tile(const LokiPruneLevel& D, const double* __restrict__ leaves,
+template <int KP = 0>
+__device__ __forceinline__ void emit_tile(
+                  const LokiPruneLevel& D, const double* __restrict__ leaves,
                   const float* __restrict__ folds, const LokiBranchInfo* __restrict__ info,
                   const int64_t* __restrict__ offsets, int64_t n_parents,
                   const float* __restrict__ seg, const int64_t* __restrict__ surv,
@@ -956,7 +970,7 @@ __device__ __forceinline__ void emit_tile(const LokiPruneLevel& D, const double*
                   float* __restrict__ sout, float* __restrict__ seout,
                   int32_t* __restrict__ bout, int64_t s0, const EmitExtra& X = EmitExtra()) {
   const int lane = threadIdx.x & 31;
-  const int nb = D.nbins, P = D.poly_order, m = P + 1;
+  const int nb = D.nbins, P = tree_order<KP>(D), m = P + 1;
   const int kmax = (int)std::min<int64_t>(32, n_surv - s0);
   const int64_t my_c = surv[s0 + min(lane, kmax - 1)];
   int64_t my_par = warp_find_parents(offsets, n_parents, my_c, kmax), my_row = 0;
@@ -1807,7 +1821,7 @@ __device__ __forceinline__ void score_child_complex(
   double pv[LOKI_MAX_PARAMS + 1];
   child_params(B, P, c - offsets[par], pv);
   pv[P] = B.d0;
-  const ChildRes r = resolve_child(D, pv, lf[(P + 1) * 2]);
+  const ChildRes r = resolve_child(D, P, pv, lf[(P + 1) * 2]);
   cidx[2 * c] = r.ia;
   cidx[2 * c + 1] = r.iff;
   cphase[c] = r.phase;
@@ -1858,6 +1872,7 @@ struct EmitRow {
 // One survivor of the complex tree: transform and backtrack, its fold's rows
 // returned.
 
+template <int KP = 0>
 __device__ __forceinline__ EmitRow emit_one_complex_leaf(
     const LokiPruneLevel& D, const double* __restrict__ leaves,
     const LokiBranchInfo* __restrict__ info, const int64_t* __restrict__ offsets,
@@ -1865,7 +1880,7 @@ __device__ __forceinline__ EmitRow emit_one_complex_leaf(
     const int32_t* __restrict__ cidx, const double* __restrict__ cphase,
     double* __restrict__ lout, float* __restrict__ sout, float* __restrict__ seout,
     int32_t* __restrict__ bout, int64_t s, int64_t par, const EmitExtra& X = EmitExtra()) {
-  const int P = D.poly_order, m = P + 1;
+  const int P = tree_order<KP>(D), m = P + 1;
   const int64_t c = surv[s];
   const LokiBranchInfo B = info[par];
   const double* lf = leaves + par * (P + 2) * 2;
@@ -3579,6 +3594,14 @@ __global__ void bj_seed_kernel(BatchTabs T) {
 // instead, sized for the largest job, most blocks only read their job's
 // counters and left (60 us a level for 64 jobs in branch alone), and the
 // descriptor's lines were fetched one dependent load after another.
+// What every wide kernel of a batch takes beside its tables.
+struct LevelArgs {
+  LokiScoreSpec sp;
+  ScoreK SK;
+  int64_t batch;  // parents a batch (circular tree)
+  int nb;         // phase bins
+};
+
 constexpr int kQueueJobs = 256;
 constexpr int kTile = kPruneWarps * 32;  // parents, children or survivors a tile
 
@@ -3657,13 +3680,14 @@ __device__ __forceinline__ const void* job_segment(const BatchTabs& T, const Lok
          (int64_t)T.seg_idx[li] * J.seg_stride * bytes;
 }
 
-__global__ void __launch_bounds__(kTile) bj_branch_kernel(BatchTabs T, int l, int j0, int nj) {
+template <int KP>
+__global__ void __launch_bounds__(kTile) bj_branch_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   __shared__ JobQueue Q;
   queue_run(Q, T, l, j0, nj, kCntPar, [&](int job, int64_t tile) {
     const LokiPruneJob& J = T.jobs[job];
     const int64_t i = tile * kTile + threadIdx.x;
     if (i < J.run.counts[kCntPar])
-      branch_one(Q.lvl, J.run.trees[(l - 1) & 1].leaves, i,
+      branch_one<KP>(Q.lvl, J.run.trees[(l - 1) & 1].leaves, i,
                  reinterpret_cast<LokiBranchInfo*>(J.run.work.info), J.run.work.offsets,
                  J.dev_err, nullptr);
   });
@@ -3724,7 +3748,7 @@ __device__ __forceinline__ int64_t job_scan_counts(int64_t* a, int64_t n, int64_
 }
 
 // After branch: the children's offsets (and, circular tree, the expansions'),
-// their number and the level's record; the circular tree's batch flags cleared.
+// their number and the level's record; the circular tree's A.batch flags cleared.
 __global__ void __launch_bounds__(kJobThreads) bj_scan_kernel(BatchTabs T, int l, int j0,
                                                               int circ, int64_t batch) {
   __shared__ int64_t wsum[32];
@@ -3878,8 +3902,9 @@ bj_select_kernel(BatchTabs T, int l, int j0, int64_t max_sugg, int64_t batch, in
 
 // ---- score and emission ------------------------------------------------------
 
-__global__ void __launch_bounds__(kTile, 4)
-bj_score_kernel(BatchTabs T, int l, int j0, int nj, LokiScoreSpec sp, ScoreK SK) {
+template <int KP>
+__global__ void __launch_bounds__(kTile, 3)
+bj_score_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   extern __shared__ float tiles[];
   __shared__ JobQueue Q;
   const int warp = threadIdx.x >> 5;
@@ -3889,10 +3914,10 @@ bj_score_kernel(BatchTabs T, int l, int j0, int nj, LokiScoreSpec sp, ScoreK SK)
     const LokiPruneTree& in = J.run.trees[(l - 1) & 1];
     const int64_t n_child = J.run.counts[kCntChild], c0 = t * kTile + warp * 32;
     if (c0 >= n_child) return;
-    float* tile = tiles + (size_t)warp * 32 * score_stride(Q.lvl.nbins, sp.wmax);
-    score_tile(Q.lvl, in.leaves, in.folds, J.run.counts[kCntPar],
+    float* tile = tiles + (size_t)warp * 32 * score_stride(Q.lvl.nbins, A.sp.wmax);
+    score_tile<KP>(Q.lvl, in.leaves, in.folds, J.run.counts[kCntPar],
                reinterpret_cast<LokiBranchInfo*>(w.info), w.offsets, n_child,
-               static_cast<const float*>(job_segment(T, J, job, l, 4)), sp, SK, w.child_scores,
+               static_cast<const float*>(job_segment(T, J, job, l, 4)), A.sp, A.SK, w.child_scores,
                w.child_idx, w.child_phase, reinterpret_cast<unsigned*>(w.minmax), tile, c0);
     __syncwarp();
   });
@@ -3911,7 +3936,8 @@ __device__ __forceinline__ EmitExtra job_extra(const LokiPruneRun& R, int l, int
   return X;
 }
 
-__global__ void __launch_bounds__(kTile, 4) bj_emit_kernel(BatchTabs T, int l, int j0, int nj) {
+template <int KP>
+__global__ void __launch_bounds__(kTile, 4) bj_emit_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   __shared__ JobQueue Q;
   const int warp = threadIdx.x >> 5;
   queue_run(Q, T, l, j0, nj, kCntSurv, [&](int job, int64_t t) {
@@ -3921,7 +3947,7 @@ __global__ void __launch_bounds__(kTile, 4) bj_emit_kernel(BatchTabs T, int l, i
     const LokiPruneTree &in = R.trees[(l - 1) & 1], &out = R.trees[l & 1];
     const int64_t n_surv = R.counts[kCntSurv], s0 = t * kTile + warp * 32;
     if (s0 >= n_surv) return;
-    emit_tile(Q.lvl, in.leaves, in.folds, reinterpret_cast<LokiBranchInfo*>(w.info), w.offsets,
+    emit_tile<KP>(Q.lvl, in.leaves, in.folds, reinterpret_cast<LokiBranchInfo*>(w.info), w.offsets,
               R.counts[kCntOldPar], static_cast<const float*>(job_segment(T, J, job, l, 4)),
               w.surv, n_surv, w.child_scores, w.child_idx, w.child_phase, out.leaves, out.folds,
               out.scores, out.scores_ep, out.backtracks, s0, job_extra(R, l, Q.lvl.poly_order));
@@ -3938,14 +3964,15 @@ __host__ __device__ inline int cplx_smem_bytes(int nbins, int wmax, bool score) 
   return score ? (int)((2 * nbins + kPruneWarps * cplx_warp_floats(nbins, stride)) * 4) : 0;
 }
 
+template <int KP>
 __global__ void __launch_bounds__(kTile)
-bj_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LokiScoreSpec sp, ScoreK SK, int nb) {
+bj_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   extern __shared__ __align__(16) float smem[];
   __shared__ JobQueue Q;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int stride = score_stride(nb, sp.wmax), nbf = nb / 2 + 1;
-  if (nb == 64) load_twiddles64(reinterpret_cast<float2*>(smem));
-  else load_twiddles(smem, nb);
+  const int stride = score_stride(A.nb, A.sp.wmax), nbf = A.nb / 2 + 1;
+  if (A.nb == 64) load_twiddles64(reinterpret_cast<float2*>(smem));
+  else load_twiddles(smem, A.nb);
   queue_run(Q, T, l, j0, nj, kCntChild, [&](int job, int64_t t) {
     const LokiPruneJob& J = T.jobs[job];
     const LokiPruneWork& w = J.run.work;
@@ -3959,10 +3986,10 @@ bj_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LokiScoreSpec sp, Sc
     if (c0 >= n_child) return;
     const int kmax = (int)min((int64_t)32, n_child - c0);
     const LokiPruneLevel& D = Q.lvl;
-    if (nb != 64) {
-      float* wbase = smem + 2 * nb + (size_t)warp * cplx_warp_floats(nb, stride);
+    if (A.nb != 64) {
+      float* wbase = smem + 2 * A.nb + (size_t)warp * cplx_warp_floats(A.nb, stride);
       if (c < n_child)
-        score_child_complex(D, in.leaves, folds, n_par, info, w.offsets, seg, sp, SK,
+        score_child_complex(D, in.leaves, folds, n_par, info, w.offsets, seg, A.sp, A.SK,
                             w.child_scores, w.child_idx, w.child_phase, keys, smem,
                             reinterpret_cast<float2*>(wbase) + (size_t)lane * 2 * nbf,
                             wbase + (size_t)32 * 2 * nbf * 2 + lane * stride, c);
@@ -3972,12 +3999,12 @@ bj_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LokiScoreSpec sp, Sc
     int64_t row = 0;
     float2 delta = make_float2(1.0f, 0.0f);
     if (lane < kmax) {
-      const int P = D.poly_order;
+      const int P = tree_order<KP>(D);
       const LokiBranchInfo B = info[par];
       double pv[LOKI_MAX_PARAMS + 1];
       child_params(B, P, c - w.offsets[par], pv);
       pv[P] = B.d0;
-      const ChildRes r = resolve_child(D, pv, in.leaves[(par * (P + 2) + P + 1) * 2]);
+      const ChildRes r = resolve_child(D, P, pv, in.leaves[(par * (P + 2) + P + 1) * 2]);
       w.child_idx[2 * c] = r.ia;
       w.child_idx[2 * c + 1] = r.iff;
       w.child_phase[c] = r.phase;
@@ -3986,14 +4013,15 @@ bj_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LokiScoreSpec sp, Sc
     }
     const int wb = max(cplx64_warp_bytes(), 32 * stride * 4);
     cplx64_score(folds, seg, par, row, delta, kmax, reinterpret_cast<const float2*>(smem),
-                 reinterpret_cast<float2*>(reinterpret_cast<char*>(smem) + 512 + warp * wb), sp,
-                 SK, w.child_scores + c0, keys);
+                 reinterpret_cast<float2*>(reinterpret_cast<char*>(smem) + 512 + warp * wb), A.sp,
+                 A.SK, w.child_scores + c0, keys);
     __syncwarp();
   });
 }
 
+template <int KP>
 __global__ void __launch_bounds__(kTile, 4)
-bj_emit_complex_kernel(BatchTabs T, int l, int j0, int nj, int nb) {
+bj_emit_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   extern __shared__ __align__(16) float smem[];
   __shared__ JobQueue Q;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -4007,23 +4035,23 @@ bj_emit_complex_kernel(BatchTabs T, int l, int j0, int nj, int nb) {
     const float2* seg = static_cast<const float2*>(job_segment(T, J, job, l, 8));
     const int64_t n_surv = R.counts[kCntSurv], s0 = t * kTile + warp * 32, s = s0 + lane;
     if (s0 >= n_surv) return;
-    const int kmax = (int)min((int64_t)32, n_surv - s0), nbf = nb / 2 + 1;
+    const int kmax = (int)min((int64_t)32, n_surv - s0), nbf = A.nb / 2 + 1;
     const int64_t par = warp_find_parents(w.offsets, R.counts[kCntOldPar],
                                           w.surv[s0 + min(lane, kmax - 1)], kmax);
     EmitRow r = {0, 0, 0.0};
     if (lane < kmax)
-      r = emit_one_complex_leaf(Q.lvl, in.leaves, info, w.offsets, w.surv, w.child_scores,
+      r = emit_one_complex_leaf<KP>(Q.lvl, in.leaves, info, w.offsets, w.surv, w.child_scores,
                                 w.child_idx, w.child_phase, out.leaves, out.scores,
                                 out.scores_ep, out.backtracks, s, par,
                                 job_extra(R, l, Q.lvl.poly_order));
     float2* fout = reinterpret_cast<float2*>(out.folds);
-    if (nb == 64)
-      cplx64_emit(folds, seg, r.par, r.row, prune_phasor(r.phase, nb), kmax,
+    if (A.nb == 64)
+      cplx64_emit(folds, seg, r.par, r.row, prune_phasor(r.phase, A.nb), kmax,
                   reinterpret_cast<float2*>(reinterpret_cast<char*>(smem) + 512 +
                                             warp * cplx64_warp_bytes()),
                   fout + s0 * 66);
     else if (lane < kmax)
-      rotate_add(seg + r.row * 2 * nbf, folds + r.par * 2 * nbf, prune_phasor(r.phase, nb), nbf,
+      rotate_add(seg + r.row * 2 * nbf, folds + r.par * 2 * nbf, prune_phasor(r.phase, A.nb), nbf,
                  fout + s * 2 * nbf);
   });
 }
@@ -4031,7 +4059,7 @@ bj_emit_complex_kernel(BatchTabs T, int l, int j0, int nj, int nb) {
 // ---- circular-orbit tree -------------------------------------------------------
 
 __global__ void __launch_bounds__(kTile)
-bj_circ_branch_kernel(BatchTabs T, int l, int j0, int nj) {
+bj_circ_branch_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   __shared__ JobQueue Q;
   queue_run(Q, T, l, j0, nj, kCntPar, [&](int job, int64_t tile) {
     const LokiPruneJob& J = T.jobs[job];
@@ -4046,21 +4074,20 @@ bj_circ_branch_kernel(BatchTabs T, int l, int j0, int nj) {
 // the batch-ordered child map and validity flags (none of a level whose
 // children exceed the workspace)
 __global__ void __launch_bounds__(kTile)
-bj_circ_map_kernel(BatchTabs T, int l, int j0, int nj, int64_t batch) {
+bj_circ_map_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   __shared__ JobQueue Q;
   queue_run(Q, T, l, j0, nj, kCntPar, [&](int job, int64_t tile) {
     const LokiPruneRun& R = T.jobs[job].run;
     const int64_t i = tile * kTile + threadIdx.x, n = R.counts[kCntPar];
     if (i < n && R.counts[kCntChild] > 0)
-      circ_map_one(Q.lvl, R.trees[(l - 1) & 1].leaves, n, batch,
+      circ_map_one(Q.lvl, R.trees[(l - 1) & 1].leaves, n, A.batch,
                    reinterpret_cast<const LokiBranchInfo*>(R.work.info), R.work.offsets,
                    R.exp_off, reinterpret_cast<CircChild*>(R.child_map), R.valid_flags, i);
   });
 }
 
 __global__ void __launch_bounds__(kTile)
-bj_circ_score_kernel(BatchTabs T, int l, int j0, int nj, LokiScoreSpec sp, ScoreK SK,
-                     int64_t batch) {
+bj_circ_score_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   extern __shared__ float tiles[];
   __shared__ JobQueue Q;
   const int warp = threadIdx.x >> 5;
@@ -4071,19 +4098,19 @@ bj_circ_score_kernel(BatchTabs T, int l, int j0, int nj, LokiScoreSpec sp, Score
     const LokiPruneTree& in = R.trees[(l - 1) & 1];
     const int64_t n_valid = R.counts[kCntValid], v0 = t * kTile + warp * 32;
     if (v0 >= n_valid) return;
-    circ_score_tile(Q.lvl, in.leaves, in.folds, batch,
+    circ_score_tile(Q.lvl, in.leaves, in.folds, A.batch,
                     reinterpret_cast<const LokiBranchInfo*>(w.info),
                     reinterpret_cast<const CircChild*>(R.child_map), R.valid_ids, n_valid,
-                    static_cast<const float*>(job_segment(T, J, job, l, 4)), sp, SK,
+                    static_cast<const float*>(job_segment(T, J, job, l, 4)), A.sp, A.SK,
                     w.child_scores, w.child_idx, w.child_phase, R.child_class, R.batch_taylor,
                     reinterpret_cast<unsigned*>(w.minmax),
-                    tiles + (size_t)warp * 32 * score_stride(Q.lvl.nbins, sp.wmax), v0);
+                    tiles + (size_t)warp * 32 * score_stride(Q.lvl.nbins, A.sp.wmax), v0);
     __syncwarp();
   });
 }
 
 __global__ void __launch_bounds__(kTile)
-bj_circ_emit_kernel(BatchTabs T, int l, int j0, int nj, int64_t batch) {
+bj_circ_emit_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   __shared__ JobQueue Q;
   const int warp = threadIdx.x >> 5;
   queue_run(Q, T, l, j0, nj, kCntSurv, [&](int job, int64_t t) {
@@ -4093,7 +4120,7 @@ bj_circ_emit_kernel(BatchTabs T, int l, int j0, int nj, int64_t batch) {
     const LokiPruneTree &in = R.trees[(l - 1) & 1], &out = R.trees[l & 1];
     const int64_t n_surv = R.counts[kCntSurv], s0 = t * kTile + warp * 32;
     if (s0 >= n_surv) return;
-    circ_emit_tile(Q.lvl, in.leaves, in.folds, batch,
+    circ_emit_tile(Q.lvl, in.leaves, in.folds, A.batch,
                    reinterpret_cast<const LokiBranchInfo*>(w.info),
                    reinterpret_cast<const CircChild*>(R.child_map), R.valid_ids,
                    static_cast<const float*>(job_segment(T, J, job, l, 4)), w.surv, n_surv,
@@ -4104,14 +4131,13 @@ bj_circ_emit_kernel(BatchTabs T, int l, int j0, int nj, int64_t batch) {
 }
 
 __global__ void __launch_bounds__(kTile)
-bj_circ_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LokiScoreSpec sp, ScoreK SK,
-                             int64_t batch, int nb) {
+bj_circ_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   extern __shared__ __align__(16) float smem[];
   __shared__ JobQueue Q;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int stride = score_stride(nb, sp.wmax), nbf = nb / 2 + 1;
-  if (nb == 64) load_twiddles64(reinterpret_cast<float2*>(smem));
-  else load_twiddles(smem, nb);
+  const int stride = score_stride(A.nb, A.sp.wmax), nbf = A.nb / 2 + 1;
+  if (A.nb == 64) load_twiddles64(reinterpret_cast<float2*>(smem));
+  else load_twiddles(smem, A.nb);
   queue_run(Q, T, l, j0, nj, kCntValid, [&](int job, int64_t t) {
     const LokiPruneJob& J = T.jobs[job];
     const LokiPruneRun& R = J.run;
@@ -4126,10 +4152,10 @@ bj_circ_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LokiScoreSpec s
     if (v0 >= n_valid) return;
     const int kmax = (int)min((int64_t)32, n_valid - v0);
     const LokiPruneLevel& D = Q.lvl;
-    if (nb != 64) {
-      float* wbase = smem + 2 * nb + (size_t)warp * cplx_warp_floats(nb, stride);
+    if (A.nb != 64) {
+      float* wbase = smem + 2 * A.nb + (size_t)warp * cplx_warp_floats(A.nb, stride);
       if (v < n_valid)
-        circ_score_one_complex(D, in.leaves, folds, batch, info, map, R.valid_ids, seg, sp, SK,
+        circ_score_one_complex(D, in.leaves, folds, A.batch, info, map, R.valid_ids, seg, A.sp, A.SK,
                                smem, reinterpret_cast<float2*>(wbase) + (size_t)lane * 2 * nbf,
                                wbase + (size_t)32 * 2 * nbf * 2 + lane * stride, w.child_scores,
                                w.child_idx, w.child_phase, R.child_class, R.batch_taylor, keys,
@@ -4146,7 +4172,7 @@ bj_circ_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LokiScoreSpec s
       circ_child(I, lf, ch, pv, ev);
       ChildRes r;
       const int cls = circ_resolve(D, pv, ev, lf[12], &r);
-      if (cls == 0) atomicOr(R.batch_taylor + ch.parent / batch, 1);
+      if (cls == 0) atomicOr(R.batch_taylor + ch.parent / A.batch, 1);
       w.child_idx[2 * v] = r.ia;
       w.child_idx[2 * v + 1] = r.iff;
       w.child_phase[v] = r.phase;
@@ -4157,14 +4183,14 @@ bj_circ_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LokiScoreSpec s
     }
     const int wb = max(cplx64_warp_bytes(), 32 * stride * 4);
     cplx64_score(folds, seg, par, row, delta, kmax, reinterpret_cast<const float2*>(smem),
-                 reinterpret_cast<float2*>(reinterpret_cast<char*>(smem) + 512 + warp * wb), sp,
-                 SK, w.child_scores + v0, keys);
+                 reinterpret_cast<float2*>(reinterpret_cast<char*>(smem) + 512 + warp * wb), A.sp,
+                 A.SK, w.child_scores + v0, keys);
     __syncwarp();
   });
 }
 
 __global__ void __launch_bounds__(kTile)
-bj_circ_emit_complex_kernel(BatchTabs T, int l, int j0, int nj, int64_t batch, int nb) {
+bj_circ_emit_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   extern __shared__ __align__(16) float smem[];
   __shared__ JobQueue Q;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -4177,10 +4203,10 @@ bj_circ_emit_complex_kernel(BatchTabs T, int l, int j0, int nj, int64_t batch, i
     const float2* seg = static_cast<const float2*>(job_segment(T, J, job, l, 8));
     const int64_t n_surv = R.counts[kCntSurv], s0 = t * kTile + warp * 32, s = s0 + lane;
     if (s0 >= n_surv) return;
-    const int kmax = (int)min((int64_t)32, n_surv - s0), nbf = nb / 2 + 1;
+    const int kmax = (int)min((int64_t)32, n_surv - s0), nbf = A.nb / 2 + 1;
     EmitRow r = {0, 0, 0.0};
     if (lane < kmax)
-      r = circ_emit_one_complex_leaf(Q.lvl, in.leaves, batch,
+      r = circ_emit_one_complex_leaf(Q.lvl, in.leaves, A.batch,
                                      reinterpret_cast<const LokiBranchInfo*>(w.info),
                                      reinterpret_cast<const CircChild*>(R.child_map),
                                      R.valid_ids, w.surv, w.child_scores, w.child_idx,
@@ -4188,15 +4214,39 @@ bj_circ_emit_complex_kernel(BatchTabs T, int l, int j0, int nj, int64_t batch, i
                                      out.scores, out.scores_ep, out.backtracks, s,
                                      job_extra(R, l, 5));
     float2* fout = reinterpret_cast<float2*>(out.folds);
-    if (nb == 64)
-      cplx64_emit(folds, seg, r.par, r.row, prune_phasor(r.phase, nb), kmax,
+    if (A.nb == 64)
+      cplx64_emit(folds, seg, r.par, r.row, prune_phasor(r.phase, A.nb), kmax,
                   reinterpret_cast<float2*>(reinterpret_cast<char*>(smem) + 512 +
                                             warp * cplx64_warp_bytes()),
                   fout + s0 * 66);
     else if (lane < kmax)
-      rotate_add(seg + r.row * 2 * nbf, folds + r.par * 2 * nbf, prune_phasor(r.phase, nb), nbf,
+      rotate_add(seg + r.row * 2 * nbf, folds + r.par * 2 * nbf, prune_phasor(r.phase, A.nb), nbf,
                  fout + s * 2 * nbf);
   });
+}
+
+// The wide kernels of a batch: of the circular tree, or of a polynomial tree whose
+// order is a constant in them (3 and 4, every configured search; KP 0: any).
+struct BatchKernels {
+  using Wide = void (*)(BatchTabs, int, int, int, LevelArgs);
+  Wide branch, map, score, emit;
+};
+
+template <int KP>
+BatchKernels tree_kernels(bool cplx) {
+  return {bj_branch_kernel<KP>, nullptr,
+          cplx ? bj_score_complex_kernel<KP> : bj_score_kernel<KP>,
+          cplx ? bj_emit_complex_kernel<KP> : bj_emit_kernel<KP>};
+}
+
+inline BatchKernels batch_kernels(bool circ, bool cplx, int order) {
+  if (circ)
+    return {bj_circ_branch_kernel, bj_circ_map_kernel,
+            cplx ? bj_circ_score_complex_kernel : bj_circ_score_kernel,
+            cplx ? bj_circ_emit_complex_kernel : bj_circ_emit_kernel};
+  return order == 3   ? tree_kernels<3>(cplx)
+         : order == 4 ? tree_kernels<4>(cplx)
+                      : tree_kernels<0>(cplx);
 }
 
 }  // namespace loki
@@ -4301,12 +4351,10 @@ static int batch_enqueue(void* dev_scratch, int32_t njobs, int32_t nlevels,
   const int smem_emit = cplx ? cplx_smem_bytes(nb, sp.wmax, false) : 0;
   if (smem > 200 * 1024)
     return set_error(LOKI_ERR_UNSUPPORTED, "nbins + wmax too large for pruning");
-  if ((cplx ? (shape.circ ? set_smem_limit(bj_circ_score_complex_kernel, smem)
-                          : set_smem_limit(bj_score_complex_kernel, smem))
-            : shape.circ ? set_smem_limit(bj_circ_score_kernel, smem)
-                         : set_smem_limit(bj_score_kernel, smem)) != cudaSuccess ||
-      (cplx && (shape.circ ? set_smem_limit(bj_circ_emit_complex_kernel, smem_emit)
-                           : set_smem_limit(bj_emit_complex_kernel, smem_emit)) != cudaSuccess))
+  const BatchKernels K = batch_kernels(shape.circ, cplx, shape.poly_order);
+  const LevelArgs A = {sp, SK, batch_size, nb};
+  if (set_smem_limit(K.score, smem) != cudaSuccess ||
+      set_smem_limit(K.emit, smem_emit) != cudaSuccess)
     return set_error(LOKI_ERR_CUDA, "cudaFuncSetAttribute failed");
   int dev = 0, nsm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -4326,33 +4374,23 @@ static int batch_enqueue(void* dev_scratch, int32_t njobs, int32_t nlevels,
   // Wide kernels: one block per resident slot (see JobQueue), no more than the
   // largest workspace has tiles. Per-job kernels: one block a job.
   const int64_t max_par = shape.max_par, max_child = shape.max_child;
-  auto wide = [&](const void* kern, int bytes, int64_t items, int nj, unsigned* g) {
+  const int nj_max = std::min<int>(njobs, kQueueJobs);
+  auto wide = [&](BatchKernels::Wide kern, int bytes, int64_t items, unsigned* g) {
     int per = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kTile, bytes) != cudaSuccess)
       return set_error(LOKI_ERR_CUDA, "occupancy query failed");
-    *g = (unsigned)std::max<int64_t>(
-        1, std::min<int64_t>((int64_t)nsm * std::max(1, per), (items + kTile - 1) / kTile * nj));
+    *g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)nsm * std::max(1, per),
+                                                          (items + kTile - 1) / kTile * nj_max));
     return (int)LOKI_OK;
   };
-  const void* k_branch = shape.circ ? (const void*)bj_circ_branch_kernel
-                                    : (const void*)bj_branch_kernel;
-  const void* k_score = shape.circ ? (cplx ? (const void*)bj_circ_score_complex_kernel
-                                           : (const void*)bj_circ_score_kernel)
-                                   : (cplx ? (const void*)bj_score_complex_kernel
-                                           : (const void*)bj_score_kernel);
-  const void* k_emit = shape.circ ? (cplx ? (const void*)bj_circ_emit_complex_kernel
-                                          : (const void*)bj_circ_emit_kernel)
-                                  : (cplx ? (const void*)bj_emit_complex_kernel
-                                          : (const void*)bj_emit_kernel);
+  unsigned g_branch = 1, g_map = 1, g_score = 1, g_emit = 1;
+  if (int rc = wide(K.branch, 0, max_par, &g_branch)) return rc;
+  if (shape.circ)
+    if (int rc = wide(K.map, 0, max_par, &g_map)) return rc;
+  if (int rc = wide(K.score, smem, max_child, &g_score)) return rc;
+  if (int rc = wide(K.emit, smem_emit, max_par, &g_emit)) return rc;
   note_launch();
   bj_seed_kernel<<<(unsigned)njobs, 1, 0, s>>>(T);
-  unsigned g_branch = 1, g_map = 1, g_score = 1, g_emit = 1;
-  const int nj_max = std::min<int>(njobs, kQueueJobs);
-  if (int rc = wide(k_branch, 0, max_par, nj_max, &g_branch)) return rc;
-  if (shape.circ)
-    if (int rc = wide((const void*)bj_circ_map_kernel, 0, max_par, nj_max, &g_map)) return rc;
-  if (int rc = wide(k_score, smem, max_child, nj_max, &g_score)) return rc;
-  if (int rc = wide(k_emit, smem_emit, max_par, nj_max, &g_emit)) return rc;
   for (int l = 1; l <= nlevels; ++l) {
     // steps of the level for every job at once, kQueueJobs jobs a launch; the
     // score launches come together so that their time can be taken
@@ -4364,40 +4402,18 @@ static int batch_enqueue(void* dev_scratch, int32_t njobs, int32_t nlevels,
         const int nj = std::min(kQueueJobs, njobs - j0);
         note_launch();
         switch (step) {
-          case 0:
-            if (shape.circ) bj_circ_branch_kernel<<<g_branch, kTile, 0, s>>>(T, l, j0, nj);
-            else bj_branch_kernel<<<g_branch, kTile, 0, s>>>(T, l, j0, nj);
-            break;
+          case 0: K.branch<<<g_branch, kTile, 0, s>>>(T, l, j0, nj, A); break;
           case 1:
             bj_scan_kernel<<<(unsigned)nj, kJobThreads, 0, s>>>(T, l, j0, shape.circ, batch_size);
             break;
-          case 2: bj_circ_map_kernel<<<g_map, kTile, 0, s>>>(T, l, j0, nj, batch_size); break;
+          case 2: K.map<<<g_map, kTile, 0, s>>>(T, l, j0, nj, A); break;
           case 3: bj_circ_valid_kernel<<<(unsigned)nj, kJobThreads, 0, s>>>(T, l, j0); break;
-          case 4:
-            if (shape.circ && cplx)
-              bj_circ_score_complex_kernel<<<g_score, kTile, smem, s>>>(T, l, j0, nj, sp, SK,
-                                                                        batch_size, nb);
-            else if (shape.circ)
-              bj_circ_score_kernel<<<g_score, kTile, smem, s>>>(T, l, j0, nj, sp, SK, batch_size);
-            else if (cplx)
-              bj_score_complex_kernel<<<g_score, kTile, smem, s>>>(T, l, j0, nj, sp, SK, nb);
-            else
-              bj_score_kernel<<<g_score, kTile, smem, s>>>(T, l, j0, nj, sp, SK);
-            break;
+          case 4: K.score<<<g_score, kTile, smem, s>>>(T, l, j0, nj, A); break;
           case 5:
             bj_select_kernel<<<(unsigned)nj, kJobThreads, 0, s>>>(T, l, j0, max_sugg, batch_size,
                                                                   shape.circ);
             break;
-          default:
-            if (shape.circ && cplx)
-              bj_circ_emit_complex_kernel<<<g_emit, kTile, smem_emit, s>>>(T, l, j0, nj,
-                                                                           batch_size, nb);
-            else if (shape.circ)
-              bj_circ_emit_kernel<<<g_emit, kTile, 0, s>>>(T, l, j0, nj, batch_size);
-            else if (cplx)
-              bj_emit_complex_kernel<<<g_emit, kTile, smem_emit, s>>>(T, l, j0, nj, nb);
-            else
-              bj_emit_kernel<<<g_emit, kTile, 0, s>>>(T, l, j0, nj);
+          default: K.emit<<<g_emit, kTile, smem_emit, s>>>(T, l, j0, nj, A);
         }
       }
     }
