@@ -307,6 +307,57 @@ __device__ __forceinline__ ChildRes resolve_child(const LokiPruneLevel& D, int P
 // branch
 // ---------------------------------------------------------------------------
 
+// The level's steps, factors and shift limit in float32, for branch_quick.
+struct BranchF {
+  float dfc[LOKI_MAX_PARAMS], fac[LOKI_MAX_PARAMS], eta;
+};
+
+__device__ __forceinline__ BranchF branch_floats(const LokiPruneLevel& D) {
+  BranchF F;
+  for (int j = 0; j < LOKI_MAX_PARAMS; ++j) {
+    F.dfc[j] = (float)D.dfc[j];
+    F.fac[j] = (float)D.fac[j];
+  }
+  F.eta = (float)D.eta_m;
+  return F;
+}
+
+// Whether parameter j (step dcur) splits, and into how many (*num), where
+// float32 settles what float64 decides: 1 or 0; -1 where it does not (a value
+// within the rounding of a limit or of a whole ratio, out of float32's range,
+// not positive, or beyond branch_max) and the float64 chain has to be run. Each
+// approximation is off by at most 10 roundings of 2^-24 (6e-7); the margins are
+// 2e-6 and more. The FP64 unit (16 clocks of the SM for an instruction of a warp)
+// was 73 % busy in the branch kernel, most of it with the divisions of the split
+// and the ratio, 9 to 13 a parent of order 4; what is left is one for each
+// parameter that splits into a count that is no power of two. 64 runs of 128
+// levels: 5.5 -> 2.8 ms; 16 of the circular tree: 4.0 -> 1.7.
+__device__ __forceinline__ int branch_quick(const BranchF& F, int j, float f0, float rf0,
+                                            double dcur, int64_t branch_max, int* num) {
+  const float dc = (float)dcur, dn = F.dfc[j] * rf0;
+  const float fb = F.fac[j] * f0 * (float)(1.0 / LOKI_C_VAL);
+  const float lo = 1e-30f, hi = 1e30f;
+  if (!(dc > lo && dc < hi && dn > lo && dn < hi && fb > lo && fb < hi && F.eta > 1e-20f &&
+        F.eta < 1e20f))
+    return -1;
+  const float shift = fabsf(dc - dn) * fb, err = (dc + dn) * fb * 2e-6f;
+  const float ratio = __fdividef(dc, dn), bm = (float)branch_max;
+  if (shift + err < F.eta * (1.0f - 2e-6f)) return ratio * (1.0f + 4e-6f) < bm ? 0 : -1;
+  if (!(shift - err > F.eta * (1.0f + 2e-6f)) || !(ratio < 1e5f)) return -1;
+  const float x = ratio - (float)LOKI_FLOAT_EPSILON, m = ratio * 4e-6f + 1e-9f;
+  const float c = ceilf(x - m);
+  if (c != ceilf(x + m) || c > bm) return -1;
+  *num = max((int)c, 1);
+  return 1;
+}
+
+// dcur / num: by a power of two exact scaling.
+__device__ __forceinline__ double branch_step(double dcur, int64_t num) {
+  return num == 1                 ? dcur
+         : (num & (num - 1)) == 0 ? __dmul_rn(dcur, 1.0 / (double)num)
+                                  : __ddiv_rn(dcur, (double)num);
+}
+
 // Parent i: per-parameter child counts, steps and first values (info[i]) and
 // its child count (counts[i]).
 template <int KP = 0>
@@ -315,11 +366,12 @@ __device__ __forceinline__ void branch_one(const LokiPruneLevel& D,
                                            LokiBranchInfo* __restrict__ info,
                                            int64_t* __restrict__ counts,
                                            int32_t* __restrict__ err,
-                                           const uint8_t* __restrict__ mask) {
+                                           const uint8_t* __restrict__ mask,
+                                           const BranchF& F) {
   const int P = tree_order<KP>(D), m = P + 1;
   const double* lf = leaves + i * (P + 2) * 2;
   const double f0 = lf[(P + 1) * 2];
-  const double fscale = __ddiv_rn(f0, LOKI_C_VAL);
+  const float f0f = (float)f0, rf0 = __frcp_rn(f0f);
   // Parent values and errors in the current domain: as stored (Taylor), or
   // shifted from the previous to the current Chebyshev domain with
   // shift_cheby_full (utils/transforms.py:650-701).
@@ -353,39 +405,40 @@ __device__ __forceinline__ void branch_one(const LokiPruneLevel& D,
   int64_t total = 1;
   for (int j = 0; j < P; ++j) {
     const double pcur = pval[j], dcur = perr[j];
-    const double dnew = __ddiv_rn(D.dfc[j], f0);
-    const double fb = __dmul_rn(D.fac[j], fscale);
-    const double shift = __dmul_rn(fabs(__dsub_rn(dcur, dnew)), fb);
-    const bool split = !(shift < D.eta_m);
-    int64_t num = 1;
-    double dact = dcur, first = pcur;
-    if (!(dcur > 0.0) || !(dnew > 0.0)) {
-      atomicOr(err, LOKI_DEVERR_BRANCH);
-    } else if (split || dcur > __dmul_rn(dnew, 0.5 * (double)D.branch_max)) {
-      // The child count is needed for a split, and for the reference's
-      // branch_max check of every parameter; a parameter that does not
-      // split and whose step is at most half of branch_max new steps cannot
-      // exceed branch_max (ratio <= branch_max / 2 up to rounding), so its
-      // division is skipped.
-      const double ratio = __ddiv_rn(dcur, dnew);
-      num = (int64_t)ceil(__dsub_rn(ratio, LOKI_FLOAT_EPSILON));
-      if (num < 1) num = 1;
-      if (num > D.branch_max) {
+    int quick_num = 1;
+    const int quick = branch_quick(F, j, f0f, rf0, dcur, D.branch_max, &quick_num);
+    bool split = quick > 0;
+    int64_t num = quick_num;
+    if (quick < 0) {
+      const double dnew = __ddiv_rn(D.dfc[j], f0);
+      const double fb = __dmul_rn(D.fac[j], __ddiv_rn(f0, LOKI_C_VAL));
+      const double shift = __dmul_rn(fabs(__dsub_rn(dcur, dnew)), fb);
+      split = !(shift < D.eta_m);
+      num = 1;
+      if (!(dcur > 0.0) || !(dnew > 0.0)) {
         atomicOr(err, LOKI_DEVERR_BRANCH);
-        num = D.branch_max;
-      }
-      if (split) {  // division by 1 or a power of two is exact scaling
-        dact = num == 1                ? dcur
-               : (num & (num - 1)) == 0 ? __dmul_rn(dcur, 1.0 / (double)num)
-                                        : __ddiv_rn(dcur, (double)num);
-        const double pmin = __dsub_rn(pcur, __dmul_rn(dcur, 0.5));
-        first = __dadd_rn(pmin, __dmul_rn(dact, 0.5));
+        split = false;
+      } else if (split || dcur > __dmul_rn(dnew, 0.5 * (double)D.branch_max)) {
+        // The child count is needed for a split, and for the reference's
+        // branch_max check of every parameter; a parameter that does not
+        // split and whose step is at most half of branch_max new steps cannot
+        // exceed branch_max (ratio <= branch_max / 2 up to rounding), so its
+        // division is skipped.
+        const double ratio = __ddiv_rn(dcur, dnew);
+        num = (int64_t)ceil(__dsub_rn(ratio, LOKI_FLOAT_EPSILON));
+        if (num < 1) num = 1;
+        if (num > D.branch_max) {
+          atomicOr(err, LOKI_DEVERR_BRANCH);
+          num = D.branch_max;
+        }
       }
     }
-    if (!split) {
+    double dact = dcur, first = pcur;
+    if (split) {
+      dact = branch_step(dcur, num);
+      first = __dadd_rn(__dsub_rn(pcur, __dmul_rn(dcur, 0.5)), __dmul_rn(dact, 0.5));
+    } else {
       num = 1;
-      dact = dcur;
-      first = pcur;
     }
     B.first[j] = first;
     B.dact[j] = dact;
@@ -404,7 +457,7 @@ __global__ void prune_branch_kernel(LokiPruneLevel D, const double* __restrict__
   if (n_dev) n = *n_dev;  // parent count held on the device
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
-  branch_one(D, leaves, i, info, counts, err, mask);
+  branch_one(D, leaves, i, info, counts, err, mask, branch_floats(D));
 }
 
 // ---------------------------------------------------------------------------
@@ -1308,7 +1361,7 @@ __device__ __forceinline__ void circ_branch_one(const LokiPruneLevel& D,
                                                 LokiBranchInfo* __restrict__ info,
                                                 int64_t* __restrict__ n_keep,
                                                 int64_t* __restrict__ n_exp,
-                                                int32_t* __restrict__ err);
+                                                int32_t* __restrict__ err, const BranchF& F);
 
 // n_dev, when not null, holds the parent count on the device (grid-stride).
 __global__ void circ_branch_kernel(LokiPruneLevel D, const double* __restrict__ leaves,
@@ -1319,11 +1372,11 @@ __global__ void circ_branch_kernel(LokiPruneLevel D, const double* __restrict__ 
     n = *n_dev;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
-      circ_branch_one(D, leaves, i, info, n_keep, n_exp, err);
+      circ_branch_one(D, leaves, i, info, n_keep, n_exp, err, branch_floats(D));
     return;
   }
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < n) circ_branch_one(D, leaves, i, info, n_keep, n_exp, err);
+  if (i < n) circ_branch_one(D, leaves, i, info, n_keep, n_exp, err, branch_floats(D));
 }
 
 __device__ __forceinline__ void circ_branch_one(const LokiPruneLevel& D,
@@ -1331,11 +1384,11 @@ __device__ __forceinline__ void circ_branch_one(const LokiPruneLevel& D,
                                                 LokiBranchInfo* __restrict__ info,
                                                 int64_t* __restrict__ n_keep,
                                                 int64_t* __restrict__ n_exp,
-                                                int32_t* __restrict__ err) {
+                                                int32_t* __restrict__ err, const BranchF& F) {
   const int P = 5;
   const double* lf = leaves + i * (P + 2) * 2;
   const double f0 = lf[(P + 1) * 2];
-  const double fscale = __ddiv_rn(f0, LOKI_C_VAL);
+  const float f0f = (float)f0, rf0 = __frcp_rn(f0f);
   LokiBranchInfo B;
   B.d0 = lf[2 * P];
   bool needs0 = false;
@@ -1343,36 +1396,41 @@ __device__ __forceinline__ void circ_branch_one(const LokiPruneLevel& D,
   int64_t total = 1;
   for (int j = 0; j < P; ++j) {
     const double pcur = lf[2 * j], dcur = lf[2 * j + 1];
-    const double dnew = __ddiv_rn(D.dfc[j], f0);
-    const double fb = __dmul_rn(D.fac[j], fscale);
-    const double shift = __dmul_rn(fabs(__dsub_rn(dcur, dnew)), fb);
-    const bool needs = shift >= D.eta_m;
-    int64_t num = 1;
-    double dact = dcur, first = pcur;
-    if (!(dcur > 0.0) || !(dnew > 0.0)) {
-      atomicOr(err, LOKI_DEVERR_BRANCH);
-    } else {
-      const double ratio = __ddiv_rn(dcur, dnew);
-      num = (int64_t)ceil(__dsub_rn(ratio, LOKI_FLOAT_EPSILON));
-      if (num < 1) num = 1;
-      if (num > D.branch_max) {
+    int quick_num = 1;
+    const int quick = branch_quick(F, j, f0f, rf0, dcur, D.branch_max, &quick_num);
+    bool needs = quick > 0;
+    int64_t num = quick_num;
+    if (quick < 0) {
+      const double dnew = __ddiv_rn(D.dfc[j], f0);
+      const double fb = __dmul_rn(D.fac[j], __ddiv_rn(f0, LOKI_C_VAL));
+      const double shift = __dmul_rn(fabs(__dsub_rn(dcur, dnew)), fb);
+      needs = shift >= D.eta_m;
+      num = 0;  // no step to split: an error, values kept
+      if (!(dcur > 0.0) || !(dnew > 0.0)) {
         atomicOr(err, LOKI_DEVERR_BRANCH);
-        num = D.branch_max;
+      } else {
+        const double ratio = __ddiv_rn(dcur, dnew);
+        num = (int64_t)ceil(__dsub_rn(ratio, LOKI_FLOAT_EPSILON));
+        if (num < 1) num = 1;
+        if (num > D.branch_max) {
+          atomicOr(err, LOKI_DEVERR_BRANCH);
+          num = D.branch_max;
+        }
       }
-      dact = __ddiv_rn(dcur, (double)num);
+    }
+    double dact = dcur, first = pcur;
+    if (needs && num > 0) {
+      dact = branch_step(dcur, num);
       first = __dadd_rn(__dsub_rn(pcur, __dmul_rn(dcur, 0.5)), __dmul_rn(dact, 0.5));
     }
+    if (num < 1) num = 1;
     if (j == 0) {  // crackle keeps the parent value; its step is the would-be child step
       needs0 = needs;
       num_c = num;
       first = pcur;
       num = 1;
     }
-    if (!needs) {
-      num = 1;
-      dact = dcur;
-      first = pcur;
-    }
+    if (!needs) num = 1;
     B.first[j] = first;
     B.dact[j] = dact;
     B.count[j] = (int32_t)num;
@@ -1383,13 +1441,14 @@ __device__ __forceinline__ void circ_branch_one(const LokiPruneLevel& D,
   const double sig = D.circ_sig_prop;
   int64_t keep = 0, exp = 0;
   double pv[LOKI_MAX_PARAMS + 1];
-  for (int64_t k = 0; k < total; ++k) {
+  if (!needs0) keep = total;  // none expands
+  for (int64_t k = 0; needs0 && k < total; ++k) {
     child_params(B, P, k, pv);
     const double snap = pv[1], jerk = pv[2], accel = pv[3];
     const bool snap_circ = fabs(snap) > __dmul_rn(sig, B.dact[1]) &&
                            fabs(accel) > __dmul_rn(sig, B.dact[3]) &&
                            __dmul_rn(-snap, accel) > 0.0;
-    const bool expand = !snap_circ && fabs(jerk) > __dmul_rn(sig, B.dact[2]) && needs0;
+    const bool expand = !snap_circ && fabs(jerk) > __dmul_rn(sig, B.dact[2]);
     if (expand) exp += num_c;
     else ++keep;
   }
@@ -3402,7 +3461,7 @@ prune_block_run_kernel(const LokiPruneJob* __restrict__ jobs,
     LokiPruneLevelStats* st = R.stats + (l - 1);
     // branch and the child offsets
     for (int64_t i = tid; i < n_par; i += blockDim.x)
-      branch_one(D, in.leaves, i, info, w.offsets, J.dev_err, nullptr);
+      branch_one(D, in.leaves, i, info, w.offsets, J.dev_err, nullptr, branch_floats(D));
     __syncthreads();
     const int64_t total = block_scan64<false>(w.offsets, n_par, 0.0, w.offsets, warp_tot);
     const int64_t n_child = total > w.child_cap ? 0 : total;
@@ -3607,6 +3666,7 @@ constexpr int kTile = kPruneWarps * 32;  // parents, children or survivors a til
 
 struct JobQueue {
   alignas(16) LokiPruneLevel lvl;
+  BranchF bf;
   int pre[kQueueJobs + 1];  // tiles before each job
 };
 
@@ -3655,6 +3715,8 @@ __device__ __forceinline__ int queue_job(JobQueue& Q, const BatchTabs& T, int j0
     uint64_t* dst = reinterpret_cast<uint64_t*>(&Q.lvl);
     for (int k = threadIdx.x; k < (int)(sizeof(LokiPruneLevel) / 8); k += blockDim.x)
       dst[k] = src[k];
+    if (threadIdx.x == 0)
+      Q.bf = branch_floats(T.levels[(size_t)(j0 + lo) * T.nlevels + (l - 1)]);
     __syncthreads();
   }
   return lo;
@@ -3681,15 +3743,16 @@ __device__ __forceinline__ const void* job_segment(const BatchTabs& T, const Lok
 }
 
 template <int KP>
-__global__ void __launch_bounds__(kTile) bj_branch_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
+__global__ void __launch_bounds__(kTile)
+bj_branch_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   __shared__ JobQueue Q;
   queue_run(Q, T, l, j0, nj, kCntPar, [&](int job, int64_t tile) {
     const LokiPruneJob& J = T.jobs[job];
     const int64_t i = tile * kTile + threadIdx.x;
     if (i < J.run.counts[kCntPar])
       branch_one<KP>(Q.lvl, J.run.trees[(l - 1) & 1].leaves, i,
-                 reinterpret_cast<LokiBranchInfo*>(J.run.work.info), J.run.work.offsets,
-                 J.dev_err, nullptr);
+                     reinterpret_cast<LokiBranchInfo*>(J.run.work.info), J.run.work.offsets,
+                     J.dev_err, nullptr, Q.bf);
   });
 }
 
@@ -3773,7 +3836,7 @@ __global__ void __launch_bounds__(kJobThreads) bj_scan_kernel(BatchTabs T, int l
 
 // Indices of the n values v with v >= thr, in order, to ids; returns how many.
 // *best: position among them of the largest, the first of equals (-1: none).
-__device__ __forceinline__ int64_t job_compact(const float* __restrict__ v, int64_t n, double thr,
+__device__ __forceinline__ int64_t job_compact(const float* __restrict__ v, int64_t n, float thr,
                                                int64_t* __restrict__ ids, int64_t* wsum,
                                                int64_t* best) {
   int64_t carry = 0, bi = -1;
@@ -3793,7 +3856,7 @@ __device__ __forceinline__ int64_t job_compact(const float* __restrict__ v, int6
       for (int k = 0; k < kJobPer; ++k) x[k] = i0 + k < n ? v[i0 + k] : nanf("");
     }
 #pragma unroll
-    for (int k = 0; k < kJobPer; ++k) f |= (double)x[k] >= thr ? 1u << k : 0u;
+    for (int k = 0; k < kJobPer; ++k) f |= x[k] >= thr ? 1u << k : 0u;
     int64_t tot, at = carry + job_scan(__popc(f), wsum, &tot);
 #pragma unroll
     for (int k = 0; k < kJobPer; ++k)
@@ -3839,7 +3902,7 @@ __global__ void __launch_bounds__(kJobThreads) bj_circ_valid_kernel(BatchTabs T,
   __shared__ int64_t wsum[32];
   const LokiPruneRun& R = T.jobs[j0 + blockIdx.x].run;
   int64_t best;
-  const int64_t n = job_compact(R.valid_flags, R.counts[kCntChild], 0.5, R.valid_ids, wsum, &best);
+  const int64_t n = job_compact(R.valid_flags, R.counts[kCntChild], 0.5f, R.valid_ids, wsum, &best);
   if (threadIdx.x == 0) {
     R.counts[kCntValid] = n;
     R.stats[l - 1].n_valid = n;
@@ -3860,8 +3923,9 @@ bj_select_kernel(BatchTabs T, int l, int j0, int64_t max_sugg, int64_t batch, in
   const int64_t n_par = cnt[kCntPar], n_valid = cnt[kCntValid];
   const double thr = T.thr[(size_t)job * T.nlevels + (l - 1)];
   int64_t best;
-  int64_t n = job_compact(w.child_scores, circ ? n_valid : cnt[kCntChild], thr, w.surv, wsum,
-                          &best);
+  // a float is at or above thr exactly if it is at or above the first float there
+  int64_t n = job_compact(w.child_scores, circ ? n_valid : cnt[kCntChild],
+                          __double2float_ru(thr), w.surv, wsum, &best);
   const bool ovf = n > max_sugg;
   if (ovf) {
     const int64_t* off = w.offsets;
@@ -4067,7 +4131,7 @@ bj_circ_branch_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
     if (i < J.run.counts[kCntPar])
       circ_branch_one(Q.lvl, J.run.trees[(l - 1) & 1].leaves, i,
                       reinterpret_cast<LokiBranchInfo*>(J.run.work.info), J.run.work.offsets,
-                      J.run.exp_off, J.dev_err);
+                      J.run.exp_off, J.dev_err, Q.bf);
   });
 }
 
