@@ -380,7 +380,7 @@ __device__ __forceinline__ void score_out(const LokiFFALevel& L, const LevelK& K
                          L.out_start + off;
     const int nout = sp.mode == 0 ? sp.nwidths : 1;
     float* row = tile + lane * stride;
-    if (SK.pow2_64) score_row64_pow2(row, sp, SK, snr + (size_t)full * nout);
+    if (SK.list64) score_row64(row, sp, SK, snr + (size_t)full * nout);
     else score_row(row, L.nbins, sp, SK, snr + (size_t)full * nout);
   }
 }

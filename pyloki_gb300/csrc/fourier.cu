@@ -408,7 +408,7 @@ fold_snr_complex64_kernel(const float2* __restrict__ folds, int64_t n, LokiScore
     x[2 * k + 1] = __fdiv_rn(a.y * (1.0f / 64.0f), __fsqrt_rn(b.y * (1.0f / 64.0f)));
   }
   const int nout = sp.mode == 0 ? sp.nwidths : 1;
-  if (SK.pow2_64) score_row64_pow2(x, sp, SK, out + (size_t)(p0 + tid) * nout);
+  if (SK.list64) score_row64(x, sp, SK, out + (size_t)(p0 + tid) * nout);
   else score_row(x, 64, sp, SK, out + (size_t)(p0 + tid) * nout);
 }
 

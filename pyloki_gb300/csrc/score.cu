@@ -52,7 +52,7 @@ score_kernel(const float* __restrict__ in, int64_t nprof, int nb, LokiScoreSpec 
   if (lane < kmax) {
     const int nout = sp.mode == 0 ? sp.nwidths : 1;
     float* row = tile + lane * stride;
-    if (SK.pow2_64) score_row64_pow2(row, sp, SK, out + (size_t)(p0 + lane) * nout);
+    if (SK.list64) score_row64(row, sp, SK, out + (size_t)(p0 + lane) * nout);
     else score_row(row, nb, sp, SK, out + (size_t)(p0 + lane) * nout);
   }
 }

@@ -53,7 +53,7 @@ sim_score_kernel(const float* __restrict__ in, const int64_t* __restrict__ src_r
   __syncwarp();
   if (lane < kmax) {
     float* row = tile + lane * stride;
-    if (SK.pow2_64) score_row64_pow2(row, sp, SK, scores + r0 + lane);
+    if (SK.list64) score_row64(row, sp, SK, scores + r0 + lane);
     else score_row(row, nb, sp, SK, scores + r0 + lane);
   }
 }
