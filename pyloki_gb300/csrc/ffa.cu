@@ -576,27 +576,34 @@ ffa_level_score_kernel(LokiFFALevel L, LevelK K, const S* __restrict__ in,
 // share the rows of the level before (L2 hits) and each of its profiles comes
 // from DRAM about once.
 //
-// Shared row layout: 64 float2 (e, v) per penultimate row (512 bytes, rows
-// 512-byte aligned), so a trial rolled by shift s reads bin (j - s) mod 64 at
-// byte (8 * (64 - s + j)) mod 512 of the row: one add and one and-or per load.
-// Compact rows let six 4-warp CTAs share an SM (36 rows per side: one final
-// other's 64 frequencies span at most 34 penultimate rows), and a chunk of two
-// final others (the usual group size of an acceleration search) is exactly
-// one 32-trial task per warp, so no warp idles while the others score.
+// Shared row layout: 64 float2 (e, v) per penultimate row and the first three
+// again, so a trial rolled by shift s reads bins j .. j + 3 at constant offsets
+// from byte (8 * (64 - s + j)) mod 512 of the row: one masked address for four
+// loads where rows of 64 need one a load (128 loads and 256 integer operations a
+// trial). A stride of 68 also moves the banks of neighbouring rows apart (the
+// kernel over the 1.5e9 trials of a 2^23-sample acceleration search: stride 67
+// 148 ms, 68 140, 69 145, 70 as 68). A chunk of two final others (the usual group
+// size of an acceleration search) by 128 frequencies is one 32-trial task per
+// warp; its rows (two sides of 64 and the shift between the others) leave room for
+// three 8-warp CTAs on an SM. Tiles of 64 frequencies in 4-warp CTAs with rows of
+// 64 took 165 ms (2400 instructions a trial, a third of them to build the rows).
 // Consecutive lanes hold consecutive final frequencies, whose rows and shifts
-// advance by about half a row and half a bin per lane, so the lanes of a warp
-// spread over the banks.
+// advance by about half a row and half a bin per lane.
 //
 // FAST: the profile is normalised as e * rsqrtf(v) (at most a few ulp from the
 // reference's e / sqrt(v)); otherwise with correctly rounded division and
-// square root, which makes the S/N bit-identical to the reference.
+// square root, which makes the S/N bit-identical to the reference. rsqrtf scales
+// subnormal arguments (three more instructions a bin): where every v of the
+// chunk's rows is at least 2^-100, no sum is subnormal and they are left out.
 // ---------------------------------------------------------------------------
 
-constexpr int kTileF = 64;        // final frequencies per tile
-constexpr int kTileWarps = 4;
-constexpr int kTileRows = 36;     // shared penultimate rows per side (tail, head)
+constexpr int kTileF = 128;       // final frequencies per tile
+constexpr int kTileWarps = 8;
+constexpr int kTileRows = 70;     // shared penultimate rows per side (tail, head)
 constexpr int kTileMembers = 8;   // final others per chunk of a group
-constexpr int kTileRowBytes = 64 * (int)sizeof(float2);
+constexpr int kTileRowBins = 68;  // 64 and the first again, three of which are read
+constexpr int kTileRowBytes = kTileRowBins * (int)sizeof(float2);
+constexpr int kTileSmem = 2 * kTileRows * kTileRowBytes;
 
 // Final others grouped by their (tail, head) penultimate other: groups[0] is
 // the group count G, groups[1 + g] the first other of group g, groups[1 + G] =
@@ -668,77 +675,90 @@ __device__ __forceinline__ float round_store<__nv_bfloat16>(float x) {
 // Builds the tile's penultimate rows (row r < nt: tail side, frequency lo_t + r
 // of penultimate other pt in segment s_t; else head side) into shared memory.
 // Warp w owns a contiguous run of rows; lane k resolves row k of the run and
-// the warp then gathers row by row.
+// the warp then gathers them, three rows in flight. Returns the smallest v.
 template <typename S>
-__device__ __forceinline__ void tile_build(const LokiFFALevel& P, const LevelK& KP,
-                                           const S* __restrict__ fold_pp,
-                                           const OtherRes* __restrict__ tab_p, int64_t no_p,
-                                           float2* rows, int nt, int nh, int64_t lo_t,
-                                           int64_t lo_h, int64_t pt, int64_t ph, int64_t s_t,
-                                           int64_t s_h, int32_t* err) {
+__device__ __forceinline__ float tile_build(const LokiFFALevel& P, const LevelK& KP,
+                                            const S* __restrict__ fold_pp,
+                                            const OtherRes* __restrict__ tab_p, int64_t no_p,
+                                            float2* rows, int nt, int nh, int64_t lo_t,
+                                            int64_t lo_h, int64_t pt, int64_t ph, int64_t s_t,
+                                            int64_t s_h, int32_t* err) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int R = nt + nh;
-  const int per = (R + kTileWarps - 1) / kTileWarps;  // <= 2 * kTileRows / 4 = 20
+  const int per = (R + kTileWarps - 1) / kTileWarps;  // <= 2 * kTileRows / 8 = 18
   const int r0 = warp * per;
   const int r1 = std::min(R, r0 + per);
   const int64_t P_in = n_in_params(P);
-  // lane k: row r0 + k
-  int32_t my_t = 0, my_h = 0, my_sh = 0;
-  bool my_ok = false;
+  // lane k: row r0 + k; its source rows and shifts (ok in bit 16)
+  int64_t my_t = 0, my_h = 0;
+  int32_t my_sh = 0;
   if (r0 + lane < r1) {
     const int r = r0 + lane;
     const bool tail = r < nt;
     const int64_t po = tail ? pt : ph;
     const int64_t f8 = tail ? lo_t + r : lo_h + (r - nt);
     const TrialRes tr = resolve_trial(P, KP, tab_p[po], tab_p[no_p + po], f8);
-    my_t = (int32_t)tr.in_tail;
-    my_h = (int32_t)tr.in_head;
-    my_sh = tr.s_tail | (tr.s_head << 8);
-    my_ok = tr.ok;
+    const int64_t seg = 2 * (tail ? s_t : s_h) * P_in;
+    if (tr.ok) {
+      my_t = (seg + tr.in_tail) * 128;
+      my_h = (seg + P_in + tr.in_head) * 128;
+    }
+    my_sh = tr.s_tail | (tr.s_head << 8) | (tr.ok ? 1 << 16 : 0);
     if (!tr.ok) atomicOr(err, LOKI_DEVERR_WINDOW);
   }
-  for (int r = r0; r < r1; ++r) {
-    const int k = r - r0;
-    const int32_t it = __shfl_sync(0xFFFFFFFFu, my_t, k);
-    const int32_t ih = __shfl_sync(0xFFFFFFFFu, my_h, k);
-    const int32_t sh2 = __shfl_sync(0xFFFFFFFFu, my_sh, k);
-    const bool ok = __shfl_sync(0xFFFFFFFFu, my_ok, k);
-    float2* dst = rows + (size_t)(r < nt ? r : kTileRows + (r - nt)) * 64;
-    if (!ok) {
-      dst[lane] = dst[lane + 32] = make_float2(0.f, 0.f);
-      continue;
+  float vmin = FLT_MAX;
+  constexpr int kU = 3;
+  for (int r = r0; r < r1; r += kU) {
+    float t[kU][4], h[kU][4];
+    int32_t sh[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int k = min(r + u, r1 - 1) - r0;  // the last row again at a ragged end
+      const S* tp = fold_pp + __shfl_sync(0xFFFFFFFFu, my_t, k);
+      const S* hp = fold_pp + __shfl_sync(0xFFFFFFFFu, my_h, k);
+      sh[u] = __shfl_sync(0xFFFFFFFFu, my_sh, k);
+      const int jt = (lane - sh[u]) & 63, jh = (lane - (sh[u] >> 8)) & 63;
+      t[u][0] = Store<S>::load(tp + jt);
+      t[u][1] = Store<S>::load(tp + (jt ^ 32));
+      t[u][2] = Store<S>::load(tp + 64 + jt);
+      t[u][3] = Store<S>::load(tp + 64 + (jt ^ 32));
+      h[u][0] = Store<S>::load(hp + jh);
+      h[u][1] = Store<S>::load(hp + (jh ^ 32));
+      h[u][2] = Store<S>::load(hp + 64 + jh);
+      h[u][3] = Store<S>::load(hp + 64 + (jh ^ 32));
     }
-    const int64_t seg8 = r < nt ? s_t : s_h;
-    const S* t = fold_pp + ((size_t)(2 * seg8) * P_in + it) * 128;
-    const S* h = fold_pp + ((size_t)(2 * seg8 + 1) * P_in + ih) * 128;
-    const int st = sh2 & 0xFF, shh = sh2 >> 8;
-    const int jt0 = (lane - st) & 63, jt1 = (lane + 32 - st) & 63;
-    const int jh0 = (lane - shh) & 63, jh1 = (lane + 32 - shh) & 63;
-    const float e0 = round_store<S>(__fadd_rn(Store<S>::load(t + jt0), Store<S>::load(h + jh0)));
-    const float e1 = round_store<S>(__fadd_rn(Store<S>::load(t + jt1), Store<S>::load(h + jh1)));
-    const float v0 =
-        round_store<S>(__fadd_rn(Store<S>::load(t + 64 + jt0), Store<S>::load(h + 64 + jh0)));
-    const float v1 =
-        round_store<S>(__fadd_rn(Store<S>::load(t + 64 + jt1), Store<S>::load(h + 64 + jh1)));
-    dst[lane] = make_float2(e0, v0);
-    dst[lane + 32] = make_float2(e1, v1);
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int rr = min(r + u, r1 - 1);
+      float x[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) x[q] = round_store<S>(__fadd_rn(t[u][q], h[u][q]));
+      if (!(sh[u] >> 16)) x[0] = x[1] = x[2] = x[3] = 0.0f;
+      float2* dst = rows + (rr < nt ? rr : kTileRows + (rr - nt)) * kTileRowBins;
+      dst[lane] = make_float2(x[0], x[2]);
+      dst[lane + 32] = make_float2(x[1], x[3]);
+      if (lane < 3) dst[lane + 64] = make_float2(x[0], x[2]);
+      vmin = fminf(vmin, fminf(x[2], x[3]));
+    }
   }
+  return vmin;
 }
 
-// (e, v) of bin j of a compact row whose roll starts at byte offset `off`
-// (= 8 * ((64 - s) mod 64)); `base` is the row's 512-aligned shared address.
-__device__ __forceinline__ float2 tile_ld(uint32_t base, uint32_t off, int j) {
-  const uint32_t a = base | ((off + 8u * (uint32_t)j) & 511u);
-  float2 r;
-  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(r.x), "=f"(r.y) : "r"(a));
+// (e, v) of bins 4 g + q, q < 4, of a row whose roll starts at byte offset `off`
+// (= 8 * ((64 - s) mod 64)), as 64-bit words: pack2(e, v) (e in the low half);
+// `a` is the masked address of bin 4 g.
+template <int Q>
+__device__ __forceinline__ unsigned long long tile_ld64(uint32_t a) {
+  unsigned long long r;
+  asm volatile("ld.shared.b64 %0, [%1+%2];" : "=l"(r) : "r"(a), "n"(8 * Q));
   return r;
 }
 
-// The same bin as one 64-bit word: pack2(e, v) (e in the low half).
-__device__ __forceinline__ unsigned long long tile_ld64(uint32_t base, uint32_t off, int j) {
-  const uint32_t a = base | ((off + 8u * (uint32_t)j) & 511u);
-  unsigned long long r;
-  asm volatile("ld.shared.b64 %0, [%1];" : "=l"(r) : "r"(a));
+// 1 / sqrt(v) of a normal v (or 0, infinity, NaN): rsqrtf's value without the
+// scaling that a subnormal v needs.
+__device__ __forceinline__ float rsqrt_normal(float v) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
   return r;
 }
 
@@ -748,7 +768,8 @@ __device__ __forceinline__ unsigned long long tile_ld64(uint32_t base, uint32_t 
 // window differences are packed f32x2 subtractions of two pairs, folded into
 // the running maximum three at a time. The differences and the maximum are
 // the reference's, so the S/N is unchanged.
-template <bool FAST, int NW>
+// NORM: 0 correctly rounded, 1 rsqrtf, 2 rsqrtf of v known to be normal.
+template <int NORM, int NW>
 __device__ __forceinline__ void tile_score_trial(uint32_t bt, uint32_t ot, uint32_t bh,
                                                  uint32_t oh, const LokiScoreSpec& sp,
                                                  const ScoreK& SK, float* __restrict__ out) {
@@ -758,19 +779,25 @@ __device__ __forceinline__ void tile_score_trial(uint32_t bt, uint32_t ot, uint3
 #pragma unroll
   for (int iw = 0; iw < NW; ++iw) m[iw] = -FLT_MAX;
   float s = 0.0f, prev = 0.0f;
+  unsigned long long ev[4];
 #pragma unroll
   for (int k = 0; k < 32; ++k) {
+    if ((k & 1) == 0) {
+      // tail + head, e and v in one packed add (each half rounded as __fadd_rn)
+      const uint32_t at = bt + ((ot + 16u * k) & 511u), ah = bh + ((oh + 16u * k) & 511u);
+      asm("add.rn.f32x2 %0, %1, %2;" : "=l"(ev[0]) : "l"(tile_ld64<0>(at)), "l"(tile_ld64<0>(ah)));
+      asm("add.rn.f32x2 %0, %1, %2;" : "=l"(ev[1]) : "l"(tile_ld64<1>(at)), "l"(tile_ld64<1>(ah)));
+      asm("add.rn.f32x2 %0, %1, %2;" : "=l"(ev[2]) : "l"(tile_ld64<2>(at)), "l"(tile_ld64<2>(ah)));
+      asm("add.rn.f32x2 %0, %1, %2;" : "=l"(ev[3]) : "l"(tile_ld64<3>(at)), "l"(tile_ld64<3>(ah)));
+    }
     float nv[2];
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      // tail + head, e and v in one packed add (each half rounded as __fadd_rn)
-      unsigned long long ev;
-      asm("add.rn.f32x2 %0, %1, %2;"
-          : "=l"(ev)
-          : "l"(tile_ld64(bt, ot, 2 * k + q)), "l"(tile_ld64(bh, oh, 2 * k + q)));
       float e, v;
-      unpack2(ev, e, v);
-      nv[q] = FAST ? __fmul_rn(e, rsqrtf(v)) : __fdiv_rn(e, __fsqrt_rn(v));
+      unpack2(ev[(k & 1) * 2 + q], e, v);
+      nv[q] = NORM == 2   ? __fmul_rn(e, rsqrt_normal(v))
+              : NORM == 1 ? __fmul_rn(e, rsqrtf(v))
+                          : __fdiv_rn(e, __fsqrt_rn(v));
     }
     const float s0 = k == 0 ? nv[0] : __fadd_rn(s, nv[0]);
     s = __fadd_rn(s0, nv[1]);
@@ -834,14 +861,13 @@ __device__ __forceinline__ void tile_score_trial(uint32_t bt, uint32_t ot, uint3
 }
 
 template <typename S, bool FAST, int NW>
-__global__ void __launch_bounds__(kTileWarps * 32, 6)
+__global__ void __launch_bounds__(kTileWarps * 32, 3)
 ffa_final_tiled64_kernel(LokiFFALevel P, LevelK KP, const S* __restrict__ fold_pp,
                          const OtherRes* __restrict__ tab_p, int64_t no_p, LokiFFALevel F,
                          LevelK KF, const OtherRes* __restrict__ tab_f, int64_t no_f,
                          const int32_t* __restrict__ groups, LokiScoreSpec sp, ScoreK SK,
                          float* __restrict__ snr, int32_t* __restrict__ err) {
-  __shared__ __align__(512) float2 rows[2 * kTileRows * 64];  // [side][row][bin]
-  __shared__ int64_t win[4];  // tail lo, tail hi, head lo, head hi
+  extern __shared__ __align__(16) float2 rows[];  // [side][row][bin]
   const uint32_t rows_sh = (uint32_t)__cvta_generic_to_shared(rows);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int n = F.nparams;
@@ -866,26 +892,28 @@ ffa_final_tiled64_kernel(LokiFFALevel P, LevelK KP, const S* __restrict__ fold_p
     while (c0 < o1) {
       const int64_t c1 = std::min<int64_t>(c0 + step, o1);
       const int m = (int)(c1 - c0);
-      __syncthreads();  // the previous chunk's rows and windows are no longer read
-      if (threadIdx.x == 0) {
-        win[0] = INT64_MAX;  // minima; indices are >= 0, so the maxima start at 0
-        win[1] = 0;
-        win[2] = INT64_MAX;
-        win[3] = 0;
+      // the chunk's windows, by every warp for itself (a barrier costs more):
+      // corners (member, first|last frequency) of the tail in even lanes, of the
+      // head in odd ones; lanes beyond repeat the last member
+      static_assert(4 * kTileMembers <= 32, "a lane for every corner");
+      int64_t lo_t, lo_h;
+      int nt, nh;
+      {
+        const int i = min(lane >> 2, m - 1), side = lane & 1, last = (lane >> 1) & 1;
+        const int64_t idx = tile_index(F, KF, tab_f[side * no_f + c0 + i],
+                                       last ? f0 + nf - 1 : f0);
+        int64_t lo = idx, hi = idx;
+#pragma unroll
+        for (int d = 2; d < 32; d <<= 1) {
+          lo = min(lo, __shfl_xor_sync(0xFFFFFFFFu, lo, d));
+          hi = max(hi, __shfl_xor_sync(0xFFFFFFFFu, hi, d));
+        }
+        const int64_t span = hi - lo + 1;
+        lo_t = __shfl_sync(0xFFFFFFFFu, lo, 0);
+        lo_h = __shfl_sync(0xFFFFFFFFu, lo, 1);
+        nt = (int)__shfl_sync(0xFFFFFFFFu, span, 0);
+        nh = (int)__shfl_sync(0xFFFFFFFFu, span, 1);
       }
-      __syncthreads();
-      if (threadIdx.x < 4 * m) {  // corners: (member, tail|head, first|last frequency)
-        const int i = threadIdx.x >> 2, side = (threadIdx.x >> 1) & 1, last = threadIdx.x & 1;
-        const int64_t o = c0 + i;
-        const int64_t idx = tile_index(F, KF, tab_f[side * no_f + o], last ? f0 + nf - 1 : f0);
-        atomicMin(reinterpret_cast<unsigned long long*>(&win[2 * side]),
-                  (unsigned long long)idx);
-        atomicMax(reinterpret_cast<unsigned long long*>(&win[2 * side + 1]),
-                  (unsigned long long)idx);
-      }
-      __syncthreads();
-      const int64_t lo_t = win[0], lo_h = win[2];
-      const int nt = (int)(win[1] - win[0] + 1), nh = (int)(win[3] - win[2] + 1);
       if (nt > kTileRows || nh > kTileRows) {  // uniform across the block
         if (step > 1) {
           step = 1;  // redo this chunk one member at a time
@@ -895,9 +923,11 @@ ffa_final_tiled64_kernel(LokiFFALevel P, LevelK KP, const S* __restrict__ fold_p
         c0 = c1;
         continue;
       }
-      tile_build<S>(P, KP, fold_pp, tab_p, no_p, rows, nt, nh, lo_t, lo_h, pt, ph, 2 * b,
-                    2 * b + 1, err);
-      __syncthreads();
+      __syncthreads();  // the previous chunk's rows are no longer read
+      const float vmin = tile_build<S>(P, KP, fold_pp, tab_p, no_p, rows, nt, nh, lo_t, lo_h,
+                                       pt, ph, 2 * b, 2 * b + 1, err);
+      // sums of two v at or above 2^-100 are normal
+      const bool quick = !__syncthreads_or(vmin < 7.8886091e-31f) && FAST;
       // trials: member-major, 32 consecutive frequencies per warp task
       const int tasks = m * (kTileF / 32);
       for (int q = warp; q < tasks; q += kTileWarps) {
@@ -920,7 +950,8 @@ ffa_final_tiled64_kernel(LokiFFALevel P, LevelK KP, const S* __restrict__ fold_p
         const uint32_t bh = rows_sh + (uint32_t)(kTileRows + rh) * kTileRowBytes;
         const uint32_t offt = 8u * (uint32_t)((64 - tr.s_tail) & 63);
         const uint32_t offh = 8u * (uint32_t)((64 - tr.s_head) & 63);
-        tile_score_trial<FAST, NW>(bt, offt, bh, offh, sp, SK, out);
+        if (quick) tile_score_trial<2, NW>(bt, offt, bh, offh, sp, SK, out);
+        else tile_score_trial<FAST ? 1 : 0, NW>(bt, offt, bh, offh, sp, SK, out);
       }
       c0 = c1;
     }
@@ -1338,12 +1369,13 @@ static int launch_tiled_t(const LokiFFALevel& P, const LevelK& KP, const void* f
   int dev = 0, nsm = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTileWarps * 32, 0) !=
+      set_smem_limit(kern, kTileSmem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTileWarps * 32, kTileSmem) !=
           cudaSuccess)
     return set_error(LOKI_ERR_CUDA, "occupancy query failed");
   const int grid = std::max(1, nsm * std::max(1, per_sm));
   note_launch();
-  kern<<<grid, kTileWarps * 32, 0, s>>>(P, KP, static_cast<const S*>(fold_pp), tab_p, no_p, F,
+  kern<<<grid, kTileWarps * 32, kTileSmem, s>>>(P, KP, static_cast<const S*>(fold_pp), tab_p, no_p, F,
                                         KF, tab_f, no_f, groups, sp, SK, snr, err);
   return LOKI_OK;
 }
