@@ -35,7 +35,15 @@ _GIB = 1 << 30
 
 
 def _cart_len(counts) -> int:
-    return int(np.prod(np.asarray(counts, dtype=np.int64)))
+    return math.prod(int(c) for c in counts)
+
+
+def _current_stream_ptr(device) -> int:
+    """The device's current stream as a pointer, without a Stream object (10 us of
+    host time; a short search asks for it at every launch)."""
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(
+        torch.cuda.current_device() if index is None else index)
 
 
 class _Grid:
@@ -45,7 +53,11 @@ class _Grid:
         self.level = level
         self.dparams = cfg.get_dparams(level)
         self.param_arr = cfg.get_param_arr(self.dparams)
-        self.counts = np.array([len(p) for p in self.param_arr], dtype=np.int64)
+        self.shape = [len(p) for p in self.param_arr]
+        self.size = math.prod(self.shape)
+        self.counts = np.array(self.shape, dtype=np.int64)
+        freqs = self.param_arr[-1]
+        self.freqs_valid = bool(np.all(np.isfinite(freqs)) and not np.any(freqs <= 0))
         self.dev = [torch.from_numpy(np.ascontiguousarray(p, dtype=np.float64)).to(device)
                     for p in self.param_arr]
         # last-dimension grid as float2 (hi, lo): f == hi + lo to ~2^-48
@@ -53,10 +65,6 @@ class _Grid:
         hi = last.astype(np.float32)
         lo = (last - hi.astype(np.float64)).astype(np.float32)
         self.split = torch.from_numpy(np.stack([hi, lo], axis=1).copy()).to(device)
-
-    @property
-    def size(self) -> int:
-        return _cart_len(self.counts)
 
 
 _GRID_CACHE: dict[tuple, _Grid] = {}
@@ -90,14 +98,13 @@ def level_desc(cfg: PulsarSearchConfig, cur: _Grid, prev: _Grid, nseg_in: int,
     d.nbins = cfg.nbins
     d.level = cur.level
     d.tseg_brute = cfg.tseg_brute
-    for i in range(n):
-        d.counts_cur[i] = int(cur.counts[i])
-        d.counts_prev[i] = int(prev.counts[i])
-        d.limits[i][0] = float(cfg.param_limits[i, 0])
-        d.limits[i][1] = float(cfg.param_limits[i, 1])
+    for i, lim in enumerate(cfg.param_limits.tolist()):
+        d.counts_cur[i] = cur.shape[i]
+        d.counts_prev[i] = prev.shape[i]
+        d.limits[i][0], d.limits[i][1] = lim
         d.param_arr[i] = cur.dev[i].data_ptr()
-    o0, ow = out_win if out_win is not None else (0, int(cur.counts[-1]))
-    i0, iw = in_win if in_win is not None else (0, int(prev.counts[-1]))
+    o0, ow = out_win if out_win is not None else (0, cur.shape[-1])
+    i0, iw = in_win if in_win is not None else (0, prev.shape[-1])
     d.out_start, d.out_width = o0, ow
     d.in_start, d.in_width = i0, iw
     d.nseg_in = nseg_in
@@ -183,6 +190,10 @@ class DynamicProgramming:
             "cuda", torch.cuda.current_device())
         self._lib = _lib.load()
         self._err = torch.zeros(1, dtype=torch.int32, device=self._device)
+        # the stream that cleared the word; None once a kernel has been given it
+        self._err_cleared_on: int | None = (
+            self._stream() if self._device.type == "cuda" else None)
+        self._grids: dict[int, _Grid] = {}
         self._data_type = np.complex64 if cfg.use_fourier else np.float32
         self._fold: torch.Tensor | None = None
         self._ffa_level = -1
@@ -231,7 +242,16 @@ class DynamicProgramming:
         return self._ffa_level
 
     def _grid(self, level: int) -> _Grid:
-        return grid(self.cfg, level, self._device)
+        g = self._grids.get(level)
+        if g is None:
+            g = self._grids[level] = grid(self.cfg, level, self._device)
+        return g
+
+    def _reset_err(self) -> None:
+        if (self._err_cleared_on is None or self._err_cleared_on != self._stream()
+                or torch.cuda.is_current_stream_capturing()):
+            self._err.zero_()
+        self._err_cleared_on = None
 
     @property
     def dparams(self) -> np.ndarray:
@@ -267,7 +287,7 @@ class DynamicProgramming:
         return self.cfg.tseg_brute * 2**self.ffa_level
 
     def _stream(self) -> int:
-        return _lib.stream_ptr(torch.cuda.current_stream(self._device))
+        return _current_stream_ptr(self._device)
 
     # ---- level 0: brute fold -------------------------------------------------
     def initialize(self) -> None:
@@ -280,8 +300,7 @@ class DynamicProgramming:
                     msg = (f"param_arr has {len(g0.param_arr[ip])} values, "
                            "should have only one")
                     raise ValueError(msg)
-        freqs = g0.param_arr[-1]
-        if not np.all(np.isfinite(freqs)) or np.any(freqs <= 0):
+        if not g0.freqs_valid:
             msg = "Frequency must be positive."
             raise ValueError(msg)
         dev = self._device
@@ -302,7 +321,7 @@ class DynamicProgramming:
             nfreq = g0.dev[-1].numel()
             nbf = cfg.nbins // 2 + 1
             fold = torch.empty((nseg, nfreq, 2, nbf), dtype=torch.complex64, device=dev)
-            self._err.zero_()
+            self._reset_err()
             v_ptr = 0 if self._unit_var else _lib.ptr(ts_v)
             need = int(self._lib.loki_brutefold_complex_scratch_bytes(
                 ts_e.numel(), cfg.bseg_brute, int(self._unit_var)))
@@ -337,7 +356,7 @@ class DynamicProgramming:
             self._fold = low
         self._fold = self._fold.reshape(nseg, *([1] * (cfg.nparams - 1)), nfreq, 2,
                                         cfg.nbins)
-        self._err.zero_()
+        self._reset_err()
         self._ffa_level = 0
 
     # ---- DP levels -----------------------------------------------------------
@@ -355,7 +374,7 @@ class DynamicProgramming:
         if self.cfg.use_fourier:  # shift_add_complex (core/common.py:344-372)
             nbf = self.nbins // 2 + 1
             desc = level_desc(self.cfg, cur, prev, nseg_in)
-            out = torch.empty((nseg_in // 2, cur.size, 2, nbf), dtype=torch.complex64,
+            out = torch.empty((nseg_in // 2, *cur.shape, 2, nbf), dtype=torch.complex64,
                               device=self._device)
             if self.nbins <= 286 and not self._tree_folds:
                 _lib.check(self._lib.loki_ffa_level_complex_rows(
@@ -369,16 +388,16 @@ class DynamicProgramming:
                 _lib.check(self._lib.loki_ffa_level_complex(
                     desc, _lib.ptr(plan), _lib.ptr(fold_in), _lib.ptr(out), self._stream()))
                 self.launches += 2
-            self._fold = out.reshape(nseg_in // 2, *cur.counts.tolist(), 2, nbf)
+            self._fold = out
             self._ffa_level += 1
             return
-        out = torch.empty((nseg_in // 2, cur.size, 2, self.nbins), dtype=self._fold_dtype,
+        out = torch.empty((nseg_in // 2, *cur.shape, 2, self.nbins), dtype=self._fold_dtype,
                           device=self._device)
         desc = level_desc(self.cfg, cur, prev, nseg_in, storage=self._storage)
         _lib.check(self._lib.loki_ffa_level(desc, _lib.ptr(fold_in), _lib.ptr(out),
                                             _lib.ptr(self._err), self._stream()))
         self.launches += 1
-        self._fold = out.reshape(nseg_in // 2, *cur.counts.tolist(), 2, self.nbins)
+        self._fold = out
         self._ffa_level += 1
 
     def get_fold_norm(self, iseg: int = 0, param_idx: tuple | None = None) -> torch.Tensor:
@@ -415,18 +434,20 @@ class DynamicProgramming:
 
             return boxcar_snr_nd(self.get_fold_norm(iseg), widths, stdnoise)
         fold = self.fold[iseg]
-        flat = fold.reshape(-1, 2, fold.shape[-1])
-        snr = torch.empty((flat.shape[0], len(widths)), dtype=torch.float32,
-                          device=self._device)
+        lead = fold.shape[:-2]
+        n = math.prod(lead)
+        if not fold.is_contiguous():
+            fold = fold.contiguous()
+        snr = torch.empty((*lead, len(widths)), dtype=torch.float32, device=self._device)
         spec = _lib.score_spec(widths, self.nbins, stdnoise, mode=0)
         if fourier:
-            _lib.check(self._lib.loki_fold_snr_complex64(_lib.ptr(flat), flat.shape[0], spec,
+            _lib.check(self._lib.loki_fold_snr_complex64(_lib.ptr(fold), n, spec,
                                                          _lib.ptr(snr), self._stream()))
         else:
-            _lib.check(self._lib.loki_fold_snr(_lib.ptr(flat), flat.shape[0], self.nbins, spec,
+            _lib.check(self._lib.loki_fold_snr(_lib.ptr(fold), n, self.nbins, spec,
                                                _lib.ptr(snr), self._stream()))
         self.launches += 1
-        return snr.reshape(*fold.shape[:-2], len(widths))
+        return snr
 
     def get_complexity(self) -> list[int]:
         return [_cart_len(self.cfg.get_param_grid_count(lvl))
@@ -478,8 +499,9 @@ class DynamicProgramming:
     # ---- fused, memory-bounded search ---------------------------------------
     def level_bytes(self, level: int) -> int:
         nseg = self.nbatch * (self.cfg.nsamps // (self.cfg.bseg_brute * 2**level))
-        return (nseg * _cart_len(self.cfg.get_param_grid_count(level)) * 2 * self.nbins
-                * self._elem_bytes)
+        g = self._grids.get(level)
+        size = g.size if g else _cart_len(self.cfg.get_param_grid_count(level))
+        return nseg * size * 2 * self.nbins * self._elem_bytes
 
     @property
     def _elem_bytes(self) -> int:
@@ -708,7 +730,7 @@ def brutefold(ts_e: torch.Tensor, ts_v: torch.Tensor, freqs: torch.Tensor, segme
     scratch = torch.empty(min(need, max(scratch_bytes, segment_len * elem)),
                           dtype=torch.uint8, device=ts_e.device)
     fold = torch.empty((nseg, nfreq, 2, nbins), dtype=torch.float32, device=ts_e.device)
-    stream = _lib.stream_ptr(torch.cuda.current_stream(ts_e.device))
+    stream = _current_stream_ptr(ts_e.device)
     if unit_variance:
         _lib.check(lib.loki_brutefold_unit_variance(
             _lib.ptr(ts_e), nsamps, _lib.ptr(freqs), nfreq, segment_len, nbins, tsamp, t_ref,

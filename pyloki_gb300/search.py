@@ -136,6 +136,7 @@ def ffa_search(tseries: TimeSeries, search_cfg: PulsarSearchConfig, *, quiet: bo
     dyp = DynamicProgramming(tseries, search_cfg, device=device)
     widths = search_cfg.score_widths
     if materialize is None:
+        dyp._grid(search_cfg.niters_ffa)  # the final grid, which either path needs
         materialize = dyp.level_bytes(search_cfg.niters_ffa) <= 1 << 30
     dyp.initialize()
     if materialize:
