@@ -2286,103 +2286,147 @@ circ_emit_complex_kernel(LokiPruneLevel D, const double* __restrict__ leaves,
 // ---------------------------------------------------------------------------
 
 // ---------------------------------------------------------------------------
-// Complex rows of 32 children at a time, 64 bins. The warp stages one component
-// of its children's parent and segment rows in shared memory (whole rows, lane
-// by harmonic), then each lane combines and transforms its own child with the
-// arithmetic of rotate_add and irfft_norm: the phasor recurrence, and every bin
-// summed over the harmonics in order with each product and sum rounded. The
-// angles of bins j, 64 - j, 32 - j and 32 + j have the same cosine and sine up
-// to sign, so their four sums share two products, and the 64 sums are
-// independent registers. A lane walking its rows in global memory and the bins
-// one after the other took 56 ms for the 7.7e6 children of a 16-run search.
+// Complex rows of 32 children at a time, 64 bins, with the arithmetic of
+// rotate_add and irfft_norm. Every lane runs its child's phasor recurrence once,
+// into a table of shared memory; then the warp combines the children's parent and
+// segment rows whole, lane by harmonic (loads and stores of full lines), and, to
+// score, each lane transforms its own child: every bin summed over the harmonics
+// in order with each product and sum rounded. The angles of bins j, 64 - j, 32 - j
+// and 32 + j have the same cosine and sine up to sign, so their four sums share
+// two products, and the 64 sums are independent registers. A lane walking its
+// rows in global memory and the bins one after the other took 56 ms for the 8.0e6
+// children of a 16-run search; now 10.5, of which 4 are the latency of the 100
+// levels with fewer than 500 children a run.
 // ---------------------------------------------------------------------------
 
 constexpr int kCplxRow = 33;  // float2 of one component; odd, so lanes miss each other's banks
 __host__ __device__ constexpr int cplx64_warp_bytes() { return 2 * 32 * kCplxRow * 8; }
 
-// One component of the rows of children k < kmax: par rows to A, seg rows to B.
-__device__ __forceinline__ void stage_rows64(const float2* __restrict__ folds,
-                                             const float2* __restrict__ seg, int64_t my_par,
-                                             int64_t my_row, int kmax, int comp, float2* A,
-                                             float2* B) {
+// Powers 0 .. 32 of each lane's phasor.
+__device__ __forceinline__ void phasor_table(float2 delta, float2* T) {
+  float2* t = T + (threadIdx.x & 31) * kCplxRow;
+  float2 ph = make_float2(1.0f, 0.0f);
+#pragma unroll 3
+  for (int k = 0; k < 33; ++k) {
+    t[k] = ph;
+    ph = cmul_rn(ph, delta);
+  }
+  __syncwarp();
+}
+
+__device__ __forceinline__ float2 rotate_add1(float2 b, float2 ph, float2 a) {
+  const float2 r = cmul_rn(b, ph);
+  return make_float2(__fadd_rn(r.x, a.x), __fadd_rn(r.y, a.y));
+}
+
+// One component of the combined rows of children k < kmax: harmonic h of child k
+// to out[k * stride + h].
+__device__ __forceinline__ void combine_rows64(const float2* __restrict__ folds,
+                                               const float2* __restrict__ seg, int64_t my_par,
+                                               int64_t my_row, int kmax, int comp,
+                                               const float2* T, float2* out, int stride) {
   const int lane = threadIdx.x & 31;
+  const float2* fa = folds + comp * 33 + lane;
+  const float2* fb = seg + comp * 33 + lane;
   constexpr int kU = 8;
   for (int k0 = 0; k0 < kmax; k0 += kU) {
     float2 a[kU], b[kU];
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
-      const int k = k0 + u, src = k < kmax ? k : 0;
-      const int64_t par = __shfl_sync(0xFFFFFFFFu, my_par, src);
-      const int64_t row = __shfl_sync(0xFFFFFFFFu, my_row, src);
-      if (k < kmax) {
-        a[u] = __ldg(folds + par * 66 + comp * 33 + lane);
-        b[u] = __ldg(seg + row * 66 + comp * 33 + lane);
-      }
+      const int k = min(k0 + u, kmax - 1);
+      a[u] = __ldg(fa + __shfl_sync(0xFFFFFFFFu, my_par, k) * 66);
+      b[u] = __ldg(fb + __shfl_sync(0xFFFFFFFFu, my_row, k) * 66);
     }
 #pragma unroll
     for (int u = 0; u < kU; ++u)
-      if (k0 + u < kmax) {
-        A[(k0 + u) * kCplxRow + lane] = a[u];
-        B[(k0 + u) * kCplxRow + lane] = b[u];
-      }
+      if (k0 + u < kmax)
+        out[(k0 + u) * stride + lane] = rotate_add1(b[u], T[(k0 + u) * kCplxRow + lane], a[u]);
   }
-  if (lane < kmax) {
-    A[lane * kCplxRow + 32] = __ldg(folds + my_par * 66 + comp * 33 + 32);
-    B[lane * kCplxRow + 32] = __ldg(seg + my_row * 66 + comp * 33 + 32);
-  }
+  if (lane < kmax)  // the last harmonic, child by lane
+    out[lane * stride + 32] =
+        rotate_add1(__ldg(seg + my_row * 66 + comp * 33 + 32), T[lane * kCplxRow + 32],
+                    __ldg(folds + my_par * 66 + comp * 33 + 32));
   __syncwarp();
 }
 
-// rotate_add of one component in place: a = b phasor^k + a.
-__device__ __forceinline__ void combine64(float2* a, const float2* b, float2 delta) {
-  float2 ph = make_float2(1.0f, 0.0f);
-#pragma unroll 3
-  for (int k = 0; k < 33; ++k) {
-    const float2 r = cmul_rn(b[k], ph), p = a[k];
-    a[k] = make_float2(__fadd_rn(r.x, p.x), __fadd_rn(r.y, p.y));
-    ph = cmul_rn(ph, delta);
-  }
-}
+// Twiddles by harmonic: W[m * 16 + j] = (cos, sin) of 2 pi m j / 64 for harmonics
+// m = 1 .. 31 (row m - 1), after the 64 angles they are taken from.
+constexpr int kTwiddle64Bytes = 512 + 31 * 16 * 8;
 
-// irfft_norm's sums of one component (unscaled); tw = (cos, sin) of 2 pi t / 64.
-__device__ __forceinline__ void irfft64_sums(const float2* __restrict__ X,
-                                             const float2* __restrict__ tw, float (&acc)[64]) {
-  const float x0 = X[0].x, nyq = X[32].x;
-#pragma unroll
-  for (int j = 0; j < 64; ++j) acc[j] = (j & 1) ? __fsub_rn(x0, nyq) : __fadd_rn(x0, nyq);
-#pragma unroll 1
-  for (int m = 1; m < 32; ++m) {
-    const float2 x = X[m];
-    const bool odd = m & 1;
-    const float sg = odd ? -2.0f : 2.0f;
-    // bins 0, 32 and 16, 48: angles that are multiples of a quarter turn
-    acc[0] = __fmaf_rn(2.0f, x.x, acc[0]);
-    acc[32] = __fmaf_rn(sg, x.x, acc[32]);
-    const float v = (m & 2) ? -2.0f : 2.0f;
-    acc[16] = __fmaf_rn(odd ? -v : v, odd ? x.y : x.x, acc[16]);
-    acc[48] = __fmaf_rn(v, odd ? x.y : x.x, acc[48]);
-    int t = 0;
-#pragma unroll
-    for (int j = 1; j < 16; ++j) {
-      t = (t + m) & 63;
-      const float2 w = tw[t];
-      const float a = __fmul_rn(x.x, w.x), b = __fmul_rn(x.y, w.y);
-      const float u = __fsub_rn(a, b), z = __fadd_rn(a, b);
-      // doubling is exact: 2 t + acc rounds once, as the sum of the doubled term
-      acc[j] = __fmaf_rn(2.0f, u, acc[j]);
-      acc[64 - j] = __fmaf_rn(2.0f, z, acc[64 - j]);
-      acc[32 - j] = __fmaf_rn(sg, z, acc[32 - j]);
-      acc[32 + j] = __fmaf_rn(sg, u, acc[32 + j]);
-    }
-  }
-}
-
-__device__ __forceinline__ void load_twiddles64(float2* tw) {
+__device__ __forceinline__ void load_twiddles64(float* smem) {
+  float2 *tw = reinterpret_cast<float2*>(smem), *W = tw + 64;
   for (int t = threadIdx.x; t < 64; t += blockDim.x) {
     double s, c;
     sincospi(2.0 * (double)t / 64.0, &s, &c);
     tw[t] = make_float2((float)c, (float)s);
   }
+  __syncthreads();
+  for (int t = threadIdx.x; t < 31 * 16; t += blockDim.x)
+    W[t] = tw[((t >> 4) + 1) * (t & 15) & 63];
+}
+
+// The 64 sums of one component: p[j] = (bin j, bin 64 - j), q[j] = (bin 32 + j,
+// bin 32 - j) for j = 1 .. 15, and bins 0, 32, 16 and 48.
+struct Sums64 {
+  unsigned long long p[16], q[16];
+  float b0, b32, b16, b48;
+};
+
+__device__ __forceinline__ unsigned long long fma2_rn(unsigned long long a, unsigned long long b,
+                                                      unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+// Harmonic m (M = m mod 4) into the sums: doubling is exact, so 2 t + acc rounds
+// once, as the sum of the doubled term.
+template <int M>
+__device__ __forceinline__ void irfft64_step(const float2 x, const float2* __restrict__ W,
+                                             Sums64& S) {
+  constexpr bool odd = M & 1;
+  constexpr float sg = odd ? -2.0f : 2.0f, v = (M & 2) ? -2.0f : 2.0f;
+  const unsigned long long two = pack2(2.0f, 2.0f), sgn = pack2(sg, sg), xx = pack2(x.x, x.y);
+  S.b0 = __fmaf_rn(2.0f, x.x, S.b0);
+  S.b32 = __fmaf_rn(sg, x.x, S.b32);
+  S.b16 = __fmaf_rn(odd ? -v : v, odd ? x.y : x.x, S.b16);
+  S.b48 = __fmaf_rn(v, odd ? x.y : x.x, S.b48);
+#pragma unroll
+  for (int j2 = 0; j2 < 16; j2 += 2) {
+    const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(W + j2);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int j = j2 + h;
+      if (j == 0) continue;
+      unsigned long long ab;
+      asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(ab) : "l"(xx), "l"(h ? w.y : w.x));
+      float a, b;
+      unpack2(ab, a, b);
+      const unsigned long long uz = pack2(__fsub_rn(a, b), __fadd_rn(a, b));
+      S.p[j] = fma2_rn(two, uz, S.p[j]);
+      S.q[j] = fma2_rn(sgn, uz, S.q[j]);
+    }
+  }
+}
+
+// irfft_norm's sums of one component (unscaled).
+__device__ __forceinline__ void irfft64_sums(const float2* __restrict__ X,
+                                             const float2* __restrict__ W, Sums64& S) {
+  const float x0 = X[0].x, nyq = X[32].x;
+  const float even = __fadd_rn(x0, nyq), odd = __fsub_rn(x0, nyq);
+  S.b0 = S.b32 = S.b16 = S.b48 = even;
+#pragma unroll
+  for (int j = 1; j < 16; ++j) S.p[j] = S.q[j] = (j & 1) ? pack2(odd, odd) : pack2(even, even);
+#pragma unroll 1
+  for (int m = 1; m < 29; m += 4) {
+    irfft64_step<1>(X[m], W + (m - 1) * 16, S);
+    irfft64_step<2>(X[m + 1], W + m * 16, S);
+    irfft64_step<3>(X[m + 2], W + (m + 1) * 16, S);
+    irfft64_step<0>(X[m + 3], W + (m + 2) * 16, S);
+  }
+  irfft64_step<1>(X[29], W + 28 * 16, S);
+  irfft64_step<2>(X[30], W + 29 * 16, S);
+  irfft64_step<3>(X[31], W + 30 * 16, S);
 }
 
 // Scores of the warp's children (rows and phasor held lane by lane).
@@ -2394,22 +2438,52 @@ __device__ __forceinline__ void cplx64_score(const float2* __restrict__ folds,
                                              float* __restrict__ scores,
                                              unsigned* __restrict__ minmax_keys) {
   const int lane = threadIdx.x & 31;
-  float2 *A = buf, *B = buf + 32 * kCplxRow;
+  float2 *A = buf, *T = buf + 32 * kCplxRow;
+  const float2* row = A + lane * kCplxRow;
+  unsigned long long* keep = reinterpret_cast<unsigned long long*>(T + lane * kCplxRow);
   const float inv = 1.0f / 64.0f;
-  float e[64], v[64];
-  stage_rows64(folds, seg, my_par, my_row, kmax, 0, A, B);
-  combine64(A + lane * kCplxRow, B + lane * kCplxRow, delta);
-  irfft64_sums(A + lane * kCplxRow, tw, e);
-  __syncwarp();
-  stage_rows64(folds, seg, my_par, my_row, kmax, 1, A, B);
-  combine64(A + lane * kCplxRow, B + lane * kCplxRow, delta);
-  irfft64_sums(A + lane * kCplxRow, tw, v);
+  phasor_table(delta, T);
+  Sums64 S;
+  combine_rows64(folds, seg, my_par, my_row, kmax, 0, T, A, kCplxRow);
+  irfft64_sums(row, tw, S);
+  __syncwarp();  // every lane has read its row
+  combine_rows64(folds, seg, my_par, my_row, kmax, 1, T, A, kCplxRow);
+  // the phasors have been used: their rows keep the first component's sums, which
+  // would be 64 more registers. (Three blocks an SM spill 108 bytes a thread: 11.0
+  // instead of 10.5 ms for the 8.0e6 children of 16 runs.)
+#pragma unroll
+  for (int j = 1; j < 16; ++j) {
+    keep[j] = S.p[j];
+    keep[16 + j] = S.q[j];
+  }
+  keep[0] = pack2(S.b0, S.b32);
+  keep[16] = pack2(S.b16, S.b48);
+  irfft64_sums(row, tw, S);
+  S.p[0] = pack2(S.b0, S.b32);
+  S.q[0] = pack2(S.b16, S.b48);
+#pragma unroll
+  for (int j = 0; j < 32; ++j) {
+    float e0, e1, v0, v1;
+    unpack2(keep[j], e0, e1);
+    unpack2(j < 16 ? S.p[j] : S.q[j - 16], v0, v1);
+    v0 = __fdiv_rn(__fmul_rn(e0, inv), __fsqrt_rn(__fmul_rn(v0, inv)));
+    v1 = __fdiv_rn(__fmul_rn(e1, inv), __fsqrt_rn(__fmul_rn(v1, inv)));
+    (j < 16 ? S.p[j] : S.q[j - 16]) = pack2(v0, v1);
+  }
   __syncwarp();  // every lane has read its rows: the buffer becomes the score tile
   const int stride = score_stride(64, sp.wmax);
   float* tile = reinterpret_cast<float*>(buf);
+  float* trow = tile + lane * stride;
 #pragma unroll
-  for (int j = 0; j < 64; ++j)
-    tile[lane * stride + j] = __fdiv_rn(__fmul_rn(e[j], inv), __fsqrt_rn(__fmul_rn(v[j], inv)));
+  for (int j = 0; j < 16; ++j) {
+    float x0, x1, y0, y1;
+    unpack2(S.p[j], x0, x1);
+    unpack2(S.q[j], y0, y1);
+    trow[j] = x0;
+    trow[j == 0 ? 32 : 64 - j] = x1;
+    trow[j == 0 ? 16 : 32 + j] = y0;
+    trow[j == 0 ? 48 : 32 - j] = y1;
+  }
   __syncwarp();
   score_tile_rows(tile, stride, 64, sp, SK, scores, kmax, minmax_keys);
 }
@@ -2419,18 +2493,9 @@ __device__ __forceinline__ void cplx64_emit(const float2* __restrict__ folds,
                                             const float2* __restrict__ seg, int64_t my_par,
                                             int64_t my_row, float2 delta, int kmax, float2* buf,
                                             float2* __restrict__ fout) {
-  const int lane = threadIdx.x & 31;
-  float2 *A = buf, *B = buf + 32 * kCplxRow;
-  for (int comp = 0; comp < 2; ++comp) {
-    stage_rows64(folds, seg, my_par, my_row, kmax, comp, A, B);
-    if (lane < kmax) combine64(A + lane * kCplxRow, B + lane * kCplxRow, delta);
-    __syncwarp();
-    for (int k = 0; k < kmax; ++k) {
-      fout[k * 66 + comp * 33 + lane] = A[k * kCplxRow + lane];
-      if (lane == 0) fout[k * 66 + comp * 33 + 32] = A[k * kCplxRow + 32];
-    }
-    __syncwarp();
-  }
+  phasor_table(delta, buf);
+  for (int comp = 0; comp < 2; ++comp)
+    combine_rows64(folds, seg, my_par, my_row, kmax, comp, buf, fout + comp * 33, 66);
 }
 
 static int check_prune(const LokiPruneLevel* D) {
@@ -4025,19 +4090,20 @@ __global__ void __launch_bounds__(kTile, 4) bj_emit_kernel(BatchTabs T, int l, i
 __host__ __device__ inline int cplx_smem_bytes(int nbins, int wmax, bool score) {
   const int stride = score_stride(nbins, wmax);
   if (nbins == 64)
-    return 512 + kPruneWarps * (score ? max(cplx64_warp_bytes(), 32 * stride * 4)
-                                      : cplx64_warp_bytes());
+    return score ? kTwiddle64Bytes + kPruneWarps * max(cplx64_warp_bytes(), 32 * stride * 4)
+                 : kPruneWarps * cplx64_warp_bytes() / 2;
   return score ? (int)((2 * nbins + kPruneWarps * cplx_warp_floats(nbins, stride)) * 4) : 0;
 }
 
 template <int KP>
-__global__ void __launch_bounds__(kTile)
+__global__ void __launch_bounds__(kTile, 2)
 bj_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   extern __shared__ __align__(16) float smem[];
   __shared__ JobQueue Q;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int stride = score_stride(A.nb, A.sp.wmax), nbf = A.nb / 2 + 1;
-  if (A.nb == 64) load_twiddles64(reinterpret_cast<float2*>(smem));
+  const float2* W = reinterpret_cast<const float2*>(smem) + 64;
+  if (A.nb == 64) load_twiddles64(smem);
   else load_twiddles(smem, A.nb);
   queue_run(Q, T, l, j0, nj, kCntChild, [&](int job, int64_t t) {
     const LokiPruneJob& J = T.jobs[job];
@@ -4078,9 +4144,10 @@ bj_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
       delta = prune_phasor(r.phase, 64);
     }
     const int wb = max(cplx64_warp_bytes(), 32 * stride * 4);
-    cplx64_score(folds, seg, par, row, delta, kmax, reinterpret_cast<const float2*>(smem),
-                 reinterpret_cast<float2*>(reinterpret_cast<char*>(smem) + 512 + warp * wb), A.sp,
-                 A.SK, w.child_scores + c0, keys);
+    cplx64_score(folds, seg, par, row, delta, kmax, W,
+                 reinterpret_cast<float2*>(reinterpret_cast<char*>(smem) + kTwiddle64Bytes +
+                                           warp * wb),
+                 A.sp, A.SK, w.child_scores + c0, keys);
     __syncwarp();
   });
 }
@@ -4113,8 +4180,7 @@ bj_emit_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
     float2* fout = reinterpret_cast<float2*>(out.folds);
     if (A.nb == 64)
       cplx64_emit(folds, seg, r.par, r.row, prune_phasor(r.phase, A.nb), kmax,
-                  reinterpret_cast<float2*>(reinterpret_cast<char*>(smem) + 512 +
-                                            warp * cplx64_warp_bytes()),
+                  reinterpret_cast<float2*>(smem) + warp * 32 * kCplxRow,
                   fout + s0 * 66);
     else if (lane < kmax)
       rotate_add(seg + r.row * 2 * nbf, folds + r.par * 2 * nbf, prune_phasor(r.phase, A.nb), nbf,
@@ -4196,13 +4262,14 @@ bj_circ_emit_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   });
 }
 
-__global__ void __launch_bounds__(kTile)
+__global__ void __launch_bounds__(kTile, 2)
 bj_circ_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   extern __shared__ __align__(16) float smem[];
   __shared__ JobQueue Q;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int stride = score_stride(A.nb, A.sp.wmax), nbf = A.nb / 2 + 1;
-  if (A.nb == 64) load_twiddles64(reinterpret_cast<float2*>(smem));
+  const float2* W = reinterpret_cast<const float2*>(smem) + 64;
+  if (A.nb == 64) load_twiddles64(smem);
   else load_twiddles(smem, A.nb);
   queue_run(Q, T, l, j0, nj, kCntValid, [&](int job, int64_t t) {
     const LokiPruneJob& J = T.jobs[job];
@@ -4248,9 +4315,10 @@ bj_circ_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
       delta = prune_phasor(r.phase, 64);
     }
     const int wb = max(cplx64_warp_bytes(), 32 * stride * 4);
-    cplx64_score(folds, seg, par, row, delta, kmax, reinterpret_cast<const float2*>(smem),
-                 reinterpret_cast<float2*>(reinterpret_cast<char*>(smem) + 512 + warp * wb), A.sp,
-                 A.SK, w.child_scores + v0, keys);
+    cplx64_score(folds, seg, par, row, delta, kmax, W,
+                 reinterpret_cast<float2*>(reinterpret_cast<char*>(smem) + kTwiddle64Bytes +
+                                           warp * wb),
+                 A.sp, A.SK, w.child_scores + v0, keys);
     __syncwarp();
   });
 }
@@ -4282,8 +4350,7 @@ bj_circ_emit_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
     float2* fout = reinterpret_cast<float2*>(out.folds);
     if (A.nb == 64)
       cplx64_emit(folds, seg, r.par, r.row, prune_phasor(r.phase, A.nb), kmax,
-                  reinterpret_cast<float2*>(reinterpret_cast<char*>(smem) + 512 +
-                                            warp * cplx64_warp_bytes()),
+                  reinterpret_cast<float2*>(smem) + warp * 32 * kCplxRow,
                   fout + s0 * 66);
     else if (lane < kmax)
       rotate_add(seg + r.row * 2 * nbf, folds + r.par * 2 * nbf, prune_phasor(r.phase, A.nb), nbf,
