@@ -60,6 +60,19 @@ __device__ __forceinline__ unsigned lanemask_lt() {
   return m;
 }
 
+// x / LOKI_C_VAL, correctly rounded, in two operations: x zh + RN(x zl) with
+// 1 / C = zh + zl (Brisebarre, Muller & Raina 2004, division by a constant known
+// in advance). The sum is off by less than 2^-105 of the quotient before its one
+// rounding, and as C is an integer of 29 bits no quotient of a double lies within
+// 2^-83 of a midpoint. Outside 2^-823 .. 2^776 (0, infinities and NaN too) the
+// division itself.
+__device__ __forceinline__ double div_c(double x) {
+  const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7FFu;
+  if (e - 200u < 1600u)
+    return __fma_rn(x, 0x1.ca726eb25f9dbp-29, __dmul_rn(x, 0x1.568bbb3de4666p-84));
+  return __ddiv_rn(x, LOKI_C_VAL);
+}
+
 // Phase bin of a periodic signal as a float in [0, nbins)
 // (utils/psr_utils.py:12-46 get_phase_idx).
 __device__ __forceinline__ double phase_idx(double proper_time, double freq,

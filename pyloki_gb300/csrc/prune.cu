@@ -294,8 +294,8 @@ __device__ __forceinline__ ChildRes resolve_child(const LokiPruneLevel& D, int P
     vel = tdot(pv, D.tm_a, P - 1, m);
     dd = tdot(pv, D.tm_a, P, m);
   }
-  const double freq = __dmul_rn(f0, __dsub_rn(1.0, __ddiv_rn(vel, LOKI_C_VAL)));
-  const double delay = __ddiv_rn(dd, LOKI_C_VAL);
+  const double freq = __dmul_rn(f0, __dsub_rn(1.0, div_c(vel)));
+  const double delay = div_c(dd);
   ChildRes r;
   r.phase = phase_idx(D.dt_phase, f0, D.nbins, delay);
   r.ia = (int32_t)axis_index(accel, D.accel_min, D.accel_inv, D.n_accel);
@@ -534,12 +534,13 @@ __device__ __forceinline__ void gather_norm_rows(const float* __restrict__ folds
       for (int u = 0; u < kU; ++u) {
         const int k = k0 + u;
         const int src = k < kmax ? k : 0;
-        const int64_t par = __shfl_sync(0xFFFFFFFFu, my_par, src);
-        const int64_t row = __shfl_sync(0xFFFFFFFFu, my_row, src);
+        // (rows of 512 bytes: their numbers fit 32 bits)
+        const uint32_t par = __shfl_sync(0xFFFFFFFFu, (uint32_t)my_par, src);
+        const uint32_t row = __shfl_sync(0xFFFFFFFFu, (uint32_t)my_row, src);
         const int sh = __shfl_sync(0xFFFFFFFFu, my_shift, src);
         if (k < kmax) {
-          const float* pf = folds + par * 128;
-          const float* sf = seg + row * 128;
+          const float* pf = folds + (size_t)par * 128;
+          const float* sf = seg + (size_t)row * 128;
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             const int j = lane + 32 * c;
@@ -617,11 +618,11 @@ __device__ __forceinline__ void score_tile(
                    int64_t n_children, const float* __restrict__ seg, const LokiScoreSpec& sp,
                    const ScoreK& SK, float* __restrict__ scores, int32_t* __restrict__ cidx,
                    double* __restrict__ cphase, unsigned* __restrict__ minmax_keys,
-                   float* tile, int64_t c0) {
+                   float* tile, int64_t c0, int width = 32) {
   const int lane = threadIdx.x & 31;
   const int nb = D.nbins, P = tree_order<KP>(D);
   const int stride = score_stride(nb, sp.wmax);
-  const int kmax = (int)std::min<int64_t>(32, n_children - c0);
+  const int kmax = (int)std::min<int64_t>(width, n_children - c0);
   // lane k resolves child c0 + k
   int64_t my_par = warp_find_parents(offsets, n_parents, c0 + lane, kmax), my_row = 0;
   int my_shift = 0;
@@ -965,12 +966,13 @@ __device__ __forceinline__ void gather_add_rows(const float* __restrict__ folds,
       for (int u = 0; u < kU; ++u) {
         const int k = k0 + u;
         const int src = k < kmax ? k : 0;
-        const int64_t par = __shfl_sync(0xFFFFFFFFu, my_par, src);
-        const int64_t row = __shfl_sync(0xFFFFFFFFu, my_row, src);
+        // (rows of 512 bytes: their numbers fit 32 bits)
+        const uint32_t par = __shfl_sync(0xFFFFFFFFu, (uint32_t)my_par, src);
+        const uint32_t row = __shfl_sync(0xFFFFFFFFu, (uint32_t)my_row, src);
         const int sh = __shfl_sync(0xFFFFFFFFu, my_shift, src);
         if (k < kmax) {
-          const float* pf = folds + par * 128;
-          const float* sf = seg + row * 128;
+          const float* pf = folds + (size_t)par * 128;
+          const float* sf = seg + (size_t)row * 128;
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             const int j = lane + 32 * c;
@@ -1023,10 +1025,11 @@ __device__ __forceinline__ void emit_tile(
                   const int32_t* __restrict__ cidx, const double* __restrict__ cphase,
                   double* __restrict__ lout, float* __restrict__ fout,
                   float* __restrict__ sout, float* __restrict__ seout,
-                  int32_t* __restrict__ bout, int64_t s0, const EmitExtra& X = EmitExtra()) {
+                  int32_t* __restrict__ bout, int64_t s0, const EmitExtra& X = EmitExtra(),
+    int width = 32) {
   const int lane = threadIdx.x & 31;
   const int nb = D.nbins, P = tree_order<KP>(D), m = P + 1;
-  const int kmax = (int)std::min<int64_t>(32, n_surv - s0);
+  const int kmax = (int)std::min<int64_t>(width, n_surv - s0);
   const int64_t my_c = surv[s0 + min(lane, kmax - 1)];
   int64_t my_par = warp_find_parents(offsets, n_parents, my_c, kmax), my_row = 0;
   int my_shift = 0;
@@ -1199,8 +1202,8 @@ __device__ __forceinline__ void ascend_tile(const LokiPruneLevel& D, const doubl
         vel = tdot(pv, T, P - 1, m);
         dd = tdot(pv, T, P, m);
       }
-      const double freq = __dmul_rn(f0, __dsub_rn(1.0, __ddiv_rn(vel, LOKI_C_VAL)));
-      const double delay = __ddiv_rn(dd, LOKI_C_VAL);
+      const double freq = __dmul_rn(f0, __dsub_rn(1.0, div_c(vel)));
+      const double delay = div_c(dd);
       const double ph = phase_idx(dt_seg[sg], f0, nb, delay);
       const int64_t ia = axis_index(accel, D.accel_min, D.accel_inv, D.n_accel);
       const int64_t iff = axis_index(freq, D.freq_min, D.freq_inv, D.n_freq);
@@ -1598,8 +1601,8 @@ __device__ __forceinline__ int circ_resolve(const LokiPruneLevel& D, const doubl
     vel = tdot(pv, D.tm_a, 4, m);
     dd = tdot(pv, D.tm_a, 5, m);
   }
-  const double freq = __dmul_rn(f0, __dsub_rn(1.0, __ddiv_rn(vel, LOKI_C_VAL)));
-  const double delay = __ddiv_rn(dd, LOKI_C_VAL);
+  const double freq = __dmul_rn(f0, __dsub_rn(1.0, div_c(vel)));
+  const double delay = div_c(dd);
   r->phase = phase_idx(D.dt_phase, f0, D.nbins, delay);
   r->ia = (int32_t)axis_index(accel, D.accel_min, D.accel_inv, D.n_accel);
   r->iff = (int32_t)axis_index(freq, D.freq_min, D.freq_inv, D.n_freq);
@@ -1615,11 +1618,11 @@ __device__ __forceinline__ void circ_score_tile(const LokiPruneLevel& D, const d
                   float* __restrict__ scores, int32_t* __restrict__ cidx,
                   double* __restrict__ cphase, int8_t* __restrict__ ccls,
                   int32_t* __restrict__ batch_taylor, unsigned* __restrict__ minmax_keys,
-                  float* tile, int64_t v0) {
+                  float* tile, int64_t v0, int width = 32) {
   const int lane = threadIdx.x & 31;
   const int nb = D.nbins, P = 5;
   const int stride = score_stride(nb, sp.wmax);
-  const int kmax = (int)std::min<int64_t>(32, n_valid - v0);
+  const int kmax = (int)std::min<int64_t>(width, n_valid - v0);
   int64_t my_par = 0, my_row = 0;
   int my_shift = 0;
   if (lane < kmax) {
@@ -1694,11 +1697,11 @@ __device__ __forceinline__ void circ_emit_tile(const LokiPruneLevel& D, const do
                  const double* __restrict__ cphase, const int8_t* __restrict__ ccls,
                  const int32_t* __restrict__ batch_taylor, double* __restrict__ lout,
                  float* __restrict__ fout, float* __restrict__ sout,
-                 float* __restrict__ seout, int32_t* __restrict__ bout, int64_t s0,
-                 const EmitExtra& X = EmitExtra()) {
+                 float* __restrict__ seout, int32_t* __restrict__ bout, int64_t s0, const EmitExtra& X = EmitExtra(),
+    int width = 32) {
   const int lane = threadIdx.x & 31;
   const int nb = D.nbins, P = 5, m = 6;
-  const int kmax = (int)std::min<int64_t>(32, n_surv - s0);
+  const int kmax = (int)std::min<int64_t>(width, n_surv - s0);
   int64_t my_par = 0, my_row = 0;
   int my_shift = 0;
   if (lane < kmax) {
@@ -2056,8 +2059,8 @@ __device__ __forceinline__ void ascend_one_complex(
       vel = tdot(pv, T, P - 1, m);
       dd = tdot(pv, T, P, m);
     }
-    const double freq = __dmul_rn(f0, __dsub_rn(1.0, __ddiv_rn(vel, LOKI_C_VAL)));
-    const double delay = __ddiv_rn(dd, LOKI_C_VAL);
+    const double freq = __dmul_rn(f0, __dsub_rn(1.0, div_c(vel)));
+    const double delay = div_c(dd);
     const double ph = phase_idx(dt_seg[sg], f0, nb, delay);
     const int64_t ia = axis_index(accel, D.accel_min, D.accel_inv, D.n_accel);
     const int64_t iff = axis_index(freq, D.freq_min, D.freq_inv, D.n_freq);
@@ -2334,8 +2337,8 @@ __device__ __forceinline__ void combine_rows64(const float2* __restrict__ folds,
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
       const int k = min(k0 + u, kmax - 1);
-      a[u] = __ldg(fa + __shfl_sync(0xFFFFFFFFu, my_par, k) * 66);
-      b[u] = __ldg(fb + __shfl_sync(0xFFFFFFFFu, my_row, k) * 66);
+      a[u] = __ldg(fa + (size_t)__shfl_sync(0xFFFFFFFFu, (uint32_t)my_par, k) * 66);
+      b[u] = __ldg(fb + (size_t)__shfl_sync(0xFFFFFFFFu, (uint32_t)my_row, k) * 66);
     }
 #pragma unroll
     for (int u = 0; u < kU; ++u)
@@ -2353,13 +2356,21 @@ __device__ __forceinline__ void combine_rows64(const float2* __restrict__ folds,
 // m = 1 .. 31 (row m - 1), after the 64 angles they are taken from.
 constexpr int kTwiddle64Bytes = 512 + 31 * 16 * 8;
 
+// cos(2 pi k / 64) to the nearest float, k = 0 .. 16.
+__constant__ float kCos64[17] = {
+    1.0f, 0.99518472f, 0.980785251f, 0.956940353f, 0.923879504f, 0.881921291f,
+    0.831469595f, 0.773010433f, 0.707106769f, 0.634393275f, 0.555570245f, 0.471396744f,
+    0.382683426f, 0.290284663f, 0.195090324f, 0.0980171412f, 0.0f};
+
+__device__ __forceinline__ float cos64(int t) {  // cos(2 pi t / 64)
+  t &= 63;
+  if (t > 32) t = 64 - t;
+  return t <= 16 ? kCos64[t] : -kCos64[32 - t];
+}
+
 __device__ __forceinline__ void load_twiddles64(float* smem) {
   float2 *tw = reinterpret_cast<float2*>(smem), *W = tw + 64;
-  for (int t = threadIdx.x; t < 64; t += blockDim.x) {
-    double s, c;
-    sincospi(2.0 * (double)t / 64.0, &s, &c);
-    tw[t] = make_float2((float)c, (float)s);
-  }
+  for (int t = threadIdx.x; t < 64; t += blockDim.x) tw[t] = make_float2(cos64(t), cos64(t - 16));
   __syncthreads();
   for (int t = threadIdx.x; t < 31 * 16; t += blockDim.x)
     W[t] = tw[((t >> 4) + 1) * (t & 15) & 63];
@@ -2429,6 +2440,81 @@ __device__ __forceinline__ void irfft64_sums(const float2* __restrict__ X,
   irfft64_step<3>(X[31], W + 30 * 16, S);
 }
 
+// The same by four lanes a child: this one's bins of j = 4 part + h, h < 4 (p[h],
+// q[h]; j = 0 stands for none), and bins 0, 32, 16 and 48.
+struct Sums16 {
+  unsigned long long p[4], q[4];
+  float b0, b32, b16, b48;
+};
+
+template <int M>
+__device__ __forceinline__ void irfft16_step(const float2 x, const float2* __restrict__ W,
+                                             Sums16& S) {
+  constexpr bool odd = M & 1;
+  constexpr float sg = odd ? -2.0f : 2.0f, v = (M & 2) ? -2.0f : 2.0f;
+  const unsigned long long two = pack2(2.0f, 2.0f), sgn = pack2(sg, sg), xx = pack2(x.x, x.y);
+  S.b0 = __fmaf_rn(2.0f, x.x, S.b0);
+  S.b32 = __fmaf_rn(sg, x.x, S.b32);
+  S.b16 = __fmaf_rn(odd ? -v : v, odd ? x.y : x.x, S.b16);
+  S.b48 = __fmaf_rn(v, odd ? x.y : x.x, S.b48);
+#pragma unroll
+  for (int h = 0; h < 4; h += 2) {
+    const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(W + h);
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      unsigned long long ab;
+      asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(ab) : "l"(xx), "l"(g ? w.y : w.x));
+      float a, b;
+      unpack2(ab, a, b);
+      const unsigned long long uz = pack2(__fsub_rn(a, b), __fadd_rn(a, b));
+      S.p[h + g] = fma2_rn(two, uz, S.p[h + g]);
+      S.q[h + g] = fma2_rn(sgn, uz, S.q[h + g]);
+    }
+  }
+}
+
+__device__ __forceinline__ void irfft16_sums(const float2* __restrict__ X,
+                                             const float2* __restrict__ W, int part, Sums16& S) {
+  const float x0 = X[0].x, nyq = X[32].x;
+  const float even = __fadd_rn(x0, nyq), odd = __fsub_rn(x0, nyq);
+  W += 4 * part;  // j has the parity of h
+  S.b0 = S.b32 = S.b16 = S.b48 = even;
+#pragma unroll
+  for (int h = 0; h < 4; ++h) S.p[h] = S.q[h] = (h & 1) ? pack2(odd, odd) : pack2(even, even);
+#pragma unroll 1
+  for (int m = 1; m < 29; m += 4) {
+    irfft16_step<1>(X[m], W + (m - 1) * 16, S);
+    irfft16_step<2>(X[m + 1], W + m * 16, S);
+    irfft16_step<3>(X[m + 2], W + (m + 1) * 16, S);
+    irfft16_step<0>(X[m + 3], W + (m + 2) * 16, S);
+  }
+  irfft16_step<1>(X[29], W + 28 * 16, S);
+  irfft16_step<2>(X[30], W + 29 * 16, S);
+  irfft16_step<3>(X[31], W + 30 * 16, S);
+}
+
+// e / sqrt(v) of two bins' sums.
+__device__ __forceinline__ unsigned long long norm64(unsigned long long e, unsigned long long v) {
+  const float inv = 1.0f / 64.0f;
+  float e0, e1, v0, v1;
+  unpack2(e, e0, e1);
+  unpack2(v, v0, v1);
+  return pack2(__fdiv_rn(__fmul_rn(e0, inv), __fsqrt_rn(__fmul_rn(v0, inv))),
+               __fdiv_rn(__fmul_rn(e1, inv), __fsqrt_rn(__fmul_rn(v1, inv))));
+}
+
+// Bins j, 64 - j, 32 + j and 32 - j (j = 0: bins 0, 32, 16 and 48) of a row.
+__device__ __forceinline__ void put_bins(float* row, int j, unsigned long long p,
+                                         unsigned long long q) {
+  float x0, x1, y0, y1;
+  unpack2(p, x0, x1);
+  unpack2(q, y0, y1);
+  row[j] = x0;
+  row[j == 0 ? 32 : 64 - j] = x1;
+  row[j == 0 ? 16 : 32 + j] = y0;
+  row[j == 0 ? 48 : 32 - j] = y1;
+}
+
 // Scores of the warp's children (rows and phasor held lane by lane).
 __device__ __forceinline__ void cplx64_score(const float2* __restrict__ folds,
                                              const float2* __restrict__ seg, int64_t my_par,
@@ -2441,8 +2527,31 @@ __device__ __forceinline__ void cplx64_score(const float2* __restrict__ folds,
   float2 *A = buf, *T = buf + 32 * kCplxRow;
   const float2* row = A + lane * kCplxRow;
   unsigned long long* keep = reinterpret_cast<unsigned long long*>(T + lane * kCplxRow);
-  const float inv = 1.0f / 64.0f;
+  const int stride = score_stride(64, sp.wmax);
+  float* tile = reinterpret_cast<float*>(buf);
   phasor_table(delta, T);
+  if (kmax <= 8) {  // four lanes a child (a level of 100 children a run: 44 -> 20 us)
+    const int part = lane & 3;
+    const float2* sub = A + (lane >> 2) * kCplxRow;
+    Sums16 E, V;
+    combine_rows64(folds, seg, my_par, my_row, kmax, 0, T, A, kCplxRow);
+    irfft16_sums(sub, tw, part, E);
+    __syncwarp();
+    combine_rows64(folds, seg, my_par, my_row, kmax, 1, T, A, kCplxRow);
+    irfft16_sums(sub, tw, part, V);
+    if (part == 0) {
+      E.p[0] = pack2(E.b0, E.b32), E.q[0] = pack2(E.b16, E.b48);
+      V.p[0] = pack2(V.b0, V.b32), V.q[0] = pack2(V.b16, V.b48);
+    }
+    __syncwarp();  // the buffer becomes the score tile
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+      put_bins(tile + (lane >> 2) * stride, 4 * part + h, norm64(E.p[h], V.p[h]),
+               norm64(E.q[h], V.q[h]));
+    __syncwarp();
+    score_tile_rows(tile, stride, 64, sp, SK, scores, kmax, minmax_keys);
+    return;
+  }
   Sums64 S;
   combine_rows64(folds, seg, my_par, my_row, kmax, 0, T, A, kCplxRow);
   irfft64_sums(row, tw, S);
@@ -2462,28 +2571,13 @@ __device__ __forceinline__ void cplx64_score(const float2* __restrict__ folds,
   S.p[0] = pack2(S.b0, S.b32);
   S.q[0] = pack2(S.b16, S.b48);
 #pragma unroll
-  for (int j = 0; j < 32; ++j) {
-    float e0, e1, v0, v1;
-    unpack2(keep[j], e0, e1);
-    unpack2(j < 16 ? S.p[j] : S.q[j - 16], v0, v1);
-    v0 = __fdiv_rn(__fmul_rn(e0, inv), __fsqrt_rn(__fmul_rn(v0, inv)));
-    v1 = __fdiv_rn(__fmul_rn(e1, inv), __fsqrt_rn(__fmul_rn(v1, inv)));
-    (j < 16 ? S.p[j] : S.q[j - 16]) = pack2(v0, v1);
+  for (int j = 0; j < 16; ++j) {
+    S.p[j] = norm64(keep[j], S.p[j]);
+    S.q[j] = norm64(keep[16 + j], S.q[j]);
   }
   __syncwarp();  // every lane has read its rows: the buffer becomes the score tile
-  const int stride = score_stride(64, sp.wmax);
-  float* tile = reinterpret_cast<float*>(buf);
-  float* trow = tile + lane * stride;
 #pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    float x0, x1, y0, y1;
-    unpack2(S.p[j], x0, x1);
-    unpack2(S.q[j], y0, y1);
-    trow[j] = x0;
-    trow[j == 0 ? 32 : 64 - j] = x1;
-    trow[j == 0 ? 16 : 32 + j] = y0;
-    trow[j == 0 ? 48 : 32 - j] = y1;
-  }
+  for (int j = 0; j < 16; ++j) put_bins(tile + lane * stride, j, S.p[j], S.q[j]);
   __syncwarp();
   score_tile_rows(tile, stride, 64, sp, SK, scores, kmax, minmax_keys);
 }
@@ -3734,32 +3828,61 @@ constexpr int kTile = kPruneWarps * 32;  // parents, children or survivors a til
 struct JobQueue {
   alignas(16) LokiPruneLevel lvl;
   BranchF bf;
+  int width;                // items a warp takes of a tile
   int pre[kQueueJobs + 1];  // tiles before each job
 };
 
-// Tiles [t0, t1) of this block over jobs j0 .. j0 + nj, counts[idx] items each.
+// Widths a warp may take: the narrowest and the widest below 32, packed.
+enum { kWide = 32 << 5, kNarrow8 = 8 << 5 | 8, kNarrow16 = 8 << 5 | 16 };
+
+// Tiles [t0, t1) of this block over jobs j0 .. j0 + nj, counts[idx] items each. A
+// warp takes 32 items of a tile; where the level is so small that the grid holds
+// all tiles at once even then, `narrow` (8) or twice that: a warp's time is latency
+// there (rows are gathered a few at a time, complex ones transformed by four lanes
+// a child), and 100 of the 127 levels of a search have a few hundred children a run
+// (score of such a level 20 -> 16 us, circular 20 -> 14, complex 44 -> 20, emission
+// 13 -> 11). The complex scores take 8 or 32: between, a lane transforms a child by
+// itself and half of the lanes would idle.
 __device__ __forceinline__ void queue_open(JobQueue& Q, const BatchTabs& T, int j0, int nj,
-                                           int idx, int* t0, int* t1) {
+                                           int idx, int narrow, int* t0, int* t1) {
   const int lane = threadIdx.x & 31;
-  for (int t = threadIdx.x; t < nj; t += blockDim.x)
-    Q.pre[t + 1] = (int)((T.jobs[j0 + t].run.counts[idx] + kTile - 1) / kTile);
-  if (threadIdx.x == 0) Q.pre[0] = 0;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    int carry = 0;
-    for (int base = 0; base < nj; base += 32) {
-      int v = base + lane < nj ? Q.pre[base + lane + 1] : 0;
+  int64_t cnt[kQueueJobs / kTile];
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xFFFFFFFFu, v, o);
-        if (lane >= o) v += y;
-      }
-      if (base + lane < nj) Q.pre[base + lane + 1] = v + carry;
-      carry += __shfl_sync(0xFFFFFFFFu, v, 31);
-    }
+  for (int k = 0; k < kQueueJobs / kTile; ++k) {
+    const int t = threadIdx.x + k * kTile;
+    cnt[k] = t < nj ? T.jobs[j0 + t].run.counts[idx] : 0;
   }
-  __syncthreads();
-  const int total = Q.pre[nj], per = (total + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int narrow_top = narrow & 31;
+  int width = narrow >> 5, total;
+  for (;; width = width < narrow_top ? 2 * width : 32) {
+    const int items = width * kPruneWarps;
+#pragma unroll
+    for (int k = 0; k < kQueueJobs / kTile; ++k) {
+      const int t = threadIdx.x + k * kTile;
+      if (t < nj) Q.pre[t + 1] = (int)((cnt[k] + items - 1) / items);
+    }
+    if (threadIdx.x == 0) Q.pre[0] = 0;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      int carry = 0;
+      for (int base = 0; base < nj; base += 32) {
+        int v = base + lane < nj ? Q.pre[base + lane + 1] : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(0xFFFFFFFFu, v, o);
+          if (lane >= o) v += y;
+        }
+        if (base + lane < nj) Q.pre[base + lane + 1] = v + carry;
+        carry += __shfl_sync(0xFFFFFFFFu, v, 31);
+      }
+    }
+    __syncthreads();
+    total = Q.pre[nj];
+    if (width == 32 || total <= (int)gridDim.x) break;
+    __syncthreads();  // every thread has read the total
+  }
+  if (threadIdx.x == 0) Q.width = width;
+  const int per = (total + (int)gridDim.x - 1) / (int)gridDim.x;
   *t0 = min((int)blockIdx.x * per, total);
   *t1 = min(*t0 + per, total);
 }
@@ -3793,9 +3916,9 @@ __device__ __forceinline__ int queue_job(JobQueue& Q, const BatchTabs& T, int j0
 // tiles.
 template <typename F>
 __device__ __forceinline__ void queue_run(JobQueue& Q, const BatchTabs& T, int l, int j0, int nj,
-                                          int idx, F body) {
+                                          int idx, int narrow, F body) {
   int t0, t1, cur = -1;
-  queue_open(Q, T, j0, nj, idx, &t0, &t1);
+  queue_open(Q, T, j0, nj, idx, narrow, &t0, &t1);
   for (int t = t0; t < t1; ++t) {
     cur = queue_job(Q, T, j0, nj, l, t, cur);
     body(j0 + cur, (int64_t)(t - Q.pre[cur]));
@@ -3813,7 +3936,7 @@ template <int KP>
 __global__ void __launch_bounds__(kTile)
 bj_branch_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   __shared__ JobQueue Q;
-  queue_run(Q, T, l, j0, nj, kCntPar, [&](int job, int64_t tile) {
+  queue_run(Q, T, l, j0, nj, kCntPar, kWide, [&](int job, int64_t tile) {
     const LokiPruneJob& J = T.jobs[job];
     const int64_t i = tile * kTile + threadIdx.x;
     if (i < J.run.counts[kCntPar])
@@ -4039,17 +4162,17 @@ bj_score_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   extern __shared__ float tiles[];
   __shared__ JobQueue Q;
   const int warp = threadIdx.x >> 5;
-  queue_run(Q, T, l, j0, nj, kCntChild, [&](int job, int64_t t) {
+  queue_run(Q, T, l, j0, nj, kCntChild, kNarrow16, [&](int job, int64_t t) {
     const LokiPruneJob& J = T.jobs[job];
     const LokiPruneWork& w = J.run.work;
     const LokiPruneTree& in = J.run.trees[(l - 1) & 1];
-    const int64_t n_child = J.run.counts[kCntChild], c0 = t * kTile + warp * 32;
+    const int64_t n_child = J.run.counts[kCntChild], c0 = (t * kPruneWarps + warp) * Q.width;
     if (c0 >= n_child) return;
     float* tile = tiles + (size_t)warp * 32 * score_stride(Q.lvl.nbins, A.sp.wmax);
     score_tile<KP>(Q.lvl, in.leaves, in.folds, J.run.counts[kCntPar],
                reinterpret_cast<LokiBranchInfo*>(w.info), w.offsets, n_child,
                static_cast<const float*>(job_segment(T, J, job, l, 4)), A.sp, A.SK, w.child_scores,
-               w.child_idx, w.child_phase, reinterpret_cast<unsigned*>(w.minmax), tile, c0);
+               w.child_idx, w.child_phase, reinterpret_cast<unsigned*>(w.minmax), tile, c0, Q.width);
     __syncwarp();
   });
 }
@@ -4071,17 +4194,18 @@ template <int KP>
 __global__ void __launch_bounds__(kTile, 4) bj_emit_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   __shared__ JobQueue Q;
   const int warp = threadIdx.x >> 5;
-  queue_run(Q, T, l, j0, nj, kCntSurv, [&](int job, int64_t t) {
+  queue_run(Q, T, l, j0, nj, kCntSurv, kNarrow16, [&](int job, int64_t t) {
     const LokiPruneJob& J = T.jobs[job];
     const LokiPruneRun& R = J.run;
     const LokiPruneWork& w = R.work;
     const LokiPruneTree &in = R.trees[(l - 1) & 1], &out = R.trees[l & 1];
-    const int64_t n_surv = R.counts[kCntSurv], s0 = t * kTile + warp * 32;
+    const int64_t n_surv = R.counts[kCntSurv], s0 = (t * kPruneWarps + warp) * Q.width;
     if (s0 >= n_surv) return;
     emit_tile<KP>(Q.lvl, in.leaves, in.folds, reinterpret_cast<LokiBranchInfo*>(w.info), w.offsets,
               R.counts[kCntOldPar], static_cast<const float*>(job_segment(T, J, job, l, 4)),
               w.surv, n_surv, w.child_scores, w.child_idx, w.child_phase, out.leaves, out.folds,
-              out.scores, out.scores_ep, out.backtracks, s0, job_extra(R, l, Q.lvl.poly_order));
+              out.scores, out.scores_ep, out.backtracks, s0, job_extra(R, l, Q.lvl.poly_order),
+                  Q.width);
   });
 }
 
@@ -4105,7 +4229,7 @@ bj_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   const float2* W = reinterpret_cast<const float2*>(smem) + 64;
   if (A.nb == 64) load_twiddles64(smem);
   else load_twiddles(smem, A.nb);
-  queue_run(Q, T, l, j0, nj, kCntChild, [&](int job, int64_t t) {
+  queue_run(Q, T, l, j0, nj, kCntChild, kNarrow8, [&](int job, int64_t t) {
     const LokiPruneJob& J = T.jobs[job];
     const LokiPruneWork& w = J.run.work;
     const LokiPruneTree& in = J.run.trees[(l - 1) & 1];
@@ -4114,13 +4238,13 @@ bj_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
     const float2* seg = static_cast<const float2*>(job_segment(T, J, job, l, 8));
     unsigned* keys = reinterpret_cast<unsigned*>(w.minmax);
     const int64_t n_par = J.run.counts[kCntPar], n_child = J.run.counts[kCntChild];
-    const int64_t c0 = t * kTile + warp * 32, c = c0 + lane;
+    const int64_t c0 = (t * kPruneWarps + warp) * Q.width, c = c0 + lane;
     if (c0 >= n_child) return;
-    const int kmax = (int)min((int64_t)32, n_child - c0);
+    const int kmax = (int)min((int64_t)Q.width, n_child - c0);
     const LokiPruneLevel& D = Q.lvl;
     if (A.nb != 64) {
       float* wbase = smem + 2 * A.nb + (size_t)warp * cplx_warp_floats(A.nb, stride);
-      if (c < n_child)
+      if (lane < kmax)
         score_child_complex(D, in.leaves, folds, n_par, info, w.offsets, seg, A.sp, A.SK,
                             w.child_scores, w.child_idx, w.child_phase, keys, smem,
                             reinterpret_cast<float2*>(wbase) + (size_t)lane * 2 * nbf,
@@ -4158,7 +4282,7 @@ bj_emit_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   extern __shared__ __align__(16) float smem[];
   __shared__ JobQueue Q;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  queue_run(Q, T, l, j0, nj, kCntSurv, [&](int job, int64_t t) {
+  queue_run(Q, T, l, j0, nj, kCntSurv, kNarrow16, [&](int job, int64_t t) {
     const LokiPruneJob& J = T.jobs[job];
     const LokiPruneRun& R = J.run;
     const LokiPruneWork& w = R.work;
@@ -4166,9 +4290,9 @@ bj_emit_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
     const LokiBranchInfo* info = reinterpret_cast<LokiBranchInfo*>(w.info);
     const float2* folds = reinterpret_cast<const float2*>(in.folds);
     const float2* seg = static_cast<const float2*>(job_segment(T, J, job, l, 8));
-    const int64_t n_surv = R.counts[kCntSurv], s0 = t * kTile + warp * 32, s = s0 + lane;
+    const int64_t n_surv = R.counts[kCntSurv], s0 = (t * kPruneWarps + warp) * Q.width, s = s0 + lane;
     if (s0 >= n_surv) return;
-    const int kmax = (int)min((int64_t)32, n_surv - s0), nbf = A.nb / 2 + 1;
+    const int kmax = (int)min((int64_t)Q.width, n_surv - s0), nbf = A.nb / 2 + 1;
     const int64_t par = warp_find_parents(w.offsets, R.counts[kCntOldPar],
                                           w.surv[s0 + min(lane, kmax - 1)], kmax);
     EmitRow r = {0, 0, 0.0};
@@ -4193,7 +4317,7 @@ bj_emit_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
 __global__ void __launch_bounds__(kTile)
 bj_circ_branch_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   __shared__ JobQueue Q;
-  queue_run(Q, T, l, j0, nj, kCntPar, [&](int job, int64_t tile) {
+  queue_run(Q, T, l, j0, nj, kCntPar, kWide, [&](int job, int64_t tile) {
     const LokiPruneJob& J = T.jobs[job];
     const int64_t i = tile * kTile + threadIdx.x;
     if (i < J.run.counts[kCntPar])
@@ -4208,7 +4332,7 @@ bj_circ_branch_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
 __global__ void __launch_bounds__(kTile)
 bj_circ_map_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   __shared__ JobQueue Q;
-  queue_run(Q, T, l, j0, nj, kCntPar, [&](int job, int64_t tile) {
+  queue_run(Q, T, l, j0, nj, kCntPar, kWide, [&](int job, int64_t tile) {
     const LokiPruneRun& R = T.jobs[job].run;
     const int64_t i = tile * kTile + threadIdx.x, n = R.counts[kCntPar];
     if (i < n && R.counts[kCntChild] > 0)
@@ -4223,12 +4347,12 @@ bj_circ_score_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   extern __shared__ float tiles[];
   __shared__ JobQueue Q;
   const int warp = threadIdx.x >> 5;
-  queue_run(Q, T, l, j0, nj, kCntValid, [&](int job, int64_t t) {
+  queue_run(Q, T, l, j0, nj, kCntValid, kNarrow16, [&](int job, int64_t t) {
     const LokiPruneJob& J = T.jobs[job];
     const LokiPruneRun& R = J.run;
     const LokiPruneWork& w = R.work;
     const LokiPruneTree& in = R.trees[(l - 1) & 1];
-    const int64_t n_valid = R.counts[kCntValid], v0 = t * kTile + warp * 32;
+    const int64_t n_valid = R.counts[kCntValid], v0 = (t * kPruneWarps + warp) * Q.width;
     if (v0 >= n_valid) return;
     circ_score_tile(Q.lvl, in.leaves, in.folds, A.batch,
                     reinterpret_cast<const LokiBranchInfo*>(w.info),
@@ -4236,7 +4360,7 @@ bj_circ_score_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
                     static_cast<const float*>(job_segment(T, J, job, l, 4)), A.sp, A.SK,
                     w.child_scores, w.child_idx, w.child_phase, R.child_class, R.batch_taylor,
                     reinterpret_cast<unsigned*>(w.minmax),
-                    tiles + (size_t)warp * 32 * score_stride(Q.lvl.nbins, A.sp.wmax), v0);
+                    tiles + (size_t)warp * 32 * score_stride(Q.lvl.nbins, A.sp.wmax), v0, Q.width);
     __syncwarp();
   });
 }
@@ -4245,12 +4369,12 @@ __global__ void __launch_bounds__(kTile)
 bj_circ_emit_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   __shared__ JobQueue Q;
   const int warp = threadIdx.x >> 5;
-  queue_run(Q, T, l, j0, nj, kCntSurv, [&](int job, int64_t t) {
+  queue_run(Q, T, l, j0, nj, kCntSurv, kNarrow16, [&](int job, int64_t t) {
     const LokiPruneJob& J = T.jobs[job];
     const LokiPruneRun& R = J.run;
     const LokiPruneWork& w = R.work;
     const LokiPruneTree &in = R.trees[(l - 1) & 1], &out = R.trees[l & 1];
-    const int64_t n_surv = R.counts[kCntSurv], s0 = t * kTile + warp * 32;
+    const int64_t n_surv = R.counts[kCntSurv], s0 = (t * kPruneWarps + warp) * Q.width;
     if (s0 >= n_surv) return;
     circ_emit_tile(Q.lvl, in.leaves, in.folds, A.batch,
                    reinterpret_cast<const LokiBranchInfo*>(w.info),
@@ -4258,7 +4382,7 @@ bj_circ_emit_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
                    static_cast<const float*>(job_segment(T, J, job, l, 4)), w.surv, n_surv,
                    w.child_scores, w.child_idx, w.child_phase, R.child_class, R.batch_taylor,
                    out.leaves, out.folds, out.scores, out.scores_ep, out.backtracks, s0,
-                   job_extra(R, l, 5));
+                   job_extra(R, l, 5), Q.width);
   });
 }
 
@@ -4271,7 +4395,7 @@ bj_circ_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   const float2* W = reinterpret_cast<const float2*>(smem) + 64;
   if (A.nb == 64) load_twiddles64(smem);
   else load_twiddles(smem, A.nb);
-  queue_run(Q, T, l, j0, nj, kCntValid, [&](int job, int64_t t) {
+  queue_run(Q, T, l, j0, nj, kCntValid, kNarrow8, [&](int job, int64_t t) {
     const LokiPruneJob& J = T.jobs[job];
     const LokiPruneRun& R = J.run;
     const LokiPruneWork& w = R.work;
@@ -4281,13 +4405,13 @@ bj_circ_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
     const float2* folds = reinterpret_cast<const float2*>(in.folds);
     const float2* seg = static_cast<const float2*>(job_segment(T, J, job, l, 8));
     unsigned* keys = reinterpret_cast<unsigned*>(w.minmax);
-    const int64_t n_valid = R.counts[kCntValid], v0 = t * kTile + warp * 32, v = v0 + lane;
+    const int64_t n_valid = R.counts[kCntValid], v0 = (t * kPruneWarps + warp) * Q.width, v = v0 + lane;
     if (v0 >= n_valid) return;
-    const int kmax = (int)min((int64_t)32, n_valid - v0);
+    const int kmax = (int)min((int64_t)Q.width, n_valid - v0);
     const LokiPruneLevel& D = Q.lvl;
     if (A.nb != 64) {
       float* wbase = smem + 2 * A.nb + (size_t)warp * cplx_warp_floats(A.nb, stride);
-      if (v < n_valid)
+      if (lane < kmax)
         circ_score_one_complex(D, in.leaves, folds, A.batch, info, map, R.valid_ids, seg, A.sp, A.SK,
                                smem, reinterpret_cast<float2*>(wbase) + (size_t)lane * 2 * nbf,
                                wbase + (size_t)32 * 2 * nbf * 2 + lane * stride, w.child_scores,
@@ -4328,16 +4452,16 @@ bj_circ_emit_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   extern __shared__ __align__(16) float smem[];
   __shared__ JobQueue Q;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  queue_run(Q, T, l, j0, nj, kCntSurv, [&](int job, int64_t t) {
+  queue_run(Q, T, l, j0, nj, kCntSurv, kNarrow16, [&](int job, int64_t t) {
     const LokiPruneJob& J = T.jobs[job];
     const LokiPruneRun& R = J.run;
     const LokiPruneWork& w = R.work;
     const LokiPruneTree &in = R.trees[(l - 1) & 1], &out = R.trees[l & 1];
     const float2* folds = reinterpret_cast<const float2*>(in.folds);
     const float2* seg = static_cast<const float2*>(job_segment(T, J, job, l, 8));
-    const int64_t n_surv = R.counts[kCntSurv], s0 = t * kTile + warp * 32, s = s0 + lane;
+    const int64_t n_surv = R.counts[kCntSurv], s0 = (t * kPruneWarps + warp) * Q.width, s = s0 + lane;
     if (s0 >= n_surv) return;
-    const int kmax = (int)min((int64_t)32, n_surv - s0), nbf = A.nb / 2 + 1;
+    const int kmax = (int)min((int64_t)Q.width, n_surv - s0), nbf = A.nb / 2 + 1;
     EmitRow r = {0, 0, 0.0};
     if (lane < kmax)
       r = circ_emit_one_complex_leaf(Q.lvl, in.leaves, A.batch,
@@ -4513,7 +4637,7 @@ static int batch_enqueue(void* dev_scratch, int32_t njobs, int32_t nlevels,
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kTile, bytes) != cudaSuccess)
       return set_error(LOKI_ERR_CUDA, "occupancy query failed");
     *g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)nsm * std::max(1, per),
-                                                          (items + kTile - 1) / kTile * nj_max));
+                                                          (items + kPruneWarps * 8 - 1) / (kPruneWarps * 8) * nj_max));
     return (int)LOKI_OK;
   };
   unsigned g_branch = 1, g_map = 1, g_score = 1, g_emit = 1;
