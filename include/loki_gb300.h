@@ -759,6 +759,12 @@ int loki_prune_seed_batch(const LokiSeedJob* jobs, int32_t njobs, int32_t nbins,
                           int32_t poly_order, const LokiScoreSpec* spec, void* dev_scratch,
                           int64_t dev_scratch_bytes, void* stream);
 
+/* loki_prune_seed_batch of complex folds: fold_rows and folds_out are
+ * n x 2 x (nbins / 2 + 1) complex64 (nbins even). */
+int loki_prune_seed_batch_complex(const LokiSeedJob* jobs, int32_t njobs, int32_t nbins,
+                                  int32_t poly_order, const LokiScoreSpec* spec,
+                                  void* dev_scratch, int64_t dev_scratch_bytes, void* stream);
+
 /* One job of loki_prune_ascend_batch: the ascend of loki_prune_ascend_dev
  * (its level descriptor, final tree, device survivor count and per-segment
  * tables) for one run. */

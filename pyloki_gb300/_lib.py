@@ -261,6 +261,8 @@ SIGNATURES: dict[str, tuple] = {
     "loki_gather_parts": (C.c_int, [_P, _I32, _P, _I64, _P, _I64, _P]),
     "loki_prune_seed_batch": (C.c_int, [_P, _I32, _I32, _I32, C.POINTER(LokiScoreSpec), _P,
                                         _I64, _P]),
+    "loki_prune_seed_batch_complex": (C.c_int, [_P, _I32, _I32, _I32, C.POINTER(LokiScoreSpec),
+                                                _P, _I64, _P]),
     "loki_ffa_plan": (C.c_int, [C.POINTER(LokiFFALevel), _P, _P, _P]),
     "loki_ffa_level": (C.c_int, [C.POINTER(LokiFFALevel), _P, _P, _P, _P]),
     "loki_ffa_level_score": (C.c_int, [C.POINTER(LokiFFALevel), _P, C.POINTER(LokiScoreSpec),

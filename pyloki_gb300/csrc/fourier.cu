@@ -435,28 +435,7 @@ __global__ void fold_norm_complex_kernel(const float2* __restrict__ folds, int64
   if (k >= n * nbins) return;
   const int64_t p = k / nbins;
   const int j = (int)(k - p * nbins);
-  float val[2];
-  for (int c = 0; c < 2; ++c) {
-    const float2* x = folds + (p * 2 + c) * nbf;
-    float acc = x[0].x;
-    int r = 0;
-    for (int m = 1; m < nbf; ++m) {
-      // the imaginary parts of the DC and (for even nbins) Nyquist terms are
-      // ignored; other terms count twice
-      r += j;
-      if (r >= nbins) r -= nbins;
-      const float cth = tw[r], s = tw[nbins + r];
-      const float2 xm = x[m];
-      if (2 * m == nbins) {
-        acc = __fmaf_rn(xm.x, cth, acc);
-      } else {
-        acc = __fmaf_rn(2.0f * xm.x, cth, acc);
-        acc = __fmaf_rn(-2.0f * xm.y, s, acc);
-      }
-    }
-    val[c] = __fdiv_rn(acc, (float)nbins);
-  }
-  out[k] = __fdiv_rn(val[0], __fsqrt_rn(val[1]));
+  out[k] = norm_bin_complex(folds + p * 2 * nbf, j, nbins, nbf, tw);
 }
 
 }  // namespace loki

@@ -4981,12 +4981,78 @@ prune_seed_batch_kernel(const LokiSeedJob* __restrict__ jobs, int nb, int P, Lok
   }
 }
 
+// The same of complex folds: rows of 2 (nb / 2 + 1) float2, eight a warp (a run's
+// few hundred seeds are one wave), normalised as fold_norm_complex_kernel does.
+// Per-run launches and copies (eight for each job) left the GPU idle for most of
+// 6 ms before the levels of 16 runs.
+constexpr int kSeedRows = 8;
+
+__global__ void __launch_bounds__(kPruneWarps * 32)
+prune_seed_batch_complex_kernel(const LokiSeedJob* __restrict__ jobs, int nb, int P,
+                                LokiScoreSpec sp, ScoreK SK) {
+  extern __shared__ float smem[];
+  const LokiSeedJob& J = jobs[blockIdx.y];
+  const int64_t n = J.n;
+  const int row_leaf = (P + 2) * 2, row_bt = P + 2, nbf = nb / 2 + 1;
+  const float2* rows = reinterpret_cast<const float2*>(J.fold_rows);
+  float2* fout = reinterpret_cast<float2*>(J.folds_out);
+  const int64_t gtid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t gstep = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = gtid; i < n * row_leaf; i += gstep) J.leaves_out[i] = J.seed_leaves[i];
+  for (int64_t i = gtid; i < n * 2 * nbf; i += gstep) fout[i] = rows[i];
+  for (int64_t i = gtid; i < n * row_bt; i += gstep) J.bt_out[i] = 0;
+  if (gtid == 0) *J.dev_err = 0;
+  load_twiddles(smem, nb);
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int stride = score_stride(nb, sp.wmax);
+  float* tile = smem + 2 * nb + (size_t)warp * kSeedRows * stride;
+  for (int64_t p0 = ((int64_t)blockIdx.x * kPruneWarps + warp) * kSeedRows; p0 < n;
+       p0 += (int64_t)gridDim.x * kPruneWarps * kSeedRows) {
+    const int kmax = (int)min((int64_t)kSeedRows, n - p0);
+    for (int k = 0; k < kmax; ++k)
+      for (int j = lane; j < nb; j += 32)
+        tile[k * stride + j] = norm_bin_complex(rows + (p0 + k) * 2 * nbf, j, nb, nbf, smem);
+    __syncwarp();
+    if (lane < kmax) {
+      float s;
+      float* row = tile + lane * stride;
+      if (SK.list64) score_row64(row, sp, SK, &s);
+      else score_row(row, nb, sp, SK, &s);
+      J.scores_out[p0 + lane] = s;
+      J.scores_ep_out[p0 + lane] = s;
+      J.seed_scores_out[p0 + lane] = s;
+    }
+    __syncwarp();
+  }
+}
+
 }  // namespace loki
+
+static int seed_batch(const LokiSeedJob* jobs, int32_t njobs, int32_t nbins, int32_t poly_order,
+                      const LokiScoreSpec* spec, void* dev_scratch, int64_t dev_scratch_bytes,
+                      bool cplx, void* stream);
 
 extern "C" int loki_prune_seed_batch(const LokiSeedJob* jobs, int32_t njobs, int32_t nbins,
                                      int32_t poly_order, const LokiScoreSpec* spec,
                                      void* dev_scratch, int64_t dev_scratch_bytes,
                                      void* stream) {
+  return seed_batch(jobs, njobs, nbins, poly_order, spec, dev_scratch, dev_scratch_bytes, false,
+                    stream);
+}
+
+extern "C" int loki_prune_seed_batch_complex(const LokiSeedJob* jobs, int32_t njobs,
+                                             int32_t nbins, int32_t poly_order,
+                                             const LokiScoreSpec* spec, void* dev_scratch,
+                                             int64_t dev_scratch_bytes, void* stream) {
+  if (nbins % 2) return set_error(LOKI_ERR_INVALID, "complex folds need an even nbins");
+  return seed_batch(jobs, njobs, nbins, poly_order, spec, dev_scratch, dev_scratch_bytes, true,
+                    stream);
+}
+
+static int seed_batch(const LokiSeedJob* jobs, int32_t njobs, int32_t nbins, int32_t poly_order,
+                      const LokiScoreSpec* spec, void* dev_scratch, int64_t dev_scratch_bytes,
+                      bool cplx, void* stream) {
   if (!jobs || njobs < 1 || njobs > 65535 || !spec || !dev_scratch || nbins < 2 ||
       poly_order < 1 || poly_order > LOKI_MAX_PARAMS)
     return set_error(LOKI_ERR_INVALID, "bad seed batch arguments");
@@ -5008,19 +5074,23 @@ extern "C" int loki_prune_seed_batch(const LokiSeedJob* jobs, int32_t njobs, int
   LokiScoreSpec sp = *spec;
   sp.mode = 1;
   const ScoreK SK = make_score_k(sp, nbins);
-  const int smem = score_smem_bytes(nbins, sp.wmax, kPruneWarps);
+  const int rows = cplx ? kSeedRows : 32;  // a warp's
+  const int smem = cplx ? (int)((2 * nbins + kPruneWarps * kSeedRows *
+                                                 score_stride(nbins, sp.wmax)) * sizeof(float))
+                        : score_smem_bytes(nbins, sp.wmax, kPruneWarps);
   if (smem > 200 * 1024) return set_error(LOKI_ERR_UNSUPPORTED, "nbins + wmax too large");
-  if (smem > 48 * 1024 && set_smem_limit(prune_seed_batch_kernel, smem) != cudaSuccess)
+  const auto kern = cplx ? prune_seed_batch_complex_kernel : prune_seed_batch_kernel;
+  if (smem > 48 * 1024 && set_smem_limit(kern, smem) != cudaSuccess)
     return set_error(LOKI_ERR_CUDA, "cudaFuncSetAttribute failed");
   cudaStream_t s = (cudaStream_t)stream;
   if (cudaMemcpyAsync(dev_scratch, jobs, njobs * sizeof(LokiSeedJob), cudaMemcpyHostToDevice,
                       s) != cudaSuccess)
     return set_error(LOKI_ERR_CUDA, "copy of the seed jobs failed");
   const unsigned bx =
-      (unsigned)std::max<int64_t>(1, std::min<int64_t>(32, (maxn + kPruneWarps * 32 - 1) /
-                                                               (kPruneWarps * 32)));
+      (unsigned)std::max<int64_t>(1, std::min<int64_t>(32, (maxn + kPruneWarps * rows - 1) /
+                                                               (kPruneWarps * rows)));
   note_launch();
-  prune_seed_batch_kernel<<<dim3(bx, njobs), kPruneWarps * 32, smem, s>>>(
+  kern<<<dim3(bx, njobs), kPruneWarps * 32, smem, s>>>(
       reinterpret_cast<const LokiSeedJob*>(dev_scratch), nbins, poly_order, sp, SK);
   return check_launch("prune_seed_batch");
 }

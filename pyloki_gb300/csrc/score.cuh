@@ -291,4 +291,33 @@ __device__ __forceinline__ void score_row(float* row, int nbins, const LokiScore
   if (sp.mode != 0) out[0] = K.inv_one ? best_f : __double2float_rn(best);
 }
 
+// Normalised bin j of a complex fold: the inverse transform of both components
+// (tw: cos, then sin, of 2 pi r / nbins), then e / sqrt(v).
+__device__ __forceinline__ float norm_bin_complex(const float2* __restrict__ fold, int j,
+                                                  int nbins, int nbf,
+                                                  const float* __restrict__ tw) {
+  float val[2];
+  for (int c = 0; c < 2; ++c) {
+    const float2* x = fold + c * nbf;
+    float acc = x[0].x;
+    int r = 0;
+    for (int m = 1; m < nbf; ++m) {
+      // the imaginary parts of the DC and (for even nbins) Nyquist terms are
+      // ignored; other terms count twice
+      r += j;
+      if (r >= nbins) r -= nbins;
+      const float cth = tw[r], s = tw[nbins + r];
+      const float2 xm = x[m];
+      if (2 * m == nbins) {
+        acc = __fmaf_rn(xm.x, cth, acc);
+      } else {
+        acc = __fmaf_rn(2.0f * xm.x, cth, acc);
+        acc = __fmaf_rn(-2.0f * xm.y, s, acc);
+      }
+    }
+    val[c] = __fdiv_rn(acc, (float)nbins);
+  }
+  return __fdiv_rn(val[0], __fsqrt_rn(val[1]));
+}
+
 }  // namespace loki

@@ -1399,7 +1399,8 @@ class _DeviceRun:
         stride = int(np.prod(prn.dyp.fold.shape[1:]))
         j = _lib.LokiSeedJob()
         j.seed_leaves = _lib.ptr(self.seed.leaves)
-        j.fold_rows = _lib.ptr(self._direct_fold) + 4 * self.ref_seg * stride
+        j.fold_rows = (_lib.ptr(self._direct_fold)
+                       + self._direct_fold.element_size() * self.ref_seg * stride)
         j.n = n
         j.leaves_out, j.folds_out = _lib.ptr(t0["leaves"]), _lib.ptr(t0["folds"])
         j.scores_out, j.scores_ep_out = _lib.ptr(t0["scores"]), _lib.ptr(t0["scores_ep"])
@@ -1911,16 +1912,18 @@ class PruneBlockBatch(PruneBatch):
         gather and one copy)."""
         nlev = runs[0][1].nlev
         n = len(runs)
-        if not fourier and all(prn.dyp.fold.dtype == torch.float32 for prn, _ in runs):
+        stored = torch.complex64 if fourier else torch.float32
+        if all(prn.dyp.fold.dtype == stored for prn, _ in runs):
             sjobs = (_lib.LokiSeedJob * n)()  # every job's seed in one launch
             for i, (prn, dr) in enumerate(runs):
                 sjobs[i] = dr.seed_job()
             p0 = runs[0][0]
             sbuf = self._dev_buf("seed", n * C.sizeof(_lib.LokiSeedJob), dev)
-            _lib.check(lib.loki_prune_seed_batch(
+            seed = lib.loki_prune_seed_batch_complex if fourier else lib.loki_prune_seed_batch
+            _lib.check(seed(
                 sjobs, n, p0.dyp.cfg.nbins, p0.poly_order, p0.spec, _lib.ptr(sbuf),
                 sbuf.numel(), _lib.stream_ptr(st)))
-        else:  # complex folds, or a fold stored in another type: per-job seeds
+        else:  # a fold stored in another type: per-job seeds
             for prn, dr in runs:
                 dr.prepare_block()
         if nlev > 0:
