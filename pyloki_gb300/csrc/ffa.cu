@@ -689,8 +689,9 @@ __device__ __forceinline__ float tile_build(const LokiFFALevel& P, const LevelK&
   const int r0 = warp * per;
   const int r1 = std::min(R, r0 + per);
   const int64_t P_in = n_in_params(P);
-  // lane k: row r0 + k; its source rows and shifts (ok in bit 16)
-  int64_t my_t = 0, my_h = 0;
+  // lane k: row r0 + k; its source rows (of 256 bytes or more: 32 bits hold their
+  // numbers) and shifts (ok in bit 16)
+  uint32_t my_t = 0, my_h = 0;
   int32_t my_sh = 0;
   if (r0 + lane < r1) {
     const int r = r0 + lane;
@@ -700,8 +701,8 @@ __device__ __forceinline__ float tile_build(const LokiFFALevel& P, const LevelK&
     const TrialRes tr = resolve_trial(P, KP, tab_p[po], tab_p[no_p + po], f8);
     const int64_t seg = 2 * (tail ? s_t : s_h) * P_in;
     if (tr.ok) {
-      my_t = (seg + tr.in_tail) * 128;
-      my_h = (seg + P_in + tr.in_head) * 128;
+      my_t = (uint32_t)(seg + tr.in_tail);
+      my_h = (uint32_t)(seg + P_in + tr.in_head);
     }
     my_sh = tr.s_tail | (tr.s_head << 8) | (tr.ok ? 1 << 16 : 0);
     if (!tr.ok) atomicOr(err, LOKI_DEVERR_WINDOW);
@@ -714,8 +715,8 @@ __device__ __forceinline__ float tile_build(const LokiFFALevel& P, const LevelK&
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
       const int k = min(r + u, r1 - 1) - r0;  // the last row again at a ragged end
-      const S* tp = fold_pp + __shfl_sync(0xFFFFFFFFu, my_t, k);
-      const S* hp = fold_pp + __shfl_sync(0xFFFFFFFFu, my_h, k);
+      const S* tp = fold_pp + (size_t)__shfl_sync(0xFFFFFFFFu, my_t, k) * 128;
+      const S* hp = fold_pp + (size_t)__shfl_sync(0xFFFFFFFFu, my_h, k) * 128;
       sh[u] = __shfl_sync(0xFFFFFFFFu, my_sh, k);
       const int jt = (lane - sh[u]) & 63, jh = (lane - (sh[u] >> 8)) & 63;
       t[u][0] = Store<S>::load(tp + jt);
