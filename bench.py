@@ -47,7 +47,7 @@ WORKLOAD = "ffa_accel_search_2^23"
 # trials); profiles/ffa_final_tiled64_kernel_ffa_accel_2^21.md. The banded
 # path's figure comes from three full-band launches at 2^21
 # (profiles/band_union64_kernel_ffa_accel_2^21.md).
-FINAL_DRAM_BYTES_PER_TRIAL = {"tiled": 70.2, "banded": 259.0}
+FINAL_DRAM_BYTES_PER_TRIAL = {"tiled": 81.1, "banded": 259.0}
 FINAL_KERNEL = {"tiled": "ffa_final_tiled64_kernel (last two levels fused per tile: "
                          "penultimate rows built in shared memory, lane-per-trial scoring)",
                 "banded": "band_union64_kernel (penultimate band + fused final-level scoring)",

@@ -2298,7 +2298,7 @@ circ_emit_complex_kernel(LokiPruneLevel D, const double* __restrict__ leaves,
 // and 32 + j have the same cosine and sine up to sign, so their four sums share
 // two products, and the 64 sums are independent registers. A lane walking its
 // rows in global memory and the bins one after the other took 56 ms for the 8.0e6
-// children of a 16-run search; now 10.5, of which 4 are the latency of the 100
+// children of a 16-run search; now 9.3, of which 2 are the latency of the 100
 // levels with fewer than 500 children a run.
 // ---------------------------------------------------------------------------
 
