@@ -255,6 +255,15 @@ __host__ __device__ inline int list_bytes(int T, int nbins, int wpf) {
   return (list_entries_off(wpf) + 4 * (T + nbins) + 15) & ~15;
 }
 
+// Bin of a warp's chain: the warps of a frequency take pairs of neighbouring bins
+// in turn. A chunk of a slow pulsar's series covers a run of neighbouring bins (10
+// of 64 at 0.2 s), which fell to one warp while the others of the block waited for
+// it when each took its bins in one piece (2^20 samples at 1-10 Hz: walk 0.55 ->
+// 0.40 ms; 100 bins at 20-150 Hz 2.58 -> 2.47; 50-500 Hz 6.76 -> 6.69).
+__host__ __device__ inline int chain_bin(int warp, int chain, int wpf) {
+  return 2 * ((chain >> 1) * wpf + warp) + (chain & 1);
+}
+
 // Rows [0, nseg) are the segments of ts_e, rows [nseg, 2 nseg) those of ts_v.
 // out: [row group][chunk][t][NS], zeros beyond the series and the last row.
 __global__ void __launch_bounds__(256)
@@ -383,9 +392,10 @@ chain_list_kernel(const double* __restrict__ freqs, int64_t seg_len, int nbins, 
     __syncwarp();
     // per bin (a lane each): the rank of every lane's first position, the
     // steps of its pair of bins and where they begin
-    int base = 0;  // steps of the bins before
-    for (int b0 = 0; b0 < nbins; b0 += 32) {
-      const int b = b0 + lane;
+    int base = 0;  // steps of the bins before (in the order of the warps' chains)
+    for (int s0 = 0; s0 < cs.wpf * cs.bpw; s0 += 32) {
+      const int kb = (s0 + lane) / cs.bpw, kc = s0 + lane - kb * cs.bpw;
+      const int b = kb < cs.wpf ? chain_bin(kb, kc, cs.wpf) : nbins;
       uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
       int c = 0;
       if (b < nbins) {
@@ -405,7 +415,6 @@ chain_list_kernel(const double* __restrict__ freqs, int64_t seg_len, int nbins, 
       }
       if (b < nbins) {
         const int at = 4 * (base + incl - st);  // the pair's first entry
-        const int kb = b / cs.bpw, kc = b - kb * cs.bpw;
         if (!(kc & 1)) steps[kb * (kChains / 2) + kc / 2] = (uint8_t)st;
         if (kc == 0) first[kb] = (uint32_t)at;
         if (counts) atomicAdd(&hist[b], c);
@@ -583,7 +592,7 @@ brutefold_chain_kernel(const float* __restrict__ rows, const uint8_t* __restrict
   if (active) {
 #pragma unroll
     for (int c = 0; c < kChains; ++c) {
-      const int b = kb * cs.bpw + c;
+      const int b = chain_bin(kb, c, cs.wpf);
       if (c < cs.bpw && b < nbins)
 #pragma unroll
         for (int v = 0; v < V; ++v) out_s[(lane * V + v) * stride + fi * nbins + b] = acc[c][v];
