@@ -612,13 +612,12 @@ __device__ __forceinline__ void score_tile_rows(float* tile, int stride, int nb,
 // Children c0 .. c0 + 31 (those below n_children) of one warp.
 template <int KP = 0>
 __device__ __forceinline__ void score_tile(
-                   const LokiPruneLevel& D, const double* __restrict__ leaves,
-                   const float* __restrict__ folds, int64_t n_parents,
-                   const LokiBranchInfo* __restrict__ info, const int64_t* __restrict__ offsets,
-                   int64_t n_children, const float* __restrict__ seg, const LokiScoreSpec& sp,
-                   const ScoreK& SK, float* __restrict__ scores, int32_t* __restrict__ cidx,
-                   double* __restrict__ cphase, unsigned* __restrict__ minmax_keys,
-                   float* tile, int64_t c0, int width = 32) {
+    const LokiPruneLevel& D, const double* __restrict__ leaves, const float* __restrict__ folds,
+    int64_t n_parents, const LokiBranchInfo* __restrict__ info,
+    const int64_t* __restrict__ offsets, int64_t n_children, const float* __restrict__ seg,
+    const LokiScoreSpec& sp, const ScoreK& SK, float* __restrict__ scores,
+    int32_t* __restrict__ cidx, double* __restrict__ cphase, unsigned* __restrict__ minmax_keys,
+    float* tile, int64_t c0, int width = 32) {
   const int lane = threadIdx.x & 31;
   const int nb = D.nbins, P = tree_order<KP>(D);
   const int stride = score_stride(nb, sp.wmax);
@@ -1017,16 +1016,13 @@ __device__ __forceinline__ void gather_add_rows(const float* __restrict__ folds,
 // Survivors s0 .. s0 + 31 (those below n_surv) of one warp.
 template <int KP = 0>
 __device__ __forceinline__ void emit_tile(
-                  const LokiPruneLevel& D, const double* __restrict__ leaves,
-                  const float* __restrict__ folds, const LokiBranchInfo* __restrict__ info,
-                  const int64_t* __restrict__ offsets, int64_t n_parents,
-                  const float* __restrict__ seg, const int64_t* __restrict__ surv,
-                  int64_t n_surv, const float* __restrict__ cscores,
-                  const int32_t* __restrict__ cidx, const double* __restrict__ cphase,
-                  double* __restrict__ lout, float* __restrict__ fout,
-                  float* __restrict__ sout, float* __restrict__ seout,
-                  int32_t* __restrict__ bout, int64_t s0, const EmitExtra& X = EmitExtra(),
-    int width = 32) {
+    const LokiPruneLevel& D, const double* __restrict__ leaves, const float* __restrict__ folds,
+    const LokiBranchInfo* __restrict__ info, const int64_t* __restrict__ offsets,
+    int64_t n_parents, const float* __restrict__ seg, const int64_t* __restrict__ surv,
+    int64_t n_surv, const float* __restrict__ cscores, const int32_t* __restrict__ cidx,
+    const double* __restrict__ cphase, double* __restrict__ lout, float* __restrict__ fout,
+    float* __restrict__ sout, float* __restrict__ seout, int32_t* __restrict__ bout, int64_t s0,
+    const EmitExtra& X = EmitExtra(), int width = 32) {
   const int lane = threadIdx.x & 31;
   const int nb = D.nbins, P = tree_order<KP>(D), m = P + 1;
   const int kmax = (int)std::min<int64_t>(width, n_surv - s0);
@@ -1153,13 +1149,12 @@ __device__ __forceinline__ void circ_shift(const double* p, double dt, bool hole
 
 // Survivors s0 .. s0 + 31 (those below n) of one warp; acc and tile are the
 // warp's accumulators (32 x 2 nb) and score tile.
-__device__ __forceinline__ void ascend_tile(const LokiPruneLevel& D, const double* __restrict__ leaves,
-                    float* __restrict__ folds, float* __restrict__ scores,
-                    float* __restrict__ scores_ep, int64_t n, int nseg,
-                    const double* __restrict__ tm_seg, const double* __restrict__ dt_seg,
-                    const int32_t* __restrict__ seg_idx, const float* __restrict__ ffa,
-                    int64_t seg_stride, const LokiScoreSpec& sp, const ScoreK& SK, float* acc,
-                    float* tile, int64_t s0) {
+__device__ __forceinline__ void ascend_tile(
+    const LokiPruneLevel& D, const double* __restrict__ leaves, float* __restrict__ folds,
+    float* __restrict__ scores, float* __restrict__ scores_ep, int64_t n, int nseg,
+    const double* __restrict__ tm_seg, const double* __restrict__ dt_seg,
+    const int32_t* __restrict__ seg_idx, const float* __restrict__ ffa, int64_t seg_stride,
+    const LokiScoreSpec& sp, const ScoreK& SK, float* acc, float* tile, int64_t s0) {
   const int lane = threadIdx.x & 31;
   const int nb = D.nbins, P = D.poly_order, m = P + 1;
   const int stride = score_stride(nb, sp.wmax);
@@ -1610,15 +1605,14 @@ __device__ __forceinline__ int circ_resolve(const LokiPruneLevel& D, const doubl
 }
 
 // Valid children v0 .. v0 + 31 (those below n_valid) of one warp.
-__device__ __forceinline__ void circ_score_tile(const LokiPruneLevel& D, const double* __restrict__ leaves,
-                  const float* __restrict__ folds, int64_t batch,
-                  const LokiBranchInfo* __restrict__ info, const CircChild* __restrict__ map,
-                  const int64_t* __restrict__ valid_ids, int64_t n_valid,
-                  const float* __restrict__ seg, const LokiScoreSpec& sp, const ScoreK& SK,
-                  float* __restrict__ scores, int32_t* __restrict__ cidx,
-                  double* __restrict__ cphase, int8_t* __restrict__ ccls,
-                  int32_t* __restrict__ batch_taylor, unsigned* __restrict__ minmax_keys,
-                  float* tile, int64_t v0, int width = 32) {
+__device__ __forceinline__ void circ_score_tile(
+    const LokiPruneLevel& D, const double* __restrict__ leaves, const float* __restrict__ folds,
+    int64_t batch, const LokiBranchInfo* __restrict__ info, const CircChild* __restrict__ map,
+    const int64_t* __restrict__ valid_ids, int64_t n_valid, const float* __restrict__ seg,
+    const LokiScoreSpec& sp, const ScoreK& SK, float* __restrict__ scores,
+    int32_t* __restrict__ cidx, double* __restrict__ cphase, int8_t* __restrict__ ccls,
+    int32_t* __restrict__ batch_taylor, unsigned* __restrict__ minmax_keys, float* tile,
+    int64_t v0, int width = 32) {
   const int lane = threadIdx.x & 31;
   const int nb = D.nbins, P = 5;
   const int stride = score_stride(nb, sp.wmax);
@@ -1688,17 +1682,16 @@ circ_score_kernel(LokiPruneLevel D, const double* __restrict__ leaves,
 // the crackle children of a batch that also holds Taylor children), backtracks
 // and folds.
 // Survivors s0 .. s0 + 31 (those below n_surv) of one warp.
-__device__ __forceinline__ void circ_emit_tile(const LokiPruneLevel& D, const double* __restrict__ leaves,
-                 const float* __restrict__ folds, int64_t batch,
-                 const LokiBranchInfo* __restrict__ info, const CircChild* __restrict__ map,
-                 const int64_t* __restrict__ valid_ids, const float* __restrict__ seg,
-                 const int64_t* __restrict__ surv, int64_t n_surv,
-                 const float* __restrict__ cscores, const int32_t* __restrict__ cidx,
-                 const double* __restrict__ cphase, const int8_t* __restrict__ ccls,
-                 const int32_t* __restrict__ batch_taylor, double* __restrict__ lout,
-                 float* __restrict__ fout, float* __restrict__ sout,
-                 float* __restrict__ seout, int32_t* __restrict__ bout, int64_t s0, const EmitExtra& X = EmitExtra(),
-    int width = 32) {
+__device__ __forceinline__ void circ_emit_tile(
+    const LokiPruneLevel& D, const double* __restrict__ leaves, const float* __restrict__ folds,
+    int64_t batch, const LokiBranchInfo* __restrict__ info, const CircChild* __restrict__ map,
+    const int64_t* __restrict__ valid_ids, const float* __restrict__ seg,
+    const int64_t* __restrict__ surv, int64_t n_surv, const float* __restrict__ cscores,
+    const int32_t* __restrict__ cidx, const double* __restrict__ cphase,
+    const int8_t* __restrict__ ccls, const int32_t* __restrict__ batch_taylor,
+    double* __restrict__ lout, float* __restrict__ fout, float* __restrict__ sout,
+    float* __restrict__ seout, int32_t* __restrict__ bout, int64_t s0,
+    const EmitExtra& X = EmitExtra(), int width = 32) {
   const int lane = threadIdx.x & 31;
   const int nb = D.nbins, P = 5, m = 6;
   const int kmax = (int)std::min<int64_t>(width, n_surv - s0);
@@ -1875,7 +1868,8 @@ __host__ __device__ inline size_t cplx_warp_floats(int nbins, int stride) {
 __device__ __forceinline__ void score_child_complex(
     const LokiPruneLevel& D, const double* __restrict__ leaves, const float2* __restrict__ folds,
     int64_t n_parents, const LokiBranchInfo* __restrict__ info,
-    const int64_t* __restrict__ offsets, const float2* __restrict__ seg, const LokiScoreSpec& sp, const ScoreK& SK,
+    const int64_t* __restrict__ offsets, const float2* __restrict__ seg, const LokiScoreSpec& sp,
+    const ScoreK& SK,
     float* __restrict__ scores, int32_t* __restrict__ cidx, double* __restrict__ cphase,
     unsigned* __restrict__ minmax_keys, const float* tw, float2* comb, float* trow, int64_t c) {
   const int nb = D.nbins, nbf = nb / 2 + 1, P = D.poly_order;
@@ -2028,7 +2022,8 @@ __device__ __forceinline__ void ascend_one_complex(
     float* __restrict__ scores, float* __restrict__ scores_ep, int nseg,
     const double* __restrict__ tm_seg, const double* __restrict__ dt_seg,
     const int32_t* __restrict__ seg_idx, const float2* __restrict__ ffa, int64_t seg_stride,
-    const LokiScoreSpec& sp, const ScoreK& SK, const float* tw, float2* comb, float* trow, int64_t r) {
+    const LokiScoreSpec& sp, const ScoreK& SK, const float* tw, float2* comb, float* trow,
+    int64_t r) {
   const int nb = D.nbins, nbf = nb / 2 + 1, P = D.poly_order, m = P + 1;
   const double* lf = leaves + r * (P + 2) * 2;
   double pv[LOKI_MAX_PARAMS + 1], ev[LOKI_MAX_PARAMS + 1];
@@ -4172,7 +4167,8 @@ bj_score_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
     score_tile<KP>(Q.lvl, in.leaves, in.folds, J.run.counts[kCntPar],
                reinterpret_cast<LokiBranchInfo*>(w.info), w.offsets, n_child,
                static_cast<const float*>(job_segment(T, J, job, l, 4)), A.sp, A.SK, w.child_scores,
-               w.child_idx, w.child_phase, reinterpret_cast<unsigned*>(w.minmax), tile, c0, Q.width);
+               w.child_idx, w.child_phase, reinterpret_cast<unsigned*>(w.minmax), tile, c0,
+               Q.width);
     __syncwarp();
   });
 }
@@ -4191,7 +4187,8 @@ __device__ __forceinline__ EmitExtra job_extra(const LokiPruneRun& R, int l, int
 }
 
 template <int KP>
-__global__ void __launch_bounds__(kTile, 4) bj_emit_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
+__global__ void __launch_bounds__(kTile, 4)
+bj_emit_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
   __shared__ JobQueue Q;
   const int warp = threadIdx.x >> 5;
   queue_run(Q, T, l, j0, nj, kCntSurv, kNarrow16, [&](int job, int64_t t) {
@@ -4290,7 +4287,8 @@ bj_emit_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
     const LokiBranchInfo* info = reinterpret_cast<LokiBranchInfo*>(w.info);
     const float2* folds = reinterpret_cast<const float2*>(in.folds);
     const float2* seg = static_cast<const float2*>(job_segment(T, J, job, l, 8));
-    const int64_t n_surv = R.counts[kCntSurv], s0 = (t * kPruneWarps + warp) * Q.width, s = s0 + lane;
+    const int64_t n_surv = R.counts[kCntSurv], s0 = (t * kPruneWarps + warp) * Q.width;
+    const int64_t s = s0 + lane;
     if (s0 >= n_surv) return;
     const int kmax = (int)min((int64_t)Q.width, n_surv - s0), nbf = A.nb / 2 + 1;
     const int64_t par = warp_find_parents(w.offsets, R.counts[kCntOldPar],
@@ -4405,15 +4403,16 @@ bj_circ_score_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
     const float2* folds = reinterpret_cast<const float2*>(in.folds);
     const float2* seg = static_cast<const float2*>(job_segment(T, J, job, l, 8));
     unsigned* keys = reinterpret_cast<unsigned*>(w.minmax);
-    const int64_t n_valid = R.counts[kCntValid], v0 = (t * kPruneWarps + warp) * Q.width, v = v0 + lane;
+    const int64_t n_valid = R.counts[kCntValid], v0 = (t * kPruneWarps + warp) * Q.width;
+    const int64_t v = v0 + lane;
     if (v0 >= n_valid) return;
     const int kmax = (int)min((int64_t)Q.width, n_valid - v0);
     const LokiPruneLevel& D = Q.lvl;
     if (A.nb != 64) {
       float* wbase = smem + 2 * A.nb + (size_t)warp * cplx_warp_floats(A.nb, stride);
       if (lane < kmax)
-        circ_score_one_complex(D, in.leaves, folds, A.batch, info, map, R.valid_ids, seg, A.sp, A.SK,
-                               smem, reinterpret_cast<float2*>(wbase) + (size_t)lane * 2 * nbf,
+        circ_score_one_complex(D, in.leaves, folds, A.batch, info, map, R.valid_ids, seg, A.sp,
+                               A.SK, smem, reinterpret_cast<float2*>(wbase) + (size_t)lane * 2 * nbf,
                                wbase + (size_t)32 * 2 * nbf * 2 + lane * stride, w.child_scores,
                                w.child_idx, w.child_phase, R.child_class, R.batch_taylor, keys,
                                v);
@@ -4459,7 +4458,8 @@ bj_circ_emit_complex_kernel(BatchTabs T, int l, int j0, int nj, LevelArgs A) {
     const LokiPruneTree &in = R.trees[(l - 1) & 1], &out = R.trees[l & 1];
     const float2* folds = reinterpret_cast<const float2*>(in.folds);
     const float2* seg = static_cast<const float2*>(job_segment(T, J, job, l, 8));
-    const int64_t n_surv = R.counts[kCntSurv], s0 = (t * kPruneWarps + warp) * Q.width, s = s0 + lane;
+    const int64_t n_surv = R.counts[kCntSurv], s0 = (t * kPruneWarps + warp) * Q.width;
+    const int64_t s = s0 + lane;
     if (s0 >= n_surv) return;
     const int kmax = (int)min((int64_t)Q.width, n_surv - s0), nbf = A.nb / 2 + 1;
     EmitRow r = {0, 0, 0.0};
@@ -4636,8 +4636,9 @@ static int batch_enqueue(void* dev_scratch, int32_t njobs, int32_t nlevels,
     int per = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kTile, bytes) != cudaSuccess)
       return set_error(LOKI_ERR_CUDA, "occupancy query failed");
-    *g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)nsm * std::max(1, per),
-                                                          (items + kPruneWarps * 8 - 1) / (kPruneWarps * 8) * nj_max));
+    const int64_t tiles = (items + kPruneWarps * 8 - 1) / (kPruneWarps * 8) * nj_max;
+    *g = (unsigned)std::max<int64_t>(1,
+                                     std::min<int64_t>((int64_t)nsm * std::max(1, per), tiles));
     return (int)LOKI_OK;
   };
   unsigned g_branch = 1, g_map = 1, g_score = 1, g_emit = 1;
