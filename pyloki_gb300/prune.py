@@ -1793,7 +1793,8 @@ class PruneBlockBatch(PruneBatch):
         """The batch's kernels over the tables just copied: enqueued directly
         the first time a shape is seen, then captured once in a CUDA graph
         and replayed (the tables are read on the device, so a replay runs
-        whatever jobs were copied in)."""
+        whatever jobs were copied in; the score spec is an argument of the
+        captured launches, so a graph serves its own widths alone)."""
         if self.__dict__.get("time_score"):  # measurement: uncaptured, timed score launches
             ms = np.zeros(nlev, np.float32)
             _lib.check(lib.loki_prune_batch_score_times(
@@ -1801,7 +1802,7 @@ class PruneBlockBatch(PruneBatch):
                 _lib.stream_ptr(st)))
             self.score_ms = ms
             return
-        key = (n, nlev, tuple(int(v) for v in shape), args[1], args[2])
+        key = (n, nlev, tuple(int(v) for v in shape), bytes(args[0]), args[1], args[2])
         graphs = self.__dict__.setdefault("_graphs", {})
         g = graphs.get(key)
         if g is None and key not in self.__dict__.setdefault("_seen", set()):

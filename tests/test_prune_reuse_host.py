@@ -1,0 +1,54 @@
+"""Batch runners used again for folds of another configuration, on the host:
+what is kept from one call to the next belongs to the configuration it was
+made for."""
+
+from __future__ import annotations
+
+import contextlib
+import types
+
+import numpy as np
+import torch
+
+from pyloki_gb300 import _lib
+from pyloki_gb300.prune import PruneBlockBatch
+
+
+def test_a_captured_batch_serves_its_own_widths_alone(monkeypatch):
+    """The score spec is baked into the captured launches: a batch of the same
+    shape with other widths is enqueued anew, and captured for itself."""
+    log = []
+    stream = types.SimpleNamespace(cuda_stream=0, wait_stream=lambda other: None)
+
+    class Graph:
+        def replay(self):
+            log.append(("replay", self.spec))
+
+    captured = []
+
+    def capture(graph, stream):
+        captured.append(graph)
+        return contextlib.nullcontext()
+
+    class Lib:
+        def loki_prune_batch_enqueue(self, scratch, n, nlev, spec, *rest):
+            log.append(("enqueue", bytes(spec)))
+            if captured and not hasattr(captured[-1], "spec"):
+                captured[-1].spec = bytes(spec)
+            return _lib.LOKI_OK
+
+    monkeypatch.setattr(torch.cuda, "Stream", lambda dev: stream)
+    monkeypatch.setattr(torch.cuda, "CUDAGraph", Graph)
+    monkeypatch.setattr(torch.cuda, "stream", lambda st: contextlib.nullcontext())
+    monkeypatch.setattr(torch.cuda, "graph", capture)
+    b = PruneBlockBatch.__new__(PruneBlockBatch)
+    b._scratch = torch.zeros(8, dtype=torch.uint8)
+    shape = np.array([64, 4, 1 << 10, 1 << 13, 0, 0], np.int64)
+    a = _lib.score_spec(np.array([1, 2, 3, 4, 6, 9]), 64, 1.0, mode=1)
+    w = _lib.score_spec(np.array([1, 2, 4, 8, 16]), 64, 1.0, mode=1)
+    for spec in (a, a, a, w, w, w, a):
+        b._enqueue_batch(Lib(), "cuda", stream, 3, 5, (spec, 1 << 10, 64), shape)
+    assert log == [(k, bytes(s)) for k, s in
+                   [("enqueue", a), ("enqueue", a), ("replay", a), ("replay", a),
+                    ("enqueue", w), ("enqueue", w), ("replay", w), ("replay", w),
+                    ("replay", a)]]
