@@ -1973,10 +1973,13 @@ class PruneBlockBatch(PruneBatch):
         device is one DMA), segment order and thresholds of ``runs``, job
         after job. They depend only on each run's configuration, reference
         segment and levels, so a call over the same runs (new folds or not)
-        reuses them."""
-        key = tuple((id(prn), dr.ref_seg, dr.nlev, id(dr)) for prn, dr in runs)
+        reuses them. A run is told by its own descriptor array, made with it;
+        the arrays of the kept tables are held, so that no later run's can
+        take the place of one in memory."""
+        descs = [dr.descs for _, dr in runs]
         cached = self.__dict__.get("_lv_cache")
-        if cached is not None and cached[0] == key:
+        if (cached is not None and len(cached[0]) == len(descs)
+                and all(a is b for a, b in zip(cached[0], descs))):
             return cached[1:4]
         n = len(runs)
         size = C.sizeof(_lib.LokiPruneLevel)
@@ -1991,7 +1994,7 @@ class PruneBlockBatch(PruneBatch):
             C.memmove(C.byref(lv, i * nlev * size), dr.descs, nlev * size)
             seg[i] = dr.seg_idx
             thr[i] = dr.thresholds
-        self._lv_cache = (key, lv, seg, thr, pin)
+        self._lv_cache = (descs, lv, seg, thr, pin)
         return lv, seg, thr
 
     def _dev_buf(self, name: str, nbytes: int, dev):

@@ -5,6 +5,7 @@ made for."""
 from __future__ import annotations
 
 import contextlib
+import gc
 import types
 
 import numpy as np
@@ -52,3 +53,41 @@ def test_a_captured_batch_serves_its_own_widths_alone(monkeypatch):
                    [("enqueue", a), ("enqueue", a), ("replay", a), ("replay", a),
                     ("enqueue", w), ("enqueue", w), ("replay", w), ("replay", w),
                     ("replay", a)]]
+
+
+def _run(ref: int, nlev: int):
+    dr = types.SimpleNamespace(ref_seg=ref, nlev=nlev)
+    dr.descs = (_lib.LokiPruneLevel * nlev)()
+    for i in range(nlev):
+        dr.descs[i].nbins = 1000 * ref + i  # a recognisable field per (run, level)
+    dr.seg_idx = np.arange(nlev, dtype=np.int32) + ref
+    dr.thresholds = np.full(nlev, float(ref))
+    return dr
+
+
+def test_level_tables_of_a_run_in_a_dropped_one_s_place(monkeypatch):
+    """A run made where a dropped one stood in memory (the same address, reference
+    segment and levels) gets its own tables."""
+    empty = torch.empty
+    monkeypatch.setattr(torch, "empty",
+                        lambda n, dtype, pin_memory=False: empty(n, dtype=dtype))
+    b = PruneBlockBatch.__new__(PruneBlockBatch)
+    prn = object()
+    dr = _run(3, 4)
+    b._level_tables([(prn, dr)], 4)
+    place = id(dr)
+    del dr
+    gc.collect()
+    held = []
+    for _ in range(10000):
+        new = types.SimpleNamespace()
+        if id(new) == place:
+            break
+        held.append(new)
+    assert id(new) == place
+    new.__dict__.update(_run(8, 4).__dict__)
+    new.ref_seg = 3
+    lv, seg, thr = b._level_tables([(prn, new)], 4)
+    assert [lv[i].nbins for i in range(4)] == [8000, 8001, 8002, 8003]
+    np.testing.assert_array_equal(seg[0], np.arange(4) + 8)
+    np.testing.assert_array_equal(thr[0], np.full(4, 8.0))
