@@ -973,13 +973,16 @@ class Pruning:
         constants and captured run graphs (they read the fold through a copy
         made before every device-resident run)."""
         a, b = self.dyp, dyp
+        keys = ["nsamps", "tsamp", "nbins", "eta", "bseg_brute", "bseg_ffa",
+                "prune_poly_order", "ducy_max", "wtsp", "use_fourier", "branch_max",
+                "tiling_strategy"]
+        if self.circular:  # the level constants of this tree hold these too
+            keys += ["p_orb_min", "x_mass_const", "propagator_significance",
+                     "validation_significance"]
         same = (a.fold.shape == b.fold.shape and a.fold.dtype == b.fold.dtype
                 and a.device == b.device and a.nsegments == b.nsegments
                 and np.array_equal(a.cfg.param_limits, b.cfg.param_limits)
-                and all(getattr(a.cfg, k) == getattr(b.cfg, k)
-                        for k in ("nsamps", "tsamp", "nbins", "eta", "bseg_brute", "bseg_ffa",
-                                  "prune_poly_order", "ducy_max", "wtsp", "use_fourier",
-                                  "branch_max", "tiling_strategy")))
+                and all(getattr(a.cfg, k) == getattr(b.cfg, k) for k in keys))
         if not same:
             msg = "rebind needs a fold of the same configuration and shape"
             raise ValueError(msg)

@@ -5,14 +5,16 @@ made for."""
 from __future__ import annotations
 
 import contextlib
+import dataclasses
 import gc
 import types
 
 import numpy as np
+import pytest
 import torch
 
-from pyloki_gb300 import _lib
-from pyloki_gb300.prune import PruneBlockBatch
+from pyloki_gb300 import ParamLimits, PulsarSearchConfig, _lib
+from pyloki_gb300.prune import PruneBlockBatch, Pruning
 
 
 def test_a_captured_batch_serves_its_own_widths_alone(monkeypatch):
@@ -91,3 +93,30 @@ def test_level_tables_of_a_run_in_a_dropped_one_s_place(monkeypatch):
     assert [lv[i].nbins for i in range(4)] == [8000, 8001, 8002, 8003]
     np.testing.assert_array_equal(seg[0], np.arange(4) + 8)
     np.testing.assert_array_equal(thr[0], np.full(4, 8.0))
+
+
+@pytest.mark.parametrize(("field", "value"),
+                         [("p_orb_min", 14400.0), ("m_c_max", 5.0), ("m_p_min", 1.2),
+                          ("propagator_significance", 3.0), ("validation_significance", 4.0)])
+def test_rebind_refuses_another_circular_configuration(field, value):
+    """The constants of the circular tree's levels are kept by a rebind, so a
+    fold of another orbit, mass or significance limit is not the same
+    configuration; the polynomial trees do not read them."""
+    lim = ParamLimits.from_circular(333.33, p_orb_min=7200.0, poly_order=5).limits
+    cfg = PulsarSearchConfig(nsamps=1 << 17, tsamp=64e-6, nbins=64, eta=1.0, param_limits=lim,
+                             use_fourier=False, bseg_ffa=1 << 15, prune_poly_order=5,
+                             p_orb_min=7200.0)
+
+    def dyp(c):
+        return types.SimpleNamespace(cfg=c, fold=torch.zeros(2, 2), device="cuda", nsegments=4)
+
+    prn = Pruning.__new__(Pruning)
+    prn._dyp = dyp(cfg)
+    other = dyp(dataclasses.replace(cfg, **{field: value}))
+    prn.circular = True
+    prn.rebind(dyp(dataclasses.replace(cfg)))
+    with pytest.raises(ValueError, match="same configuration"):
+        prn.rebind(other)
+    prn.circular = False
+    prn.rebind(other)
+    assert prn.dyp is other
