@@ -1185,7 +1185,15 @@ class Pruning:
 class _DeviceBuffers:
     """Trees and workspace of device-resident runs on one Pruning object."""
 
+    @staticmethod
+    def layout_of(prn: Pruning) -> tuple:
+        """What the sizes of the buffers hang on beside their capacities: rows
+        of another order, bin count or domain would run over their ends."""
+        return (prn.poly_order, prn.dyp.cfg.nbins, prn.fourier, prn.circular, prn.max_sugg,
+                prn.batch_size, prn.dyp.nsegments, str(prn._device))
+
     def __init__(self, prn: Pruning, child_cap: int, bt_rows: int) -> None:
+        self.layout = self.layout_of(prn)
         dev = prn._device
         P, nb, cap = prn.poly_order, prn.dyp.cfg.nbins, prn.max_sugg
         nlev = max(prn.dyp.nsegments - 1, 1)
@@ -1289,8 +1297,10 @@ class _DeviceRun:
         if grow is not None:
             child_cap = max(child_cap, grow.need_child, bufs.child_cap if bufs else 0)
             bt_rows = max(bt_rows, grow.need_bt, bufs.bt_rows if bufs else 0)
-        if (bufs is None or bufs.child_cap < child_cap or bufs.bt_rows < bt_rows
-                or bufs.mem["mirror"].numel() < dyp.fold.numel()):
+        if (bufs is None or bufs.layout != _DeviceBuffers.layout_of(prn)
+                or bufs.child_cap < child_cap or bufs.bt_rows < bt_rows
+                or bufs.mem["mirror"].numel() < dyp.fold.numel()
+                or bufs.mem["mirror"].dtype != dyp.fold.dtype):
             prn.__dict__.pop("_device_runs", None)  # their graphs hold the old buffers
             bufs = prn._device_bufs = _DeviceBuffers(prn, child_cap, bt_rows)
         self.bufs = bufs

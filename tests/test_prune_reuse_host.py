@@ -14,7 +14,7 @@ import pytest
 import torch
 
 from pyloki_gb300 import ParamLimits, PulsarSearchConfig, _lib
-from pyloki_gb300.prune import PruneBlockBatch, Pruning
+from pyloki_gb300.prune import PruneBatch, PruneBlockBatch, Pruning, _DeviceRun
 
 
 def test_a_captured_batch_serves_its_own_widths_alone(monkeypatch):
@@ -120,3 +120,44 @@ def test_rebind_refuses_another_circular_configuration(field, value):
     prn.circular = False
     prn.rebind(other)
     assert prn.dyp is other
+
+
+def _pruning(order, nbins, fourier, cap, nseg=4, batch=8):
+    cols, dtype = (nbins // 2 + 1, torch.complex64) if fourier else (nbins, torch.float32)
+    dyp = types.SimpleNamespace(cfg=types.SimpleNamespace(nbins=nbins), nsegments=nseg, tseg=1.0,
+                                fold=torch.zeros((nseg, 3, 2, cols), dtype=dtype))
+    return types.SimpleNamespace(
+        dyp=dyp, poly_order=order, fourier=fourier, circular=order == 5, max_sugg=cap,
+        batch_size=batch, device_child_cap=64, _device=torch.device("cpu"),
+        _lib=types.SimpleNamespace(loki_scan_scratch_bytes=lambda n: 64),
+        threshold_scheme=np.ones(nseg - 1), _fold_segment=lambda ref: None,
+        _seed=lambda seg: types.SimpleNamespace(size=3),
+        level_desc=lambda lvl: _lib.LokiPruneLevel(), rebind=None)
+
+
+@pytest.mark.parametrize("other", [(4, 128, False, 16), (6, 64, False, 16), (5, 64, False, 16),
+                                   (4, 64, True, 16), (4, 64, False, 32), (4, 64, False, 16, 9),
+                                   (4, 64, False, 16, 4, 2)])
+def test_run_buffers_are_not_taken_over_by_rows_of_another_size(monkeypatch, other):
+    """A stream of a batch hands its run buffers to the next Pruning on it. A
+    tree of other rows (order, bins, domain), capacity or length gets its own."""
+    made = [_pruning(4, 64, False, 16), _pruning(*other), _pruning(*other)]
+    monkeypatch.setattr("pyloki_gb300.prune.Pruning", lambda dyp, scheme: made.pop(0))
+    b = PruneBatch(np.ones(3), n_streams=1)
+    b._prns, b._bufs = [{}], [None]
+    bufs = []
+    for k in range(3):
+        b._prns[0].clear()
+        prn = b._pruning(0, None)
+        bufs.append(_DeviceRun(prn, 1, prn.dyp.nsegments - 1).bufs)
+        b._bufs[0] = prn._device_bufs
+        P, nb, fourier, cap = (4, 64, False, 16) if k == 0 else other[:4]
+        for tree in bufs[k].trees:
+            assert tree["leaves"].shape == (cap, P + 2, 2)
+            assert tree["bt"].shape == (cap, P + 2)
+            assert tree["folds"].shape == (cap, 2, nb // 2 + 1 if fourier else nb)
+            assert tree["folds"].is_complex() == fourier
+        assert len(bufs[k].mem["best_scores"]) == prn.dyp.nsegments - 1
+        assert ("btay" in bufs[k].mem) == (P == 5)
+    assert bufs[1] is not bufs[0]
+    assert bufs[2] is bufs[1]  # the same rows: handed on
