@@ -102,9 +102,9 @@ int64_t loki_launch_count(void);
  * the FFA. Replaces core/fold.py:108-171 brutefold_start (called through
  * ffa_taylor_init, core/fold.py:527-569). Per (segment, freq, bin) the sum is
  * taken in sample order, so the result is bit-identical to the reference.
- * phase_scratch holds the (freq, sample) phase-bin map; it may be smaller
- * than nfreqs * segment_len bytes (nbins <= 256) or 2x that (nbins > 256),
- * in which case the frequencies are processed in chunks. */
+ * phase_scratch holds at least one frequency's phase-bin map (segment_len
+ * bytes with nbins <= 256, twice that above); with less than
+ * loki_brutefold_series_scratch_bytes() the work is done in pieces. */
 int loki_brutefold(const float* ts_e, const float* ts_v, int64_t nsamps,
                    const double* freqs, int64_t nfreqs, int64_t segment_len,
                    int32_t nbins, double tsamp, double t_ref,
@@ -114,14 +114,15 @@ int loki_brutefold(const float* ts_e, const float* ts_v, int64_t nsamps,
 /* Scratch bytes with which loki_brutefold / loki_brutefold_unit_variance fold
  * nsamps samples at all nfreqs frequencies in one pass. With nbins <= 256 that
  * is the series laid out by time chunk plus, per frequency and chunk, the
- * chunk's positions sorted by bin; a smaller scratch takes the frequencies,
- * then the segments, in chunks, and one too small for 32 segments and a
- * frequency of that layout uses the phase map alone (segment_len bytes a
- * frequency, twice that with nbins > 256). No reference counterpart. */
+ * chunk's positions sorted by bin. A smaller scratch takes the frequencies, or
+ * runs of chunks and the frequencies, in pieces; one too small for a chunk of
+ * every segment and the lists of frequencies that fill the GPU uses the phase
+ * map (segment_len bytes a frequency, twice that with nbins > 256). No
+ * reference counterpart. */
 int64_t loki_brutefold_series_scratch_bytes(int64_t nsamps, int64_t nfreqs,
                                             int64_t segment_len, int32_t nbins,
                                             int32_t unit_variance);
-/* The same for 64 segments of a series (longer ones are taken in chunks). */
+/* The same for 64 segments of a series (longer ones are taken in pieces). */
 int64_t loki_brutefold_scratch_bytes(int64_t nfreqs, int64_t segment_len, int32_t nbins);
 
 /* loki_brutefold for a series whose ts_v is all ones (the normalised series
@@ -141,9 +142,10 @@ int loki_brutefold_unit_variance(const float* ts_e, int64_t nsamps, const double
  * not allocate device memory: cudaMalloc and cudaFree synchronise the whole
  * device, stalling a host pipeline that keeps other streams busy, and a host
  * that holds a fixed device-memory budget has nothing left to hand out.
- * The map lives in a fixed 16 MiB device array of the library (its size is
- * returned by loki_brutefold_noalloc_scratch_bytes), so segment_len is
- * limited to 16 Mi samples for nbins <= 256 and 8 Mi for nbins > 256;
+ * The scratch is a fixed 16 MiB device array of the library (its size is
+ * returned by loki_brutefold_noalloc_scratch_bytes), which has to hold one
+ * frequency's phase map: segment_len is limited to 16 Mi samples for
+ * nbins <= 256 and 8 Mi for nbins > 256;
  * beyond that it returns LOKI_ERR_CAPACITY. The array is shared by all calls
  * on one device: calls that overlap on the GPU (different streams, no
  * ordering between them) race on it; calls on one stream are ordered. */

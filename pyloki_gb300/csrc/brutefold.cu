@@ -208,18 +208,20 @@ brutefold_count_kernel(const T* __restrict__ map, int64_t nfreq_chunk, int64_t f
 // segment, so the order is built once per frequency, not once per row:
 //
 // 1. series_rows_kernel lays the series out by time chunk: for a group of NS
-//    rows (32 V lanes' worth) and a chunk of T samples, [t][row], so that a
-//    chunk is one contiguous copy and the rows of one sample are one
-//    conflict-free shared-memory load.
+//    rows and a chunk of T samples, [t][row], so that a chunk is one contiguous
+//    copy and the rows of one sample are one conflict-free shared-memory load.
 // 2. chain_list_kernel sorts each chunk's T positions by bin (stable) for one
 //    frequency and writes them as steps of two neighbouring bins: two
 //    positions of the even bin, two of the odd one, in time order, padded with
 //    position T, a row of zeros. Adding +0 leaves a sum unchanged (a sum that
 //    starts at +0 is never -0).
-// 3. brutefold_chain_kernel: each lane owns V rows, each warp up to 32 chains
-//    (consecutive bins of one frequency) whose sums stay in registers over the
-//    whole segment. A step loads its four positions (one broadcast) and four
-//    samples of V rows and adds them in order, two chains side by side.
+// 3. brutefold_chain_kernel: each lane owns V rows (NS = 32 V; groups of 4 rows
+//    where there are no more, which 28 lanes then read with the others), each warp
+//    up to 32 chains (bins of one frequency) whose sums stay in registers over the
+//    whole segment (or, with little scratch, over a run of chunks: the sums then
+//    pass from launch to launch through the fold). A step loads its four positions
+//    (one broadcast) and four samples of V rows and adds them in order, two chains
+//    side by side.
 //
 // Bound: shared-memory bandwidth, 4 bytes per add at 128 bytes a clock and SM:
 // 4.6 ms with padding for 2^21 samples x 15 100 frequencies, 64 bins, 128
@@ -235,7 +237,7 @@ constexpr int kMaxPer = 16;      // samples of a chunk per lane of the list kern
 
 // Shape of one chain launch, fixed by nbins, the rows and the frequencies.
 struct ChainShape {
-  int V;    // rows per lane (0: the chain path does not apply)
+  int NS;   // rows per group: 4, 32 or 64 (0: the chain path does not apply)
   int T;    // samples per time chunk, a multiple of 32, at most 32 kMaxPer
   int wpf;  // warps per frequency
   int bpw;  // bins per warp (even)
@@ -265,31 +267,33 @@ __host__ __device__ inline int chain_bin(int warp, int chain, int wpf) {
 }
 
 // Rows [0, nseg) are the segments of ts_e, rows [nseg, 2 nseg) those of ts_v.
-// out: [row group][chunk][t][NS], zeros beyond the series and the last row.
+// out: [row group][chunk - c0][t][NS] for nc chunks from c0, zeros beyond the
+// series and the last row.
+template <int NS>
 __global__ void __launch_bounds__(256)
 series_rows_kernel(const float* __restrict__ ts_e, const float* __restrict__ ts_v,
-                   int64_t nsamps, int64_t seg_len, int64_t nseg, int64_t nrows, int64_t rg0,
-                   int T, int NS, int64_t nch, float* __restrict__ out) {
-  __shared__ float tile[32][33];
+                   int64_t nsamps, int64_t seg_len, int64_t nseg, int64_t nrows, int T,
+                   int64_t c0, int64_t nc, float* __restrict__ out) {
+  __shared__ float tile[NS][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int64_t nt = T / 32;  // a block per 32 positions of a chunk; rg: within this launch
-  const int64_t tc = blockIdx.x / nt, t = tc % nch, rg = tc / nch;
+  const int64_t nt = T / 32;  // a block per 32 positions of a chunk
+  const int64_t tc = blockIdx.x / nt, t = tc % nc, rg = tc / nc;
   const int t0 = (int)(blockIdx.x - tc * nt) * 32;
-  float* o = out + (rg * nch + t) * (int64_t)T * NS;
-  for (int r0 = 0; r0 < NS; r0 += 32) {
-    __syncthreads();
-    for (int q = ty; q < 32; q += 8) {
-      const int64_t row = (rg0 + rg) * NS + r0 + q;
-      const int64_t seg = row < nseg ? row : row - nseg;
-      const int64_t i = t * T + t0 + tx;  // position within the segment
-      const int64_t p = seg * seg_len + i;
-      float x = 0.0f;
-      if (row < nrows && i < seg_len && p < nsamps) x = __ldg((row < nseg ? ts_e : ts_v) + p);
-      tile[q][tx] = x;
-    }
-    __syncthreads();
-    for (int q = ty; q < 32; q += 8) o[(int64_t)(t0 + q) * NS + r0 + tx] = tile[tx][q];
+  const int64_t i = (c0 + t) * T + t0 + tx;  // position within the segment
+#pragma unroll
+  for (int q0 = 0; q0 < NS; q0 += 8) {
+    const int q = q0 + ty;
+    const int64_t row = rg * NS + q, seg = row < nseg ? row : row - nseg;
+    const int64_t p = seg * seg_len + i;
+    float x = 0.0f;
+    if (q < NS && row < nrows && i < seg_len && p < nsamps)
+      x = __ldg((row < nseg ? ts_e : ts_v) + p);
+    if (q < NS) tile[q][tx] = x;
   }
+  __syncthreads();
+  float* o = out + ((rg * nc + t) * (int64_t)T + t0) * NS;
+#pragma unroll
+  for (int k = threadIdx.x; k < 32 * NS; k += 256) o[k] = tile[k % NS][k / NS];
 }
 
 // Turns per sample (and at position 0) of one frequency as 64-bit fixed-point
@@ -331,8 +335,11 @@ static __device__ __noinline__ int bin_exact(int64_t i, double f, int nbins, dou
   return b < 0 || b >= nbins ? 0 : b;  // as phase_map_kernel
 }
 
-// One block per frequency, a warp per time chunk. counts (unit variance):
-// [frequency][2][nbins] sample counts of a full and of the last segment. The
+// Lists of nc chunks from c0. The blocks of a frequency (grid y) share its chunks,
+// a warp per chunk. counts (unit variance): [frequency][2][nbins] sample counts of
+// these chunks of a full and of the last segment, added up over the blocks where
+// there are several (whole numbers below 2^24: exact in any order; the caller
+// clears them). The
 // bins are integer arithmetic kept in registers and sorted by per-lane counts
 // whose rows are padded to an odd number of words (without the padding 16-way
 // bank conflicts made it 2.2 ms instead of 1.0). Bound: instruction issue (79 %).
@@ -344,7 +351,7 @@ __host__ __device__ inline int list_warp_bytes(int nbins, int LB) {
 
 __global__ void __launch_bounds__(256, 3)
 chain_list_kernel(const double* __restrict__ freqs, int64_t seg_len, int nbins, double tsamp,
-                  double t_ref, ChainShape cs, int64_t nch, int64_t last_len,
+                  double t_ref, ChainShape cs, int64_t c0, int64_t nc, int64_t last_len,
                   uint8_t* __restrict__ lists, float* __restrict__ counts) {
   extern __shared__ __align__(16) uint8_t lsm[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
@@ -363,7 +370,9 @@ chain_list_kernel(const double* __restrict__ freqs, int64_t seg_len, int nbins, 
   for (int k = tid; k < 2 * nbins; k += blockDim.x) hist[k] = 0;
   for (int k = lane; k < list_entries_off(cs.wpf); k += 32) list[k] = 0;
   __syncthreads();
-  for (int64_t t = warp; t < nch; t += nwarps) {
+  for (int64_t tl = (int64_t)blockIdx.y * nwarps + warp; tl < nc;
+       tl += (int64_t)gridDim.y * nwarps) {
+    const int64_t t = c0 + tl;
     const int clen = (int)min((int64_t)cs.T, seg_len - t * cs.T);
     for (int k = lane; k < nbins * (kCntRow / 4); k += 32) reinterpret_cast<uint32_t*>(cnt)[k] = 0;
     __syncwarp();
@@ -443,7 +452,7 @@ chain_list_kernel(const double* __restrict__ freqs, int64_t seg_len, int nbins, 
         entry[o[32] + 4 * (r >> 1) + (r & 1)] = (uint16_t)(2 * (i0 + k));
       }
     __syncwarp();
-    uint4* dst = reinterpret_cast<uint4*>(lists + (f * nch + t) * cs.LB);
+    uint4* dst = reinterpret_cast<uint4*>(lists + (f * nc + tl) * cs.LB);
     const int used = (list_entries_off(cs.wpf) + 8 * base + 15) / 16;
     for (int k = lane; k < used; k += 32) dst[k] = reinterpret_cast<const uint4*>(list)[k];
     __syncwarp();
@@ -451,8 +460,14 @@ chain_list_kernel(const double* __restrict__ freqs, int64_t seg_len, int nbins, 
   if (!counts) return;
   __syncthreads();
   for (int b = tid; b < nbins; b += blockDim.x) {
-    counts[(f * 2) * nbins + b] = (float)hist[b];
-    counts[(f * 2 + 1) * nbins + b] = (float)hist[last_len < seg_len ? nbins + b : b];
+    const float full = (float)hist[b], end = (float)hist[last_len < seg_len ? nbins + b : b];
+    if (gridDim.y == 1) {
+      counts[(f * 2) * nbins + b] = full;
+      counts[(f * 2 + 1) * nbins + b] = end;
+    } else {
+      atomicAdd(counts + (f * 2) * nbins + b, full);
+      atomicAdd(counts + (f * 2 + 1) * nbins + b, end);
+    }
   }
 }
 
@@ -476,25 +491,27 @@ __device__ __forceinline__ void lds_rows(uint32_t addr, float (&x)[2]) {
   asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(x[0]), "=f"(x[1]) : "r"(addr));
 }
 
-// Block: NS = 32 V rows x F frequencies, F * wpf warps. Shared memory, double
-// buffered by chunk: rows [T + 1][NS] f32 (row T zeros), lists [F][LB]; the
-// next chunk is copied while this one is walked. The sums leave through the
-// same memory, whole profiles at a time.
-template <int V>
+// Block: NS rows x F frequencies, F * wpf warps, over nc chunks. Shared
+// memory, double buffered by chunk: rows [T + 1][NS] f32 (row T zeros), lists
+// [F][LB]; the next chunk is copied while this one is walked. The sums leave
+// through the same memory, whole profiles at a time; `go_on`: they start from
+// what an earlier launch left in the fold.
+template <int NS>
 __global__ void __launch_bounds__(kChainWarps * 32, 1)
 brutefold_chain_kernel(const float* __restrict__ rows, const uint8_t* __restrict__ lists,
                        const float* __restrict__ counts, ChainShape cs, int64_t nfreq_chunk,
-                       int64_t f_offset, int64_t nfreq_total, int64_t nch, int64_t nseg,
-                       int64_t nrows, int64_t rg0, int64_t nrg, int nbins,
+                       int64_t f_offset, int64_t nfreq_total, int64_t nc, int64_t nseg,
+                       int64_t nrows, int64_t nrg, int nbins, int go_on,
                        float* __restrict__ fold) {
-  constexpr int NS = 32 * V;
+  constexpr int V = NS == 64 ? 2 : 1;    // rows per lane
+  constexpr int kU = NS < 16 ? NS : 16;  // rows of the fold in flight
   extern __shared__ __align__(16) uint8_t csm[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x;
   const int64_t rg = blockIdx.x % nrg, f0 = blockIdx.x / nrg * cs.F;
   const int nfb = (int)min((int64_t)cs.F, nfreq_chunk - f0);
   const int rbytes = (cs.T + 1) * NS * 4, lbytes = cs.F * cs.LB + 16;
   uint8_t* buf[2] = {csm, csm + rbytes + lbytes};
-  const float* src_r = rows + rg * nch * (int64_t)cs.T * NS;
+  const float* src_r = rows + rg * nc * (int64_t)cs.T * NS;
   auto fetch = [&](int64_t t) {
     uint8_t* b = buf[t & 1];
     const uint8_t* r = reinterpret_cast<const uint8_t*>(src_r + t * (int64_t)cs.T * NS);
@@ -502,22 +519,55 @@ brutefold_chain_kernel(const float* __restrict__ rows, const uint8_t* __restrict
     const int lq = cs.LB / 16;
     for (int k = tid; k < nfb * lq; k += nthr) {
       const int fi = k / lq, q = k - fi * lq;
-      cp_async16(b + rbytes + 16 * k, lists + ((f0 + fi) * nch + t) * cs.LB + 16 * q);
+      cp_async16(b + rbytes + 16 * k, lists + ((f0 + fi) * nc + t) * cs.LB + 16 * q);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  for (int k = tid; k < NS; k += nthr)
-    for (int q = 0; q < 2; ++q) reinterpret_cast<float*>(buf[q])[cs.T * NS + k] = 0.0f;
+  // the frequencies side by side: those of a slow pulsar are all in the same bins,
+  // whose warps would otherwise share one of the SM's four schedulers
+  const int kb = warp / cs.F, fi = warp - kb * cs.F;
+  const bool active = fi < nfb;
+  const int nv = (int)min((int64_t)NS, nrows - rg * NS);  // rows of this block
+  // a row's profiles of the block's frequencies in the fold
+  auto profiles = [&](int r) {
+    const int64_t row = rg * NS + r, seg = row < nseg ? row : row - nseg;
+    return fold + ((size_t)seg * nfreq_total + f_offset + f0) * 2 * nbins +
+           (row < nseg ? 0 : nbins);
+  };
+  float* out_s = reinterpret_cast<float*>(csm);  // [row][F nbins]
+  const int fn = cs.F * nbins, stride = fn + 1;
   float acc[kChains][V];
 #pragma unroll
   for (int c = 0; c < kChains; ++c)
 #pragma unroll
     for (int v = 0; v < V; ++v) acc[c][v] = 0.0f;
-  const int fi = warp / cs.wpf, kb = warp - fi * cs.wpf;
-  const bool active = fi < nfb;
+  if (go_on) {
+    for (int k = tid; k < nfb * nbins; k += nthr) {
+      const int q = k / nbins, at = q * 2 * nbins + (k - q * nbins);
+      for (int r0 = 0; r0 < nv; r0 += kU) {
+        float x[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) x[u] = profiles(min(r0 + u, nv - 1))[at];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) out_s[min(r0 + u, nv - 1) * stride + k] = x[u];
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < kChains; ++c) {
+      const int b = chain_bin(kb, c, cs.wpf);
+      if (active && c < cs.bpw && b < nbins)
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+          if (lane * V + v < nv) acc[c][v] = out_s[(lane * V + v) * stride + fi * nbins + b];
+    }
+    __syncthreads();
+  }
+  for (int k = tid; k < NS; k += nthr)
+    for (int q = 0; q < 2; ++q) reinterpret_cast<float*>(buf[q])[cs.T * NS + k] = 0.0f;
   fetch(0);
-  for (int64_t t = 0; t < nch; ++t) {
-    if (t + 1 < nch) {
+  for (int64_t t = 0; t < nc; ++t) {
+    if (t + 1 < nc) {
       fetch(t + 1);
       asm volatile("cp.async.wait_group 1;" ::: "memory");
     } else {
@@ -530,37 +580,40 @@ brutefold_chain_kernel(const float* __restrict__ rows, const uint8_t* __restrict
                                                        kb * (kChains / 2));
       const uint32_t cw[4] = {c4.x, c4.y, c4.z, c4.w};
       // 32-bit shared addresses: this lane's rows, the warp's entries
-      const uint32_t xb = (uint32_t)__cvta_generic_to_shared(buf[t & 1]) + lane * (4 * V);
+      const uint32_t xb =
+          (uint32_t)__cvta_generic_to_shared(buf[t & 1]) + lane % (NS / V) * (4 * V);
       uint32_t e = (uint32_t)__cvta_generic_to_shared(l) + list_entries_off(cs.wpf) +
                    2 * reinterpret_cast<const uint32_t*>(l)[kb];
-      // a row's bytes are 64 V per unit of an entry: one 16 x 8-bit dot product per address
-      constexpr uint32_t kLo = 64 * V, kHi = kLo << 8;
+      // a sample's bytes are 2 NS per unit of an entry: one 16 x 8-bit dot product per address
+      constexpr uint32_t kLo = 2 * NS, kHi = kLo << 8;
       uint2 next = lds_u32x2(e);  // one step ahead: the warp's steps are one run
 #pragma unroll
       for (int c = 0; c < kChains; c += 2) {
         const uint32_t end = e + ((cw[c >> 3] >> (8 * ((c >> 1) & 3))) & 0xFFu) * 8;
         // One row a lane is where a walk has few warps and, at the low
         // frequencies of few segments, long runs of one bin: four steps' loads
-        // in flight there (32 segments at 1-10 Hz: 0.66 -> 0.55 ms).
+        // in flight there (32 segments at 1-10 Hz: 0.66 -> 0.55 ms; eight: 7 %
+        // slower than four).
         if constexpr (V == 1) {
+          constexpr int N = 4;
 #pragma unroll 1
-          while (end - e >= 32) {
-            uint2 w[4];
+          while (end - e >= 8 * N) {
+            uint2 w[N];
             w[0] = next;
 #pragma unroll
-            for (int k = 1; k < 4; ++k) w[k] = lds_u32x2(e + 8 * k);
-            e += 32;
+            for (int k = 1; k < N; ++k) w[k] = lds_u32x2(e + 8 * k);
+            e += 8 * N;
             next = lds_u32x2(e);
-            float x[4][4][V];
+            float x[N][4][V];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
+            for (int k = 0; k < N; ++k) {
               lds_rows(__dp2a_lo(w[k].x, kLo, xb), x[k][0]);
               lds_rows(__dp2a_lo(w[k].x, kHi, xb), x[k][1]);
               lds_rows(__dp2a_lo(w[k].y, kLo, xb), x[k][2]);
               lds_rows(__dp2a_lo(w[k].y, kHi, xb), x[k][3]);
             }
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
+            for (int k = 0; k < N; ++k) {
               acc[c][0] = __fadd_rn(__fadd_rn(acc[c][0], x[k][0][0]), x[k][1][0]);
               acc[c + 1][0] = __fadd_rn(__fadd_rn(acc[c + 1][0], x[k][2][0]), x[k][3][0]);
             }
@@ -586,38 +639,33 @@ brutefold_chain_kernel(const float* __restrict__ rows, const uint8_t* __restrict
     }
     __syncthreads();
   }
-  // sums to shared memory [row][F nbins], then whole profiles to the fold
-  float* out_s = reinterpret_cast<float*>(csm);
-  const int fn = cs.F * nbins, stride = fn + 1;
+  // sums to shared memory, then whole profiles to the fold
   if (active) {
 #pragma unroll
     for (int c = 0; c < kChains; ++c) {
       const int b = chain_bin(kb, c, cs.wpf);
-      if (c < cs.bpw && b < nbins)
+      if (c < cs.bpw && b < nbins && lane < NS / V)
 #pragma unroll
         for (int v = 0; v < V; ++v) out_s[(lane * V + v) * stride + fi * nbins + b] = acc[c][v];
     }
   }
   __syncthreads();
-  const int ncomp = counts ? 1 : 2;
-  for (int r = 0; r < NS; ++r) {
-    const int64_t row = (rg0 + rg) * NS + r;
-    if (row >= nrows) break;
-    const int64_t seg = row < nseg ? row : row - nseg;
-    float* o = fold + ((size_t)seg * nfreq_total + f_offset + f0) * 2 * nbins +
-               (row < nseg ? 0 : nbins);
-    if (ncomp == 1) {
-      const float* cn = counts + (f0 * 2 + (seg == nseg - 1 ? 1 : 0)) * nbins;
-      for (int k = tid; k < nfb * 2 * nbins; k += nthr) {
-        const int q = k / (2 * nbins), j = k - q * 2 * nbins;
-        o[k] = j < nbins ? out_s[r * stride + q * nbins + j]
-                         : __ldg(cn + q * 2 * nbins + j - nbins);
-      }
-    } else {
-      for (int k = tid; k < nfb * nbins; k += nthr) {
-        const int q = k / nbins;
-        o[q * 2 * nbins + (k - q * nbins)] = out_s[r * stride + k];
-      }
+  const int per = counts ? 2 * nbins : nbins;  // unit variance: every row is a segment's
+  for (int k = tid; k < nfb * per; k += nthr) {
+    const int q = k / per, j = k - q * per, at = q * 2 * nbins + j;
+    if (j < nbins) {
+      for (int r = 0; r < nv; ++r) profiles(r)[at] = out_s[r * stride + q * nbins + j];
+      continue;
+    }
+    const float* cn = counts + (f0 + q) * 2 * nbins + j - nbins;
+    const float full = __ldg(cn), end = __ldg(cn + nbins);
+    for (int r0 = 0; r0 < nv; r0 += kU) {
+      float x[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) x[u] = go_on ? profiles(min(r0 + u, nv - 1))[at] : 0.0f;
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+        if (r0 + u < nv) profiles(r0 + u)[at] = x[u] + (rg * NS + r0 + u == nseg - 1 ? end : full);
     }
   }
 }
@@ -633,76 +681,119 @@ static int64_t round256(int64_t x) { return (x + 255) & ~int64_t(255); }
 constexpr int kChainSmem = 226 * 1024;
 
 static int chain_smem(const ChainShape& c, int nbins) {
-  const int ns = 32 * c.V;
-  const int walk = 2 * ((c.T + 1) * ns * 4 + c.F * c.LB + 16);
-  const int out = ns * (c.F * nbins + 1) * 4;
+  const int walk = 2 * ((c.T + 1) * c.NS * 4 + c.F * c.LB + 16);
+  const int out = c.NS * (c.F * nbins + 1) * 4;
   return std::max(walk, out);
 }
 
-// V: two rows a lane (64 rows share a list walk, 8-byte loads) once there are
-// more than 32. F: as many frequencies as 16 warps hold, fewer where that
-// leaves SMs without a block. T: the longest chunk two buffers of which
-// fit, since each (chain, chunk) pays a loop and half a padding entry.
-static ChainShape chain_shape(int nbins, int64_t nrows, int64_t nfreqs, int V) {
+constexpr int64_t kChainSms = 152;
+
+// NS: two rows a lane (64 rows share a list walk, 8-byte loads) once there are
+// more than 32, unless blocks of 32 rows and one frequency all fit on the GPU
+// at once; four rows where there are no more (one fold of 2^23 samples: 28 ms,
+// and 56 with copies of 32 rows, most of them zeros). F: as many frequencies as
+// 16 warps hold, fewer where that leaves SMs without a block; the warps that
+// this leaves free share a frequency's bins. T: the longest chunk two buffers of
+// which fit, since each (chain, chunk) pays a loop and half a padding entry, but
+// no longer than an even share of a segment.
+static ChainShape chain_shape(int nbins, int64_t nrows, int64_t nfreqs, int64_t seg_len) {
   ChainShape c{0, 0, 0, 0, 0, 0};
   if (nbins < 1 || nbins > 256) return c;
-  c.wpf = (nbins + kChains - 1) / kChains;
-  c.bpw = ((nbins + c.wpf - 1) / c.wpf + 1) & ~1;
-  c.F = kChainWarps / c.wpf;
-  const int64_t nrg = (nrows + 32 * V - 1) / (32 * V);
+  const int ns = nrows <= 4                                            ? 4
+                 : nrows > 32 && (nrows + 31) / 32 * nfreqs > kChainSms ? 64
+                                                                        : 32;
+  const int least = (nbins + kChains - 1) / kChains;  // warps that hold a frequency's bins
+  c.F = kChainWarps / least;
+  const int64_t nrg = (nrows + ns - 1) / ns;
   // waves of blocks times the work of one (its copies cost about 0.8 of a frequency's walk)
   const int fmax = c.F;
   double best = 0.0;
   for (int f = fmax; f >= 1; --f) {
     const int64_t blocks = nrg * ((nfreqs + f - 1) / f);
-    const double cost = (double)((blocks + 151) / 152) * (f + 0.8);
+    const double cost = (double)((blocks + kChainSms - 1) / kChainSms) * (f + 0.8);
     if (f == fmax || cost < best) {
       best = cost;
       c.F = f;
     }
   }
-  for (c.T = V == 1 ? 480 : 384; c.T >= 32; c.T -= 32) {
+  c.wpf = std::max(least, std::min(kChainWarps / c.F, (nbins + 1) / 2));
+  c.bpw = ((nbins + c.wpf - 1) / c.wpf + 1) & ~1;
+  for (c.T = ns < 64 ? 480 : 384; c.T >= 32; c.T -= 32) {
     c.LB = list_bytes(c.T, nbins, c.wpf);
-    c.V = V;
-    if (chain_smem(c, nbins) <= kChainSmem) return c;
+    c.NS = ns;
+    if (chain_smem(c, nbins) > kChainSmem) continue;
+    const int64_t nch = (seg_len + c.T - 1) / c.T;
+    c.T = (int)(((seg_len + nch - 1) / nch + 31) / 32 * 32);
+    c.LB = list_bytes(c.T, nbins, c.wpf);
+    return c;
   }
-  c.V = 0;
+  c.NS = 0;
   return c;
 }
 
 static int64_t chain_chunks(const ChainShape& c, int64_t seg_len) {
   return (seg_len + c.T - 1) / c.T;
 }
-// Scratch bytes of one row group of the series layout, and of one frequency
-// (lists and counts).
-static int64_t chain_group_bytes(const ChainShape& c, int64_t seg_len) {
-  return chain_chunks(c, seg_len) * c.T * 32 * c.V * 4;
-}
-static int64_t chain_freq_bytes(const ChainShape& c, int64_t seg_len, int nbins) {
-  return chain_chunks(c, seg_len) * c.LB + 2 * nbins * 4;
+static int64_t chain_groups(const ChainShape& c, int64_t nrows) {
+  return (nrows + c.NS - 1) / c.NS;
 }
 
-// Scratch of the chain path: `groups` row groups of the series at a time (all
-// of them when they fit in half of it) and `chunk` frequencies.
+// Scratch of the chain path: the series layout of `run` chunks of every
+// segment, then their lists (and sample counts) for `freqs` frequencies (0: the
+// path does not apply).
 struct ChainPlan {
   ChainShape c;
-  int64_t groups, chunk;
+  int64_t run, freqs;
 };
+
+static int64_t chain_rows_bytes(const ChainShape& c, int64_t nrows, int64_t run) {
+  return chain_groups(c, nrows) * run * c.T * c.NS * 4;
+}
+static int64_t chain_freq_bytes(const ChainShape& c, int64_t run, int nbins) {
+  return run * c.LB + 2 * nbins * 4;
+}
+static int64_t chain_bytes(const ChainPlan& p, int64_t nrows, int nbins) {
+  return 4 * 256 + chain_rows_bytes(p.c, nrows, p.run) +
+         p.freqs * chain_freq_bytes(p.c, p.run, nbins);
+}
+
+// Everything in one run over all frequencies where that fits. Otherwise a run of
+// fewer chunks, of every row: the layout is made once and each list once whatever
+// the split, but every run after the first reads the sums back from the fold, so
+// runs are as long as leaves room for frequencies that fill the GPU twice; where
+// one chunk at a time does not, the phase map is made instead.
+// (16 MiB for 2^23 samples of general
+// variance, 15 100 frequencies: a launch of 20 blocks for every 64 rows and 157
+// frequencies took 432 ms.) Of five to eight rows, padded to 32, the runs keep the
+// layout within kPadded.
+constexpr int64_t kPadded = int64_t(64) << 20;
 
 static ChainPlan chain_plan(int nbins, int64_t nrows, int64_t nfreqs, int64_t seg_len,
                             int64_t scratch_bytes) {
-  for (int V = nrows > 32 ? 2 : 1; V >= 1; --V) {
-    const ChainShape c = chain_shape(nbins, nrows, nfreqs, V);
-    if (!c.V) continue;
-    const int64_t avail = scratch_bytes - 4 * 256;
-    const int64_t g = chain_group_bytes(c, seg_len), q = chain_freq_bytes(c, seg_len, nbins);
-    const int64_t nrg = (nrows + 32 * V - 1) / (32 * V);
-    if (avail < g + q) continue;
-    int64_t groups = nrg;
-    if (nrg * g + nfreqs * q > avail) groups = std::min(nrg, std::max<int64_t>(1, avail / 2 / g));
-    return {c, groups, std::min(nfreqs, std::max<int64_t>(1, (avail - groups * g) / q))};
+  const ChainPlan none = {{0, 0, 0, 0, 0, 0}, 0, 0};
+  ChainPlan p = {chain_shape(nbins, nrows, nfreqs, seg_len), 0, nfreqs};
+  if (!p.c.NS) return none;
+  const int64_t nch = chain_chunks(p.c, seg_len);
+  p.run = nch;
+  if (p.c.NS == 32 && nrows <= 8)
+    p.run = std::max<int64_t>(1, std::min(nch, kPadded / chain_rows_bytes(p.c, nrows, 1)));
+  if (chain_bytes(p, nrows, nbins) <= scratch_bytes) return p;
+  for (int64_t run = p.run; run >= 1; run = run == 1 ? 0 : (run + 1) / 2) {
+    // where a launch does not fill the GPU, the shape is one for its frequencies
+    int64_t nf = nfreqs;
+    for (int pass = 0; pass < 3 && nf > 0; ++pass) {
+      const ChainShape c = chain_shape(nbins, nrows, nf, seg_len);
+      const int64_t avail = scratch_bytes - 4 * 256 - chain_rows_bytes(c, nrows, run);
+      const int64_t fit = avail < 0 ? 0 : avail / chain_freq_bytes(c, run, nbins);
+      const int64_t take = std::min(fit, nf);
+      if (take < 1) break;
+      const int64_t blocks = chain_groups(c, nrows) * ((take + c.F - 1) / c.F);
+      if (take == nfreqs || blocks >= 2 * kChainSms) return {c, run, take};
+      if (take == nf) break;
+      nf = take;
+    }
   }
-  return {{0, 0, 0, 0, 0, 0}, 0, 0};
+  return none;
 }
 
 static int brutefold_chain(const float* ts_e, const float* ts_v, bool unit, int64_t nsamps,
@@ -711,9 +802,14 @@ static int brutefold_chain(const float* ts_e, const float* ts_v, bool unit, int6
                            float* fold_out, cudaStream_t s) {
   const ChainShape& c = p.c;
   const int64_t nseg = (nsamps + seg_len - 1) / seg_len, nrows = nseg * (unit ? 1 : 2);
-  const int64_t nch = chain_chunks(c, seg_len), nrg = (nrows + 32 * c.V - 1) / (32 * c.V);
+  const int64_t nch = chain_chunks(c, seg_len), nrg = chain_groups(c, nrows);
   const int64_t last_len = nsamps - (nseg - 1) * seg_len;
-  auto kf = c.V == 1 ? brutefold_chain_kernel<1> : brutefold_chain_kernel<2>;
+  auto kf = c.NS == 4    ? brutefold_chain_kernel<4>
+            : c.NS == 32 ? brutefold_chain_kernel<32>
+                         : brutefold_chain_kernel<64>;
+  auto kr = c.NS == 4    ? series_rows_kernel<4>
+            : c.NS == 32 ? series_rows_kernel<32>
+                         : series_rows_kernel<64>;
   const int smem = chain_smem(c, nbins);
   const int lwarps = nbins <= 128 ? 8 : 4;  // about 230 KB at 256 bins and 8 warps
   const int lsmem = lwarps * list_warp_bytes(nbins, c.LB) + 2 * nbins * (int)sizeof(int);
@@ -721,31 +817,32 @@ static int brutefold_chain(const float* ts_e, const float* ts_v, bool unit, int6
       set_smem_limit(chain_list_kernel, lsmem) != cudaSuccess)
     return set_error(LOKI_ERR_CUDA, "cudaFuncSetAttribute failed");
   float* rows = reinterpret_cast<float*>(scratch);
-  char* at = scratch + round256(p.groups * chain_group_bytes(c, seg_len));
+  char* at = scratch + round256(chain_rows_bytes(c, nrows, p.run));
   float* counts = unit ? reinterpret_cast<float*>(at) : nullptr;
-  uint8_t* lists = reinterpret_cast<uint8_t*>(at + round256(p.chunk * 2 * nbins * 4));
-  const int threads = c.F * c.wpf * 32;
-  auto lay_out = [&](int64_t rg0, int64_t n) {
-    note_launch();
-    series_rows_kernel<<<(unsigned)(n * nch * (c.T / 32)), 256, 0, s>>>(ts_e, ts_v, nsamps, seg_len, nseg,
-                                                           nrows, rg0, c.T, 32 * c.V, nch, rows);
-  };
-  if (p.groups * nch * (c.T / 32) > 0x7FFFFFFF || p.chunk > 0x7FFFFFFF ||
-      p.groups * ((p.chunk + c.F - 1) / c.F) > 0x7FFFFFFF)
+  uint8_t* lists = reinterpret_cast<uint8_t*>(at + round256(p.freqs * 2 * nbins * 4));
+  if (nrg * p.run * (c.T / 32) > 0x7FFFFFFF || p.freqs > 0x7FFFFFFF ||
+      nrg * ((p.freqs + c.F - 1) / c.F) > 0x7FFFFFFF)
     return set_error(LOKI_ERR_UNSUPPORTED, "grid too large");
-  if (p.groups == nrg) lay_out(0, nrg);
-  for (int64_t f0 = 0; f0 < nfreqs; f0 += p.chunk) {
-    const int64_t nf = std::min(p.chunk, nfreqs - f0);
+  for (int64_t c0 = 0; c0 < nch; c0 += p.run) {
+    const int64_t nc = std::min(p.run, nch - c0);
     note_launch();
-    chain_list_kernel<<<(unsigned)nf, 32 * lwarps, lsmem, s>>>(freqs + f0, seg_len, nbins, tsamp,
-                                                              t_ref, c, nch, last_len, lists,
-                                                              counts);
-    for (int64_t r0 = 0; r0 < nrg; r0 += p.groups) {
-      const int64_t n = std::min(p.groups, nrg - r0);
-      if (p.groups < nrg) lay_out(r0, n);
+    kr<<<(unsigned)(nrg * nc * (c.T / 32)), 256, 0, s>>>(ts_e, ts_v, nsamps, seg_len, nseg,
+                                                          nrows, c.T, c0, nc, rows);
+    for (int64_t f0 = 0; f0 < nfreqs; f0 += p.freqs) {
+      const int64_t nf = std::min(p.freqs, nfreqs - f0);
+      // blocks a frequency: three on every SM, two chunks a warp at least (the counts
+      // of several have to be cleared first)
+      const int64_t ny = std::max<int64_t>(
+          1, std::min<int64_t>((3 * kChainSms + nf - 1) / nf, nc / (2 * lwarps)));
+      if (counts && ny > 1 &&
+          cudaMemsetAsync(counts, 0, nf * 2 * nbins * sizeof(float), s) != cudaSuccess)
+        return set_error(LOKI_ERR_CUDA, "cudaMemsetAsync failed");
       note_launch();
-      kf<<<(unsigned)(n * ((nf + c.F - 1) / c.F)), threads, smem, s>>>(
-          rows, lists, counts, c, nf, f0, nfreqs, nch, nseg, nrows, r0, n, nbins, fold_out);
+      chain_list_kernel<<<dim3((unsigned)nf, (unsigned)ny), 32 * lwarps, lsmem, s>>>(
+          freqs + f0, seg_len, nbins, tsamp, t_ref, c, c0, nc, last_len, lists, counts);
+      note_launch();
+      kf<<<(unsigned)(nrg * ((nf + c.F - 1) / c.F)), c.F * c.wpf * 32, smem, s>>>(
+          rows, lists, counts, c, nf, f0, nfreqs, nc, nseg, nrows, nrg, nbins, c0 > 0, fold_out);
     }
     int rc = check_launch("brutefold_chain");
     if (rc) return rc;
@@ -753,8 +850,8 @@ static int brutefold_chain(const float* ts_e, const float* ts_v, bool unit, int6
   return LOKI_OK;
 }
 
-// unit: ts_v is all ones (ts_v may be NULL); the ts_e sums come from the
-// sequential kernel and the variance rows from the per-frequency counts.
+// unit: ts_v is all ones (ts_v may be NULL): only the ts_e sums are made from
+// samples, the variance rows are the per-frequency sample counts.
 static int brutefold_impl(const float* ts_e, const float* ts_v, bool unit, int64_t nsamps,
                           const double* freqs, int64_t nfreqs, int64_t segment_len,
                           int32_t nbins, double tsamp, double t_ref, void* phase_scratch,
@@ -770,18 +867,17 @@ static int brutefold_impl(const float* ts_e, const float* ts_v, bool unit, int64
   cudaStream_t s = (cudaStream_t)stream;
   const int nc = unit ? 1 : 2;
   const int64_t nseg = (nsamps + segment_len - 1) / segment_len;
-  {  // the chain path when it applies and one row group and frequency of it fit
+  const int elem = nbins <= 256 ? 1 : 2;
+  if (scratch_bytes / (segment_len * elem) < 1)
+    return set_error(LOKI_ERR_CAPACITY, "phase scratch of %lld bytes holds no frequency",
+                     (long long)scratch_bytes);
+  {  // the chain path when it applies and a chunk of every row and one frequency's list fit
     const ChainPlan p = chain_plan(nbins, nseg * nc, nfreqs, segment_len, scratch_bytes);
-    if (p.chunk > 0 && (reinterpret_cast<uintptr_t>(phase_scratch) & 15) == 0)
+    if (p.freqs > 0 && (reinterpret_cast<uintptr_t>(phase_scratch) & 15) == 0)
       return brutefold_chain(ts_e, ts_v, unit, nsamps, freqs, nfreqs, segment_len, nbins, tsamp,
                              t_ref, reinterpret_cast<char*>(phase_scratch), p, fold_out, s);
   }
-  const int elem = nbins <= 256 ? 1 : 2;
-  int64_t chunk = scratch_bytes / (segment_len * elem);
-  if (chunk < 1)
-    return set_error(LOKI_ERR_CAPACITY, "phase scratch of %lld bytes holds no frequency",
-                     (long long)scratch_bytes);
-  chunk = std::min(chunk, nfreqs);
+  const int64_t chunk = std::min(scratch_bytes / (segment_len * elem), nfreqs);
   int bs = 128;  // nc * nbins floats of shared memory per thread, <= 200 KB a block
   while (bs > 32 && (size_t)bs * nc * nbins * sizeof(float) > 200 * 1024) bs >>= 1;
   const size_t smem = (size_t)bs * nc * nbins * sizeof(float);
@@ -835,11 +931,9 @@ extern "C" int64_t loki_brutefold_series_scratch_bytes(int64_t nsamps, int64_t n
                                                       int32_t unit_variance) {
   if (nsamps <= 0 || nfreqs <= 0 || segment_len <= 0 || nbins < 1) return 0;
   const int64_t nrows = (nsamps + segment_len - 1) / segment_len * (unit_variance ? 1 : 2);
-  const int V = nrows > 32 ? 2 : 1;
-  const ChainShape c = chain_shape(nbins, nrows, nfreqs, V);
-  if (!c.V) return nfreqs * segment_len * (nbins <= 256 ? 1 : 2);
-  return 4 * 256 + (nrows + 32 * V - 1) / (32 * V) * chain_group_bytes(c, segment_len) +
-         nfreqs * chain_freq_bytes(c, segment_len, nbins);
+  const ChainPlan p = chain_plan(nbins, nrows, nfreqs, segment_len, INT64_MAX / 2);
+  if (!p.freqs) return nfreqs * segment_len * (nbins <= 256 ? 1 : 2);
+  return chain_bytes(p, nrows, nbins);
 }
 
 extern "C" int64_t loki_brutefold_scratch_bytes(int64_t nfreqs, int64_t segment_len,
@@ -865,10 +959,10 @@ extern "C" int loki_brutefold_unit_variance(const float* ts_e, int64_t nsamps,
                         t_ref, phase_scratch, scratch_bytes, fold_out, stream);
 }
 
-// Fixed phase-map scratch of loki_brutefold_noalloc. 16 MiB holds the map of
-// one frequency for segments of up to 16 Mi samples (nbins <= 256, one byte a
-// sample) or 8 Mi samples (nbins > 256, two bytes); larger frequency grids are
-// processed in chunks of as many frequencies as the array holds.
+// Fixed scratch of loki_brutefold_noalloc: the series layout and the sample lists
+// of a run of chunks (chain_plan), or the phase map of as many frequencies as it
+// holds. The limits on segment_len are the map's: 16 MiB hold one frequency of
+// up to 16 Mi samples (nbins <= 256, one byte a sample) or 8 Mi (two bytes).
 static constexpr int64_t kNoAllocScratchBytes = int64_t(16) << 20;
 static __device__ __align__(256) unsigned char g_noalloc_phase_scratch[kNoAllocScratchBytes];
 
@@ -909,8 +1003,9 @@ extern "C" int loki_brutefold_noalloc(const float* ts_e, const float* ts_v, int6
   void* scratch = nullptr;
   const int rc = noalloc_scratch(&scratch);
   if (rc) return rc;
-  // Every map entry a fold reads is written by the phase-map launch of the same
-  // chunk, and every fold_out element by one fold thread: nothing is cleared.
+  // What a launch reads of the scratch (rows and lists, or the map) is written by
+  // launches of the same call before it, and every fold_out element by one thread
+  // (which reads it again where its sums go on): nothing is left to be cleared.
   return loki_brutefold(ts_e, ts_v, nsamps, freqs, nfreqs, segment_len, nbins, tsamp, t_ref,
                         scratch, kNoAllocScratchBytes, fold_out, stream);
 }
