@@ -276,7 +276,7 @@ int loki_brutefold_complex(const float* ts_e, const float* ts_v, int64_t nsamps,
  * loki_brutefold_complex_scratch_bytes() device bytes (16-byte aligned) for
  * the segments split into bfloat16 parts; float32 results, as close to float64
  * as loki_brutefold_complex's. segment_len <= 2^24. A bounded wait that runs
- * out sets LOKI_DEVERR_TIMEOUT. */
+ * out sets LOKI_DEVERR_TIMEOUT, and the sums not finished by then are NaN. */
 int loki_brutefold_complex_scratch(const float* ts_e, const float* ts_v, int64_t nsamps,
                                    const double* freqs, int64_t nfreqs, int64_t segment_len,
                                    int32_t nbins, double tsamp, double t_ref, void* scratch,
@@ -284,6 +284,12 @@ int loki_brutefold_complex_scratch(const float* ts_e, const float* ts_v, int64_t
                                    void* stream);
 int64_t loki_brutefold_complex_scratch_bytes(int64_t nsamps, int64_t segment_len,
                                              int32_t unit_variance);
+
+/* Test hook for that fold's bounded waits (current device): with wait 1 or 2 a
+ * wait that completed (1: of the warp that issues the products, 2: of those
+ * that sum them) counts as run out; 0 restores normal operation. Synchronous.
+ * No reference counterpart (error-path testing only). */
+int loki_fourier_force_timeout(int32_t wait);
 
 /* One complex DP level (dynamic/dyn_pffa.py:435-489 with shift_add_complex,
  * core/common.py:344-372): out[ipair, p] = tail * e^{-2 pi i k s_t / nbins}

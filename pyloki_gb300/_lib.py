@@ -325,6 +325,7 @@ SIGNATURES: dict[str, tuple] = {
     "loki_brutefold_complex_scratch": (C.c_int, [_P, _P, _I64, _P, _I64, _I64, _I32, _D, _D, _P,
                                                  _I64, _P, _P, _P]),
     "loki_brutefold_complex_scratch_bytes": (C.c_int64, [_I64, _I64, _I32]),
+    "loki_fourier_force_timeout": (C.c_int, [_I32]),
     "loki_brutefold_complex": (C.c_int, [_P, _P, _I64, _P, _I64, _I64, _I32, _D, _D, _P, _P]),
     "loki_ffa_level_complex": (C.c_int, [C.POINTER(LokiFFALevel), _P, _P, _P, _P]),
     "loki_fold_norm_complex": (C.c_int, [_P, _I64, _I32, _P, _P]),

@@ -19,7 +19,9 @@
 // each, and put its cosine and sine parts into tensor memory as the A operands;
 // warp 16 fetches the segments' parts (B, laid out in global memory as the MMA
 // reads them, one bulk copy a chunk) and issues the MMAs. Chunks of 48 samples
-// pass through two stages with mbarriers both ways, every wait bounded.
+// pass through two stages with mbarriers both ways, every wait bounded: where
+// one runs out the CTA waits (bounded again) for its MMAs and copies in flight,
+// writes NaN for the sums that it did not finish and sets the error word.
 //
 // Bound: making the basis (about 48 instructions per (f, h, sample) with the
 // splitting: 10.5 ms at full issue for 15 100 frequencies x 33 harmonics x
@@ -201,19 +203,33 @@ __device__ __forceinline__ void fm_commit(uint64_t* bar) {
       : "memory");
 }
 
+// Test hook (loki_fourier_force_timeout): one wait that completed counts as run
+// out, 1: the issuing warp's for the basis of the second chunk, 2: the basis
+// warps' for the first sums. Nothing of the tensor cores' is left in flight by
+// it that a wait that really ran out would not leave.
+__device__ int g_fm_force_timeout = 0;
+
 struct FmBars {
   uint64_t full[3], empty[3], done, drained, last;
   uint32_t tmem;
-  int dead;  // a wait ran out: nothing more is issued or waited for
+  int dead;    // a wait ran out: nothing more is issued, arrived at or waited for
+  int loaded;  // chunks that were copied for, of a CTA whose wait ran out
+  int force;   // g_fm_force_timeout
 };
 
-// Bounded wait; returns at once (and for good) after any wait ran out.
-__device__ __forceinline__ void fm_wait(FmBars& S, uint64_t* bar, uint32_t parity) {
+// Bounded wait. False, at once and for good in every thread that has to wait,
+// after any wait ran out; `expired`: one that completed counts as run out.
+__device__ __forceinline__ bool fm_wait(FmBars& S, uint64_t* bar, uint32_t parity,
+                                        bool expired = false) {
   for (long long i = 0; i < kSpinLimit; ++i) {
-    if (mbar_try_wait(bar, parity)) return;
-    if (*reinterpret_cast<volatile int*>(&S.dead)) return;
+    if (mbar_try_wait(bar, parity)) {
+      if (!expired) return true;
+      break;
+    }
+    if (*reinterpret_cast<volatile int*>(&S.dead)) return false;
   }
   *reinterpret_cast<volatile int*>(&S.dead) = 1;
+  return false;
 }
 
 template <int N>
@@ -243,64 +259,70 @@ brutefold_complex_mma_kernel(const uint8_t* __restrict__ parts, const float* __r
     mbar_init(&B.drained, kFmGen);
     mbar_init(&B.last, 1);
     B.dead = 0;
+    B.force = g_fm_force_timeout;
   }
   if (warp == kFmGen / 32) tmem_alloc(&B.tmem, 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tm = B.tmem;
+  // chunks whose copy was waited for, or (basis warps) arrived for: nch unless a
+  // wait ran out
+  int mine = nch;
 
   if (warp == kFmGen / 32) {
-    {
-      const uint8_t* src = parts + (int64_t)blockIdx.y * nch * kB;
-      for (int i = 0; i < S && i < nch; ++i) {
-        if (lane == 0) {
-          mbar_expect(&B.full[i], kB);
-          bulk_load(bs + i * kB, src + i * kB, kB, &B.full[i]);
-        }
-      }
-      constexpr uint32_t idesc = idesc_bf16(128, N);
-      int loaded = std::min(S, nch);
-      for (int i = 0; i < nch; ++i) {
-        const int s = i % S;
-        fm_wait(B, &B.full[s], (uint32_t)(i / S) & 1u);
-        const bool first = i % kGroup == 0;
-        if (first && i > 0) fm_wait(B, &B.drained, (uint32_t)(i / kGroup - 1) & 1u);
-        if (*reinterpret_cast<volatile int*>(&B.dead)) break;
-        __syncwarp();
-        tc_fence_after();
-        const uint32_t a = tm + kColA + s * fm_acols(N);
-        const uint32_t b = smem_u32(bs + s * kB);
-#pragma unroll
-        for (int ks = 0; ks < K / 16; ++ks)
-#pragma unroll
-          for (int comp = 0; comp < 2; ++comp)
-#pragma unroll
-            for (int p = 0; p < 6; ++p)
-              mma_bf16_ta(tm + comp * N, a + (comp * 3 + kFmPart[p][0]) * (K / 2) + ks * 8,
-                          smem_desc(b + kFmPart[p][1] * (N * K * 2) + ks * 256, 128,
-                                    K / 8 * 128),
-                          idesc, first && ks == 0 && p == 0 ? 0u : 1u);
-        fm_commit(&B.empty[s]);
-        if (i % kGroup == kGroup - 1 || i == nch - 1) fm_commit(&B.done);
-        // refill the stage of the chunk before this one, whose MMAs are done first
-        if (i > 0 && loaded < nch) {
-          const int r = (i - 1) % S;
-          fm_wait(B, &B.empty[r], (uint32_t)((i - 1) / S) & 1u);
-          if (*reinterpret_cast<volatile int*>(&B.dead)) break;
-          if (lane == 0) {
-            mbar_expect(&B.full[r], kB);
-            bulk_load(bs + r * kB, src + (int64_t)loaded * kB, kB, &B.full[r]);
-          }
-          __syncwarp();
-          ++loaded;
-        }
-      }
-      // nothing of this CTA's is in flight when its tensor memory is freed
-      fm_commit(&B.last);
-      for (long long k = 0; k < kSpinLimit && !mbar_try_wait(&B.last, 0); ++k) {
+    const uint8_t* src = parts + (int64_t)blockIdx.y * nch * kB;
+    int loaded = std::min(S, nch), taken = 0;  // chunks copied for, and waited for
+    for (int i = 0; i < loaded; ++i) {
+      if (lane == 0) {
+        mbar_expect(&B.full[i], kB);
+        bulk_load(bs + i * kB, src + i * kB, kB, &B.full[i]);
       }
     }
+    // the warp's wait: all of its lanes go on, or none
+    auto wait = [&](uint64_t* bar, uint32_t parity, bool expired = false) {
+      return __all_sync(0xFFFFFFFFu, fm_wait(B, bar, parity, expired));
+    };
+    constexpr uint32_t idesc = idesc_bf16(128, N);
+    for (int i = 0; i < nch; ++i) {
+      const int s = i % S;
+      const bool expired = i == 1 && B.force == 1;
+      if (!wait(&B.full[s], (uint32_t)(i / S) & 1u, expired)) break;
+      ++taken;
+      const bool first = i % kGroup == 0;
+      if (first && i > 0 && !wait(&B.drained, (uint32_t)(i / kGroup - 1) & 1u)) break;
+      tc_fence_after();
+      const uint32_t a = tm + kColA + s * fm_acols(N);
+      const uint32_t b = smem_u32(bs + s * kB);
+#pragma unroll
+      for (int ks = 0; ks < K / 16; ++ks)
+#pragma unroll
+        for (int comp = 0; comp < 2; ++comp)
+#pragma unroll
+          for (int p = 0; p < 6; ++p)
+            mma_bf16_ta(tm + comp * N, a + (comp * 3 + kFmPart[p][0]) * (K / 2) + ks * 8,
+                        smem_desc(b + kFmPart[p][1] * (N * K * 2) + ks * 256, 128, K / 8 * 128),
+                        idesc, first && ks == 0 && p == 0 ? 0u : 1u);
+      fm_commit(&B.empty[s]);
+      if (i % kGroup == kGroup - 1 || i == nch - 1) fm_commit(&B.done);
+      // refill the stage of the chunk before this one, whose MMAs are done first
+      if (i > 0 && loaded < nch) {
+        const int r = (i - 1) % S;
+        if (!wait(&B.empty[r], (uint32_t)((i - 1) / S) & 1u)) break;
+        if (lane == 0) {
+          mbar_expect(&B.full[r], kB);
+          bulk_load(bs + r * kB, src + (int64_t)loaded * kB, kB, &B.full[r]);
+        }
+        __syncwarp();
+        ++loaded;
+      }
+    }
+    // no MMA of this CTA's is in flight when its tensor memory is freed
+    fm_commit(&B.last);
+    for (long long k = 0; k < kSpinLimit && !mbar_try_wait(&B.last, 0); ++k) {
+    }
+    if (lane == 0) B.loaded = loaded;
+    mine = taken;
     __syncwarp();
   } else {
     const int quad = warp & 3, g = warp >> 2;  // tensor-memory lanes, sample group
@@ -315,8 +337,10 @@ brutefold_complex_mma_kernel(const uint8_t* __restrict__ parts, const float* __r
 #pragma unroll
     for (int j = 0; j < kCols; ++j) accc[j] = accs[j] = 0.0f;
     // sums of a finished group of chunks out of tensor memory
-    auto drain = [&](int group) {
-      fm_wait(B, &B.done, (uint32_t)group & 1u);
+    // (`arrived`: chunks arrived for so far)
+    auto drain = [&](int group, int arrived) {
+      if (mine == nch && !fm_wait(B, &B.done, (uint32_t)group & 1u, group == 0 && B.force == 2))
+        mine = arrived + (arrived == nch);  // another number than that of a sum that is whole
       __syncwarp();
       tc_fence_after();
 #pragma unroll
@@ -332,8 +356,10 @@ brutefold_complex_mma_kernel(const uint8_t* __restrict__ parts, const float* __r
         }
       }
       tc_fence_before();
-      mbar_arrive(&B.drained);
+      if (mine == nch) mbar_arrive(&B.drained);
     };
+    // after a wait that ran out a thread arrives at no barrier any more; its warp
+    // goes on together, as tcgen05.st and ld want it, to the next group's end
     for (int i = 0; i < nch; ++i) {
       const int s = i % S;
       float tv[kPer];
@@ -343,7 +369,7 @@ brutefold_complex_mma_kernel(const uint8_t* __restrict__ parts, const float* __r
         tv[q] = v.x, tv[q + 1] = v.y, tv[q + 2] = v.z, tv[q + 3] = v.w;
       }
       if (i >= S) {
-        fm_wait(B, &B.empty[s], (uint32_t)(i / S - 1) & 1u);
+        if (mine == nch && !fm_wait(B, &B.empty[s], (uint32_t)(i / S - 1) & 1u)) mine = i;
         tc_fence_after();
       }
       uint32_t pc[3][kPer / 2], ps[3][kPer / 2];
@@ -376,10 +402,17 @@ brutefold_complex_mma_kernel(const uint8_t* __restrict__ parts, const float* __r
       }
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
-      mbar_arrive(&B.full[s]);
-      if (i % kGroup == 0 && i > 0) drain(i / kGroup - 1);
+      if (mine == nch) mbar_arrive(&B.full[s]);
+      if (i % kGroup == 0 && i > 0) {
+        drain(i / kGroup - 1, i + 1);
+        if (!__all_sync(0xFFFFFFFFu, mine == nch)) break;
+      }
     }
-    drain((nch - 1) / kGroup);
+    drain((nch - 1) / kGroup, nch);
+    if (mine != nch) {  // sums that were not finished are not handed out as numbers
+#pragma unroll
+      for (int j = 0; j < kCols; ++j) accc[j] = accs[j] = nanf("");
+    }
     // correction phasor exp(i * float32(corr_factor * f_h)), complex64 multiply
     if (comb < ncomb) {
       float cs_c, sn_c;
@@ -405,6 +438,19 @@ brutefold_complex_mma_kernel(const uint8_t* __restrict__ parts, const float* __r
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (B.dead) {
+    // Copies ahead of the products may still be on their way into this CTA's
+    // shared memory. Each lands on a barrier that the basis warps had not all
+    // arrived at: they arrive now, and the issuing warp waits (bounded).
+    if (warp < kFmGen / 32) {
+      for (int j = mine; j < B.loaded; ++j) mbar_arrive(&B.full[j % S]);
+    } else {
+      for (int j = mine; j < B.loaded; ++j)
+        for (long long k = 0;
+             k < kSpinLimit && !mbar_try_wait(&B.full[j % S], (uint32_t)(j / S) & 1u); ++k) {
+        }
+    }
+  }
   if (warp == kFmGen / 32) {
     if (lane == 0 && B.dead) atomicOr(err, LOKI_DEVERR_TIMEOUT);
     __syncwarp();
@@ -415,6 +461,14 @@ brutefold_complex_mma_kernel(const uint8_t* __restrict__ parts, const float* __r
 }  // namespace loki
 
 using namespace loki;
+
+extern "C" int loki_fourier_force_timeout(int32_t wait) {
+  const int v = wait;
+  if (wait < 0 || wait > 2) return set_error(LOKI_ERR_INVALID, "wait %d outside 0..2", wait);
+  if (cudaMemcpyToSymbol(g_fm_force_timeout, &v, sizeof(v)) != cudaSuccess)
+    return set_error(LOKI_ERR_CUDA, "cudaMemcpyToSymbol failed");
+  return LOKI_OK;
+}
 
 extern "C" int64_t loki_brutefold_complex_scratch_bytes(int64_t nsamps, int64_t segment_len,
                                                         int32_t unit_variance) {
