@@ -251,12 +251,19 @@ class TimeSeries:
             raise ValueError(msg)
         out = torch.empty_like(e)
         lib, stream = _lib.load(), _lib.stream_ptr(torch.cuda.current_stream(dev))
-        need = int(lib.loki_running_median_scratch_bytes(e.numel(), nwin))
+        # The sliding window takes 0.7 us an output, one block of at least 4
+        # windows' outputs after the other on each SM; the wavelet matrix 34
+        # launches whatever the size. Up to 256 outputs a block the first is
+        # faster (10 000 samples and a window of 17: 178 us a call against 351;
+        # 100 000 samples: 598 against 358).
+        per_block = max(4 * nwin, -(-e.numel() // 152))
+        need = 0 if per_block <= 256 else int(
+            lib.loki_running_median_scratch_bytes(e.numel(), nwin))
         if need:
             scratch = torch.empty(need, dtype=torch.uint8, device=dev)
             _lib.check(lib.loki_running_median_scratch(
                 _lib.ptr(e), e.numel(), nwin, 1, _lib.ptr(out), _lib.ptr(scratch), need, stream))
-        else:  # a size only the sliding window takes, or its error
+        else:  # or a size only the sliding window takes, or its error
             _lib.check(lib.loki_running_median(_lib.ptr(e), e.numel(), nwin, 1, _lib.ptr(out),
                                                stream))
         return TimeSeries(out.cpu().numpy() if host else out,
