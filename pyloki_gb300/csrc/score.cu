@@ -16,6 +16,37 @@ int score_warps_per_block(int nbins, int wmax);
 // widths took 0.71 ms with a normalisation pass before and take 0.25 ms.
 constexpr int kRowsInFlight = 8;
 
+// n <= R rows, R by C loads in flight a lane: rows side by side, or (one or two
+// profiles, whose columns a lane would wait for one by one) columns.
+template <bool FROM_EV, int R, int C>
+__device__ __forceinline__ void stage_rows(const float* __restrict__ src, int row, int nb, int n,
+                                           float* trow, int stride) {
+  for (int j0 = threadIdx.x & 31; j0 < nb; j0 += 32 * C) {
+    float e[R][C], v[R][C];
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      if (u >= n) break;
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        const int j = j0 + 32 * c;
+        if (j >= nb) break;
+        e[u][c] = src[(size_t)u * row + j];
+        if (FROM_EV) v[u][c] = src[(size_t)u * row + nb + j];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      if (u >= n) break;
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        const int j = j0 + 32 * c;
+        if (j >= nb) break;
+        trow[u * stride + j] = FROM_EV ? __fdiv_rn(e[u][c], __fsqrt_rn(v[u][c])) : e[u][c];
+      }
+    }
+  }
+}
+
 template <bool FROM_EV>
 __global__ void __launch_bounds__(128)
 score_kernel(const float* __restrict__ in, int64_t nprof, int nb, LokiScoreSpec sp, ScoreK SK,
@@ -30,23 +61,11 @@ score_kernel(const float* __restrict__ in, int64_t nprof, int nb, LokiScoreSpec 
   const int kmax = (int)min((int64_t)32, nprof - p0);
   const int row = FROM_EV ? 2 * nb : nb;
   for (int k0 = 0; k0 < kmax; k0 += kRowsInFlight) {
+    const int n = min(kRowsInFlight, kmax - k0);
     const float* src = in + (size_t)(p0 + k0) * row;
     float* trow = tile + k0 * stride;
-    const int n = min(kRowsInFlight, kmax - k0);
-    for (int j = lane; j < nb; j += 32) {
-      float e[kRowsInFlight], v[kRowsInFlight];
-#pragma unroll
-      for (int u = 0; u < kRowsInFlight; ++u) {
-        if (u >= n) break;
-        e[u] = src[(size_t)u * row + j];
-        if (FROM_EV) v[u] = src[(size_t)u * row + nb + j];
-      }
-#pragma unroll
-      for (int u = 0; u < kRowsInFlight; ++u) {
-        if (u >= n) break;
-        trow[u * stride + j] = FROM_EV ? __fdiv_rn(e[u], __fsqrt_rn(v[u])) : e[u];
-      }
-    }
+    if (n > 2 || nb <= 64) stage_rows<FROM_EV, kRowsInFlight, 1>(src, row, nb, n, trow, stride);
+    else stage_rows<FROM_EV, 2, 4>(src, row, nb, n, trow, stride);
   }
   __syncwarp();
   if (lane < kmax) {
