@@ -25,21 +25,10 @@ __device__ __forceinline__ void sincos_reduced(float a, float* s, float* c) {
   }
 }
 
-// The same for a caller that knows |a| < 2e5: reduction by pi / 2 in four
-// parts (the first three with 7 significant bits, so k times them is exact for
-// |k| < 2^17 and the subtractions are exact; the parts, truncations of pi / 2
-// to 60 digits, sum to it within 6e-15), then minimax polynomials on [-pi/4,
-// pi/4] in r^2 (Remez exchange in float64, rounded: sin to 4e-9, cos to 1e-10
-// before rounding). Both results are within 1.3 x 2^-24 of the exact values:
-// as accurate as sincosf there, in about half its instructions.
-__device__ __forceinline__ void sincos_small(float a, float* s, float* c) {
-  const float kf = __fmaf_rn(a, 0x1.45f306p-1f, 12582912.0f);  // 2^23 + 2^22: k in the low bits
-  const unsigned q = __float_as_uint(kf);
-  const float k = __fsub_rn(kf, 12582912.0f);
-  float r = __fmaf_rn(-k, 0x1.9p+0f, a);
-  r = __fmaf_rn(-k, 0x1.0cp-7f, r);
-  r = __fmaf_rn(-k, 0x1.ecp-14f, r);
-  r = __fmaf_rn(-k, 0x1.5110b4p-22f, r);
+// Sine and cosine of r, |r| < 0.86, by minimax polynomials on [-pi/4, pi/4] in
+// r^2 (Remez exchange in float64, rounded: sin to 4e-9, cos to 1e-10 before
+// rounding), turned by the quadrant q.
+__device__ __forceinline__ void sincos_poly(float r, unsigned q, float* s, float* c) {
   const float r2 = __fmul_rn(r, r);
   float p = __fmaf_rn(r2, -0x1.994cfap-13f, 0x1.11075cp-7f);
   p = __fmaf_rn(r2, p, -0x1.555546p-3f);
@@ -50,6 +39,33 @@ __device__ __forceinline__ void sincos_small(float a, float* s, float* c) {
   const float sv = q & 1u ? cr : sr, cv = q & 1u ? sr : cr;
   *s = __uint_as_float(__float_as_uint(sv) ^ ((q << 30) & 0x80000000u));
   *c = __uint_as_float(__float_as_uint(cv) ^ (((q + 1u) << 30) & 0x80000000u));
+}
+
+// The same for a caller that knows |a| < 2e5: reduction by pi / 2 in four
+// parts (the first three with 7 significant bits, so k times them is exact for
+// |k| < 2^17 and the subtractions are exact; the parts, truncations of pi / 2
+// to 60 digits, sum to it within 6e-15). Both results are within 1.6 x 2^-24 of
+// the exact values (1.56 over 1.2e7 angles): as accurate as sincosf there, in
+// about half its instructions.
+__device__ __forceinline__ void sincos_small(float a, float* s, float* c) {
+  const float kf = __fmaf_rn(a, 0x1.45f306p-1f, 12582912.0f);  // 2^23 + 2^22: k in the low bits
+  const float k = __fsub_rn(kf, 12582912.0f);
+  float r = __fmaf_rn(-k, 0x1.9p+0f, a);
+  r = __fmaf_rn(-k, 0x1.0cp-7f, r);
+  r = __fmaf_rn(-k, 0x1.ecp-14f, r);
+  r = __fmaf_rn(-k, 0x1.5110b4p-22f, r);
+  sincos_poly(r, __float_as_uint(kf), s, c);
+}
+
+// For |a| < 1.6e6 (|k| < 2^20), as accurate: pi / 2 = C1 + C2 to 2^-49, C1 its
+// nearest float. a and k C1 are multiples of 2^-23 (or, |a| < 1, of 2^-24) and
+// differ by less than 1, so the first subtraction is exact and the second rounds
+// once. k may be off by 0.043 before it is rounded: |r| < 0.86.
+__device__ __forceinline__ void sincos_mid(float a, float* s, float* c) {
+  const float kf = __fmaf_rn(a, 0x1.45f306p-1f, 12582912.0f);
+  const float k = __fsub_rn(kf, 12582912.0f);
+  const float r = __fmaf_rn(-k, -0x1.777a5cp-25f, __fmaf_rn(-k, 0x1.921fb6p+0f, a));
+  sincos_poly(r, __float_as_uint(kf), s, c);
 }
 
 }  // namespace loki
