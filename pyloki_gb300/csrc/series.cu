@@ -29,9 +29,11 @@ __device__ __forceinline__ int64_t reflect_idx(int64_t j, int64_t n) {
   return m < n ? m : p - 1 - m;
 }
 
-// Order-preserving map of a float to an unsigned key (NaN after +inf).
-__device__ __forceinline__ unsigned f2key(float f) {
-  const unsigned u = __float_as_uint(f);
+// Order-preserving key of the float at p (NaN after +inf). Its bits are loaded
+// as an integer: made from a loaded float, u | 0x80000000 (which is -|x|) of a
+// positive NaN came out as 0x7FFFFFFF, the key of -0.
+__device__ __forceinline__ unsigned load_key(const float* __restrict__ p) {
+  const unsigned u = __ldg(reinterpret_cast<const unsigned*>(p));
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 __device__ __forceinline__ float key2f(unsigned k) {
@@ -185,7 +187,7 @@ wm_keys_kernel(const float* __restrict__ x, int64_t n, int half, int64_t m, WmSc
   int ones = 0;
   for (int k = threadIdx.x; k < kWmTile; k += kWmThreads) {
     const int64_t p = base + k;
-    const uint32_t key = p < m ? f2key(x[reflect_idx(p - half, n)]) : 0u;
+    const uint32_t key = p < m ? load_key(x + reflect_idx(p - half, n)) : 0u;
     W.keys[p] = key;
     ones += (int)(key >> 31);
   }
@@ -343,7 +345,7 @@ select_multi_kernel(const float* __restrict__ x, int64_t n, int digit, SelRanks 
   __syncthreads();
   for (int64_t i = blockIdx.x * (int64_t)kSelThreads + tid; i < n;
        i += (int64_t)gridDim.x * kSelThreads) {
-    const unsigned key = f2key(__ldg(x + i));
+    const unsigned key = load_key(x + i);
 #pragma unroll
     for (int q = 0; q < kSelRanks; ++q)
       if (q < nh && (key & mask) == prefix[q])
