@@ -44,9 +44,7 @@ METRIC = "period-trials/s"
 WORKLOAD = "ffa_accel_search_2^23"
 # DRAM bytes (read + write) per final trial of the fused last two levels:
 # ncu capture of one launch of the same search at 2^21 samples (13 x 1932736
-# trials); profiles/ffa_final_tiled64_kernel_ffa_accel_2^21.md. The banded
-# path's figure comes from three full-band launches at 2^21
-# (profiles/band_union64_kernel_ffa_accel_2^21.md).
+# trials). The banded path's figure comes from three full-band launches at 2^21.
 FINAL_DRAM_BYTES_PER_TRIAL = {"tiled": 81.1, "banded": 259.0}
 FINAL_KERNEL = {"tiled": "ffa_final_tiled64_kernel (last two levels fused per tile: "
                          "penultimate rows built in shared memory, lane-per-trial scoring)",

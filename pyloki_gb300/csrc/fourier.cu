@@ -321,18 +321,6 @@ ffa_level_complex_rows_kernel(LokiFFALevel L, LevelK K, int pw, int64_t pairs,
 constexpr int kSnrThreads = 64;
 constexpr int kSnrRow = 67;  // float2 of a staged fold (66) and one of padding
 
-// cos and sin of 2 pi k / 64, k = 0 .. 16, for compile-time twiddles.
-__device__ constexpr float kCos64[17] = {
-    1.0f, 0.99518472667219693f, 0.98078528040323043f, 0.95694033573220882f, 0.92387953251128674f,
-    0.88192126434835505f, 0.83146961230254524f, 0.77301045336273699f, 0.70710678118654752f,
-    0.63439328416364549f, 0.55557023301960218f, 0.47139673682599764f, 0.38268343236508977f,
-    0.29028467725446233f, 0.19509032201612825f, 0.09801714032956060f, 0.0f};
-__device__ __forceinline__ constexpr float cos64(int k) {
-  k &= 63;
-  return k <= 16 ? kCos64[k] : k <= 32 ? -kCos64[32 - k] : k <= 48 ? -kCos64[k - 32] : kCos64[64 - k];
-}
-__device__ __forceinline__ constexpr float sin64(int k) { return cos64(k + 48); }
-
 // In-place inverse transform (positive exponent, unscaled) of 2^LOG complex
 // values in registers, decimation in frequency; the output is bit-reversed.
 template <int LOG>

@@ -79,7 +79,7 @@ static FmRows fm_rows(int64_t nseg, bool unit) {
   return r;
 }
 
-// The segments' bfloat16 parts: [tile][chunk][part][N x 32, K-major core
+// The segments' bfloat16 parts: [tile][chunk][part][N x K, K-major core
 // matrices of 8 rows x 16 bytes]; one thread makes 8 samples of one row. times:
 // float32(t * tfac) of every sample.
 template <int K>
@@ -105,7 +105,9 @@ fm_split_kernel(const float* __restrict__ ts_e, const float* __restrict__ ts_v, 
       const int64_t t = t0 + 2 * q + z;
       x[z] = 0.0f;
       if (row < rows && t < seg_len)
-        x[z] = row < nseg ? ts_e[row * seg_len + t] : ts_v ? ts_v[(row - nseg) * seg_len + t] : 1.0f;
+        x[z] = row < nseg ? ts_e[row * seg_len + t]
+               : ts_v     ? ts_v[(row - nseg) * seg_len + t]
+                          : 1.0f;
     }
 #pragma unroll
     for (int s = 0; s < 3; ++s) {
@@ -167,12 +169,6 @@ __device__ __forceinline__ void tmem_store(uint32_t taddr, const uint32_t (&r)[6
   asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(taddr + 4),
                "r"(r[4]), "r"(r[5])
                : "memory");
-}
-__device__ __forceinline__ void tmem_store(uint32_t taddr, const uint32_t (&r)[8]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-      : "memory");
 }
 __device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
@@ -479,8 +475,8 @@ extern "C" int64_t loki_brutefold_complex_scratch_bytes(int64_t nsamps, int64_t 
 }
 
 template <int N>
-static int launch_fm(dim3 grid, const uint8_t* parts, const float* times, const double* freqs, int64_t nfreqs,
-                     int64_t seg_len, int64_t nseg, int64_t rows, int unit, int nbf, float tfac,
+static int launch_fm(dim3 grid, const uint8_t* parts, const float* times, const double* freqs,
+                     int64_t nfreqs, int64_t seg_len, int64_t nseg, int64_t rows, int unit, int nbf, float tfac,
                      float corr, int64_t nch, float2* fold, int32_t* err, cudaStream_t s) {
   // more than half of an SM's shared memory: tensor memory has room for one CTA
   const int smem = std::max(116 * 1024, fm_stages(N) * fm_b_bytes(N));

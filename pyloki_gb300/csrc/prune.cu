@@ -18,6 +18,7 @@
 
 #include "loki_common.cuh"
 #include "score.cuh"
+#include "sincos.cuh"
 
 namespace loki {
 
@@ -1919,8 +1920,6 @@ prune_score_complex_kernel(LokiPruneLevel D, const double* __restrict__ leaves,
                       minmax_keys, tw, comb, tile + lane * stride, c);
 }
 
-// Survivors of the complex tree: transform / backtrack exactly as
-// prune_emit_kernel, the fold written as the complex sum.
 // The rows one survivor's fold is made of.
 struct EmitRow {
   int64_t par, row;
@@ -1929,7 +1928,6 @@ struct EmitRow {
 
 // One survivor of the complex tree: transform and backtrack, its fold's rows
 // returned.
-
 template <int KP = 0>
 __device__ __forceinline__ EmitRow emit_one_complex_leaf(
     const LokiPruneLevel& D, const double* __restrict__ leaves,
@@ -1996,6 +1994,8 @@ __device__ __forceinline__ void emit_one_complex(
              fout + s * 2 * nbf);
 }
 
+// Survivors of the complex tree: transform / backtrack exactly as
+// prune_emit_kernel, the fold written as the complex sum.
 __global__ void __launch_bounds__(kPruneWarps * 32)
 prune_emit_complex_kernel(LokiPruneLevel D, const double* __restrict__ leaves,
                           const float2* __restrict__ folds,
@@ -2280,10 +2280,6 @@ circ_emit_complex_kernel(LokiPruneLevel D, const double* __restrict__ leaves,
 }
 
 // ---------------------------------------------------------------------------
-// launchers
-// ---------------------------------------------------------------------------
-
-// ---------------------------------------------------------------------------
 // Complex rows of 32 children at a time, 64 bins, with the arithmetic of
 // rotate_add and irfft_norm. Every lane runs its child's phasor recurrence once,
 // into a table of shared memory; then the warp combines the children's parent and
@@ -2293,7 +2289,7 @@ circ_emit_complex_kernel(LokiPruneLevel D, const double* __restrict__ leaves,
 // and 32 + j have the same cosine and sine up to sign, so their four sums share
 // two products, and the 64 sums are independent registers. A lane walking its
 // rows in global memory and the bins one after the other took 56 ms for the 8.0e6
-// children of a 16-run search; now 9.3, of which 2 are the latency of the 100
+// children of a 16-run search; now 9.4, of which 2 are the latency of the 100
 // levels with fewer than 500 children a run.
 // ---------------------------------------------------------------------------
 
@@ -2351,21 +2347,9 @@ __device__ __forceinline__ void combine_rows64(const float2* __restrict__ folds,
 // m = 1 .. 31 (row m - 1), after the 64 angles they are taken from.
 constexpr int kTwiddle64Bytes = 512 + 31 * 16 * 8;
 
-// cos(2 pi k / 64) to the nearest float, k = 0 .. 16.
-__constant__ float kCos64[17] = {
-    1.0f, 0.99518472f, 0.980785251f, 0.956940353f, 0.923879504f, 0.881921291f,
-    0.831469595f, 0.773010433f, 0.707106769f, 0.634393275f, 0.555570245f, 0.471396744f,
-    0.382683426f, 0.290284663f, 0.195090324f, 0.0980171412f, 0.0f};
-
-__device__ __forceinline__ float cos64(int t) {  // cos(2 pi t / 64)
-  t &= 63;
-  if (t > 32) t = 64 - t;
-  return t <= 16 ? kCos64[t] : -kCos64[32 - t];
-}
-
 __device__ __forceinline__ void load_twiddles64(float* smem) {
   float2 *tw = reinterpret_cast<float2*>(smem), *W = tw + 64;
-  for (int t = threadIdx.x; t < 64; t += blockDim.x) tw[t] = make_float2(cos64(t), cos64(t - 16));
+  for (int t = threadIdx.x; t < 64; t += blockDim.x) tw[t] = make_float2(cos64(t), sin64(t));
   __syncthreads();
   for (int t = threadIdx.x; t < 31 * 16; t += blockDim.x)
     W[t] = tw[((t >> 4) + 1) * (t & 15) & 63];
@@ -2553,8 +2537,8 @@ __device__ __forceinline__ void cplx64_score(const float2* __restrict__ folds,
   __syncwarp();  // every lane has read its row
   combine_rows64(folds, seg, my_par, my_row, kmax, 1, T, A, kCplxRow);
   // the phasors have been used: their rows keep the first component's sums, which
-  // would be 64 more registers. (Three blocks an SM spill 108 bytes a thread: 11.0
-  // instead of 10.5 ms for the 8.0e6 children of 16 runs.)
+  // would be 64 more registers. (Three blocks an SM spill 108 bytes a thread and
+  // were 5 % slower.)
 #pragma unroll
   for (int j = 1; j < 16; ++j) {
     keep[j] = S.p[j];
@@ -2586,6 +2570,10 @@ __device__ __forceinline__ void cplx64_emit(const float2* __restrict__ folds,
   for (int comp = 0; comp < 2; ++comp)
     combine_rows64(folds, seg, my_par, my_row, kmax, comp, buf, fout + comp * 33, 66);
 }
+
+// ---------------------------------------------------------------------------
+// launchers
+// ---------------------------------------------------------------------------
 
 static int check_prune(const LokiPruneLevel* D) {
   if (!D) return set_error(LOKI_ERR_INVALID, "null prune level descriptor");

@@ -1,9 +1,22 @@
-// Sine and cosine of the Fourier folds' float32 angles.
+// Sine and cosine of the Fourier folds' float32 angles and of 64 bins.
 #pragma once
 
 #include "loki_common.cuh"
 
 namespace loki {
+
+// cos and sin of 2 pi k / 64, the nearest floats.
+__device__ constexpr float kCos64[17] = {
+    1.0f, 0.99518472667219693f, 0.98078528040323043f, 0.95694033573220882f, 0.92387953251128674f,
+    0.88192126434835505f, 0.83146961230254524f, 0.77301045336273699f, 0.70710678118654752f,
+    0.63439328416364549f, 0.55557023301960218f, 0.47139673682599764f, 0.38268343236508977f,
+    0.29028467725446233f, 0.19509032201612825f, 0.09801714032956060f, 0.0f};
+__device__ __forceinline__ constexpr float cos64(int k) {
+  k &= 63;
+  if (k > 32) k = 64 - k;
+  return k <= 16 ? kCos64[k] : -kCos64[32 - k];
+}
+__device__ __forceinline__ constexpr float sin64(int k) { return cos64(k + 48); }
 
 // sin and cos of a float32 angle by Cody and Waite's additive reduction
 // ("Software Manual for the Elementary Functions", 1980): 2 pi split into
