@@ -225,7 +225,7 @@ brutefold_count_kernel(const T* __restrict__ map, int64_t nfreq_chunk, int64_t f
 //
 // Bound: shared-memory bandwidth, 4 bytes per add at 128 bytes a clock and SM:
 // 4.6 ms with padding for 2^21 samples x 15 100 frequencies, 64 bins, 128
-// segments, where the walk takes 6.8 ms and the lists 1.1 ms. A walk of
+// segments, where the walk takes 6.2 ms and the lists 1.1 ms. A walk of
 // 512-sample chunks with one row a lane and the sums in shared memory took
 // 13.6 ms (four loads of loop state per 10 samples of a chain), its float64
 // phase map 4.5 ms and the sort of it by warp matches 2.7 ms.
