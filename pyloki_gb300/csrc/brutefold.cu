@@ -933,7 +933,7 @@ extern "C" int64_t loki_brutefold_series_scratch_bytes(int64_t nsamps, int64_t n
   const int64_t nrows = (nsamps + segment_len - 1) / segment_len * (unit_variance ? 1 : 2);
   const ChainPlan p = chain_plan(nbins, nrows, nfreqs, segment_len, INT64_MAX / 2);
   if (!p.freqs) return nfreqs * segment_len * (nbins <= 256 ? 1 : 2);
-  return chain_bytes(p, nrows, nbins);
+  return std::max(segment_len, chain_bytes(p, nrows, nbins));  // what any fold asks for at least
 }
 
 extern "C" int64_t loki_brutefold_scratch_bytes(int64_t nfreqs, int64_t segment_len,

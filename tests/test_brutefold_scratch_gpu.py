@@ -84,3 +84,19 @@ def test_one_long_fold_needs_little_scratch(nfreq):
     for unit in (0, 1):
         need = lib.loki_brutefold_series_scratch_bytes(n, nfreq, n, 64, unit)
         assert need <= (5.5 * nfreq + 16.5) * n
+
+
+@pytest.mark.parametrize("nseg", [1, 3, 5, 8, 40])
+def test_scratch_for_all_is_never_refused(nseg):
+    """Less than one frequency's phase map is refused, also where the chain path
+    would do with less: the scratch for a whole fold is at least that."""
+    from pyloki_gb300 import _lib
+
+    try:
+        lib = _lib.load()
+    except RuntimeError:
+        pytest.skip("libloki_gb300.so not built")
+    for seg in (1000, 1 << 20, 1 << 28):
+        for nbins in (1, 64, 256, 300):
+            need = lib.loki_brutefold_series_scratch_bytes(nseg * seg, 1, seg, nbins, 1)
+            assert need >= seg * (1 if nbins <= 256 else 2)
