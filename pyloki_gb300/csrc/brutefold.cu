@@ -787,8 +787,10 @@ static ChainPlan chain_plan(int nbins, int64_t nrows, int64_t nfreqs, int64_t se
       const int64_t fit = avail < 0 ? 0 : avail / chain_freq_bytes(c, run, nbins);
       const int64_t take = std::min(fit, nf);
       if (take < 1) break;
-      const int64_t blocks = chain_groups(c, nrows) * ((take + c.F - 1) / c.F);
-      if (take == nfreqs || blocks >= 2 * kChainSms) return {c, run, take};
+      const int64_t nrg = chain_groups(c, nrows), blocks = nrg * ((take + c.F - 1) / c.F);
+      if (take == nfreqs) return {c, run, take};
+      if (blocks >= 2 * kChainSms)  // whole waves of blocks
+        return {c, run, std::min(take, blocks / kChainSms * kChainSms / nrg * c.F)};
       if (take == nf) break;
       nf = take;
     }
